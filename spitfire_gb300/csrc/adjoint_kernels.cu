@@ -38,33 +38,16 @@ struct AdjParams {
 
 // d ln q_r / d ln k_r (the factor s_r / q_r above) of a falloff reaction at the state of the group's scratch
 __device__ double falloff_factor(const DevMech &m, const Blob &b, const ScratchLayout &L, const double *scr,
-                                 const StateCtx &s, int r, int kind, int kform, int info)
+                                 const StateCtx &s, int r, int kind, int info)
 {
-  const double *kc = b.d + m.d_kf + 3 * r;
-  double kf;
-  switch (kform) {
-  case 0: kf = kc[0]; break;
-  case 1: kf = kc[0] * s.T; break;
-  case 2: kf = kc[0] * s.T * s.T; break;
-  case 3: kf = kc[0] * s.invT; break;
-  default: kf = kc[0] * tab_exp(kc[1] * s.logT - kc[2] * s.invT, b.d + m.d_exptab); break;
-  }
-  const double *y = scr + L.y;
-  const int t0 = b.i[m.i_tb_off + r], t1 = b.i[m.i_tb_off + r + 1];
-  double sumtb = 0.;
-  for (int j = t0; j < t1; ++j) sumtb += b.d[m.d_tbeff + j] * y[b.i[m.i_tb + j]];
-  const double M = b.d[m.d_beff + r] * s.ct + s.rho * sumtb;
+  const double M = third_body(m, b, s, r, scr + L.C);
   const int f = b.i[m.i_fall + r];
   const double *kp = b.d + m.d_kp + 3 * f;
-  const double pr = kp[0] * tab_exp(kp[1] * s.logT - kp[2] * s.invT, b.d + m.d_exptab) / kf * M;
+  const double pr = kp[0] * tab_exp(fma(kp[1], s.logT, -(kp[2] * s.invT)), b.d + m.d_exptab) * M;
   double fac = pr / (1. + pr);
   if (kind == 4 && pr > 1.e-300) {
-    const double *tr = b.d + m.d_troe + 4 * f;
-    const int terms = (info >> RI_TROE_SHIFT) & 7;
-    double fc = 0.;
-    if (terms & 1) fc += (1 - tr[0]) * tab_exp(-s.T / tr[1], b.d + m.d_exptab);
-    if (terms & 2) fc += tr[0] * tab_exp(-s.T / tr[2], b.d + m.d_exptab);
-    if (terms & 4) fc += tab_exp(-s.invT * tr[3], b.d + m.d_exptab);
+    double Tdfc;
+    const double fc = troe_center<false>(m, b, s, f, (info >> RI_TROE_SHIFT) & 7, Tdfc);
     const double lfc = log10(fc);
     const double nn = 0.75 - 1.27 * lfc;
     const double lpc = log10(pr) + (-0.4 - 0.67 * lfc);
@@ -107,31 +90,20 @@ __global__ void __launch_bounds__(256) rate_param_adjoint_kernel(const AdjParams
         sim += scr[L.y + i] * b.d[m.d_invmw + i];
         cmix += scr[L.y + i] * scr[L.cpv + i];
       }
-      sim = grp.sum(sim);
-      cmix = grp.sum(cmix);
-      const double mmw = 1. / sim;
-      const double rho = isochoric ? qs[0] : pres * mmw / (T * m.Ru);
-      StateCtx s;
-      s.T = T;
-      s.logT = log(T);
-      s.invT = 1. / T;
-      s.rho = rho;
-      s.invRho = 1. / rho;
-      s.mmw = mmw;
-      s.invM = sim;
-      s.ct = rho * sim;
+      grp.sum2(sim, cmix);
+      const StateCtx s = state_ctx<G>(m, grp, T, isochoric ? qs[0] : 0., sim, pres, isochoric, 0);
+      const double icmix = 1. / cmix;
       for (int r = lane; r < nr; r += G) {
         const int info = b.i[m.i_info + r];
         const int kind = (info >> RI_KIND_SHIFT) & 7;
-        const int kform = (info >> RI_KFORM_SHIFT) & 7;
         double sr = scr[L.q + r];
-        if (kind == 3 || kind == 4) sr *= falloff_factor(m, b, L, scr, s, r, kind, kform, info);
+        if (kind == 3 || kind == 4) sr *= falloff_factor(m, b, L, scr, s, r, kind, info);
         const int n0 = b.i[m.i_net_off + r], n1 = b.i[m.i_net_off + r + 1];
         const int ro = b.i[m.i_orig + r];  // reported in the order the mechanism was described
         for (int o = 0; o < p.wsets; ++o) {  // the rates above serve every adjoint vector of this state
           const double *w = p.w + (((size_t)it * p.wsets + o) * p.stages + st) * neq;
           double *out = p.out + ((size_t)it * p.wsets + o) * 2 * nr;
-          const double wTc = w[tix] / cmix;
+          const double wTc = w[tix] * icmix;
           double B = 0.;
           for (int j = n0; j < n1; ++j) {
             const int sp = b.i[m.i_net + j] & 0xFFFF;

@@ -79,6 +79,10 @@ __device__ inline bool stage_to_smem(void *dst, const void *src, uint32_t bytes,
 }
 
 // ----------------------------------------------------------------------------------------------- state groups
+// Sums over a group are formed together where the caller has several (sum2, sum4): on GB300 every FP64 instruction of
+// a warp costs the same 64-76 cycles of its scheduler's FP64 unit however many lanes carry a value, and the
+// transposed reduction below adds four 32-lane sums in 6 instructions instead of 20 (the first two exchanges leave
+// each quarter of the lanes with one of the four sums).
 template <int G>
 struct Group {
   int lane;       // 0..G-1
@@ -95,6 +99,51 @@ struct Group {
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o, G);
     return v;
+  }
+  __device__ __forceinline__ void sum2(double &a, double &b) const
+  {
+    if (G == 1) return;
+    constexpr int H = G > 1 ? G / 2 : 1;
+    const bool up = (lane & H) != 0;
+    double r = (up ? b : a) + __shfl_xor_sync(mask, up ? a : b, H, G);
+#pragma unroll
+    for (int o = H / 2; o > 0; o >>= 1) r += __shfl_xor_sync(mask, r, o, G);
+    a = __shfl_sync(mask, r, 0, G);
+    b = __shfl_sync(mask, r, H, G);
+  }
+  __device__ __forceinline__ void sum4(double &a, double &b, double &c, double &d) const
+  {
+    if (G < 4) {
+      sum2(a, b);
+      sum2(c, d);
+      return;
+    }
+    constexpr int H = G / 2, Q = G > 2 ? G / 4 : 1;
+    const bool up = (lane & H) != 0, uq = (lane & Q) != 0;
+    const double x = (up ? b : a) + __shfl_xor_sync(mask, up ? a : b, H, G);
+    const double y = (up ? d : c) + __shfl_xor_sync(mask, up ? c : d, H, G);
+    double r = (uq ? y : x) + __shfl_xor_sync(mask, uq ? x : y, Q, G);
+#pragma unroll
+    for (int o = Q / 2; o > 0; o >>= 1) r += __shfl_xor_sync(mask, r, o, G);
+    a = __shfl_sync(mask, r, 0, G);
+    b = __shfl_sync(mask, r, H, G);
+    c = __shfl_sync(mask, r, Q, G);
+    d = __shfl_sync(mask, r, H + Q, G);
+  }
+  // reciprocals of three values that all lanes hold: one division instruction sequence for all three where the
+  // group has lanes to share it (an FP64 division is about eight FP64 instructions)
+  __device__ __forceinline__ void recip3(double a, double b, double c, double &ia, double &ib, double &ic) const
+  {
+    if (G < 4) {
+      ia = 1. / a;
+      ib = 1. / b;
+      ic = 1. / c;
+      return;
+    }
+    const double r = 1. / (lane == 1 ? b : (lane == 2 ? c : a));
+    ia = __shfl_sync(mask, r, 0, G);
+    ib = __shfl_sync(mask, r, 1, G);
+    ic = __shfl_sync(mask, r, G < 4 ? 0 : 2, G);
   }
 };
 
@@ -127,47 +176,57 @@ __device__ __forceinline__ Blob blob_at(const DevMech &m, const void *base)
 // (thermodynamics_kernels.cpp:45-131, 183-260, 262-351; chemistry_kernels.cpp:56-97;
 //  rates_sensitivities_exact.cpp:83-124).
 struct SpeciesThermo {
-  double cp, h, dcp, g, dB;
+  double cp, h, dcp, g, TdB;  // TdB: T times the B term
 };
 
+// Magnitude tests on temperatures as integers: non-negative doubles order like their bit patterns (and a negative one
+// below every positive), so that a comparison does not take an FP64 instruction.
+__device__ __forceinline__ bool le_bits(double a, double b) { return __double_as_longlong(a) <= __double_as_longlong(b); }
+
+// The four temperature terms t_j = A_j T^j of a NASA7 polynomial (A_j the stored, scaled coefficients) serve g, h, cp
+// and their derivatives together inside the polynomials' range: about 20 FP64 instructions per species for the
+// right-hand side where three separate Horner forms took 45 and six FP64 comparisons. Outside the range, where cp is
+// clamped and h extrapolated, the general form below runs.
 __device__ __forceinline__ SpeciesThermo species_thermo(const DevMech &m, Blob b, int k, double T, double logT,
                                                         double invT, bool want_sens)
 {
   SpeciesThermo s;
   const double *c = b.d + m.d_nasa + 15 * k;
   const double invmw = b.d[m.d_invmw + k];
+  s.dcp = 0.;
+  s.TdB = 0.;
   if (m.all_nasa7 || b.i[m.i_thermo + k] == 2) {
     const double tmin = b.d[m.d_tmin + k], tmax = b.d[m.d_tmax + k];
-    // polynomial for g and dB: chosen by Tmid only
-    const int gb = (T <= c[0]) ? 8 : 1;
-    const double *a = c + gb;
-    const double a6 = (T <= c[0]) ? c[13] : c[6];
-    const double a7 = (T <= c[0]) ? c[14] : c[7];
-    s.g = a6 + T * (a[0] - a7 - a[0] * logT - T * (a[1] + T * (a[2] + T * (a[3] + T * a[4]))));
-    // cp / h / dcp on the clamped temperature
+    const double *a = c + (le_bits(T, c[0]) ? 8 : 1);  // polynomial for g and B: chosen by Tmid only
+    if (le_bits(tmin, T) && le_bits(T, tmax)) {
+      const double T2 = T * T;
+      const double t1 = a[1] * T, t2 = a[2] * T2, t3 = a[3] * (T2 * T), t4 = a[4] * (T2 * T2);
+      s.g = fma(T, (a[0] - a[6]) - fma(a[0], logT, (t1 + t2) + (t3 + t4)), a[5]);
+      const double hm = fma(T, fma(4., t4, fma(3., t3, fma(2., t2, a[0] + t1))), a[5]);
+      s.h = invmw * hm;
+      s.cp = invmw * fma(20., t4, fma(12., t3, fma(6., t2, fma(2., t1, a[0]))));
+      if (want_sens) {
+        s.dcp = invmw * invT * fma(80., t4, fma(36., t3, fma(12., t2, 2. * t1)));
+        s.TdB = fma(hm, invT * m.invRu, -1.);
+      }
+      return s;
+    }
+    s.g = a[5] + T * (a[0] - a[6] - a[0] * logT - T * (a[1] + T * (a[2] + T * (a[3] + T * a[4]))));
+    // cp / h on the clamped temperature (dcp/dT is zero outside the range)
     const double tt = fmin(fmax(T, tmin), tmax);
-    const bool inside = (T >= tmin) && (T <= tmax);
-    const int hb = (tt <= c[0]) ? 8 : 1;
-    const double *p = c + hb;
-    const double p6 = (tt <= c[0]) ? c[13] : c[6];
+    const double *p = c + ((tt <= c[0]) ? 8 : 1);
     const double cpm = p[0] + tt * (2. * p[1] + tt * (6. * p[2] + tt * (12. * p[3] + 20. * tt * p[4])));
     s.cp = invmw * cpm;
-    const double hm = p6 + tt * (p[0] + tt * (p[1] + tt * (2. * p[2] + tt * (3. * p[3] + tt * 4. * p[4]))));
-    s.h = invmw * (inside ? hm : hm + cpm * (T - tt));
-    if (want_sens) {
-      s.dcp = inside ? invmw * (2. * p[1] + tt * (12. * p[2] + tt * (36. * p[3] + 80. * tt * p[4]))) : 0.;
-      s.dB = m.invRu * ((a[0] - m.Ru) * invT + a[1] + T * (2 * a[2] + T * (3 * a[3] + T * 4 * a[4])) + a6 * invT * invT);
-    } else {
-      s.dcp = 0.;
-      s.dB = 0.;
-    }
+    const double hm = p[5] + tt * (p[0] + tt * (p[1] + tt * (2. * p[2] + tt * (3. * p[3] + tt * 4. * p[4]))));
+    s.h = invmw * (hm + cpm * (T - tt));
+    if (want_sens)
+      s.TdB = m.invRu * ((a[0] - m.Ru) + T * (a[1] + T * (2 * a[2] + T * (3 * a[3] + T * 4 * a[4]))) + a[5] * invT);
   } else {
     // constant cp: c = [T0, h0, s0, cp, log T0] (thermodynamics_kernels.cpp:60-63, chemistry_kernels.cpp:88-89)
     s.cp = invmw * c[3];
     s.h = invmw * (c[1] + c[3] * (T - c[0]));
     s.g = c[1] + c[3] * (T - c[0]) - T * (c[2] + c[3] * (logT - c[4]));
-    s.dcp = 0.;
-    s.dB = want_sens ? invT * (b.d[m.d_mw + k] * m.invRu * (c[3] - invT * (c[3] * c[0] - c[1])) - 1) : 0.;
+    if (want_sens) s.TdB = b.d[m.d_mw + k] * m.invRu * (c[3] - invT * (c[3] * c[0] - c[1])) - 1;
   }
   return s;
 }
@@ -251,15 +310,19 @@ __device__ __forceinline__ void store_gibbs_factor(S scr, const ScratchLayout &L
   const double ep = O + E, em = E - O;                                        // e^r - 1, e^-r - 1
   scr[L.gm + i] = t.x + fma(t.x, ep, t.y);
   scr[L.gmi + i] = ui * (u.x + fma(u.x, em, u.y));
-  scr[L.gk + i] = __longlong_as_double((long long)(N >> 6));
+  scr[L.gk + i] = __hiloint2double(0, N >> 6);
 }
 
 // x 2^K, exact unless the result leaves the normal range; |K| beyond 2044 already takes any factor of a rate
-// expression to 0 or infinity.
+// expression to 0 or infinity. A normal x whose result is normal has K added to its exponent field.
 __device__ __forceinline__ double scale_pow2(double x, long long K)
 {
-  const int k = (int)(K < -2044 ? -2044 : (K > 2046 ? 2046 : K));
-  const int k1 = k / 2, k2 = k - k1;  // both within [-1022, 1023]
+  const int e = (__double2hiint(x) >> 20) & 0x7ff;
+  const int k = (int)(K < -4096 ? -4096 : (K > 4096 ? 4096 : K));
+  if ((unsigned)(e - 1) < 2046u && (unsigned)(e + k - 1) < 2046u)
+    return __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
+  const int kc = k < -2044 ? -2044 : (k > 2046 ? 2046 : k);
+  const int k1 = kc / 2, k2 = kc - k1;  // both within [-1022, 1023]
   const double f1 = __longlong_as_double((long long)(k1 + 1023) << 52);
   const double f2 = __longlong_as_double((long long)(k2 + 1023) << 52);
   return x * f1 * f2;
@@ -280,11 +343,10 @@ struct StateCtx {
   int option;  // rates-sensitivity option: 0 / 2 exact, 1 without third-body/falloff derivatives
 };
 
-// Product of C_j^nu_j over a reactant/product list, with the factor of list position `at` differentiated
-// with respect to Y of that species (nu * rho/M * C^(nu-1)); at < 0: no differentiation.
+// Product of C_j^nu_j over a reactant/product list, with the factor of list position `at` differentiated with
+// respect to its concentration (nu * C^(nu-1)); at < 0: no differentiation.
 template <class SC>
-__device__ __forceinline__ double mass_action(const int *lst, int n, const SC &C, const double *invmw_d,
-                                              double rho, int at)
+__device__ __forceinline__ double mass_action(const int *lst, int n, const SC &C, int at)
 {
   double v = 1.;
   for (int j = 0; j < n; ++j) {
@@ -292,61 +354,67 @@ __device__ __forceinline__ double mass_action(const int *lst, int n, const SC &C
     const int s = e & 0xFFFF, nu = e >> 16;
     const double c = C[s];
     if (j == at)
-      v *= nu * rho * invmw_d[s] * ipow(c, nu - 1);
+      v *= nu * ipow(c, nu - 1);
     else
       v *= ipow(c, nu);
   }
   return v;
 }
 
-// Mass-action factors of a reactant or product list of at most three entries, formed once per reaction: the
-// product P = prod_i C_i^nu_i and, per list position j, g_j = d P / d Y_j / rho = nu_j / M_j C_j^(nu_j - 1)
-// prod_{i != j} C_i^nu_i (C_i = rho Y_i / M_i). The Jacobian slots of the reaction then cost one multiply each.
-struct MassAction3 {
-  double P, g0, g1, g2;
-  __device__ __forceinline__ double g(int j) const { return j == 0 ? g0 : (j == 1 ? g1 : g2); }
+// One side of a reaction with at most three species: the rate R = k prod_i C_i^nu_i and, with JAC, its derivatives
+// t_j = dR/dC_j of list position j. The products are shared: a side of two species with unit coefficients takes
+// three multiplications for all three values, one of three species six.
+struct Side3 {
+  double R, t0, t1, t2;
+  __device__ __forceinline__ double t(int j) const { return j == 0 ? t0 : (j == 1 ? t1 : t2); }
 };
 
-template <class SC>
-__device__ __forceinline__ MassAction3 mass_action3(const int *lst, int n, const SC &C, const double *invmw_d)
+template <bool JAC, class SC>
+__device__ __forceinline__ Side3 side3(const int *lst, int n, const SC &C, double k, const double *smallint)
 {
-  double p[3], d[3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    p[j] = 1.;
-    d[j] = 0.;
-    if (j < n) {
-      const int e = lst[j];
-      const int sp = e & 0xFFFF, nu = e >> 16;
-      const double c = C[sp];
-      const double im = invmw_d[sp];
-      if (nu == 1) {
-        p[j] = c;
-        d[j] = im;
-      } else {
-        const double cm = ipow(c, nu - 1);
-        p[j] = cm * c;
-        d[j] = (double)nu * im * cm;
-      }
-    }
+  Side3 o;
+  o.t1 = o.t2 = 0.;
+  // position j: p_j = C_j^nu_j and kd_j = k nu_j C_j^(nu_j - 1)
+  const int e0 = lst[0];
+  double p0 = C[e0 & 0xFFFF], kd0 = k;
+  const bool unit0 = (e0 >> 16) == 1;
+  if (!unit0) {
+    const double cm = ipow(p0, (e0 >> 16) - 1);
+    p0 *= cm;
+    kd0 *= small_int(smallint, e0 >> 16) * cm;
   }
-  MassAction3 o;
-  if (n <= 1) {
-    o.P = p[0];
-    o.g0 = d[0];
-    o.g1 = o.g2 = 0.;
-  } else if (n == 2) {
-    o.P = p[0] * p[1];
-    o.g0 = d[0] * p[1];
-    o.g1 = p[0] * d[1];
-    o.g2 = 0.;
-  } else {
-    const double t = p[0] * p[1];
-    o.P = t * p[2];
-    o.g0 = d[0] * (p[1] * p[2]);
-    o.g1 = d[1] * (p[0] * p[2]);
-    o.g2 = d[2] * t;
+  if (n == 1) {
+    o.R = k * p0;
+    o.t0 = kd0;
+    return o;
   }
+  const int e1 = lst[1];
+  double p1 = C[e1 & 0xFFFF], kd1 = k;
+  if ((e1 >> 16) != 1) {
+    const double cm = ipow(p1, (e1 >> 16) - 1);
+    p1 *= cm;
+    kd1 *= small_int(smallint, e1 >> 16) * cm;
+  }
+  if (n == 2) {
+    o.t0 = kd0 * p1;
+    o.R = unit0 ? o.t0 * p0 : k * p0 * p1;
+    if (JAC) o.t1 = kd1 * p0;
+    return o;
+  }
+  const int e2 = lst[2];
+  double p2 = C[e2 & 0xFFFF], kd2 = k;
+  if ((e2 >> 16) != 1) {
+    const double cm = ipow(p2, (e2 >> 16) - 1);
+    p2 *= cm;
+    kd2 *= small_int(smallint, e2 >> 16) * cm;
+  }
+  if (JAC) {
+    o.t0 = kd0 * p1 * p2;
+    o.t1 = kd1 * p0 * p2;
+  }
+  const double p01 = p0 * p1;
+  o.t2 = kd2 * p01;
+  o.R = (e2 >> 16) == 1 ? o.t2 * p2 : k * p01 * p2;
   return o;
 }
 
@@ -379,186 +447,212 @@ __device__ __forceinline__ double special_orders(const DevMech &m, Blob b, int r
   return v;
 }
 
-template <bool JAC>
-struct RxnOut {
-  double q;
-};
+// Forward rate constant of reaction r (chemistry_kernels.cpp:140-157).
+__device__ __forceinline__ double forward_constant(const DevMech &m, const Blob &b, const StateCtx &s, int r, int kform)
+{
+  const double *kc = b.d + m.d_kf + 3 * r;
+  switch (kform) {
+  case 0: return kc[0];
+  case 1: return kc[0] * s.T;
+  case 2: return kc[0] * (s.T * s.T);
+  case 3: return kc[0] * s.invT;
+  default: return kc[0] * tab_exp(fma(kc[1], s.logT, -(kc[2] * s.invT)), b.d + m.d_exptab);
+  }
+}
 
-// Evaluate reaction r. Always writes q[r]; with JAC also dq/drho, dq/dT, the sparse slot derivatives D (scaled by
-// 1/rho), the dense coefficients alpha, beta (scaled by 1/rho) and E_r = sum_i c_ir * eh_i.
+// F_cent of a Troe reaction and, with JAC, T dF_cent/dT. d_troe holds (a, -1/T3, -1/T1, T2).
+template <bool JAC>
+__device__ __forceinline__ double troe_center(const DevMech &m, const Blob &b, const StateCtx &s, int f, int terms,
+                                              double &Tdfc)
+{
+  const double *tr = b.d + m.d_troe + 4 * f;
+  double fc = 0.;
+  Tdfc = 0.;
+  if (terms & 1) {
+    const double x = s.T * tr[1];
+    const double e = (1. - tr[0]) * tab_exp(x, b.d + m.d_exptab);
+    fc += e;
+    if (JAC) Tdfc = x * e;
+  }
+  if (terms & 2) {
+    const double x = s.T * tr[2];
+    const double e = tr[0] * tab_exp(x, b.d + m.d_exptab);
+    fc += e;
+    if (JAC) Tdfc = fma(x, e, Tdfc);
+  }
+  if (terms & 4) {
+    const double x = -(s.invT * tr[3]);
+    const double e = tab_exp(x, b.d + m.d_exptab);
+    fc += e;
+    if (JAC) Tdfc = fma(-x, e, Tdfc);
+  }
+  return fc;
+}
+
+// Third-body concentration of reaction r: the default efficiency times the total plus the listed excesses.
+template <class SC>
+__device__ __forceinline__ double third_body(const DevMech &m, const Blob &b, const StateCtx &s, int r, const SC &C)
+{
+  const int t0 = b.i[m.i_tb_off + r], t1 = b.i[m.i_tb_off + r + 1];
+  double M = b.d[m.d_beff + r] * s.ct;
+  for (int j = t0; j < t1; ++j) M = fma(b.d[m.d_tbeff + j], C[b.i[m.i_tb + j]], M);
+  return M;
+}
+
+// Evaluate reaction r. Always writes its net rate q[r]; with JAC also
+//   dqdrho = rho dq/drho, dqdT = T dq/dT, the sparse slots D_j = dq/dC_j (concentration C = rho Y / M), the dense
+//   coefficients alpha, beta of dq/dY_k / rho = D_k / M_k + alpha u_k + beta, and E = sum_i c_ir e_i.
+// The kernels are bound by FP64 instructions, so the scaled forms were chosen for what they leave out: the factors 1/M,
+// 1/rho and 1/T belong to a species or a state and are applied once there (1/M in the gather programs' coefficients),
+// a reaction without a third body multiplies by no such factor, the products of a side are shared by its rate and
+// derivatives (side3), and the product side carries its minus sign in the constant. About 45 FP64 instructions for
+// a reversible 2+2 reaction with its derivatives (a third of them the exponential) where the form with every
+// factor in place took 110.
 template <bool JAC, class S>
 __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const ScratchLayout &L, S scr,
                                               const StateCtx &s, int r, double *Eacc_a, double *Eacc_b)
 {
   const int info = b.i[m.i_info + r];
   const int kind = (info >> RI_KIND_SHIFT) & 7;
-  const int kform = (info >> RI_KFORM_SHIFT) & 7;
   const bool rev = (info >> RI_REV_BIT) & 1;
   const bool has_ord = (info >> RI_ORD_BIT) & 1;
-  const double *kc = b.d + m.d_kf + 3 * r;
   const auto C = scr + L.C;
-  const auto y = scr + L.y;
-  const double *invmw_d = b.d + m.d_invmw;
-  // forward rate constant (chemistry_kernels.cpp:140-157)
-  double kf;
-  switch (kform) {
-  case 0: kf = kc[0]; break;
-  case 1: kf = kc[0] * s.T; break;
-  case 2: kf = kc[0] * s.T * s.T; break;
-  case 3: kf = kc[0] * s.invT; break;
-  default: kf = kc[0] * tab_exp(kc[1] * s.logT - kc[2] * s.invT, b.d + m.d_exptab); break;
-  }
-  const double dlogkf = s.invT * (kc[1] + kc[2] * s.invT);
-  // third-body / falloff factor (chemistry_kernels.cpp:158-314; rates_sensitivities_exact.cpp:826-1000)
-  double Ctbaf = 1., dCdrho = 0., dCdT = 0., K = 0.;
+  const double *smallint = b.d + m.d_smallint;
+  const double kf = forward_constant(m, b, s, r, (info >> RI_KFORM_SHIFT) & 7);
+  const double *kc = b.d + m.d_kf + 3 * r;
+  const double Tdlogkf = fma(kc[2], s.invT, kc[1]);  // T d ln kf / dT
+  // third-body / falloff factor (chemistry_kernels.cpp:158-314; rates_sensitivities_exact.cpp:826-1000); K = dCtbaf/dM
+  double Ctbaf = 1., TdCdT = 0., K = 0., M = 0.;
   if (kind != 1) {
-    const int t0 = b.i[m.i_tb_off + r], t1 = b.i[m.i_tb_off + r + 1];
-    double sumtb = 0.;
-    for (int j = t0; j < t1; ++j) sumtb += b.d[m.d_tbeff + j] * y[b.i[m.i_tb + j]];
-    const double beff = b.d[m.d_beff + r];
-    const double M = beff * s.ct + s.rho * sumtb;
-    const double dMdrho = beff * s.invM + sumtb;
+    M = third_body(m, b, s, r, C);
     if (kind == 2) {
       Ctbaf = M;
       K = 1.;
-      dCdrho = dMdrho;
     } else {
       const int f = b.i[m.i_fall + r];
-      const double *kp = b.d + m.d_kp + 3 * f;
-      const double kpf = kp[0] * tab_exp(kp[1] * s.logT - kp[2] * s.invT, b.d + m.d_exptab) / kf;
+      const double *kp = b.d + m.d_kp + 3 * f;  // the ratio k0 / kinf as A, b, E/R
+      const double kpf = kp[0] * tab_exp(fma(kp[1], s.logT, -(kp[2] * s.invT)), b.d + m.d_exptab);
       const double pr = kpf * M;
-      const double dlogk = s.invT * (kp[1] + kp[2] * s.invT) - dlogkf;
+      const double i1 = 1. / (1. + pr), hf = pr * i1;
+      const double Tdlogk = fma(kp[2], s.invT, kp[1]);
       if (kind == 3) {
-        Ctbaf = pr / (1. + pr);
+        Ctbaf = hf;
         if (JAC) {
-          dCdT = Ctbaf / (1. + pr) * dlogk;
-          K = kpf / ((1. + pr) * (1. + pr));
+          TdCdT = hf * i1 * Tdlogk;
+          K = kpf * i1 * i1;
         }
       } else {
-        const double *tr = b.d + m.d_troe + 4 * f;
-        const int terms = (info >> RI_TROE_SHIFT) & 7;
-        double fc = 0., dfc = 0.;
-        if (terms & 1) {
-          const double e1 = tab_exp(-s.T / tr[1], b.d + m.d_exptab);
-          fc += (1 - tr[0]) * e1;
-          dfc += (tr[0] - 1) / tr[1] * e1;
-        }
-        if (terms & 2) {
-          const double e2 = tab_exp(-s.T / tr[2], b.d + m.d_exptab);
-          fc += tr[0] * e2;
-          dfc += -tr[0] / tr[2] * e2;
-        }
-        if (terms & 4) {
-          const double e3 = tab_exp(-s.invT * tr[3], b.d + m.d_exptab);
-          fc += e3;
-          dfc += e3 * tr[3] * s.invT * s.invT;
-        }
-        if (!JAC) {
-          // chemistry_kernels.cpp:280-312: F = 10^(log10 Fc / (1 + f1^2)), no clamp on Fc
-          const double lfc = log10(fc);
-          const double lpc = log10(fmax(pr, 1.e-300)) + (-0.4 - 0.67 * lfc);
-          const double f1 = lpc / ((0.75 - 1.27 * lfc) - 0.14 * lpc);
-          Ctbaf = tab_exp(2.302585092994046 * (lfc / (1 + f1 * f1)), b.d + m.d_exptab) * pr / (1 + pr);
-        } else {
-          // rates_sensitivities_exact.cpp:949-985: F = Fc^g with Fc clamped at 1e-300
-          const double l10pr = log10(fmax(pr, 1.e-300));
-          const double lnfc = log(fmax(fc, 1.e-300));
-          const double l10fc = lnfc * 0.43429448190325176;
-          const double a = l10pr - 0.67 * l10fc - 0.4;
-          const double bb = -0.14 * l10pr - 1.1762 * l10fc + 0.806;
-          const double gt = 1 / (1 + (a / bb) * (a / bb));
-          const double F = tab_exp(gt * lnfc, b.d + m.d_exptab);
-          Ctbaf = F * pr / (1 + pr);
-          const double ln10 = 2.302585092994046;
-          const double dFdT = F * (gt / fc * dfc + lnfc * (-2.0 * gt * gt / ln10 * a / (bb * bb * bb) *
-                                                          ((bb + 0.14 * a) * dlogk - (0.67 * bb - 1.1762 * a) * dfc / fc)));
-          dCdT = 1. / (1. + 1. / pr) * dFdT + F * pr / ((1. + pr) * (1. + pr)) * dlogk;
-          K = kpf * (-2.0 / (1. + pr) * F * lnfc * gt * gt / ln10 * a / (bb * bb * bb) * (bb + 0.14 * a) +
-                     F / ((1. + pr) * (1 + pr)));
+        double Tdfc;
+        const double fc = troe_center<JAC>(m, b, s, f, (info >> RI_TROE_SHIFT) & 7, Tdfc);
+        constexpr double kLog10e = 0.43429448190325176;
+        const double l10pr = log(fmax(pr, 1.e-300)) * kLog10e;
+        // Fc clamped at 1e-300 in the sensitivities (rates_sensitivities_exact.cpp:949-985), not in the rates
+        // (chemistry_kernels.cpp:280-312): log10 F = log10 Fc / (1 + (a / bb)^2)
+        const double lnfc = log(JAC ? fmax(fc, 1.e-300) : fc);
+        const double l10fc = lnfc * kLog10e;
+        const double a = l10pr - 0.67 * l10fc - 0.4;
+        const double bb = 0.806 - 0.14 * l10pr - 1.1762 * l10fc;
+        const double b2 = bb * bb;
+        const double iq = 1. / fma(a, a, b2);
+        const double gt = b2 * iq;
+        const double F = tab_exp(gt * lnfc, b.d + m.d_exptab);
+        Ctbaf = F * hf;
+        if (JAC) {
+          const double dlfc = Tdfc / fc;
+          const double c1 = (-2. * kLog10e) * lnfc * (a * bb) * (iq * iq);
+          const double p1 = fma(0.14, a, bb) * c1;
+          const double TdlnF = fma(gt, dlfc, fma(p1, Tdlogk, -(c1 * (0.67 * bb - 1.1762 * a) * dlfc)));
+          TdCdT = Ctbaf * fma(i1, Tdlogk, TdlnF);
+          K = kpf * F * i1 * (p1 + i1);
         }
       }
-      if (JAC) dCdrho = K * dMdrho;
     }
   }
   const bool orders = has_ord && !(JAC && s.option == 1);
   const int ro0 = b.i[m.i_reac_off + r], nre = b.i[m.i_reac_off + r + 1] - ro0;
   const int po0 = b.i[m.i_prod_off + r], npr = b.i[m.i_prod_off + r + 1] - po0;
+  const int n0 = b.i[m.i_net_off + r], n1 = b.i[m.i_net_off + r + 1];
   const int *rl = b.i + m.i_reac + ro0;
   const int *pl = b.i + m.i_prod + po0;
-  double Rf, kr = 0., Rr = 0.;
+  double Rf, nkr = 0., nRr = 0.;  // the reverse side carries its minus sign
   const int sums = b.i[m.i_sums + r];
   const int sum_nu = (int)(short)(sums & 0xFFFF);
   // lists of at most three entries (every reaction of common mechanisms) use the factored form
-  const bool short_lists = !orders && nre <= 3 && npr <= 3;
-  MassAction3 mr, mp;
-  mp.P = mp.g0 = mp.g1 = mp.g2 = 0.;
+  const bool short_lists = !orders && (unsigned)(nre - 1) < 3u && (unsigned)(npr - 1) < 3u;
+  Side3 fr, fp;
+  fp.t0 = fp.t1 = fp.t2 = 0.;
   if (orders) {
     Rf = kf * special_orders(m, b, r, C, s.rho, -1, false);
   } else {
     if (short_lists) {
-      mr = mass_action3(rl, nre, C, invmw_d);
-      Rf = kf * mr.P;
+      fr = side3<JAC>(rl, nre, C, kf, smallint);
+      Rf = fr.R;
     } else {
-      Rf = kf * mass_action(rl, nre, C, invmw_d, s.rho, -1);
+      Rf = kf * mass_action(rl, nre, C, -1);
     }
     // rates of a special-order reaction have no reverse part (chemistry_kernels.cpp:316-326)
     if (rev && !has_ord) {
       // kr = kf exp(sum_nu ln(p_ref/RT) - sum_i nu_i g_i/RT) (chemistry_kernels.cpp:327-341), with
       // exp(-g_i/RT) = gm_i 2^gk_i
-      const int n0 = b.i[m.i_net_off + r], n1 = b.i[m.i_net_off + r + 1];
-      double mant = 1.;
-      long long K = 0;
+      nkr = -kf;
+      if (sum_nu) nkr *= sum_nu > 0 ? ipow(s.port, sum_nu) : ipow(s.invport, -sum_nu);
+      long long Kp = 0;
       for (int j = n0; j < n1; ++j) {
         const int e = b.i[m.i_net + j];
         const int sp = e & 0xFFFF, nu = (e >> 16) - 128;
         const double mi = scr[(nu > 0 ? L.gm : L.gmi) + sp];
         const int a = nu > 0 ? nu : -nu;
-        mant *= a == 1 ? mi : ipow(mi, a);
-        K += (long long)nu * __double_as_longlong(scr[L.gk + sp]);
+        nkr *= a == 1 ? mi : ipow(mi, a);
+        Kp += (long long)nu * __double2loint(scr[L.gk + sp]);
       }
-      const double pw = sum_nu >= 0 ? ipow(s.port, sum_nu) : ipow(s.invport, -sum_nu);
-      kr = scale_pow2(kf * pw * mant, K);
+      nkr = scale_pow2(nkr, Kp);
       if (short_lists) {
-        mp = mass_action3(pl, npr, C, invmw_d);
-        Rr = kr * mp.P;
+        fp = side3<JAC>(pl, npr, C, nkr, smallint);
+        nRr = fp.R;
       } else {
-        Rr = kr * mass_action(pl, npr, C, invmw_d, s.rho, -1);
+        nRr = nkr * mass_action(pl, npr, C, -1);
       }
     }
   }
-  const double Rnet = Rf - Rr;
-  scr[L.q + r] = Rnet * Ctbaf;
+  const double Rnet = Rf + nRr;
+  const double q = kind == 1 ? Rnet : Rnet * Ctbaf;
+  scr[L.q + r] = q;
   if (!JAC) return;
 
-  const double *smallint = b.d + m.d_smallint;
-  const double sum_reac_nu = small_int(smallint, (sums >> 16) & 0xFF),
-               sum_prod_nu = small_int(smallint, (sums >> 24) & 0xFF);
-  double dRdrho, dRdT;
+  const int snr = (sums >> 16) & 0xFF, snp = (sums >> 24) & 0xFF;
+  double rdRdrho, TdRdT = Rnet * Tdlogkf;
   if (orders) {
     double sumo = 0.;
     const int o0 = b.i[m.i_ord_off + r], o1 = b.i[m.i_ord_off + r + 1];
     for (int j = o0; j < o1; ++j)
       if (b.i[m.i_ord + j] >> 16) sumo += b.d[m.d_ord + j];
-    dRdrho = Rf * s.invRho * sumo;
-    dRdT = Rf * dlogkf;
+    rdRdrho = Rf * sumo;
   } else {
-    double dKc = 0.;
+    rdRdrho = snr == snp ? Rnet * small_int(smallint, snr)
+                         : fma(nRr, small_int(smallint, snp), Rf * small_int(smallint, snr));
     if (rev && !has_ord) {
-      const int n0 = b.i[m.i_net_off + r], n1 = b.i[m.i_net_off + r + 1];
+      double dKc = 0.;
       for (int j = n0; j < n1; ++j) {
         const int e = b.i[m.i_net + j];
-        dKc -= small_int(smallint, (e >> 16) - 128) * scr[L.dB + (e & 0xFFFF)];
+        dKc = fma(small_int(smallint, (e >> 16) - 128), scr[L.dB + (e & 0xFFFF)], dKc);
       }
+      TdRdT = fma(nRr, dKc, TdRdT);
     }
-    dRdrho = (Rf * sum_reac_nu - Rr * sum_prod_nu) * s.invRho;
-    dRdT = Rf * dlogkf - Rr * (dlogkf - dKc);
   }
-  const bool tbaf = s.option != 1;
-  scr[L.dqdrho + r] = dRdrho * Ctbaf + (tbaf ? dCdrho * Rnet : 0.);
-  scr[L.dqdT + r] = dRdT * Ctbaf + (tbaf ? dCdT * Rnet : 0.);
-  // d q / d Y_k / rho through the third-body concentration: rho * Rnet * K * eff_k / rho
-  const double RK = tbaf ? Rnet * K : 0.;
-  // sparse slots: D_j = d q / d Y_k / rho for the slot's species k
+  // d q / d Y_k / rho through the third-body concentration: Rnet K d M / d C_k
+  double RK = 0.;
+  if (kind != 1) {
+    rdRdrho *= Ctbaf;
+    TdRdT *= Ctbaf;
+    if (s.option != 1) {
+      RK = Rnet * K;
+      rdRdrho = fma(RK, M, rdRdrho);  // rho dM/drho = M
+      TdRdT = fma(Rnet, TdCdT, TdRdT);
+    }
+  }
+  scr[L.dqdrho + r] = rdRdrho;
+  scr[L.dqdT + r] = TdRdT;
+  // sparse slots: D_j = d q / d C_k for the slot's species k
   const int ns = m.ns;
   const int s0 = b.i[m.i_slot_off + r], s1 = b.i[m.i_slot_off + r + 1];
   const int tb0 = b.i[m.i_tb_off + r];
@@ -566,70 +660,69 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
     const int e = b.i[m.i_slot + j];
     const int rp = ((e >> 16) & 15) - 1, pp = ((e >> 20) & 15) - 1, tp = ((e >> 24) & 15) - 1;
     const int op = ((unsigned)e >> 28) - 1;
-    double v = 0.;  // d (Rf - Rr) / d Y_k / rho
+    double v = 0.;  // d (Rf - Rr) / d C_k
     if (orders) {
       if (op >= 0) {
         const int oe = b.i[m.i_ord + b.i[m.i_ord_off + r] + op];
-        if (oe >> 16) v = kf * special_orders(m, b, r, C, s.rho, op, false) * s.invRho;
+        if (oe >> 16)
+          v = kf * special_orders(m, b, r, C, s.rho, op, false) * s.invRho * b.d[m.d_mw + (e & 0xFFFF)];
       }
     } else if (short_lists) {
-      if (rp >= 0) v += kf * mr.g(rp);
-      if (pp >= 0 && kr != 0.) v -= kr * mp.g(pp);
+      if (rp >= 0) v = fr.t(rp);
+      if (pp >= 0) v = rp >= 0 ? v + fp.t(pp) : fp.t(pp);
     } else {
-      if (rp >= 0) v += kf * mass_action(rl, nre, C, invmw_d, s.rho, rp) * s.invRho;
-      if (pp >= 0 && kr != 0.) v -= kr * mass_action(pl, npr, C, invmw_d, s.rho, pp) * s.invRho;
+      if (rp >= 0) v += kf * mass_action(rl, nre, C, rp);
+      if (pp >= 0) v += nkr * mass_action(pl, npr, C, pp);
     }
-    double Dv = Ctbaf * v;
-    if (tp >= 0) Dv += RK * b.d[m.d_tbeff + tb0 + tp];
-    scr[L.D + j] = Dv;
+    if (kind != 1) {
+      v *= Ctbaf;
+      if (tp >= 0) v = fma(RK, b.d[m.d_tbeff + tb0 + tp], v);
+    }
+    scr[L.D + j] = v;
   }
   const int di = b.i[m.i_dense + r];
   double Er = 0.;
-  {
-    const int n0 = b.i[m.i_net_off + r], n1 = b.i[m.i_net_off + r + 1];
-    for (int j = n0; j < n1; ++j) Er += b.d[m.d_netc + j] * scr[L.eh + (b.i[m.i_net + j] & 0xFFFF)];
-  }
+  for (int j = n0; j < n1; ++j) Er = fma(b.d[m.d_netc + j], scr[L.eh + (b.i[m.i_net + j] & 0xFFFF)], Er);
   scr[L.E + r] = Er;
   if (di >= 0) {
     // closure species ns-1 and third-body terms common to every Y column (all divided by rho)
-    double closure = 0.;
+    double closure = 0.;  // -d (Rf - Rr) / d C_{ns-1}
     if (orders) {
       const int o0 = b.i[m.i_ord_off + r], o1 = b.i[m.i_ord_off + r + 1];
       for (int j = o0; j < o1; ++j) {
         const int oe = b.i[m.i_ord + j];
         if ((oe & 0xFFFF) == ns - 1 && (oe >> 16))
-          closure -= kf * special_orders(m, b, r, C, s.rho, j - o0, true) * s.invRho;
+          closure -= kf * special_orders(m, b, r, C, s.rho, j - o0, true) * s.invRho * b.d[m.d_mw + ns - 1];
       }
-    } else if (short_lists) {
-      for (int j = 0; j < nre; ++j)
-        if ((rl[j] & 0xFFFF) == ns - 1) closure -= kf * mr.g(j);
-      if (kr != 0.)
-        for (int j = 0; j < npr; ++j)
-          if ((pl[j] & 0xFFFF) == ns - 1) closure += kr * mp.g(j);
     } else {
       for (int j = 0; j < nre; ++j)
-        if ((rl[j] & 0xFFFF) == ns - 1) closure -= kf * mass_action(rl, nre, C, invmw_d, s.rho, j) * s.invRho;
-      if (kr != 0.)
+        if ((rl[j] & 0xFFFF) == ns - 1) closure -= short_lists ? fr.t(j) : kf * mass_action(rl, nre, C, j);
+      if (rev && !has_ord)
         for (int j = 0; j < npr; ++j)
-          if ((pl[j] & 0xFFFF) == ns - 1) closure += kr * mass_action(pl, npr, C, invmw_d, s.rho, j) * s.invRho;
+          if ((pl[j] & 0xFFFF) == ns - 1) closure -= short_lists ? fp.t(j) : nkr * mass_action(pl, npr, C, j);
     }
-    double beta = Ctbaf * closure;
-    if (tbaf && kind != 1) {
-      const int t1 = b.i[m.i_tb_off + r + 1];
-      for (int j = tb0; j < t1; ++j)
-        if (b.i[m.i_tb + j] == ns - 1) beta -= RK * b.d[m.d_tbeff + j];
+    double beta = closure;
+    double alpha = 0.;
+    if (kind != 1) {
+      beta *= Ctbaf;
+      if (s.option != 1) {
+        const int t1 = b.i[m.i_tb_off + r + 1];
+        for (int j = tb0; j < t1; ++j)
+          if (b.i[m.i_tb + j] == ns - 1) beta -= RK * b.d[m.d_tbeff + j];
+      }
+      alpha = RK * b.d[m.d_beff + r];
     }
-    const double alpha = (kind != 1) ? RK * b.d[m.d_beff + r] : 0.;
+    beta *= b.d[m.d_invmw + ns - 1];
     scr[L.alpha + di] = alpha;
     scr[L.beta + di] = beta;
-    *Eacc_a += Er * alpha;
-    *Eacc_b += Er * beta;
+    *Eacc_a = fma(Er, alpha, *Eacc_a);
+    *Eacc_b = fma(Er, beta, *Eacc_b);
   }
 }
 
 // ------------------------------------------------------------------------------------------ gather programs
-// Execute a gather program for one state: every lane runs prog.len items (see sf_mech.h). Destination kinds:
-// DST_SCRATCH / DST_TROW write scratch[index]; DST_JBLOCK calls jw(row, col, value).
+// Execute a gather program for one state: every lane runs prog.len items (see sf_mech.h). Scratch destinations are
+// written to scratch, Jacobian ones passed to jw(row, col, value), their sums starting from scratch[qoff + row].
 // Items are processed in batches of U (each lane's item count is padded to a multiple of GATHER_UNROLL): the
 // operands of a whole batch are loaded before its FMAs, and the next batch's items while they run. This is sound
 // because no program reads a scratch location that it writes (checked when the program is built), so no load
@@ -639,55 +732,59 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
 // (scratch in shared memory or L2) take half the batch, which keeps their larger kernels free of register spills.
 __host__ __device__ constexpr int default_unroll(int G) { return G == 1 ? GATHER_UNROLL : GATHER_UNROLL / 2; }
 
-template <class S>
-__device__ __forceinline__ double gather_operand(uint32_t ref, const double *blobd, const S &scr)
-{
-  return (ref & REF_SCRATCH) ? scr[ref & ~REF_SCRATCH] : blobd[ref];
-}
-
-template <int G, int U = default_unroll(G), class JW, class S>
-__device__ __forceinline__ void run_program(const DevProgram &prog, int lane, const double *blobd, S scr,
-                                            JW &jw)
+template <int G, int U, class JW, class S>
+__device__ __forceinline__ void run_items(const DevProgram &prog, int lane, S scr, int qoff, JW &jw)
 {
   static_assert(GATHER_UNROLL % U == 0, "batch must divide the program padding");
   const uint4 *it = reinterpret_cast<const uint4 *>(prog.items) + lane;
   uint4 x[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) x[u] = prog.len > 0 ? __ldg(it + u * G) : make_uint4(0, 0, 0, F_NOP);
+  for (int u = 0; u < U; ++u) x[u] = prog.len > 0 ? __ldg(it + u * G) : make_uint4(0, 0, 0, IT_NOP);
   double acc = 0.;
   for (int j = 0; j < prog.len; j += U) {
     double a[U], bv[U], c0[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      a[u] = gather_operand(x[u].x, blobd, scr);
-      bv[u] = gather_operand(x[u].y, blobd, scr);
-      const uint32_t ii = x[u].w & INIT_MASK;
-      c0[u] = ((x[u].w & F_START) && ii) ? scr[ii - 1] : 0.;
+      a[u] = __hiloint2double((int)x[u].y, (int)x[u].x);
+      if (x[u].w & IT_PAIR) a[u] = scr[x[u].x];
+      bv[u] = scr[x[u].z];
+      c0[u] = 0.;
+      if ((x[u].w & (IT_START | IT_JAC)) == (IT_START | IT_JAC)) c0[u] = scr[qoff + (x[u].w & IT_ROW_MASK)];
     }
     uint4 y[U];
     const bool more = j + U < prog.len;
 #pragma unroll
-    for (int u = 0; u < U; ++u) y[u] = more ? __ldg(it + (j + U + u) * G) : make_uint4(0, 0, 0, F_NOP);
+    for (int u = 0; u < U; ++u) y[u] = more ? __ldg(it + (j + U + u) * G) : make_uint4(0, 0, 0, IT_NOP);
     bool stop = false;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (x[u].w & F_NOP) {
+      if (x[u].w & IT_NOP) {
         stop = true;  // padding only follows a lane's last real item
       } else {
-        if (x[u].w & F_START) acc = c0[u];
-        acc = fma(a[u], bv[u], acc);
-        if (x[u].w & F_END) {
-          const uint32_t kindd = x[u].z & DST_KIND_MASK;
-          if (kindd == DST_JBLOCK)
-            jw(x[u].z & 0x7FFF, (x[u].z >> 15) & 0x7FFF, acc);
+        acc = fma(a[u], bv[u], (x[u].w & IT_START) ? c0[u] : acc);
+        if (x[u].w & IT_END) {
+          if (x[u].w & IT_JAC)
+            jw((int)(x[u].w & IT_ROW_MASK), (int)((x[u].w >> IT_COL_SHIFT) & IT_ROW_MASK), acc);
           else
-            scr[x[u].z & ~DST_KIND_MASK] = acc;
+            scr[x[u].w & IT_DST_MASK] = acc;
         }
       }
     }
     if (stop) break;
 #pragma unroll
     for (int u = 0; u < U; ++u) x[u] = y[u];
+  }
+}
+
+// A program and, where it has one, the second pass that adds the partial sums of its split entries.
+template <int G, int U = default_unroll(G), class JW, class S>
+__device__ __forceinline__ void run_program(const DevProgram &prog, const Group<G> &grp, S scr, int qoff, JW &jw)
+{
+  run_items<G, U>(prog, grp.lane, scr, qoff, jw);
+  if (prog.fix_len > 0) {
+    grp.sync();
+    DevProgram fix{prog.fix_items, prog.fix_len};
+    run_items<G, U>(fix, grp.lane, scr, qoff, jw);
   }
 }
 

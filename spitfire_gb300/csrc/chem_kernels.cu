@@ -93,19 +93,7 @@ __device__ __forceinline__ void eval_state(const KParams &p, const DevMech &m, c
   double sim = 0.;
   for (int i = lane; i < ns; i += G) sim += scr[L.y + i] * b.d[m.d_invmw + i];
   sim = grp.sum(sim);
-  const double mmw = 1. / sim;
-  StateCtx s;
-  s.T = T;
-  s.logT = log(T);
-  s.invT = 1. / T;
-  s.rho = rho;
-  s.invRho = 1. / rho;
-  s.mmw = mmw;
-  s.invM = 1. / mmw;
-  s.ct = rho / mmw;
-  s.port = m.pref * s.invT * m.invRu;
-  s.invport = 1. / s.port;
-  s.option = p.option;
+  const StateCtx s = state_ctx<G>(m, grp, T, rho, sim, 0., true, p.option);
   prep_species<G, JAC>(m, b, L, scr, grp, s, false, MODE == MODE_SENS);
   reactions_and_gathers<G, JAC>(m, b, L, scr, grp, s, pg);
   if (MODE == MODE_RATES) {
@@ -118,13 +106,13 @@ __device__ __forceinline__ void eval_state(const KParams &p, const DevMech &m, c
   double *Sb = p.out_S + (size_t)st * n1 * n1;
   for (int i = lane; i < ns; i += G) {
     p.out_w[(size_t)st * ns + i] = scr[L.w + i];
-    Sb[i] = scr[L.Srho + i];
-    Sb[n1 + i] = scr[L.ST + i];
+    Sb[i] = scr[L.Srho + i] * s.invRho;  // the gathers hold rho S_rho and T S_T
+    Sb[n1 + i] = scr[L.ST + i] * s.invT;
   }
   for (int k = lane; k < n1; k += G) Sb[k * n1 + ns] = 0.;
   grp.sync();
   JWriter<G> jw{Sb, n1, 0, 2, rho};
-  run_program<G>(p.prog_j, lane, b.d, scr, jw);
+  run_program<G>(p.prog_j, grp, scr, L.Q, jw);
   grp.sync();
 }
 

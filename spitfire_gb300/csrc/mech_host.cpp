@@ -24,8 +24,7 @@ static int pack_sp(int s, int hi) { return (s & 0xFFFF) | (hi << 16); }
 HostMech::~HostMech()
 {
   for (auto &kv : programs) {
-    for (auto &p : kv.second.progs)
-      if (p.items) cudaFree((void *)p.items);
+    for (GatherItem *p : kv.second.owned) cudaFree(p);
   }
   if (d_blob) cudaFree(d_blob);
   if (d_status) cudaFree(d_status);
@@ -45,6 +44,7 @@ void HostMech::build(const sf_mech_desc *d)
   m.Ru = d->gas_constant;
   m.invRu = 1. / d->gas_constant;
   m.pref = d->ref_pressure;
+  m.ipref = 1. / m.pref;
 
   // ---------------- species
   invmw.resize(ns);
@@ -106,7 +106,7 @@ void HostMech::build(const sf_mech_desc *d)
       for (int i = d->eff_offsets[r]; i < d->eff_offsets[r + 1]; ++i) {
         const int s = d->eff_species[i];
         x.tb.push_back(s);
-        x.tbeff.push_back(invmw[s] * (d->eff_values[i] - x.beff));
+        x.tbeff.push_back(d->eff_values[i] - x.beff);
       }
     if (d->order_offsets && d->order_offsets[r + 1] > d->order_offsets[r]) {
       x.has_orders = true;
@@ -172,15 +172,18 @@ void HostMech::build(const sf_mech_desc *d)
     x.dense = (x.kind != SF_RXN_SIMPLE) || last_involved;
     x.dense_idx = x.dense ? n_dense++ : -1;
   }
-  // Device order: reactions grouped by kind and, within a kind, by their number of Jacobian slots (stable).
-  // Lanes of a state group take reactions in strides of the group width, so the per-reaction slot loop of a
-  // group iteration then runs about as many times for every lane. Per-reaction outputs map back through i_orig.
+  // Device order: reactions grouped by kind and, within a kind, by the form of their forward constant (those without an
+  // exponential first), the lengths of their sides and their number of Jacobian slots (stable). Lanes of a state
+  // group take reactions in strides of the group width, so the lanes of a pass then mostly take the same paths and
+  // run the slot loop about as many times. Per-reaction outputs map back through i_orig.
   std::vector<int> order(nr);
   std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    if (rx[a].kind != rx[b].kind) return rx[a].kind < rx[b].kind;
-    return rx[a].slots.size() < rx[b].slots.size();
-  });
+  auto key = [&](int r) {
+    const HRxn &x = rx[r];
+    return std::array<int, 6>{x.kind, x.kform == 4 ? 1 : 0, x.reversible ? 0 : 1, (int)x.reac.size(),
+                              (int)x.prod.size(), (int)x.slots.size()};
+  };
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key(a) < key(b); });
   {
     std::vector<HRxn> sorted(nr);
     for (int k = 0; k < nr; ++k) sorted[k] = std::move(rx[order[k]]);
@@ -223,8 +226,10 @@ void HostMech::build(const sf_mech_desc *d)
     const HRxn &x = rx[r];
     for (int j = 0; j < 3; ++j) D[m.d_kf + 3 * r + j] = x.kf[j];
     if (x.fall >= 0) {
-      for (int j = 0; j < 3; ++j) D[m.d_kp + 3 * x.fall + j] = x.kp[j];
-      for (int j = 0; j < 4; ++j) D[m.d_troe + 4 * x.fall + j] = x.troe[j];
+      D[m.d_kp + 3 * x.fall] = x.kp[0] / x.kf[0];
+      for (int j = 1; j < 3; ++j) D[m.d_kp + 3 * x.fall + j] = x.kp[j] - x.kf[j];
+      const double tr[4] = {x.troe[0], -1. / x.troe[1], -1. / x.troe[2], x.troe[3]};
+      for (int j = 0; j < 4; ++j) D[m.d_troe + 4 * x.fall + j] = tr[j];
     }
     D[m.d_beff + r] = x.beff;
   }
@@ -361,27 +366,34 @@ void ensure_dynamic_smem(const void *kernel, size_t bytes)
 
 // ------------------------------------------------------------------------------------------ gather programs
 namespace {
+struct Item {
+  double c;
+  uint32_t ref;
+  int pair;  // >= 0: scratch index of the coefficient
+};
 struct Entry {
-  std::vector<std::pair<uint32_t, uint32_t>> items;  // (a, b)
-  uint32_t init;  // scratch index + 1, or 0
-  uint32_t dst;
+  std::vector<Item> items;
+  uint32_t dst;  // IT_JAC | row | col << IT_COL_SHIFT, or a scratch index
 };
 
 // The device runner loads operands ahead of the stores of earlier items, so a program must never read a scratch
 // location that it writes (as a destination or through an entry's initial value).
-void check_no_read_after_write(const std::vector<Entry> &entries)
+void check_no_read_after_write(const std::vector<Entry> &entries, int qoff)
 {
   std::vector<uint32_t> written;
   for (const Entry &e : entries)
-    if ((e.dst & DST_KIND_MASK) != DST_JBLOCK) written.push_back(e.dst & ~DST_KIND_MASK);
+    if (!(e.dst & IT_JAC)) written.push_back(e.dst);
   std::sort(written.begin(), written.end());
-  auto is_written = [&](uint32_t idx) { return std::binary_search(written.begin(), written.end(), idx); };
+  auto check = [&](uint32_t idx) {
+    if (std::binary_search(written.begin(), written.end(), idx))
+      throw sf_error(SF_ERR_MECHANISM, "internal: gather program reads what it writes");
+  };
   for (const Entry &e : entries) {
-    if (e.init && is_written(e.init - 1)) throw sf_error(SF_ERR_MECHANISM, "internal: gather program reads what it writes");
-    for (auto &it : e.items)
-      for (uint32_t ref : {it.first, it.second})
-        if ((ref & REF_SCRATCH) && is_written(ref & ~REF_SCRATCH))
-          throw sf_error(SF_ERR_MECHANISM, "internal: gather program reads what it writes");
+    if (e.dst & IT_JAC) check(qoff + (e.dst & IT_ROW_MASK));
+    for (const Item &it : e.items) {
+      check(it.ref);
+      if (it.pair >= 0) check(it.pair);
+    }
   }
 }
 
@@ -389,18 +401,16 @@ void check_no_read_after_write(const std::vector<Entry> &entries)
 // multiple of the device runner's batch. G > 1: longest-processing-time assignment (balanced lanes). G = 1 (one
 // lane per state): entries in destination order, Jacobian entries column-major, so that each thread writes its
 // Jacobian block sequentially through memory.
-std::vector<GatherItem> schedule(std::vector<Entry> &entries, int G, int *len_out)
+std::vector<GatherItem> schedule(const std::vector<Entry> &entries, int G, int qoff, int *len_out)
 {
-  check_no_read_after_write(entries);
+  check_no_read_after_write(entries, qoff);
   std::vector<int> order(entries.size());
   std::iota(order.begin(), order.end(), 0);
   if (G == 1) {
     auto key = [&](int e) {
       const uint32_t d = entries[e].dst;
-      const uint64_t kind = d & DST_KIND_MASK;
-      const uint64_t pos = kind == DST_JBLOCK ? (uint64_t)((d >> 15) & 0x7FFF) << 15 | (d & 0x7FFF)
-                                              : (uint64_t)(d & ~DST_KIND_MASK);
-      return kind << 32 | pos;
+      const uint64_t jac = (d & IT_JAC) ? 0 : 1;  // the Jacobian first
+      return jac << 32 | (d & IT_DST_MASK);       // col << 13 | row: column-major
     };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key(a) < key(b); });
   } else {
@@ -419,23 +429,59 @@ std::vector<GatherItem> schedule(std::vector<Entry> &entries, int G, int *len_ou
   size_t len = 0;
   for (int l = 0; l < G; ++l) len = std::max(len, load[l]);
   len = (len + GATHER_UNROLL - 1) / GATHER_UNROLL * GATHER_UNROLL;
-  std::vector<GatherItem> out(len * G, GatherItem{0, 0, 0, F_NOP});
+  std::vector<GatherItem> out(len * G, GatherItem{0., 0, IT_NOP});
   for (int l = 0; l < G; ++l) {
     size_t j = 0;
     for (int e : lane[l]) {
       const Entry &E = entries[e];
       for (size_t k = 0; k < E.items.size(); ++k, ++j) {
-        GatherItem it;
-        it.a = E.items[k].first;
-        it.b = E.items[k].second;
-        it.dst = E.dst;
-        it.flags = (k == 0 ? F_START | (E.init & INIT_MASK) : 0) | (k + 1 == E.items.size() ? F_END : 0);
+        const Item &x = E.items[k];
+        GatherItem it{x.c, x.ref, E.dst};
+        if (x.pair >= 0) {
+          const uint64_t bits = (uint32_t)x.pair;
+          std::memcpy(&it.c, &bits, 8);
+          it.ctl |= IT_PAIR;
+        }
+        if (k == 0) it.ctl |= IT_START;
+        if (k + 1 == E.items.size()) it.ctl |= IT_END;
         out[j * G + l] = it;
       }
     }
   }
   *len_out = (int)len;
   return out;
+}
+
+// Entries longer than a lane's share are cut into parts of about that share, which sum into the scratch slots
+// part .. part + cap - 1 and are added up by the entries put into `fix`. (GRI-3.0's species rates on 32 lanes: 137
+// items for H against a share of 39.) A Jacobian entry's first item, u_k P_i on top of Q_i, stays in its fix entry.
+std::vector<Entry> split_entries(const std::vector<Entry> &entries, int G, int part, int cap, std::vector<Entry> *fix)
+{
+  if (G == 1) return entries;
+  size_t total = 0;
+  for (const Entry &e : entries) total += e.items.size();
+  for (size_t share = std::max<size_t>(4, (total + G - 1) / G);; share += (share + 3) / 4) {
+    std::vector<Entry> out;
+    fix->clear();
+    int used = 0;
+    for (const Entry &e : entries) {
+      const size_t keep = (e.dst & IT_JAC) ? 1 : 0, n = e.items.size() - std::min(keep, e.items.size());
+      if (e.items.size() <= share + share / 8) {
+        out.push_back(e);
+        continue;
+      }
+      const size_t parts = (n + share - 1) / share;
+      Entry f{{e.items.begin(), e.items.begin() + keep}, e.dst};
+      for (size_t p = 0; p < parts; ++p) {
+        const size_t a = keep + n * p / parts, b = keep + n * (p + 1) / parts;
+        out.push_back(Entry{{e.items.begin() + a, e.items.begin() + b}, (uint32_t)(part + used)});
+        f.items.push_back(Item{1., (uint32_t)(part + used), -1});
+        ++used;
+      }
+      fix->push_back(f);
+    }
+    if (used <= cap) return out;
+  }
 }
 }  // namespace
 
@@ -444,94 +490,87 @@ void HostMech::build_programs(int G)
   if (programs.count(G)) return;
   const int ns = dm.ns, nr = dm.nr;
   const ScratchLayout &L = sl;
-  auto S = [](int idx) { return REF_SCRATCH | (uint32_t)idx; };
-  auto B = [](int idx) { return (uint32_t)idx; };
-  // species -> list of (reaction, net entry) in increasing reaction order
-  std::vector<std::vector<std::pair<int, int>>> by_species(ns);
+  // species -> list of (reaction, coefficient of its rate) in increasing reaction order
+  std::vector<std::vector<std::pair<int, double>>> by_species(ns);
   for (int r = 0; r < nr; ++r)
-    for (size_t i = 0; i < rx[r].net.size(); ++i) by_species[rx[r].net[i]].push_back({r, net_entry_of[r][i]});
-  Programs P;
+    for (size_t i = 0; i < rx[r].net.size(); ++i)
+      by_species[rx[r].net[i]].push_back({r, host_dbl[dm.d_netc + net_entry_of[r][i]]});
+  std::vector<Entry> E[4];
+  auto item = [](double c, int ref) { return Item{c, (uint32_t)ref, -1}; };
   // program 0: production rates only  w_i = sum_r c_ir q_r
-  {
-    std::vector<Entry> E;
-    for (int i = 0; i < ns; ++i) {
-      Entry e{{}, 0, DST_SCRATCH | (uint32_t)(L.w + i)};
-      for (auto &re : by_species[i]) e.items.push_back({B(dm.d_netc + re.second), S(L.q + re.first)});
-      E.push_back(e);
-    }
-    auto items = schedule(E, G, &P.progs[0].len);
-    P.host_items[0] = items;
+  for (int i = 0; i < ns; ++i) {
+    Entry e{{}, (uint32_t)(L.w + i)};
+    for (auto &re : by_species[i]) e.items.push_back(item(re.second, L.q + re.first));
+    E[0].push_back(e);
   }
   // program 1: w, S_rho, S_T, P, Q for all species
-  {
-    std::vector<Entry> E;
-    for (int i = 0; i < ns; ++i) {
-      Entry ew{{}, 0, DST_SCRATCH | (uint32_t)(L.w + i)};
-      Entry er{{}, 0, DST_SCRATCH | (uint32_t)(L.Srho + i)};
-      Entry et{{}, 0, DST_SCRATCH | (uint32_t)(L.ST + i)};
-      Entry ep{{}, 0, DST_SCRATCH | (uint32_t)(L.P + i)};
-      Entry eq{{}, 0, DST_SCRATCH | (uint32_t)(L.Q + i)};
-      for (auto &re : by_species[i]) {
-        const uint32_t c = B(dm.d_netc + re.second);
-        ew.items.push_back({c, S(L.q + re.first)});
-        er.items.push_back({c, S(L.dqdrho + re.first)});
-        et.items.push_back({c, S(L.dqdT + re.first)});
-        const int di = rx[re.first].dense_idx;
-        if (di >= 0) {
-          ep.items.push_back({c, S(L.alpha + di)});
-          eq.items.push_back({c, S(L.beta + di)});
-        }
+  for (int i = 0; i < ns; ++i) {
+    Entry ew{{}, (uint32_t)(L.w + i)}, er{{}, (uint32_t)(L.Srho + i)}, et{{}, (uint32_t)(L.ST + i)},
+        ep{{}, (uint32_t)(L.P + i)}, eq{{}, (uint32_t)(L.Q + i)};
+    for (auto &re : by_species[i]) {
+      const double c = re.second;
+      ew.items.push_back(item(c, L.q + re.first));
+      er.items.push_back(item(c, L.dqdrho + re.first));
+      et.items.push_back(item(c, L.dqdT + re.first));
+      const int di = rx[re.first].dense_idx;
+      if (di >= 0) {
+        ep.items.push_back(item(c, L.alpha + di));
+        eq.items.push_back(item(c, L.beta + di));
       }
-      for (Entry *e : {&ew, &er, &et, &ep, &eq}) E.push_back(*e);
     }
-    auto items = schedule(E, G, &P.progs[1].len);
-    P.host_items[1] = items;
+    for (Entry *e : {&ew, &er, &et, &ep, &eq}) E[1].push_back(*e);
   }
-  // program 2: the Y block (rows/cols 0..ns-2) and the T-row sums
+  // program 2: the Y block (rows/cols 0..ns-2) and the T-row sums; program 3: every species row (the (ns+1)^2
+  // sensitivity block of prod_rates_primitive_sensitivities)
   {
-    std::vector<std::vector<std::vector<std::pair<int, int>>>> contrib(ns);  // [row][col] -> (net entry, slot)
+    std::vector<std::vector<std::vector<std::pair<double, int>>>> contrib(ns);  // [row][col] -> (coefficient, slot)
     for (int i = 0; i < ns; ++i) contrib[i].resize(ns - 1);
     std::vector<std::vector<std::pair<int, int>>> tcontrib(ns - 1);  // [col] -> (reaction, slot)
     for (int r = 0; r < nr; ++r) {
       const HRxn &x = rx[r];
       for (size_t j = 0; j < x.slots.size(); ++j) {
-        const int s = x.slots[j] & 0xFFFF;
-        tcontrib[s].push_back({r, slot_entry_of[r][j]});
-        for (size_t i = 0; i < x.net.size(); ++i) {
-          contrib[x.net[i]][s].push_back({net_entry_of[r][i], slot_entry_of[r][j]});
-        }
+        const int k = x.slots[j] & 0xFFFF;
+        tcontrib[k].push_back({r, slot_entry_of[r][j]});
+        for (size_t i = 0; i < x.net.size(); ++i)
+          contrib[x.net[i]][k].push_back({host_dbl[dm.d_netc + net_entry_of[r][i]] * invmw[k], slot_entry_of[r][j]});
       }
     }
     for (int variant = 2; variant <= 3; ++variant) {
-      // variant 2: reactor Y block (species rows 0..ns-2) + T-row sums; variant 3: every species row (the
-      // (ns+1)^2 sensitivity block of prod_rates_primitive_sensitivities)
       const int nrows = variant == 2 ? ns - 1 : ns;
-      std::vector<Entry> E;
       for (int i = 0; i < nrows; ++i)
         for (int k = 0; k < ns - 1; ++k) {
-          Entry e{{}, (uint32_t)(L.Q + i + 1), DST_JBLOCK | (uint32_t)i | ((uint32_t)k << 15)};
-          e.items.push_back({S(L.P + i), B(dm.d_u + k)});
-          for (auto &c : contrib[i][k]) e.items.push_back({B(dm.d_netc + c.first), S(L.D + c.second)});
-          E.push_back(e);
+          Entry e{{}, IT_JAC | (uint32_t)i | ((uint32_t)k << IT_COL_SHIFT)};
+          e.items.push_back(item(host_dbl[dm.d_u + k], L.P + i));
+          for (auto &c : contrib[i][k]) e.items.push_back(item(c.first, L.D + c.second));
+          E[variant].push_back(e);
         }
       if (variant == 2)
         for (int k = 0; k < ns - 1; ++k) {
-          Entry e{{}, 0, DST_TROW | (uint32_t)(L.trow + k)};
-          for (auto &c : tcontrib[k]) e.items.push_back({S(L.E + c.first), S(L.D + c.second)});
-          E.push_back(e);
+          Entry e{{}, (uint32_t)(L.trow + k)};
+          for (auto &c : tcontrib[k]) e.items.push_back(Item{0., (uint32_t)(L.D + c.second), L.E + c.first});
+          E[variant].push_back(e);
         }
-      auto items = schedule(E, G, &P.progs[variant].len);
-      P.host_items[variant] = items;
     }
   }
+  Programs P;
   for (int k = 0; k < 4; ++k) {
-    P.progs[k].G = G;
-    const auto &items = P.host_items[k];
-    GatherItem *dptr = nullptr;
-    const size_t bytes = std::max<size_t>(items.size(), 1) * sizeof(GatherItem);
-    CUDA_THROW(cudaMalloc(&dptr, bytes));
-    if (!items.empty()) CUDA_THROW(cudaMemcpy(dptr, items.data(), items.size() * sizeof(GatherItem), cudaMemcpyHostToDevice));
-    P.progs[k].items = dptr;
+    // partial sums: the Gibbs factors are dead after the reactions, dqdrho and dqdT after the species gathers
+    const int part = k < 2 ? L.gm : L.dqdrho, cap = k < 2 ? L.q - L.gm : L.E - L.dqdrho;
+    std::vector<Entry> fix;
+    const std::vector<Entry> main = split_entries(E[k], G, part, cap, &fix);
+    auto upload = [&](const std::vector<Entry> &entries, int *len) -> const GatherItem * {
+      const std::vector<GatherItem> items = schedule(entries, G, L.Q, len);
+      GatherItem *dptr = nullptr;
+      CUDA_THROW(cudaMalloc(&dptr, std::max<size_t>(items.size(), 1) * sizeof(GatherItem)));
+      P.owned.push_back(dptr);
+      if (!items.empty())
+        CUDA_THROW(cudaMemcpy(dptr, items.data(), items.size() * sizeof(GatherItem), cudaMemcpyHostToDevice));
+      return dptr;
+    };
+    P.progs[k].items = upload(main, &P.progs[k].len);
+    P.progs[k].fix_items = nullptr;
+    P.progs[k].fix_len = 0;
+    if (!fix.empty()) P.progs[k].fix_items = upload(fix, &P.progs[k].fix_len);
   }
   programs.emplace(G, std::move(P));
 }

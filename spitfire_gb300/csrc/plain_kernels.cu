@@ -7,7 +7,7 @@
 // Also: the plain form of the batched ignition integrator, one thread per reactor running the same ESDIRK64 step
 // logic over plain_state and a serial LU (the comparison point of integrate_kernels.cu), and the thermodynamic
 // property kernel behind sf_thermo_batch (thermodynamics_kernels.cpp:18-382).
-#include "chem_device.cuh"
+#include "reactor_eval.cuh"
 #include "esdirk64.cuh"
 #include "sf_internal.h"
 
@@ -47,27 +47,27 @@ __device__ void plain_state(const DevMech &m, const Blob &b, const ScratchLayout
   scr[L.y + ns - 1] = 1. - ysum;
   double sim = 0.;
   for (int i = 0; i < ns; ++i) sim += scr[L.y + i] * b.d[m.d_invmw + i];
-  const double mmw = 1. / sim;
   if (iso) {
     rho = qs[0];
     T = qs[1];
   } else {
+    rho = 0.;
     T = qs[0];
-    rho = pressure * mmw / (T * m.Ru);
   }
-  StateCtx s;
-  s.T = T; s.logT = log(T); s.invT = 1. / T; s.rho = rho; s.invRho = 1. / rho; s.mmw = mmw; s.invM = 1. / mmw;
-  s.ct = rho / mmw; s.port = m.pref * s.invT * m.invRu; s.invport = 1. / s.port; s.option = 0;
+  const Group<1> one;
+  const StateCtx s = state_ctx<1>(m, one, T, rho, sim, pressure, iso, 0);
+  rho = s.rho;
+  const double mmw = s.mmw;
   double cpmix = 0., cpsens = 0.;
   for (int i = 0; i < ns; ++i) {
     const double invmw = b.d[m.d_invmw + i];
     scr[L.C + i] = scr[L.y + i] * rho * invmw;
     const SpeciesThermo th = species_thermo(m, b, i, T, s.logT, s.invT, JAC);
-    store_gibbs_factor(scr, L, i, th.g * s.invT * m.invRu, b.d + m.d_exptab);
+    store_gibbs_factor(scr, L, i, th.g * (s.invT * m.invRu), b.d + m.d_exptab);
     scr[L.eh + i] = iso ? th.h - m.Ru * T * invmw : th.h;
     scr[L.cpv + i] = iso ? th.cp - m.Ru * invmw : th.cp;
     if (JAC) {
-      scr[L.dB + i] = th.dB;
+      scr[L.dB + i] = th.TdB;
       scr[L.dcp + i] = th.dcp;
       cpsens += scr[L.y + i] * th.dcp;
     }
@@ -86,15 +86,15 @@ __device__ void plain_state(const DevMech &m, const Blob &b, const ScratchLayout
       const double al = di >= 0 ? scr[L.alpha + di] : 0., be = di >= 0 ? scr[L.beta + di] : 0.;
       for (int k = 0; k < ns - 1; ++k) dq[k] = al * b.d[m.d_u + k] + be;
       for (int j = b.i[m.i_slot_off + r]; j < b.i[m.i_slot_off + r + 1]; ++j)
-        dq[b.i[m.i_slot + j] & 0xFFFF] += scr[L.D + j];
+        dq[b.i[m.i_slot + j] & 0xFFFF] += scr[L.D + j] * b.d[m.d_invmw + (b.i[m.i_slot + j] & 0xFFFF)];
     }
     for (int j = b.i[m.i_net_off + r]; j < b.i[m.i_net_off + r + 1]; ++j) {
       const int i = b.i[m.i_net + j] & 0xFFFF;
       const double c = b.d[m.d_netc + j];
       scr[L.w + i] += c * scr[L.q + r];
       if (JAC) {
-        S[i] += c * scr[L.dqdrho + r];
-        S[i + n1] += c * scr[L.dqdT + r];
+        S[i] += c * (scr[L.dqdrho + r] * s.invRho);
+        S[i + n1] += c * (scr[L.dqdT + r] * s.invT);
         for (int k = 0; k < ns - 1; ++k) S[i + (2 + k) * n1] += c * dq[k];
       }
     }

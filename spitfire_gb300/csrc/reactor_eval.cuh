@@ -46,7 +46,7 @@ __device__ __forceinline__ SpeciesSums prep_species(const DevMech &m, const Blob
     const double invmw = b.d[m.d_invmw + i];
     scr[L.C + i] = yi * s.rho * invmw;
     const SpeciesThermo th = species_thermo(m, b, i, s.T, s.logT, s.invT, JAC);
-    store_gibbs_factor(scr, L, i, th.g * s.invT * m.invRu, b.d + m.d_exptab);
+    store_gibbs_factor(scr, L, i, th.g * (s.invT * m.invRu), b.d + m.d_exptab);
     if (want_eh) {
       scr[L.eh + i] = isochoric ? th.h - m.Ru * s.T * invmw : th.h;
       scr[L.cpv + i] = isochoric ? th.cp - m.Ru * invmw : th.cp;
@@ -57,7 +57,7 @@ __device__ __forceinline__ SpeciesSums prep_species(const DevMech &m, const Blob
     // gather destinations start at zero: an entry with no contributions (an inert species) is never written
     scr[L.w + i] = 0.;
     if (JAC) {
-      scr[L.dB + i] = th.dB;
+      scr[L.dB + i] = th.TdB;
       scr[L.dcp + i] = th.dcp;
       cpsens += yi * th.dcp;
       scr[L.Srho + i] = 0.;
@@ -66,11 +66,39 @@ __device__ __forceinline__ SpeciesSums prep_species(const DevMech &m, const Blob
       scr[L.Q + i] = 0.;
     }
   }
-  SpeciesSums r;
-  r.cpmix = grp.sum(cpmix);
-  r.cpsens = JAC ? grp.sum(cpsens) : 0.;
+  SpeciesSums r{cpmix, cpsens};
+  if (JAC) {
+    grp.sum2(r.cpmix, r.cpsens);
+  } else {
+    r.cpmix = grp.sum(r.cpmix);
+  }
   grp.sync();
   return r;
+}
+
+// Scalars of a state: three reciprocals in one division sequence, everything else products.
+template <int G>
+__device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &grp, double T, double rho, double sim,
+                                              double pres, bool isochoric, int option)
+{
+  StateCtx s;
+  s.T = T;
+  s.logT = log(T);
+  double ix;  // 1 / rho isochoric, 1 / p isobaric
+  grp.recip3(T, sim, isochoric ? rho : pres, s.invT, s.mmw, ix);
+  s.invM = sim;
+  if (isochoric) {
+    s.rho = rho;
+    s.invRho = ix;
+  } else {
+    s.rho = pres * s.mmw * (s.invT * m.invRu);
+    s.invRho = T * m.Ru * (sim * ix);
+  }
+  s.ct = s.rho * sim;
+  s.port = m.pref * s.invT * m.invRu;
+  s.invport = T * (m.Ru * m.ipref);
+  s.option = option;
+  return s;
 }
 
 // P2 + P3: reaction rates (and derivatives) and the species gathers. Returns (EA, EB) of the T-row dense terms.
@@ -81,13 +109,10 @@ __device__ __forceinline__ double2 reactions_and_gathers(const DevMech &m, const
 {
   double EA = 0., EB = 0.;
   for (int r = grp.lane; r < m.nr; r += G) eval_reaction<JAC>(m, b, L, scr, s, r, &EA, &EB);
-  if (JAC) {
-    EA = grp.sum(EA);
-    EB = grp.sum(EB);
-  }
+  if (JAC) grp.sum2(EA, EB);
   grp.sync();
   NoJ noj;
-  run_program<G, U>(JAC ? pg.full : pg.w, grp.lane, b.d, scr, noj);
+  run_program<G, U>(JAC ? pg.full : pg.w, grp, scr, L.Q, noj);
   grp.sync();
   return make_double2(EA, EB);
 }
@@ -113,37 +138,28 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
   } else {
     T = qs[0];
   }
-  double sy = 0.;
+  // the last mass fraction is 1 - sum y (extract_y, combustion_kernels.h:526-535), so 1 / mmw = sum y_i / M_i =
+  // 1 / M_last + sum y_i u_i
+  double sy = 0., sim = 0.;
   for (int i = lane; i < ns - 1; i += G) {
     const double yi = qs[(isochoric ? 2 : 1) + i];
     scr[L.y + i] = yi;
     sy += yi;
+    sim = fma(yi, b.d[m.d_u + i], sim);
   }
-  sy = grp.sum(sy);
-  if (lane == 0) scr[L.y + ns - 1] = 1. - sy;  // extract_y (combustion_kernels.h:526-535)
+  grp.sum2(sy, sim);
+  if (lane == 0) scr[L.y + ns - 1] = 1. - sy;
   grp.sync();
-  double sim = 0.;
-  for (int i = lane; i < ns; i += G) sim += scr[L.y + i] * b.d[m.d_invmw + i];
-  sim = grp.sum(sim);
-  const double mmw = 1. / sim;
-  if (!isochoric) rho = pres * mmw / (T * m.Ru);
-  StateCtx s;
-  s.T = T;
-  s.logT = log(T);
-  s.invT = 1. / T;
-  s.rho = rho;
-  s.invRho = 1. / rho;
-  s.mmw = mmw;
-  s.invM = 1. / mmw;
-  s.ct = rho / mmw;
-  s.port = m.pref * s.invT * m.invRu;
-  s.invport = 1. / s.port;
-  s.option = c.option;
+  sim += b.d[m.d_invmw + ns - 1];
+  const StateCtx s = state_ctx<G>(m, grp, T, rho, sim, pres, isochoric, c.option);
+  rho = s.rho;
+  const double mmw = s.mmw;
   // ---------------- P1-P3
   const SpeciesSums sums = prep_species<G, JAC>(m, b, L, scr, grp, s, isochoric, true);
   const double2 E = reactions_and_gathers<G, JAC, U>(m, b, L, scr, grp, s, pg);
   const double EA = E.x, EB = E.y;
-  const double cmix = isochoric ? sums.cpmix - m.Ru / mmw : sums.cpmix;  // cv or cp
+  const double cmix = isochoric ? sums.cpmix - m.Ru * sim : sums.cpmix;  // cv or cp
+  const double invRho = s.invRho, iC = 1. / cmix, iRC = iC * invRho;
   const double cpsens = sums.cpsens;
   // feed of an open reactor (isochoric_reactor_kernels.cpp:39-154, isobaric_reactor_kernels.cpp:31-168):
   // fe = sum_i (e_i(Tin) - e_i(T)) yin_i (enthalpies when isobaric), fc = sum_i yin_i cv_i(T) (cp_i)
@@ -157,15 +173,14 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
       fe += (ein - scr[L.eh + i]) * yi;
       fc += yi * scr[L.cpv + i];
     }
-    fe = grp.sum(fe);
-    fc = grp.sum(fc);
+    grp.sum2(fe, fc);
   }
   // mass-exchange factor of the species and energy equations: rho_in / (tau rho) isochoric, 1 / tau isobaric
   const double itau = open_ ? 1. / c.tau : 0.;
-  const double mfac = open_ ? (isochoric ? itau * c.rho_in / rho : itau) : 0.;
-  const double mrT = open_ ? fe / cmix * mfac : 0.;  // feed term of the temperature equation
+  const double mfac = open_ ? (isochoric ? itau * c.rho_in * invRho : itau) : 0.;
+  const double mrT = open_ ? fe * iC * mfac : 0.;  // feed term of the temperature equation
 
-  // ---------------- P4: right-hand side and rho/T columns
+  // ---------------- P4: right-hand side and rho/T columns. The gathers hold rho S_rho and T S_T.
   double swe = 0., sre = 0., ste = 0., swc = 0.;
   for (int i = lane; i < ns; i += G) {
     const double e = scr[L.eh + i];
@@ -176,18 +191,14 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
       swc += scr[L.w + i] * scr[L.cpv + i];
     }
   }
-  swe = grp.sum(swe);
-  if (JAC) {
-    sre = grp.sum(sre);
-    ste = grp.sum(ste);
-    swc = grp.sum(swc);
-  }
-  const double invRho = s.invRho;
-  const double iC = 1. / cmix, iRC = 1. / (rho * cmix);
-  const double rhsT = -swe / (rho * cmix);
+  if (JAC)
+    grp.sum4(swe, sre, ste, swc);
+  else
+    swe = grp.sum(swe);
+  const double rhsT = -swe * iRC;
   double qheat = 0.;
   if (c.heat == 2)
-    qheat = c.SoV / (rho * cmix) * (c.hc * (c.Tc - T) + c.eps * 5.67e-8 * (c.Tr * c.Tr * c.Tr * c.Tr - T * T * T * T));
+    qheat = c.SoV * iRC * (c.hc * (c.Tc - T) + c.eps * 5.67e-8 * (c.Tr * c.Tr * c.Tr * c.Tr - T * T * T * T));
   const int tix = isochoric ? 1 : 0;  // index of T in the state
   for (int i = lane; i < ns - 1; i += G) {
     double v = scr[L.w + i] * invRho;
@@ -203,25 +214,25 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
     return;
   }
   // primitive rho and T columns of the T row (chem_jac_isochoric / chem_jac_isobaric)
-  const double JTrho = -iRC * sre - invRho * rhsT;
-  const double JTT = -iC * (invRho * (ste + swc) + rhsT * cpsens);
+  const double JTrho = -invRho * fma(iRC, sre, rhsT);
+  const double JTT = -iC * (invRho * fma(s.invT, ste, swc) + rhsT * cpsens);
   const double cpv_last = scr[L.cpv + ns - 1];
   if (isochoric) {
+    const double ir2 = invRho * invRho, irt = invRho * s.invT;
     for (int i = lane; i < ns - 1; i += G) {
-      double v = invRho * (scr[L.Srho + i] - invRho * scr[L.w + i]);
+      double v = ir2 * (scr[L.Srho + i] - scr[L.w + i]);
       if (open_) v -= (c.yin[i] - scr[L.y + i]) * mfac * invRho;
       jset(2 + i, 0, v);
-      jset(2 + i, 1, invRho * scr[L.ST + i]);
+      jset(2 + i, 1, irt * scr[L.ST + i]);
     }
   } else {
     // isobaric transform (isobaric_reactor_kernels.cpp:319-343): T column = PJ_T - rho/T * PJ_rho, and the Y
-    // columns get (-rho*mmw) * u_k * PJ_rho, folded into P
-    const double roT = rho / T, nrm = -rho * mmw;
+    // columns get (-rho*mmw) * u_k * PJ_rho, folded into P; PJ_rho = (rho S_rho - w) / rho^2
+    const double irt = invRho * s.invT, nmr = -(mmw * invRho);
     for (int i = lane; i < ns - 1; i += G) {
-      const double pjr = invRho * (scr[L.Srho + i] - invRho * scr[L.w + i]);
-      const double pjt = invRho * scr[L.ST + i];
-      jset(1 + i, 0, pjt - roT * pjr);
-      scr[L.P + i] += nrm * pjr;
+      const double d = scr[L.Srho + i] - scr[L.w + i];
+      jset(1 + i, 0, irt * (scr[L.ST + i] - d));
+      scr[L.P + i] = fma(nmr, d, scr[L.P + i]);
     }
   }
   for (int k = lane; k < ns; k += G) scr[L.trow + k] = 0.;
@@ -237,18 +248,17 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
       if (diag && row == col) v += dyy;
       jset(off + row, off + col, v);
     };
-    run_program<G, U>(pg.j, lane, b.d, scr, yblock);
+    run_program<G, U>(pg.j, grp, scr, L.Q, yblock);
   }
   grp.sync();
 
-  // ---------------- P6: T row (and the zero rho row of the isochoric Jacobian)
+  // ---------------- P6: T row (and the zero rho row of the isochoric Jacobian). trow holds the sums over D = dq/dC.
   const double iso_heat = (c.heat == 1) ? 0. : 1.;
+  const double fT = rhsT + mrT + qheat;  // every heat term of dT/dt varies with Y_k through the mixture's heat capacity
   if (isochoric) {
     for (int k = lane; k < ns - 1; k += G) {
-      const double ts = scr[L.trow + k] + b.d[m.d_u + k] * EA + EB;
-      double v = -iC * ts - rhsT * (scr[L.cpv + k] - cpv_last) * iC;
-      if (open_) v += -iC * mrT * (scr[L.cpv + k] - cpv_last);
-      if (c.heat == 2) v += iC * qheat * (cpv_last - scr[L.cpv + k]);
+      const double ts = fma(scr[L.trow + k], b.d[m.d_invmw + k], fma(b.d[m.d_u + k], EA, EB));
+      const double v = -iC * fma(fT, scr[L.cpv + k] - cpv_last, ts);
       jset(1, 2 + k, v * iso_heat);
     }
     for (int k = lane; k < neq; k += G) jset(0, k, (k == 0 && open_) ? -itau : 0.);
@@ -259,28 +269,27 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
         j11 += -iC * (itau * invRho * c.rho_in * fc + cpsens * mrT);
       }
       if (c.heat == 2) {
-        j10 += -qheat / rho;
+        j10 += -qheat * invRho;
         j11 += -iC * cpsens * qheat - c.SoV * iRC * (c.hc + 4. * c.eps * 5.67e-8 * T * T * T);
       }
       jset(1, 0, j10 * iso_heat);
       jset(1, 1, j11 * iso_heat);
     }
   } else {
-    const double roT = rho / T, nrm = -rho * mmw;
+    const double roT = rho * s.invT, nrm = -rho * mmw;
     double pjr = JTrho, pjt = JTT;
     if (open_) pjt += -iC * (cpsens * mrT + itau * fc);
     if (c.heat == 2) {
-      pjr += -qheat / rho;
+      pjr += -qheat * invRho;
       pjt += -iC * cpsens * qheat - c.SoV * iRC * (c.hc + 4. * c.eps * 5.67e-8 * T * T * T);
     }
     pjr *= iso_heat;
     pjt *= iso_heat;
+    const double upj = nrm * pjr, niC = -iC * iso_heat;
     for (int k = lane; k < ns - 1; k += G) {
-      const double ts = scr[L.trow + k] + b.d[m.d_u + k] * EA + EB;
-      double v = -iC * ts - rhsT * (scr[L.cpv + k] - cpv_last) * iC;
-      if (open_) v += -mrT * (scr[L.cpv + k] - cpv_last) * iC;
-      if (c.heat == 2) v += iC * qheat * (cpv_last - scr[L.cpv + k]);
-      jset(0, 1 + k, v * iso_heat + nrm * b.d[m.d_u + k] * pjr);
+      const double u = b.d[m.d_u + k];
+      const double ts = fma(scr[L.trow + k], b.d[m.d_invmw + k], fma(u, EA, EB));
+      jset(0, 1 + k, fma(niC, fma(fT, scr[L.cpv + k] - cpv_last, ts), u * upj));
     }
     if (lane == 0) jset(0, 0, pjt - roT * pjr);
   }

@@ -54,7 +54,7 @@ struct HostMech {
 
   struct Programs {
     DevProgram progs[4]{};  // 0: w only, 1: w/S_rho/S_T/P/Q, 2: Y block + T row, 3: all species rows (sens)
-    std::vector<GatherItem> host_items[4];
+    std::vector<GatherItem *> owned;  // device allocations of the items
   };
   std::map<int, Programs> programs;
 

@@ -31,16 +31,16 @@ struct DevMech {
   int blob_doubles; // size of the double section
   int blob_ints;    // size of the int section
   int blob_bytes;   // total, multiple of 16
-  double Ru, invRu, pref;
+  double Ru, invRu, pref, ipref;
 
   // ---- double section offsets ----
   int d_nasa;    // [ns][15] Griffon NASA7 storage (chemistry_setup.cpp:102-130); const-cp: [T0, h0, s0, cp, ...]
   int d_tmin, d_tmax, d_invmw, d_mw, d_u;  // [ns]; u_s = 1/M_s - 1/M_{ns-1}
   int d_kf;      // [nr][3] A, b, Ea/R
-  int d_kp;      // [n_fall][3]
-  int d_troe;    // [n_fall][4]
+  int d_kp;      // [n_fall][3] the ratio k0 / kinf: A0/A, b0 - b, (E0 - E)/R
+  int d_troe;    // [n_fall][4] a, -1/T3, -1/T1, T2
   int d_beff;    // [nr] default third-body efficiency
-  int d_tbeff;   // [tb entries] invM*(eff - default)
+  int d_tbeff;   // [tb entries] eff - default
   int d_netc;    // [net entries] -nu*M (coefficient of q_r in w_i)
   int d_ord;     // [order entries] special orders
   int d_one;     // 1.0
@@ -64,29 +64,31 @@ struct DevMech {
 };
 
 // ---------------------------------------------------------------------------------------- gather programs
-// A gather program computes many sums  acc = init + sum_k a_k * b_k  with one FMA per item, spread over the G
-// lanes of a state group in a static, load-balanced schedule: item j of lane l sits at items[j*G + l] and every
-// lane executes exactly `len` items, so the loop has no divergence. Operand references name a double either in
-// the mechanism blob (shared memory) or in the state's scratch area.
+// A gather program computes many sums  acc = init + sum_k c_k x_k  with one FMA per item, spread over the G
+// lanes of a state group in a static, load-balanced schedule: item j of lane l sits at items[j*G + l]. The item holds
+// the coefficient itself, so that an FMA needs one 16-byte item and one scratch load; x_k is a double of the state's
+// scratch area (in a pair item, so is the coefficient). An entry longer than a lane's share is split into partial sums
+// on several lanes, which a second short program (fix) adds up.
 struct GatherItem {
-  uint32_t a;      // operand ref
-  uint32_t b;      // operand ref
-  uint32_t dst;    // destination (see DST_*), valid on END items
-  uint32_t flags;  // START | END | NOP, init ref in the low 24 bits (0 = start from zero)
+  double c;      // coefficient (pair items: scratch index of the other factor in the low word)
+  uint32_t ref;  // scratch index of x
+  uint32_t ctl;  // IT_* flags; Jacobian entries: row | col << IT_COL_SHIFT; scratch destinations: their index
 };
-constexpr uint32_t REF_SCRATCH = 0x80000000u;  // else blob double table
-constexpr uint32_t F_START = 0x80000000u, F_END = 0x40000000u, F_NOP = 0x20000000u;
-constexpr uint32_t INIT_MASK = 0x00FFFFFFu;    // scratch index + 1 of the initial value
-constexpr uint32_t DST_SCRATCH = 0u << 30, DST_JBLOCK = 1u << 30, DST_TROW = 2u << 30;
-constexpr uint32_t DST_KIND_MASK = 3u << 30;
+constexpr uint32_t IT_START = 0x80000000u, IT_END = 0x40000000u, IT_NOP = 0x20000000u, IT_PAIR = 0x10000000u;
+constexpr uint32_t IT_JAC = 0x08000000u;       // Jacobian entry (init: scratch[Q + row]); else scratch destination
+constexpr uint32_t IT_DST_MASK = 0x03FFFFFFu;
+constexpr uint32_t IT_ROW_MASK = 0x1FFFu;
+constexpr int IT_COL_SHIFT = 13;
 constexpr int GATHER_UNROLL = 8;  // items per batch of the device runner; each lane's item count is a multiple
 
 // Per-state scratch layout (doubles), shared by every kernel of one mechanism.
 struct ScratchLayout {
   int y, C, dB, eh, cpv, dcp;          // species arrays [ns]
-  int gm, gmi, gk;                     // [ns] exp(-g/RT) = gm * 2^gk (gk as integer bits), gmi = 1 / gm
+  int gm, gmi, gk;                     // [ns] exp(-g/RT) = gm * 2^gk (gk an int in the low word), gmi = 1 / gm; dead
+                                       // after the reactions: partial sums of the species gathers
   int w, Srho, ST, P, Q, trow;         // gather destinations [ns]
-  int q, dqdrho, dqdT, E;              // reaction arrays [nr]
+  int q, dqdrho, dqdT, E;              // reaction arrays [nr]; dqdrho, dqdT: dead after the species gathers, then
+                                       // partial sums of the Jacobian gathers
   int alpha, beta;                     // [n_dense]
   int D;                               // [n_slots]
   int misc;                            // 16 scalars
@@ -95,9 +97,10 @@ struct ScratchLayout {
 };
 
 struct DevProgram {
-  const GatherItem *items;  // device
-  int len;                  // items per lane
-  int G;                    // lanes per group
+  const GatherItem *items;      // device
+  int len;                      // items per lane
+  const GatherItem *fix_items;  // sums of split entries, after the items and a group barrier
+  int fix_len;
 };
 
 }  // namespace sfgb
