@@ -2,13 +2,13 @@
 
 For one mechanism on the current device it times the candidate shapes on a sample of the caller's workload with
 CUDA events and applies the fastest through ``sf_mech_set_tuning``:
-  * lanes per state (8, 16, 32, or 1: the thread-per-state kernels, with their resident blocks per SM) of the
-    production-rate, right-hand-side and Jacobian kernels;
+  * lanes per state (0: the library's own rule on the batch size; 8, 16, 32; or 1: the thread-per-state kernels, with
+    their resident blocks per SM) of the production-rate, right-hand-side and Jacobian kernels;
   * for the persistent ESDIRK64 integrator: where each warp keeps its Griffon scratch and iteration matrix (shared
     memory, or L2-resident global slots, which leave room for more warps per SM) and how many warps (reactors)
-    share a block.
-The knobs change launch shapes only. The integrator's candidates produce bit-identical results; the lane-group
-width changes the order of the per-species sums, so those candidates agree to rounding (the tuner checks both).
+    share a block, against the library's own choice (0, 0), which for large mechanisms is eight warps per reactor.
+The knobs change launch shapes only. The integrator's one-warp candidates produce bit-identical results; the group
+width changes the order of the per-species sums, so other candidates agree to rounding (the tuner checks both).
 Choices are cached per (mechanism, device) in spitfire_gb300/_tuning (created on first use).
 """
 
@@ -67,8 +67,8 @@ def _key(mech):
 def tune_chemistry(mech, states, pressures=None, configuration='isochoric', kinds=('rates', 'rhs', 'jac'), reps=3,
                    thread_per_state=True):
     """Choose lanes per state for each kernel family on `states` (a batch of reactor states of the given
-    configuration): 8, 16 or 32, or (with thread_per_state) 1 at a few resident-block counts of the thread-per-state
-    kernels. Returns {knob: (best value, {candidate: ms})}, candidates labelled G or '1/<blocks per SM>', and, when
+    configuration): 0 (the library's rule), 8, 16 or 32, or (with thread_per_state) 1 at a few resident-block counts of
+    the thread-per-state kernels. Returns {knob: (best value, {candidate: ms})}, candidates labelled G or '1/<blocks per SM>', and, when
     a family chose 1, 'tps_ctas': (blocks per SM, None)."""
     torch = _torch()
     from ._desc import reactor_params
@@ -93,7 +93,7 @@ def tune_chemistry(mech, states, pressures=None, configuration='isochoric', kind
         knob = 'group_' + kind
         times = {}
         ref = None
-        cands = {8: 8, 16: 16, 32: 32}
+        cands = {0: 0, 8: 8, 16: 16, 32: 32}
         if thread_per_state:
             cands.update({f'1/{c}': (1, c) for c in (0, 2, 1)})  # label '1/<blocks per SM>' (0: all that fit)
         for label, cand in cands.items():
@@ -134,8 +134,8 @@ def tune_chemistry(mech, states, pressures=None, configuration='isochoric', kind
 def tune_integrator(integrator, q0, pressures=None, reps=1, **controls):
     """Choose the integrator's memory placement and warps per block on a sample batch (q0 rows): scratch 3 (all in
     shared memory), 1 (Griffon scratch in an L2-resident global slot per warp) or 2 (the iteration matrix there
-    too). The sample should fill the largest candidate's resident warps (16 per SM at 8 warps per block), or the
-    smaller shapes win on it. Returns (best (scratch, warps), {(scratch, warps): ms})."""
+    too), or (0, 0), the library's own choice. The sample should fill the largest candidate's resident warps (16 per SM
+    at 8 warps per block), or the smaller shapes win on it. Returns (best (scratch, warps), {(scratch, warps): ms})."""
     torch = _torch()
     mech = integrator.mech
     times = {}
@@ -157,6 +157,16 @@ def tune_integrator(integrator, q0, pressures=None, reps=1, **controls):
                 raise RuntimeError(f'integrator shape {(scratch, warps)} changed the results')
             times[(scratch, warps)] = _time(lambda: integrator.run(q0, pressures=pressures, **controls), reps)
     best = pick_integrator_shape(times)
+    # the library's own shape: other groupings of the same sums, so the delays agree to the integration's sensitivity
+    set_tuning(mech, 'integrate_scratch', 0)
+    set_tuning(mech, 'integrate_warps', 0)
+    res = integrator.run(q0, pressures=pressures, **controls)
+    torch.cuda.synchronize()
+    if not torch.equal(ref['status'], res['status']) or float(((ref['t'] - res['t']).abs() / ref['t']).max()) > 1.e-6:
+        raise RuntimeError('integrator shape (0, 0) changed the results beyond rounding')
+    times[(0, 0)] = _time(lambda: integrator.run(q0, pressures=pressures, **controls), reps)
+    if times[(0, 0)] <= times[best]:
+        best = (0, 0)
     set_tuning(mech, 'integrate_scratch', best[0])
     set_tuning(mech, 'integrate_warps', best[1])
     return best, times

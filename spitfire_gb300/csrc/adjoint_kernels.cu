@@ -61,7 +61,7 @@ __device__ double falloff_factor(const DevMech &m, const Blob &b, const ScratchL
 }
 
 template <int G>
-__global__ void __launch_bounds__(256) rate_param_adjoint_kernel(const AdjParams p)
+__global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) rate_param_adjoint_kernel(const AdjParams p)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t bar;
@@ -70,9 +70,11 @@ __global__ void __launch_bounds__(256) rate_param_adjoint_kernel(const AdjParams
   const Blob b = blob_at(m, smem);
   const ScratchLayout &L = p.L;
   const int gid = threadIdx.x / G;
-  double *scr = reinterpret_cast<double *>(smem + m.blob_bytes) + (size_t)gid * (L.total_rhs + p.neq + 2);
+  double *shared = reinterpret_cast<double *>(smem + m.blob_bytes) +
+                   (size_t)gid * (L.total_rhs + p.neq + 2 + Group<G>::kShared);
+  double *scr = shared + Group<G>::kShared;
   double *rhs_tmp = scr + L.total_rhs;
-  const Group<G> grp;
+  const Group<G> grp(shared, gid);
   const int lane = grp.lane;
   const int ns = m.ns, nr = m.nr, neq = p.neq;
   const bool isochoric = p.cfg.configuration == 1;
@@ -90,7 +92,7 @@ __global__ void __launch_bounds__(256) rate_param_adjoint_kernel(const AdjParams
         sim += scr[L.y + i] * b.d[m.d_invmw + i];
         cmix += scr[L.y + i] * scr[L.cpv + i];
       }
-      grp.sum2(sim, cmix);
+      grp.sum2(sim, cmix, ns);
       const StateCtx s = state_ctx<G>(m, grp, T, isochoric ? qs[0] : 0., sim, pres, isochoric, 0);
       const double icmix = 1. / cmix;
       for (int r = lane; r < nr; r += G) {
@@ -127,7 +129,11 @@ void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pre
                                cudaStream_t st)
 {
   if (n_items == 0) return;
-  constexpr int G = 32;
+  int dev, smem_max, nsm;
+  CUDA_THROW(cudaGetDevice(&dev));
+  CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int G = n_items <= 2 * nsm ? 256 : (n_items <= 8 * nsm ? 64 : 32);
   const auto &progs = hm.programs_for(G);
   AdjParams p{};
   p.m = hm.dm;
@@ -149,21 +155,21 @@ void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pre
   p.q = q;
   p.w = w;
   p.out = out;
-  int dev, smem_max, nsm;
-  CUDA_THROW(cudaGetDevice(&dev));
-  CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t per = (size_t)(hm.sl.total_rhs + p.neq + 2) * 8;
+  const int shared = wide_group_doubles(G);
+  const size_t per = (size_t)(hm.sl.total_rhs + p.neq + 2 + shared) * 8;
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
-  const int groups = (int)std::min<size_t>(avail / per, 256 / G);
+  int groups = (int)std::min<size_t>(avail / per, (G > 32 ? 512 : 256) / G);
   if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the parameter-adjoint kernel");
+  groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)n_items + nsm - 1) / nsm));
   p.groups_per_cta = groups;
   const size_t smem = hm.dm.blob_bytes + per * groups;
-  ensure_dynamic_smem((const void *)rate_param_adjoint_kernel<G>, smem);
+  auto kern = G == 256 ? rate_param_adjoint_kernel<256>
+                       : (G == 64 ? rate_param_adjoint_kernel<64> : rate_param_adjoint_kernel<32>);
+  ensure_dynamic_smem((const void *)kern, smem);
   const int bps = std::max(1, (int)((size_t)smem_max / smem));
   const int grid = (int)std::max<long long>(
       1, std::min<long long>(((long long)n_items + groups - 1) / groups, (long long)nsm * bps));
-  rate_param_adjoint_kernel<G><<<grid, groups * G, smem, st>>>(p);
+  kern<<<grid, groups * G, smem, st>>>(p);
   CUDA_THROW(cudaGetLastError());
 }
 

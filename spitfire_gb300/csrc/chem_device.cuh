@@ -83,24 +83,35 @@ __device__ inline bool stage_to_smem(void *dst, const void *src, uint32_t bytes,
 // a warp costs the same 64-76 cycles of its scheduler's FP64 unit however many lanes carry a value, and the
 // transposed reduction below adds four 32-lane sums in 6 instructions instead of 20 (the first two exchanges leave
 // each quarter of the lanes with one of the four sums).
-template <int G>
+//
+// Group<G>, G <= 32: part of a warp. Group<G>, G = 128 or 256: several warps of a block, for launches with too few
+// states to give every scheduler of the GPU a warp of its own (below).
+template <int G, bool WIDE = (G > 32)>
 struct Group {
+  static constexpr int kShared = 0;  // doubles of shared memory the group's reductions take
   int lane;       // 0..G-1
   unsigned mask;  // lanes of this group within the warp
-  __device__ __forceinline__ Group()
+  __device__ __forceinline__ Group(double * = nullptr, int = 0)
   {
     const int wl = threadIdx.x & 31;
     lane = wl & (G - 1);
     mask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (wl & ~(G - 1)));
   }
   __device__ __forceinline__ void sync() const { __syncwarp(mask); }
-  __device__ __forceinline__ double sum(double v) const
+  // The sums take the number of leading lanes that hold a value (a wide group's other warps then add nothing).
+  __device__ __forceinline__ double max(double v, int = G) const
+  {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(mask, v, o, G));
+    return v;
+  }
+  __device__ __forceinline__ double sum(double v, int = G, int = 0) const
   {
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o, G);
     return v;
   }
-  __device__ __forceinline__ void sum2(double &a, double &b) const
+  __device__ __forceinline__ void sum2(double &a, double &b, int = G, int = 0) const
   {
     if (G == 1) return;
     constexpr int H = G > 1 ? G / 2 : 1;
@@ -111,7 +122,7 @@ struct Group {
     a = __shfl_sync(mask, r, 0, G);
     b = __shfl_sync(mask, r, H, G);
   }
-  __device__ __forceinline__ void sum4(double &a, double &b, double &c, double &d) const
+  __device__ __forceinline__ void sum4(double &a, double &b, double &c, double &d, int = G) const
   {
     if (G < 4) {
       sum2(a, b);
@@ -146,6 +157,92 @@ struct Group {
     ic = __shfl_sync(mask, r, G < 4 ? 0 : 2, G);
   }
 };
+
+// A state group of several whole warps of one block (G = 128 or 256 threads). An SM's FP64 rate is shared by four
+// schedulers and one warp can use only its own scheduler's quarter, so a launch whose states are fewer than about
+// four per SM runs each of them on all four. Warps meet at the group's own named barrier; a reduction goes through
+// shared memory, with two alternating buffers so that one barrier per reduction is enough (a thread reuses a buffer only
+// after the next reduction's barrier, which every thread passes after its reads of this one).
+template <int G>
+struct Group<G, true> {
+  static constexpr int W = G / 32;
+  static constexpr int kScalars = 16;
+  static constexpr int kShared = 2 * 4 * W + kScalars;
+  int lane, warp, id;
+  double *red, *scalars;
+  mutable int flip;
+  __device__ __forceinline__ Group(double *shared, int group_in_block)
+      : lane(threadIdx.x % G), warp((threadIdx.x % G) >> 5), id(1 + group_in_block), red(shared),
+        scalars(shared + 2 * 4 * W), flip(0)
+  {
+  }
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(G) : "memory"); }
+  // N values per warp published by its first lane; the warps that hold data are those of the lanes first .. first +
+  // count - 1
+  template <int N, class Op>
+  __device__ __forceinline__ void combine(double (&v)[N], int count, int first, Op op) const
+  {
+    const int w0 = first >> 5, w1 = min(W, (first + count + 31) >> 5);
+    double *buf = red + flip * 4 * W;
+    flip ^= 1;
+    if (warp >= w0 && warp < w1 && (lane & 31) == 0) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) buf[4 * warp + j] = v[j];
+    }
+    sync();
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = buf[4 * w0 + j];
+    for (int w = w0 + 1; w < w1; ++w) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] = op(v[j], buf[4 * w + j]);
+    }
+  }
+  __device__ __forceinline__ bool holds(int count, int first) const
+  {
+    return warp * 32 < first + count && warp * 32 + 31 >= first;
+  }
+  static __device__ __forceinline__ double add(double a, double b) { return a + b; }
+  static __device__ __forceinline__ double larger(double a, double b) { return fmax(a, b); }
+  __device__ __forceinline__ double max(double v, int count = G) const
+  {
+    if (holds(count, 0)) v = Group<32>().max(v);
+    double t[1] = {v};
+    combine(t, count, 0, larger);
+    return t[0];
+  }
+  __device__ __forceinline__ double sum(double v, int count = G, int first = 0) const
+  {
+    if (holds(count, first)) v = Group<32>().sum(v);
+    double t[1] = {v};
+    combine(t, count, first, add);
+    return t[0];
+  }
+  __device__ __forceinline__ void sum2(double &a, double &b, int count = G, int first = 0) const
+  {
+    // a warp whose lanes hold only zeros (as most do in the sums over third-body reactions) skips the exchange
+    const bool any = ((__double_as_longlong(a) | __double_as_longlong(b)) << 1) != 0;
+    if (holds(count, first) && __any_sync(0xffffffffu, any)) Group<32>().sum2(a, b);
+    double t[2] = {a, b};
+    combine(t, count, first, add);
+    a = t[0];
+    b = t[1];
+  }
+  __device__ __forceinline__ void sum4(double &a, double &b, double &c, double &d, int count = G) const
+  {
+    if (holds(count, 0)) Group<32>().sum4(a, b, c, d);
+    double t[4] = {a, b, c, d};
+    combine(t, count, 0, add);
+    a = t[0];
+    b = t[1];
+    c = t[2];
+    d = t[3];
+  }
+};
+
+inline int wide_group_doubles(int G)
+{
+  return G == 256 ? Group<256>::kShared : (G == 128 ? Group<128>::kShared : (G == 64 ? Group<64>::kShared : 0));
+}
 
 struct Blob {
   const double *d;

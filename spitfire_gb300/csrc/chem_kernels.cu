@@ -136,7 +136,7 @@ __device__ __forceinline__ ReactorCfg cfg_of(const KParams &p)
 }
 
 template <int G, int MODE>
-__global__ void __launch_bounds__(256) chem_kernel(const KParams p)
+__global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) chem_kernel(const KParams p)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t bar;
@@ -146,8 +146,9 @@ __global__ void __launch_bounds__(256) chem_kernel(const KParams p)
   const ScratchLayout &L = p.L;
   const int gid = threadIdx.x / G;
   const int scr_doubles = jac_mode(MODE) ? L.total : L.total_rhs;
-  double *scr = reinterpret_cast<double *>(smem + m.blob_bytes) + (size_t)gid * scr_doubles;
-  const Group<G> grp;
+  double *shared = reinterpret_cast<double *>(smem + m.blob_bytes) + (size_t)gid * (scr_doubles + Group<G>::kShared);
+  double *scr = shared + Group<G>::kShared;
+  const Group<G> grp(shared, gid);
   const Progs pg{p.prog_w, p.prog_full, p.prog_j};
   const ReactorCfg cfg = cfg_of(p);
   for (int st = blockIdx.x * p.groups_per_cta + gid; st < p.n; st += gridDim.x * p.groups_per_cta)
@@ -209,10 +210,31 @@ size_t tps_scratch_bytes(const HostMech &hm, int mode, long long n)
   return per_warp * warps;
 }
 
+// Threads per state for n states when no lane width was set: narrow groups waste the fewest FP64 instructions on empty
+// lanes, wide ones put few states on all four schedulers of every SM, and the shared memory decides how many states an
+// SM holds at once. Measured on 152 SMs (microseconds, GRI-3.0, 53 species / 325 reactions; h2-burke, 11 / 27):
+//   GRI Jacobians   n = 1: 41 with 256 threads, 135 with 32; 608: 90 (128), 88 (64), 139 (32); 2432: 337 (128), 380
+//                   (64), 569 (32); 4864: 652 (64), 668 (128); 65,536: 8,108 (64), 12,266 (32), 9,129 (thread per state)
+//   GRI rates       n = 152: 28 (128), 55 (32); 608: 44 (64), 58 (32); 1216: 75 (64), 83 (32), 90 (16); 4864: 248 (16),
+//                   278 (64), 297 (32); 20,011: 1,049 (8), 1,094 (16); 65,536: 2,961 (8), 3,262 (16)
+//   h2 Jacobians    n = 1: 33 (64), 40 (16); 1216: 42 (16), 53 (64); 4096: 74 (8), 96 (16); 65,536: 677 (1), 1,063 (8)
+//   h2 rates        n = 1216: 25 (16), 30 (8); 4096: 41 (8), 63 (16); 20,000: 155 (1), 204 (8)
+// The lines lie at the SM count times the states of one SM; thread per state only where the caller's workspace has its
+// scratch (allowed), and for small mechanisms: GRI's 29 KB of scratch per state do not stay in L2.
+int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_allowed)
+{
+  const long long per_sm = (n + nsm - 1) / nsm;
+  if (m.nr >= 96 || m.ns >= 24) {
+    if (jac) return per_sm <= 2 ? 256 : (per_sm <= 24 ? 128 : 64);
+    return per_sm <= 1 ? 128 : (per_sm <= 10 ? 64 : (per_sm <= 80 ? 16 : 8));
+  }
+  if (per_sm <= 2 && jac) return 64;
+  if (per_sm <= 16) return 16;
+  return per_sm > 100 && tps_allowed ? 1 : 8;
+}
+
 // ------------------------------------------------------------------------------------------------ launchers
 namespace {
-
-int pick_group(const DevMech &m) { return m.nr >= 96 || m.ns >= 24 ? 32 : (m.nr >= 24 ? 16 : 8); }
 
 template <int MODE>
 int launch_tps(const HostMech &hm, KParams &p, cudaStream_t st, void *ws, size_t ws_bytes)
@@ -247,8 +269,14 @@ int launch_tps(const HostMech &hm, KParams &p, cudaStream_t st, void *ws, size_t
 template <int MODE>
 int launch_mode(const HostMech &hm, KParams &p, cudaStream_t st, int G_req, void *ws, size_t ws_bytes)
 {
-  if (G_req == 1) return launch_tps<MODE>(hm, p, st, ws, ws_bytes);
-  const int G = G_req > 0 ? G_req : pick_group(hm.dm);
+  int dev;
+  CUDA_THROW(cudaGetDevice(&dev));
+  int smem_max, nsm;
+  CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const bool room = ws && ws_bytes >= tps_scratch_bytes(hm, MODE, p.n);
+  const int G = G_req > 0 ? G_req : default_group(hm.dm, jac_mode(MODE), p.n, nsm, room);
+  if (G == 1) return launch_tps<MODE>(hm, p, st, ws, ws_bytes);
   const auto &progs = hm.programs_for(G);
   p.m = hm.dm;
   p.blob = hm.d_blob;
@@ -258,17 +286,14 @@ int launch_mode(const HostMech &hm, KParams &p, cudaStream_t st, int G_req, void
   p.prog_full = progs.progs[1];
   p.prog_j = (MODE == MODE_SENS) ? progs.progs[3] : progs.progs[2];
   const int scr_doubles = jac_mode(MODE) ? hm.sl.total : hm.sl.total_rhs;
-  int dev;
-  CUDA_THROW(cudaGetDevice(&dev));
-  int smem_max, nsm;
-  CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t per_group = (size_t)scr_doubles * 8;
+  const int shared = wide_group_doubles(G);
+  const size_t per_group = (size_t)(scr_doubles + shared) * 8;
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
   if ((size_t)smem_max <= (size_t)hm.dm.blob_bytes + per_group)
     throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the shared-memory kernels");
-  int groups = (int)std::min<size_t>(avail / per_group, 256 / G);
-  groups = std::max(groups, 1);
+  int groups = (int)std::min<size_t>(avail / per_group, (G > 32 ? 512 : 256) / G);
+  // no more groups per block than spread the states over all SMs
+  groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)p.n + nsm - 1) / nsm));
   p.groups_per_cta = groups;
   const size_t smem = hm.dm.blob_bytes + per_group * groups;
   const int threads = groups * G;
@@ -276,6 +301,9 @@ int launch_mode(const HostMech &hm, KParams &p, cudaStream_t st, int G_req, void
   switch (G) {
   case 8: kern = chem_kernel<8, MODE>; break;
   case 16: kern = chem_kernel<16, MODE>; break;
+  case 64: kern = chem_kernel<64, MODE>; break;
+  case 128: kern = chem_kernel<128, MODE>; break;
+  case 256: kern = chem_kernel<256, MODE>; break;
   default: kern = chem_kernel<32, MODE>; break;
   }
   ensure_dynamic_smem((const void *)kern, smem);
@@ -529,8 +557,12 @@ size_t sf_chem_workspace_size(const sf_mech *mech, int kind, int n)
   if (!mech || n <= 0 || kind < SF_CHEM_RATES || kind > SF_CHEM_JAC) return 0;
   static const int knob[4] = {SF_TUNE_GROUP_RATES, SF_TUNE_GROUP_SENS, SF_TUNE_GROUP_RHS, SF_TUNE_GROUP_JAC};
   static const int mode[4] = {MODE_RATES, MODE_SENS, MODE_RHS, MODE_JAC};
-  if (group_of(mech->m, knob[kind]) != 1) return 0;
   try {
+    int dev, nsm;
+    CUDA_THROW(cudaGetDevice(&dev));
+    CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const int g = group_of(mech->m, knob[kind]);
+    if ((g ? g : default_group(mech->m.dm, jac_mode(mode[kind]), n, nsm, true)) != 1) return 0;
     return tps_scratch_bytes(mech->m, mode[kind], n);
   } catch (sf_error &e) {
     t_err = e.what();

@@ -66,8 +66,7 @@ __device__ __forceinline__ double cp_of_state(const DevMech &m, const Blob &b, c
     cp += st[1 + i] * th.cp;
     ys += st[1 + i];
   }
-  ys = grp.sum(ys);
-  cp = grp.sum(cp);
+  grp.sum2(ys, cp, ns);
   const SpeciesThermo thn = species_thermo(m, b, ns - 1, T, logT, invT, false);
   return cp + (1. - ys) * thn.cp;
 }
@@ -106,8 +105,7 @@ __device__ __forceinline__ void heat_loss_cfg(const FlmParams &p, const Group<G>
   if (p.scaled_heat_loss) {
     double mx = -1.;
     for (int j = grp.lane; j < nzi; j += G) mx = fmax(mx, p.state[(size_t)(z0 + j) * p.m.ns]);
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(grp.mask, mx, o, G));
+    mx = grp.max(mx);
     const double Tr4 = Tr * Tr * Tr * Tr;
     hc = hc / (mx - Tc);
     hr = hr / (mx * mx * mx * mx - Tr4);
@@ -121,7 +119,7 @@ __device__ __forceinline__ void heat_loss_cfg(const FlmParams &p, const Group<G>
 }
 
 template <int G, bool JAC>
-__global__ void __launch_bounds__(256) flamelet_point_kernel(const FlmParams p)
+__global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) flamelet_point_kernel(const FlmParams p)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t bar;
@@ -131,8 +129,10 @@ __global__ void __launch_bounds__(256) flamelet_point_kernel(const FlmParams p)
   const ScratchLayout &L = p.L;
   const int gid = threadIdx.x / G;
   // per group: Griffon scratch + ns doubles for the (unused) right-hand side of the Jacobian evaluation
-  double *scr = reinterpret_cast<double *>(smem + m.blob_bytes) + (size_t)gid * ((JAC ? L.total : L.total_rhs) + m.ns + 2);
-  const Group<G> grp;
+  double *shared = reinterpret_cast<double *>(smem + m.blob_bytes) +
+                   (size_t)gid * ((JAC ? L.total : L.total_rhs) + m.ns + 2 + Group<G>::kShared);
+  double *scr = shared + Group<G>::kShared;
+  const Group<G> grp(shared, gid);
   const int lane = grp.lane;
   const int ns = m.ns;
   ReactorCfg cfg{};
@@ -159,14 +159,14 @@ __global__ void __launch_bounds__(256) flamelet_point_kernel(const FlmParams p)
       // enthalpy-flux and variable-cp terms of the temperature equation (flamelet_kernels.cpp:1141-1206)
       double cp = 0.;
       for (int i = lane; i < ns; i += G) cp += scr[L.y + i] * scr[L.cpv + i];
-      cp = grp.sum(cp);
+      cp = grp.sum(cp, ns);
       const double dTdZ = mcf * sm1[0] + ncf * sp1[0];
       double extra = 0.;
       if (p.eflux) {
         const double cpn = scr[L.cpv + ns - 1];
         double s = 0.;
         for (int j = lane; j < ns - 1; j += G) s += (scr[L.cpv + j] - cpn) * (mcf * sm1[1 + j] + ncf * sp1[1 + j]);
-        s = grp.sum(s);
+        s = grp.sum(s, ns);
         extra += 0.5 * chi / cp * dTdZ * s;
       }
       if (p.vcp) {
@@ -197,8 +197,7 @@ __global__ void __launch_bounds__(256) flamelet_point_kernel(const FlmParams p)
           cp += scr[L.y + i] * scr[L.cpv + i];
           cps += scr[L.y + i] * scr[L.dcp + i];
         }
-        cp = grp.sum(cp);
-        cps = grp.sum(cps);
+        grp.sum2(cp, cps, ns);
         const double cpm = cp_of_state<G>(m, b, grp, sm1);
         const double cpp = cp_of_state<G>(m, b, grp, sp1);
         const double dTdZ = mcf * sm1[0] + ncf * sp1[0];
@@ -913,7 +912,11 @@ __global__ void btddod_scale_diag_kernel(int nf, int ns, const int *offz, const 
 
 int launch_points(HostMech &hm, FlmParams &p, bool jac, cudaStream_t st)
 {
-  const int G = 32;
+  int dev, smem_max, nsm;
+  CUDA_THROW(cudaGetDevice(&dev));
+  CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int G = default_group(hm.dm, jac, p.n_points, nsm, false);
   const auto &progs = hm.programs_for(G);
   p.m = hm.dm;
   p.blob = hm.d_blob;
@@ -922,17 +925,22 @@ int launch_points(HostMech &hm, FlmParams &p, bool jac, cudaStream_t st)
   p.pg.w = progs.progs[0];
   p.pg.full = progs.progs[1];
   p.pg.j = progs.progs[2];
-  int dev, smem_max, nsm;
-  CUDA_THROW(cudaGetDevice(&dev));
-  CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const size_t per = (size_t)((jac ? hm.sl.total : hm.sl.total_rhs) + hm.dm.ns + 2) * 8;
+  const int shared = wide_group_doubles(G);
+  const size_t per = (size_t)((jac ? hm.sl.total : hm.sl.total_rhs) + hm.dm.ns + 2 + shared) * 8;
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
-  int groups = (int)std::min<size_t>(avail / per, 256 / G);
+  int groups = (int)std::min<size_t>(avail / per, (G > 32 ? 512 : 256) / G);
   if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the flamelet kernels");
+  groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)p.n_points + nsm - 1) / nsm));
   p.groups_per_cta = groups;
   const size_t smem = hm.dm.blob_bytes + per * groups;
-  void (*k)(const FlmParams) = jac ? flamelet_point_kernel<32, true> : flamelet_point_kernel<32, false>;
+  void (*k)(const FlmParams);
+  switch (G) {
+  case 8: k = jac ? flamelet_point_kernel<8, true> : flamelet_point_kernel<8, false>; break;
+  case 16: k = jac ? flamelet_point_kernel<16, true> : flamelet_point_kernel<16, false>; break;
+  case 64: k = jac ? flamelet_point_kernel<64, true> : flamelet_point_kernel<64, false>; break;
+  case 128: k = jac ? flamelet_point_kernel<128, true> : flamelet_point_kernel<128, false>; break;
+  default: k = jac ? flamelet_point_kernel<256, true> : flamelet_point_kernel<256, false>; break;
+  }
   ensure_dynamic_smem((const void *)k, smem);
   const int bps = std::max(1, (int)((size_t)smem_max / smem));
   const int grid = (int)std::max<long long>(1, std::min<long long>(((long long)p.n_points + groups - 1) / groups,

@@ -24,8 +24,9 @@ namespace sfgb {
 namespace {
 
 // Gather batch of the reactor evaluations inside the integrator: unbatched measured fastest there (the warp's scratch
-// is in shared memory or L2, and the integrator kernel has no registers to spare for operands in flight).
-constexpr int kIntegratorUnroll = 1;
+// is in shared memory or L2, and the integrator kernel has no registers to spare for operands in flight). A wide
+// group's lanes have only a few items each, whose latency counts.
+__host__ __device__ constexpr int int_unroll(int G) { return G > 32 ? 4 : 1; }
 
 struct IntParams {
   DevMech m;
@@ -89,12 +90,168 @@ struct IterMatrix {
   }
 };
 
+// The same, row-major with an odd leading dimension (wide groups: threads that each walk one row then touch
+// different banks).
+struct IterMatrixRows {
+  double *A;
+  int ld;
+  double pref;
+  __device__ __forceinline__ void operator()(int row, int col, double v) const
+  {
+    A[row * ld + col] = pref * v - (row == col ? 1. : 0.);
+  }
+};
+
+// Inverse of the n x n row-major matrix in S (leading dimension ld) by Gauss-Jordan elimination with partial pivoting
+// by one wide group; the scheme of the block-Thomas factorization's elimination (flamelet_kernels.cu), one group
+// barrier per column: warp 0 forms the next column, chooses the next pivot (largest magnitude, lowest row on ties) and
+// its multipliers while the other warps update the block from S to D. Returns the buffer Z with inverse(r, c) =
+// Z[piv[r]][pinv[c]]. ws: 2n + 2 doubles; used: n ints; n <= 128. A zero pivot column gives no inverse (the step then
+// ends in values that are not finite and is rejected).
+template <int G>
+__device__ __forceinline__ double *group_gj_inverse(const Group<G> &grp, double *S, double *D, int n, int ld, int *piv,
+                                                    int *pinv, double *ws, int *used)
+{
+  const int lane = grp.lane & 31, warp = grp.warp;
+  double *ipb = ws + 2 * n;
+  auto choose = [&](int j, const double (&v)[4]) {
+    unsigned long long best = 0ull;
+    int bp = n;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int i = lane + 32 * s;
+      if (i < n && !used[i]) {
+        const unsigned long long key = abs_key(v[s]);
+        if (bp == n || key > best) { best = key; bp = i; }
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bp, o);
+      if (oi < n && (bp >= n || ob > best || (ob == best && oi < bp))) { best = ob; bp = oi; }
+    }
+    double pv = 0.;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const double t = __shfl_sync(0xffffffffu, v[s], bp & 31);
+      if ((bp >> 5) == s) pv = t;
+    }
+    const double ip = 1. / pv;
+    double *f = ws + (j & 1) * n;  // the negated multipliers
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int i = lane + 32 * s;
+      if (i < n) f[i] = -(v[s] * ip);
+    }
+    if (lane == 0) {
+      ipb[j & 1] = ip;
+      piv[j] = bp;
+      pinv[bp] = j;
+      used[bp] = 1;
+    }
+    __syncwarp();
+  };
+  if (warp == 0) {
+    for (int i = lane; i < n; i += 32) used[i] = 0;
+    __syncwarp();
+    double v[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int i = lane + 32 * s;
+      v[s] = i < n ? S[i * ld] : 0.;
+    }
+    choose(0, v);
+  }
+  grp.sync();
+  constexpr int stride = G - 32;
+  const int ut = grp.lane - 32;
+  const int i0 = ut / n, j0 = ut - i0 * n, di = stride / n, dj = stride - di * n;
+  for (int k = 0; k < n; ++k) {
+    const int p = piv[k];
+    const double ip = ipb[k & 1];
+    const double *nf = ws + (k & 1) * n;  // -f_i
+    const double *Sp = S + (size_t)p * ld;
+    if (warp == 0) {
+      if (k + 1 < n) {
+        const int j = k + 1;
+        const double spj = Sp[j];
+        double v[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          const int i = lane + 32 * s;
+          double val = 0.;
+          if (i < n) {
+            val = S[i * ld + j] + nf[i] * spj;
+            if (i == p) val = spj * ip;
+            D[i * ld + j] = val;
+          }
+          v[s] = val;
+        }
+        choose(j, v);
+      }
+    } else {
+      const int kn = k + 1;
+      int i = i0, j = j0;
+      while (i < n) {
+        if (j != kn) {  // column k+1 is warp 0's
+          const double nfi = nf[i];
+          double val = S[i * ld + j] + nfi * Sp[j];
+          if (j == k) val = nfi;
+          if (i == p) val = j == k ? ip : Sp[j] * ip;
+          D[i * ld + j] = val;
+        }
+        i += di;
+        j += dj;
+        if (j >= n) {
+          j -= n;
+          ++i;
+        }
+      }
+    }
+    grp.sync();
+    double *t = S;
+    S = D;
+    D = t;
+  }
+  return S;
+}
+
+// x[pinv[i]] = sum_k Z[i][k] b[piv[k]] for the permuted inverse of group_gj_inverse: the row sums are cut into parts
+// over the group's warps (part: G doubles), b permuted into xb first. Ends with a barrier; x is then complete.
+template <int G>
+__device__ __forceinline__ void group_apply_inverse(const Group<G> &grp, const double *Z, int n, int ld, const int *piv,
+                                                    const int *pinv, const double *b, double *xb, double *part,
+                                                    double *x)
+{
+  const int rows = (n + 31) & ~31;
+  for (int i = grp.lane; i < n; i += G) xb[i] = b[piv[i]];
+  grp.sync();
+  const int parts = G / rows, p = grp.lane / rows, i = grp.lane - p * rows;
+  if (p < parts && i < n) {
+    const int a = n * p / parts, e = n * (p + 1) / parts;
+    const double *row = Z + (size_t)i * ld;
+    double s0 = 0.;
+    for (int k = a; k < e; ++k) s0 = fma(row[k], xb[k], s0);
+    part[p * rows + i] = s0;
+  }
+  grp.sync();
+  for (int r = grp.lane; r < n; r += G) {
+    double v = part[r];
+    for (int q = 1; q < parts; ++q) v += part[q * rows + r];
+    x[pinv[r]] = v;
+  }
+  grp.sync();
+}
+
 // Time-dependent reactor parameters at integration-local time t: every column of the time table is its 4-point
 // (cubic) Lagrange interpolant in time, held constant beyond the table's ends. At a spacing of the first time step
 // the interpolation error, fourth order in the spacing, is far below the rounding of the values, so the right-hand
 // side sees the parameter functions themselves. Sets the parameters of time_columns in cf; the feed mass fractions
 // go to ybuf (ns doubles of the warp's shared memory), which cf.yin then points to.
-__device__ __noinline__ void apply_time_params(const IntParams &p, ReactorCfg &cf, double t, double *ybuf, int ns)
+// lanes, lane: the group's width and this thread's place in it, for the feed mass fractions, which the group's next
+// barrier orders before their use.
+__device__ __noinline__ void apply_time_params(const IntParams &p, ReactorCfg &cf, double t, double *ybuf, int ns,
+                                               int lane, int lanes)
 {
   const sf_integrate_params &ip = p.ip;
   const double *tab = ip.time_table;
@@ -137,16 +294,10 @@ __device__ __noinline__ void apply_time_params(const IntParams &p, ReactorCfg &c
   if (m & SF_TIME_RAD_EPS) cf.eps = val(c++);
   if ((m & SF_TIME_FEED_Y) && ybuf) {
     __syncwarp();
-    for (int k = threadIdx.x & 31; k < ns; k += 32) ybuf[k] = val(c + k);
+    for (int k = lane; k < ns; k += lanes) ybuf[k] = val(c + k);
     __syncwarp();
     cf.yin = ybuf;
   }
-}
-
-__device__ __forceinline__ double warp_max(double v)
-{
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
 }
 
 // The right-hand side of a step's first stage and of every Newton iteration, as one function that both call sites
@@ -154,44 +305,54 @@ __device__ __forceinline__ double warp_max(double v)
 // phases of their steps (ncu: instruction-fetch stalls, "no instruction", were the largest stall reason); one
 // shared copy ran the 8192-reactor GRI ignition batch 4.8 % faster with the same results bit for bit. Making the
 // Jacobian evaluation and the LU separate functions as well was slower (register spills in the Jacobian).
-template <bool OPEN>
+// A wide group's reduction buffers start over here: its callers pass a barrier after their last reduction.
+template <bool OPEN, int G>
 __device__ __noinline__ void int_rhs(const IntParams &p, Blob b, double *scr, const double *q, double pres,
-                                     const ReactorCfg &cf, double *out)
+                                     const ReactorCfg &cf, double *out, double *group_shared, int group_in_block)
 {
-  const Group<32> grp;
+  const Group<G> grp(group_shared, group_in_block);
   NoJ noj;
-  reactor_eval<32, false, kIntegratorUnroll, OPEN>(p.m, b, p.L, scr, grp, q, pres, cf, p.pg, out, noj);
+  reactor_eval<G, false, int_unroll(G), OPEN>(p.m, b, p.L, scr, grp, q, pres, cf, p.pg, out, noj);
 }
 
+// One reactor per group of G threads. G = 32: one warp per reactor, LU factors, data in shared memory or in global
+// slots. G = 256: eight warps per reactor for batches that leave most schedulers without a warp otherwise; everything
+// in shared memory, the iteration matrix inverted once per setup so that each Newton solve is a matrix-vector product
+// over all warps instead of two serial triangular sweeps of one.
 // p is a __grid_constant__ parameter so that int_rhs reads it in place, without a per-thread copy.
-template <bool OPEN>
-__global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ IntParams p)
+template <bool OPEN, int G>
+__global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) integrate_kernel(const __grid_constant__ IntParams p)
 {
+  constexpr bool WIDE = G > 32;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t bar;
   const DevMech &m = p.m;
   if (!stage_to_smem(smem, p.blob, m.blob_bytes, &bar, p.status)) return;
   const Blob b = blob_at(m, smem);
   const ScratchLayout &L = p.L;
-  const Group<32> grp;
-  const int lane = grp.lane;
-  const int warp = threadIdx.x >> 5;
+  const int gid = threadIdx.x / G;
   const int neq = p.neq;
+  const int ld = neq | 1;  // WIDE: leading dimension of the iteration matrix and its inverse
   const sf_integrate_params &ip = p.ip;
-  double *base = reinterpret_cast<double *>(smem + m.blob_bytes) + (size_t)warp * p.per_warp;
-  const size_t slot = (size_t)blockIdx.x * p.warps + warp;  // this warp's global slots
+  double *base = reinterpret_cast<double *>(smem + m.blob_bytes) + (size_t)gid * p.per_warp;
+  double *group_shared = base;
+  base += Group<G>::kShared;
+  const Group<G> grp(group_shared, gid);
+  const int lane = grp.lane;
+  const size_t slot = (size_t)blockIdx.x * p.warps + gid;  // this group's global slots
   // iteration matrix: in shared memory, or with the FP32 factors in this warp's global slot (L2-resident)
-  double *A = p.gmat ? p.gmat + slot * p.mat_doubles : base;  // neq*neq
-  double *y = p.gmat ? base : A + neq * neq;              // current state
+  double *A = p.gmat ? p.gmat + slot * p.mat_doubles : base;
+  double *y = p.gmat ? base : A + (WIDE ? neq * ld : neq * neq);  // current state
   double *Y = y + neq;                                    // stage iterate
   double *res = Y + neq;                                  // Newton residual / step update
   double *f = res + neq;                                  // RHS at the iterate
   double *prior = f + neq;                                // sum_j a_sj k_j
   double *x = prior + neq;                                // linear-solve work vector
   double *k = x + neq;                                    // 6 stage derivatives
-  // Griffon scratch: in shared memory, or in this warp's slot of the global scratch array (L2-resident)
+  // Griffon scratch: in shared memory, or in this warp's slot of the global scratch array (L2-resident). WIDE: also the
+  // second buffer of the inversion
   double *scr = p.gscratch ? p.gscratch + slot * L.total : k + 6 * neq;
-  double *after = p.gscratch ? k + 6 * neq : scr + L.total;
+  double *after = p.gscratch ? k + 6 * neq : scr + (WIDE ? max(L.total, neq * ld) : L.total);
   const int lu32_doubles = (p.prec == 1 && !p.gmat) ? (neq * neq + 1) / 2 : 0;
   // FP32 factors (precision 1)
   float *LU32 = p.gmat ? reinterpret_cast<float *>(A + neq * neq) : reinterpret_cast<float *>(after);
@@ -200,25 +361,36 @@ __global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ 
   int *piv = reinterpret_cast<int *>(after + (p.prec == 1 ? lu32_doubles + neq : 0));
   double *dinv = after + (p.prec == 1 ? lu32_doubles + neq : 0) + (neq + 1) / 2 + 1;
   float *rf = xf + neq;
+  // WIDE: pivot order and its inverse, rows used, multipliers (3 neq ints, 2 neq + 2 doubles), parts (G doubles)
+  int *pinv = piv + neq, *used = pinv + neq;
+  double *ws = after + (3 * neq + 1) / 2 + 1;
+  double *part = ws + 2 * neq + 2;
   const int Tidx = p.cfg.configuration == 1 ? 1 : 0;
-  // feed mass fractions of a time table: the last ns doubles of the warp's shared region
-  double *ybuf = (p.ip.time_table && (p.ip.time_columns & SF_TIME_FEED_Y)) ? base + p.per_warp - m.ns : nullptr;
+  // feed mass fractions of a time table: the last ns doubles of the group's shared region
+  double *ybuf = (p.ip.time_table && (p.ip.time_columns & SF_TIME_FEED_Y)) ? group_shared + p.per_warp - m.ns : nullptr;
 
   for (;;) {
     unsigned int r = 0;
     if (lane == 0) r = atomicAdd(p.queue, 1u);
-    r = __shfl_sync(0xffffffffu, r, 0);
+    if constexpr (WIDE) {
+      if (lane == 0) grp.scalars[9] = (double)r;
+      grp.sync();
+      r = (unsigned)grp.scalars[9];
+    } else {
+      r = __shfl_sync(0xffffffffu, r, 0);
+    }
     if (r >= (unsigned)p.n) break;
     const double pres = p.cfg.configuration == 1 ? 0. : (p.pressures ? p.pressures[r] : p.pressure);
-    for (int i = lane; i < neq; i += 32) y[i] = p.q0[(size_t)r * neq + i];
-    __syncwarp();
+    for (int i = lane; i < neq; i += G) y[i] = p.q0[(size_t)r * neq + i];
+    grp.sync();
     const double T0 = y[Tidx];
     // reactor options with the feed temperature of the current evaluation; t_rhs: time of the most recent
     // right-hand side, whose feed the next Jacobian uses
     ReactorCfg cf = p.cfg;
     double t_rhs = ip.time_jac_t0;
     double t = 0., dt = ip.first_time_step;
-    double tau_interp = nan("");  // first crossing of T0 + delta, Hermite-interpolated
+    double tau_interp = nan("");  // first crossing of T0 + delta, Hermite-interpolated (WIDE: in the first warp)
+    bool crossed = false;
     bool setup = true;
     int count = 0, nsteps = 0, nnewton = 0, njac = 0, nfail = 0, status = 0, attempts = 0;
     const bool coerce = ip.stop_at_time > 0.;
@@ -229,18 +401,26 @@ __global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ 
       }
       if (coerce && t + dt > ip.stop_at_time) dt = ip.stop_at_time - t;
       if (setup) {
-        IterMatrix im{A, neq, dt * kGamma};
-        if (p.ip.time_table) apply_time_params(p, cf, t_rhs, ybuf, m.ns);
-        reactor_eval<32, true, kIntegratorUnroll, OPEN>(m, b, L, scr, grp, y, pres, cf, p.pg, f, im);
-        __syncwarp();
-        if (p.prec == 1) {
-          for (int e = lane; e < neq * neq; e += 32) LU32[e] = (float)A[e];
-          __syncwarp();
-          warp_lu_pd(LU32, neq, piv, reinterpret_cast<float *>(dinv));
+        if (p.ip.time_table) apply_time_params(p, cf, t_rhs, ybuf, m.ns, lane, G);
+        if constexpr (WIDE) {
+          IterMatrixRows im{A, ld, dt * kGamma};
+          reactor_eval<G, true, int_unroll(G), OPEN>(m, b, L, scr, grp, y, pres, cf, p.pg, f, im);
+          const double *Z = group_gj_inverse<G>(grp, A, scr, neq, ld, piv, pinv, ws, used);
+          if (Z != A)  // an odd number of columns ends in the scratch, which the next right-hand side overwrites
+            for (int e = lane; e < neq * ld; e += G) A[e] = Z[e];
         } else {
-          warp_lu_pd(A, neq, piv, dinv);
+          IterMatrix im{A, neq, dt * kGamma};
+          reactor_eval<G, true, int_unroll(G), OPEN>(m, b, L, scr, grp, y, pres, cf, p.pg, f, im);
+          __syncwarp();
+          if (p.prec == 1) {
+            for (int e = lane; e < neq * neq; e += 32) LU32[e] = (float)A[e];
+            __syncwarp();
+            warp_lu_pd(LU32, neq, piv, reinterpret_cast<float *>(dinv));
+          } else {
+            warp_lu_pd(A, neq, piv, dinv);
+          }
         }
-        __syncwarp();
+        grp.sync();
         ++njac;
       }
       ++count;
@@ -256,30 +436,32 @@ __global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ 
           slot[0] = t;
           slot[1] = dt;
         }
-        for (int i = lane; i < neq; i += 32) slot[2 + i] = y[i];
+        for (int i = lane; i < neq; i += G) slot[2 + i] = y[i];
       }
       // ---------------- one ESDIRK64 step (methods.py:502-612)
       t_rhs = t;
-      if (p.ip.time_table) apply_time_params(p, cf, t_rhs, ybuf, m.ns);
-      int_rhs<OPEN>(p, b, scr, y, pres, cf, k);
-      for (int i = lane; i < neq; i += 32) Y[i] = y[i];
-      __syncwarp();
+      if (p.ip.time_table) apply_time_params(p, cf, t_rhs, ybuf, m.ns, lane, G);
+      int_rhs<OPEN, G>(p, b, scr, y, pres, cf, k, group_shared, gid);
+      for (int i = lane; i < neq; i += G) Y[i] = y[i];
+      grp.sync();
       bool nl_ok = true;
       for (int s = 1; s < 6; ++s) {
         const double *kprev = k + (s - 1) * neq;
         t_rhs = t + c_c[s] * dt;
-        if (p.ip.time_table) apply_time_params(p, cf, t_rhs, ybuf, m.ns);
-        for (int i = lane; i < neq; i += 32) {
+        if (p.ip.time_table) apply_time_params(p, cf, t_rhs, ybuf, m.ns, lane, G);
+        for (int i = lane; i < neq; i += G) {
           double pr = 0.;
           for (int j = s - 1; j >= 0; --j) pr += c_a[s][j] * k[j * neq + i];  // a_s,s-1 k_s-1 + ... + a_s1 k_1
           prior[i] = pr;
           res[i] = dt * (kGamma * kprev[i] + pr) - (Y[i] - y[i]);
         }
-        __syncwarp();
+        grp.sync();
         bool conv = false;
         for (int it = 1; it <= ip.max_nonlinear_iter; ++it) {
           // dx = A^-1 res
-          if (p.prec == 1) {
+          if constexpr (WIDE) {
+            group_apply_inverse<G>(grp, A, neq, ld, piv, pinv, res, f, part, x);
+          } else if (p.prec == 1) {
             // FP32 triangular solves of the FP32 factors, FP64 residual refinement r = res - A x
             for (int i = lane; i < neq; i += 32) xf[i] = (float)res[piv[i]];
             warp_lu_solve_pd(LU32, neq, reinterpret_cast<const float *>(dinv), xf);
@@ -300,32 +482,31 @@ __global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ 
             for (int i = lane; i < neq; i += 32) x[i] = res[piv[i]];
             warp_lu_solve_pd(A, neq, dinv, x);
           }
-          for (int i = lane; i < neq; i += 32) Y[i] -= x[i];
-          __syncwarp();
-          int_rhs<OPEN>(p, b, scr, Y, pres, cf, f);
+          for (int i = lane; i < neq; i += G) Y[i] -= x[i];
+          grp.sync();
+          int_rhs<OPEN, G>(p, b, scr, Y, pres, cf, f, group_shared, gid);
           double nrm = 0.;
-          for (int i = lane; i < neq; i += 32) {
+          for (int i = lane; i < neq; i += G) {
             res[i] = dt * (kGamma * f[i] + prior[i]) - (Y[i] - y[i]);
             nrm = fmax(nrm, fabs(res[i]) * (i == Tidx ? 1.e-3 : 1.));
           }
-          nrm = warp_max(nrm);
+          nrm = grp.max(nrm, neq);
           ++nnewton;
-          __syncwarp();
+          grp.sync();
           if (nrm < ip.nonlinear_tolerance) {
             conv = true;
             break;
           }
         }
-        for (int i = lane; i < neq; i += 32) k[s * neq + i] = f[i];
+        for (int i = lane; i < neq; i += G) k[s * neq + i] = f[i];
         if (slot)
-          for (int i = lane; i < neq; i += 32) slot[2 + (size_t)s * neq + i] = Y[i];
-        __syncwarp();
+          for (int i = lane; i < neq; i += G) slot[2 + (size_t)s * neq + i] = Y[i];
+        grp.sync();
         if (!conv) nl_ok = false;
       }
       // ---------------- update, error estimate, residual
-      double err = 0., rsd = 0.;
-      bool finite = true;
-      for (int i = lane; i < neq; i += 32) {
+      double err = 0., rsd = 0., bad = 0.;
+      for (int i = lane; i < neq; i += G) {
         double ds = 0., dh = 0.;
         for (int j = 0; j < 6; ++j) {
           ds += c_b[j] * k[j * neq + i];
@@ -337,30 +518,39 @@ __global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ 
         const double wi = (i == Tidx) ? 1.e-3 : 1.;
         err = fmax(err, fabs((ds - dh) * wi));
         rsd = fmax(rsd, fabs(ds * wi));
-        finite = finite && isfinite(ds);
+        if (!isfinite(ds)) bad = 1.;
       }
-      err = warp_max(err);
-      rsd = warp_max(rsd) / dt;
-      finite = __all_sync(0xffffffffu, finite);
+      err = grp.max(err, neq);
+      rsd = grp.max(rsd, neq) / dt;
+      const bool finite = grp.max(bad, neq) == 0.;
       const double T_start = y[Tidx];
-      __syncwarp();
+      grp.sync();
       const double recent = dt;
       if (finite) {
-        for (int i = lane; i < neq; i += 32) {
+        for (int i = lane; i < neq; i += G) {
           const double v = y[i] + res[i];
           y[i] = v < 0. ? 0. : v;  // post_step_callback (reactors.py:506-508)
         }
-        __syncwarp();
-        if (ip.delta_temperature_ignition > 0. && isnan(tau_interp) &&
-            y[Tidx] > T0 + ip.delta_temperature_ignition)  // this step crossed: dT/dt at its ends are k_1 and k_6
-          tau_interp = hermite_crossing(t, dt, T_start, y[Tidx], k[Tidx], k[5 * neq + Tidx],
-                                        T0 + ip.delta_temperature_ignition);
+        grp.sync();
+        if (ip.delta_temperature_ignition > 0. && !crossed && y[Tidx] > T0 + ip.delta_temperature_ignition) {
+          crossed = true;  // this step crossed: dT/dt at its ends are k_1 and k_6
+          if (!WIDE || lane < 32)
+            tau_interp = hermite_crossing(t, dt, T_start, y[Tidx], k[Tidx], k[5 * neq + Tidx],
+                                          T0 + ip.delta_temperature_ignition);
+        }
         t += dt;
         ++nsteps;
-        if (err < 1.e-16)
-          dt = fmin(dt * 1.1, ip.max_time_step);
-        else
-          dt = fmin(dt * fmin(1.1, pow(ip.transient_tolerance / err, 0.1333333333)), ip.max_time_step);
+        if (!WIDE || lane < 32) {
+          if (err < 1.e-16)
+            dt = fmin(dt * 1.1, ip.max_time_step);
+          else
+            dt = fmin(dt * fmin(1.1, pow(ip.transient_tolerance / err, 0.1333333333)), ip.max_time_step);
+        }
+        if constexpr (WIDE) {  // the power is formed by one warp for the group
+          if (lane == 0) grp.scalars[10] = dt;
+          grp.sync();
+          dt = grp.scalars[10];
+        }
         if (count == ip.maximum_steps_per_jacobian) {
           count = 0;
           setup = true;
@@ -405,7 +595,7 @@ __global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ 
       }
       if (!cont) break;
     }
-    for (int i = lane; i < neq; i += 32) p.out_q[(size_t)r * neq + i] = y[i];
+    for (int i = lane; i < neq; i += G) p.out_q[(size_t)r * neq + i] = y[i];
     if (lane == 0) {
       p.out_t[r] = t;
       p.out_counts[4 * (size_t)r + 0] = nsteps;
@@ -415,7 +605,7 @@ __global__ void __launch_bounds__(256) integrate_kernel(const __grid_constant__ 
       p.out_status[r] = status;
       if (ip.ignition_time_interp) ip.ignition_time_interp[r] = tau_interp;
     }
-    __syncwarp();
+    grp.sync();
   }
 }
 
@@ -447,8 +637,18 @@ size_t matrix_doubles(int neq, int prec)
   return n2 + (prec == 1 ? (n2 + 1) / 2 : 0);
 }
 
+// Wide groups (256 threads per reactor): shared memory per group.
+constexpr int kWideG = 256;
+size_t wide_doubles(const HostMech &hm, int G, int neq, bool feed_y_table)
+{
+  const size_t ld = neq | 1;
+  return wide_group_doubles(G) + neq * ld + 12 * (size_t)neq + std::max<size_t>(hm.sl.total, neq * ld) +
+         (3 * (size_t)neq + 1) / 2 + 1 + 2 * (size_t)neq + 2 + G + (feed_y_table ? (size_t)hm.dm.ns : 0);
+}
+
 struct IntShape {
-  int warps, grid;
+  int group;         // threads per reactor
+  int warps, grid;   // warps: reactors (groups) per block
   size_t per_warp, smem, scratch_bytes, mat_bytes;
 };
 
@@ -460,6 +660,24 @@ IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   IntShape s{};
+  // A mechanism of more than 64 reactions runs eight warps per reactor up to 12 reactors per SM, unless a launch shape
+  // was set (the autotuner's) or the factors are FP32. (GRI-3.0 to 20 us: one reactor 4.0 ms against 13.0 with one
+  // warp, 300 16.7 against 66.1, 1000 38.1 against 66.9, 2000 64.0 against 89.0; ignitions to 0.1 s: 2048 reactors
+  // 0.88 s against 0.90, 8192 3.29 against 2.73. h2-burke's 27 reactions fit one warp: 1000 reactors 171 ms with one,
+  // 243 with eight.)
+  if (prec == 0 && hm.dm.nr > 64 && n <= 12 * nsm && hm.tune[SF_TUNE_INTEGRATE_SCRATCH] == 0 && hm.tune[SF_TUNE_INTEGRATE_WARPS] == 0) {
+    constexpr int wg = kWideG;
+    s.per_warp = wide_doubles(hm, wg, neq, feed_y_table);
+    const int fit = (int)std::min<size_t>(512 / wg, ((size_t)smem_max - hm.dm.blob_bytes - 64) / (s.per_warp * 8));
+    if (fit >= 1) {
+      s.group = wg;
+      s.warps = (int)std::min<long long>(fit, ((long long)n + nsm - 1) / nsm);
+      s.smem = hm.dm.blob_bytes + (size_t)s.warps * s.per_warp * 8;
+      s.grid = (int)std::max<long long>(1, std::min<long long>(nsm, ((long long)n + s.warps - 1) / s.warps));
+      return s;
+    }
+  }
+  s.group = 32;
   const int place = integrate_placement(hm);
   const bool gs = place >= 1, gm = place == 2;
   s.per_warp = per_warp_doubles(hm, neq, prec, gs, gm, feed_y_table);
@@ -539,15 +757,11 @@ static int integrate_impl(const sf_mech *mech, const sf_reactor_params *rp, cons
     if (mech->m.dm.ns + 1 > 128) throw sf_error(SF_ERR_UNSUPPORTED, "the integrator supports up to 127 species");
     if (n == 0) return SF_OK;
     HostMech &hm = const_cast<HostMech &>(mech->m);
-    const auto &progs = hm.programs_for(32);
     IntParams p{};
     p.m = hm.dm;
     p.blob = hm.d_blob;
     p.status = hm.d_status;
     p.L = hm.sl;
-    p.pg.w = progs.progs[0];
-    p.pg.full = progs.progs[1];
-    p.pg.j = progs.progs[2];
     p.cfg.configuration = rp->configuration;
     p.cfg.heat = rp->heat_transfer;
     p.cfg.option = ip->rates_option;
@@ -580,17 +794,22 @@ static int integrate_impl(const sf_mech *mech, const sf_reactor_params *rp, cons
                                         ip->time_table && (ip->time_columns & SF_TIME_FEED_Y));
     if (workspace_bytes < 256 + sh.scratch_bytes + sh.mat_bytes)
       throw sf_error(SF_ERR_WORKSPACE, "workspace smaller than sf_integrate_workspace_size reports");
+    const auto &progs = hm.programs_for(sh.group);
+    p.pg.w = progs.progs[0];
+    p.pg.full = progs.progs[1];
+    p.pg.j = progs.progs[2];
     p.per_warp = sh.per_warp;
     p.warps = sh.warps;
     p.gscratch = sh.scratch_bytes ? reinterpret_cast<double *>(static_cast<char *>(workspace) + 256) : nullptr;
     p.gmat = sh.mat_bytes ? reinterpret_cast<double *>(static_cast<char *>(workspace) + 256 + sh.scratch_bytes)
                           : nullptr;
     p.mat_doubles = matrix_doubles(p.neq, p.prec);
-    auto kern = p.cfg.open ? integrate_kernel<true> : integrate_kernel<false>;
+    auto kern = sh.group == 32 ? (p.cfg.open ? integrate_kernel<true, 32> : integrate_kernel<false, 32>)
+                               : (p.cfg.open ? integrate_kernel<true, kWideG> : integrate_kernel<false, kWideG>);
     ensure_dynamic_smem((const void *)kern, sh.smem);
     cudaStream_t st = (cudaStream_t)stream;
     CUDA_THROW(cudaMemsetAsync(workspace, 0, 256, st));
-    kern<<<sh.grid, 32 * sh.warps, sh.smem, st>>>(p);
+    kern<<<sh.grid, sh.group * sh.warps, sh.smem, st>>>(p);
     CUDA_THROW(cudaGetLastError());
     return SF_OK;
   } catch (sf_error &e) {

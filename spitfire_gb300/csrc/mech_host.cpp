@@ -341,7 +341,7 @@ void HostMech::build(const sf_mech_desc *d)
   CUDA_THROW(cudaMemset(d_status, 0, 16));
   CUDA_THROW(cudaGetDevice(&device));
   // every gather program the kernels use, built here so that no evaluation call builds or allocates one
-  for (int G : {1, 8, 16, 32}) build_programs(G);
+  for (int G : {1, 8, 16, 32, 64, 128, 256}) build_programs(G);
 }
 
 const HostMech::Programs &HostMech::programs_for(int G) const

@@ -39,65 +39,108 @@ __device__ __forceinline__ SpeciesSums prep_species(const DevMech &m, const Blob
                                                     S scr, const Group<G> &grp, const StateCtx &s,
                                                     bool isochoric, bool want_eh)
 {
-  const int ns = m.ns, lane = grp.lane;
+  const int ns = m.ns;
   double cpmix = 0., cpsens = 0.;
-  for (int i = lane; i < ns; i += G) {
+  // A wide group's first half takes the Gibbs factors and its second half the heat capacities and enthalpies: the
+  // two parts need about the same number of FP64 instructions and one warp can issue only one every 64 cycles.
+  constexpr int H = G > 32 ? G / 2 : G;
+  const bool gibbs = G <= 32 || grp.lane < H, caloric = G <= 32 || grp.lane >= H;
+  for (int i = grp.lane & (H - 1); i < ns; i += H) {
     const double yi = scr[L.y + i];
     const double invmw = b.d[m.d_invmw + i];
-    scr[L.C + i] = yi * s.rho * invmw;
     const SpeciesThermo th = species_thermo(m, b, i, s.T, s.logT, s.invT, JAC);
-    store_gibbs_factor(scr, L, i, th.g * (s.invT * m.invRu), b.d + m.d_exptab);
-    if (want_eh) {
-      scr[L.eh + i] = isochoric ? th.h - m.Ru * s.T * invmw : th.h;
-      scr[L.cpv + i] = isochoric ? th.cp - m.Ru * invmw : th.cp;
-      cpmix += yi * th.cp;
-    } else {
-      scr[L.eh + i] = 0.;
+    if (gibbs) {
+      scr[L.C + i] = yi * s.rho * invmw;
+      store_gibbs_factor(scr, L, i, th.g * (s.invT * m.invRu), b.d + m.d_exptab);
+      // gather destinations start at zero: an entry with no contributions (an inert species) is never written
+      scr[L.w + i] = 0.;
+      if (JAC) {
+        scr[L.Srho + i] = 0.;
+        scr[L.ST + i] = 0.;
+        scr[L.P + i] = 0.;
+        scr[L.Q + i] = 0.;
+      }
     }
-    // gather destinations start at zero: an entry with no contributions (an inert species) is never written
-    scr[L.w + i] = 0.;
-    if (JAC) {
-      scr[L.dB + i] = th.TdB;
-      scr[L.dcp + i] = th.dcp;
-      cpsens += yi * th.dcp;
-      scr[L.Srho + i] = 0.;
-      scr[L.ST + i] = 0.;
-      scr[L.P + i] = 0.;
-      scr[L.Q + i] = 0.;
+    if (caloric) {
+      if (want_eh) {
+        scr[L.eh + i] = isochoric ? th.h - m.Ru * s.T * invmw : th.h;
+        scr[L.cpv + i] = isochoric ? th.cp - m.Ru * invmw : th.cp;
+        cpmix += yi * th.cp;
+      } else {
+        scr[L.eh + i] = 0.;
+      }
+      if (JAC) {
+        scr[L.dB + i] = th.TdB;
+        scr[L.dcp + i] = th.dcp;
+        cpsens += yi * th.dcp;
+      }
     }
   }
   SpeciesSums r{cpmix, cpsens};
+  const int first = G <= 32 ? 0 : H, count = min(ns, H);
   if (JAC) {
-    grp.sum2(r.cpmix, r.cpsens);
+    grp.sum2(r.cpmix, r.cpsens, count, first);
   } else {
-    r.cpmix = grp.sum(r.cpmix);
+    r.cpmix = grp.sum(r.cpmix, count, first);
   }
-  grp.sync();
+  if (G <= 32) grp.sync();  // a wide group's reduction has a barrier after the stores above
   return r;
 }
 
-// Scalars of a state: three reciprocals in one division sequence, everything else products.
+// Scalars of a state: three reciprocals in one division sequence, everything else products. In a wide group the first
+// warp forms them and the second one the logarithm, for all.
 template <int G>
 __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &grp, double T, double rho, double sim,
                                               double pres, bool isochoric, int option)
 {
   StateCtx s;
   s.T = T;
-  s.logT = log(T);
-  double ix;  // 1 / rho isochoric, 1 / p isobaric
-  grp.recip3(T, sim, isochoric ? rho : pres, s.invT, s.mmw, ix);
   s.invM = sim;
-  if (isochoric) {
-    s.rho = rho;
-    s.invRho = ix;
-  } else {
-    s.rho = pres * s.mmw * (s.invT * m.invRu);
-    s.invRho = T * m.Ru * (sim * ix);
-  }
-  s.ct = s.rho * sim;
-  s.port = m.pref * s.invT * m.invRu;
-  s.invport = T * (m.Ru * m.ipref);
   s.option = option;
+  auto scalars = [&](const auto &g) {
+    double ix;  // 1 / rho isochoric, 1 / p isobaric
+    g.recip3(T, sim, isochoric ? rho : pres, s.invT, s.mmw, ix);
+    if (isochoric) {
+      s.rho = rho;
+      s.invRho = ix;
+    } else {
+      s.rho = pres * s.mmw * (s.invT * m.invRu);
+      s.invRho = T * m.Ru * (sim * ix);
+    }
+    s.ct = s.rho * sim;
+    s.port = m.pref * s.invT * m.invRu;
+    s.invport = T * (m.Ru * m.ipref);
+  };
+  if constexpr (G <= 32) {
+    s.logT = log(T);
+    scalars(grp);
+  } else {
+    double *sh = grp.scalars;
+    if (grp.warp == 0) {
+      scalars(Group<32>());
+      if (grp.lane == 0) {
+        sh[0] = s.invT;
+        sh[1] = s.mmw;
+        sh[2] = s.rho;
+        sh[3] = s.invRho;
+        sh[4] = s.ct;
+        sh[5] = s.port;
+        sh[6] = s.invport;
+      }
+    } else if (grp.warp == 1) {
+      s.logT = log(T);
+      if (grp.lane == 32) sh[7] = s.logT;
+    }
+    grp.sync();
+    s.invT = sh[0];
+    s.mmw = sh[1];
+    s.rho = sh[2];
+    s.invRho = sh[3];
+    s.ct = sh[4];
+    s.port = sh[5];
+    s.invport = sh[6];
+    s.logT = sh[7];
+  }
   return s;
 }
 
@@ -108,9 +151,18 @@ __device__ __forceinline__ double2 reactions_and_gathers(const DevMech &m, const
                                                          const Progs &pg)
 {
   double EA = 0., EB = 0.;
-  for (int r = grp.lane; r < m.nr; r += G) eval_reaction<JAC>(m, b, L, scr, s, r, &EA, &EB);
+  if constexpr (G <= 32) {
+    for (int r = grp.lane; r < m.nr; r += G) eval_reaction<JAC>(m, b, L, scr, s, r, &EA, &EB);
+  } else {
+    // the last reactions in device order, the falloff ones, cost several times the others: the first warps take
+    // those in the first pass, and the last warps start the second
+    for (int p = 0; p * G < m.nr; ++p) {
+      const int r = m.nr - 1 - p * G - ((p & 1) ? G - 1 - grp.lane : grp.lane);
+      if (r >= 0) eval_reaction<JAC>(m, b, L, scr, s, r, &EA, &EB);
+    }
+  }
   if (JAC) grp.sum2(EA, EB);
-  grp.sync();
+  if (G <= 32 || !JAC) grp.sync();  // a wide group's reduction has a barrier of its own
   NoJ noj;
   run_program<G, U>(JAC ? pg.full : pg.w, grp, scr, L.Q, noj);
   grp.sync();
@@ -147,19 +199,28 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
     sy += yi;
     sim = fma(yi, b.d[m.d_u + i], sim);
   }
-  grp.sum2(sy, sim);
+  grp.sum2(sy, sim, ns - 1);
   if (lane == 0) scr[L.y + ns - 1] = 1. - sy;
-  grp.sync();
+  if (G <= 32) grp.sync();  // else the barrier in state_ctx
   sim += b.d[m.d_invmw + ns - 1];
   const StateCtx s = state_ctx<G>(m, grp, T, rho, sim, pres, isochoric, c.option);
   rho = s.rho;
   const double mmw = s.mmw;
   // ---------------- P1-P3
   const SpeciesSums sums = prep_species<G, JAC>(m, b, L, scr, grp, s, isochoric, true);
+  const double cmix = isochoric ? sums.cpmix - m.Ru * sim : sums.cpmix;  // cv or cp
+  const double invRho = s.invRho;
+  double iC;
+  if constexpr (G <= 32) {
+    iC = 1. / cmix;
+  } else if (grp.warp == Group<G>::W / 2) {  // read after the reactions' barrier
+    iC = 1. / cmix;
+    if ((lane & 31) == 0) grp.scalars[8] = iC;
+  }
   const double2 E = reactions_and_gathers<G, JAC, U>(m, b, L, scr, grp, s, pg);
   const double EA = E.x, EB = E.y;
-  const double cmix = isochoric ? sums.cpmix - m.Ru * sim : sums.cpmix;  // cv or cp
-  const double invRho = s.invRho, iC = 1. / cmix, iRC = iC * invRho;
+  if constexpr (G > 32) iC = grp.scalars[8];
+  const double iRC = iC * invRho;
   const double cpsens = sums.cpsens;
   // feed of an open reactor (isochoric_reactor_kernels.cpp:39-154, isobaric_reactor_kernels.cpp:31-168):
   // fe = sum_i (e_i(Tin) - e_i(T)) yin_i (enthalpies when isobaric), fc = sum_i yin_i cv_i(T) (cp_i)
@@ -173,7 +234,7 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
       fe += (ein - scr[L.eh + i]) * yi;
       fc += yi * scr[L.cpv + i];
     }
-    grp.sum2(fe, fc);
+    grp.sum2(fe, fc, ns);
   }
   // mass-exchange factor of the species and energy equations: rho_in / (tau rho) isochoric, 1 / tau isobaric
   const double itau = open_ ? 1. / c.tau : 0.;
@@ -192,9 +253,9 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
     }
   }
   if (JAC)
-    grp.sum4(swe, sre, ste, swc);
+    grp.sum4(swe, sre, ste, swc, ns);
   else
-    swe = grp.sum(swe);
+    swe = grp.sum(swe, ns);
   const double rhsT = -swe * iRC;
   double qheat = 0.;
   if (c.heat == 2)

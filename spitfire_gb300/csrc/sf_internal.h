@@ -59,7 +59,7 @@ struct HostMech {
   std::map<int, Programs> programs;
 
   void build(const sf_mech_desc *d);
-  const Programs &programs_for(int G) const;  // the gather programs of lane width G (1, 8, 16 or 32), built by build()
+  const Programs &programs_for(int G) const;  // the gather programs of group width G (1, 8, 16, 32, 128 or 256), built by build()
   ~HostMech();
 
  private:
@@ -76,6 +76,8 @@ void ensure_dynamic_smem(const void *kernel, size_t bytes);
 // Thread-per-state chemistry kernels: warps that can be resident at once, and the bytes of interleaved scratch a
 // launch of n states takes (at most one slot per resident warp).
 size_t tps_resident_warps(const HostMech &hm);
+// Threads per state (8 to 256, or 1) of the chemistry kernels for n states when none was set.
+int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_allowed);
 // sf_reactor_jac_batch with an explicit lane width G (8, 16 or 32; no workspace). Throws sf_error.
 void reactor_jac_lanes(const sf_mech *mech, const sf_reactor_params *rp, int rates_option, int n, const double *q,
                        const double *pressures, double *out_rhs, double *out_jac, int G, cudaStream_t st);
