@@ -11,6 +11,7 @@
 #include "reactor_eval.cuh"
 #include "sf_internal.h"
 #include "eig_device.cuh"
+#include "gj_device.cuh"
 
 namespace sfgb {
 namespace {
@@ -289,155 +290,34 @@ __global__ void flamelet_expeig_kernel(int n_points, int nf, int ns, const int *
 // elimination with one CTA barrier per column, and the inverse is what the solve applies.
 // Storage: values block i holds the inverse of the eliminated block i; l_values block i holds L_i for
 // 1 <= i <= m and U_i for m < i < nzi (block 0 unused).
-constexpr int kFactorThreads = 512;  // 16 warps: warp 0 runs the pivot look-ahead, 12 update the block
-static_assert(kFactorThreads >= 64 && kFactorThreads % 32 == 0, "the elimination needs updating warps");
+constexpr int kFactorThreads = 384;  // 12 warps: warp 0 runs the pivot look-ahead, the others update the block
 
-// Inverse of the n x n row-major matrix in S by Gauss-Jordan elimination with partial pivoting (G. H. Golub and
-// C. F. Van Loan, "Matrix Computations", section 3.2; rows are not moved, the pivot order is recorded). Phase k
-// maps the source buffer to the destination (S and D alternate): with pivot row p, ip = 1/S[p][k] and
-// f_i = S[i][k] ip,
-//   D[p][j] = S[p][j] ip,   D[i][j] = S[i][j] - f_i S[p][j]   (j != k),   D[p][k] = ip,   D[i][k] = -f_i.
-// The other warps update the block while warp 0 forms column k+1 of D and, before the phase's barrier, chooses the
-// next pivot among the unused rows (largest magnitude, lowest row on ties, as idamax) and its multipliers: one
-// barrier per column. Returns the buffer Z holding the inverse permuted: inverse(r, c) = Z[piv[r]][pinv[c]], where
-// pinv[piv[k]] = k. ws: 2n + 2 doubles (the negated multipliers and pivot reciprocals of two phases); used: n ints.
-// A pivot column of zeros gives ip = 0 (a singular block; the output is then not an inverse). n <= 128.
-__device__ double *cta_gj_inverse(double *S, double *D, int n, int *piv, int *pinv, double *ws, int *used)
-{
-  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
-  double *ipb = ws + 2 * n;
-  // The updating warps leave warp 0's scheduler partition (warps 4, 8, ... share it; warps are dealt to the four
-  // partitions by warp index) to warp 0 alone, so that its serial look-ahead does not queue for the FP64 unit
-  // behind their updates. Elements are dealt to the updating threads in row-major order with incremental indices.
-  const int nw = nt >> 5;
-  const int uw = (warp & 3) ? warp - (warp >> 2) - 1 : -1;
-  const int ustride = 32 * (nw - (nw + 3) / 4);
-  const int ut = uw * 32 + lane;
-  const int i0 = ut / n, j0 = ut - (ut / n) * n, di = ustride / n, dj = ustride - (ustride / n) * n;
-  // warp 0: choose the pivot of column j among the unused rows from the lane-held column values v (row lane+32s),
-  // publish it with its multipliers for phase j
-  auto choose = [&](int j, const double (&v)[4]) {
-    unsigned long long best = 0ull;
-    int bp = n;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = lane + 32 * s;
-      if (i < n && !used[i]) {
-        const unsigned long long key = (unsigned long long)__double_as_longlong(v[s]) & 0x7fffffffffffffffull;
-        if (bp == n || key > best) { best = key; bp = i; }
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bp, o);
-      if (oi < n && (bp >= n || ob > best || (ob == best && oi < bp))) { best = ob; bp = oi; }
-    }
-    double pv = 0.;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const double t = __shfl_sync(0xffffffffu, v[s], bp & 31);
-      if ((bp >> 5) == s) pv = t;
-    }
-    const double ip = pv != 0. ? 1. / pv : 0.;
-    const double nip = -ip;
-    double *f = ws + (j & 1) * n;  // the negated multipliers -f_i
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = lane + 32 * s;
-      if (i < n) f[i] = v[s] * nip;
-    }
-    if (lane == 0) {
-      ipb[j & 1] = ip;
-      piv[j] = bp;
-      pinv[bp] = j;
-      used[bp] = 1;
-    }
-    __syncwarp();
-  };
-  if (warp == 0) {
-    for (int i = lane; i < n; i += 32) used[i] = 0;
-    __syncwarp();
-    double v[4];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = lane + 32 * s;
-      v[s] = i < n ? S[i * n] : 0.;
-    }
-    choose(0, v);
-  }
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    const int p = piv[k];
-    const double ip = ipb[k & 1];
-    const double *nf = ws + (k & 1) * n;  // -f_i
-    const double *Sp = S + (size_t)p * n;
-    if (warp == 0) {
-      if (k + 1 < n) {
-        const int j = k + 1;
-        const double spj = Sp[j];
-        double v[4];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          const int i = lane + 32 * s;
-          double val = 0.;
-          if (i < n) {
-            val = S[i * n + j] + nf[i] * spj;
-            if (i == p) val = spj * ip;
-            D[i * n + j] = val;
-          }
-          v[s] = val;
-        }
-        choose(j, v);
-      }
-    } else if (uw >= 0) {
-      const int kn = k + 1;
-      int i = i0, j = j0;
-      for (int e = ut; e < n * n; e += ustride) {
-        if (j != kn) {  // column k+1 is warp 0's
-          // one FMA per element and warp; the column-k value is a select, the pivot row (in at most two of a warp's
-          // iterations) a multiplication
-          const double nfi = nf[i];
-          double val = S[e] + nfi * Sp[j];
-          if (j == k) val = nfi;
-          if (i == p) val = j == k ? ip : Sp[j] * ip;
-          D[e] = val;
-        }
-        i += di;
-        j += dj;
-        if (j >= n) {
-          j -= n;
-          ++i;
-        }
-      }
-    }
-    __syncthreads();
-    double *t = S;
-    S = D;
-    D = t;
-  }
-  return S;
-}
-
-// Shared-memory bytes of the factorization kernels: two row-major blocks, the elimination's multipliers and pivot
-// reciprocals, three index arrays.
+// Shared-memory bytes of the factorization kernels: two row-major blocks with an odd leading dimension, the
+// elimination's multipliers, two index arrays.
 inline size_t factor_smem_bytes(int ns)
 {
-  return (size_t)2 * ns * ns * 8 + (size_t)(2 * ns + 2) * 8 + (size_t)3 * ns * 4 + 16;
+  return (size_t)2 * ns * (ns | 1) * 8 + (size_t)2 * ns * 8 + (size_t)2 * ns * 4 + 16;
 }
 
 struct FactorShared {
   double *buf0, *buf1, *ws;
-  int *piv, *pinv, *used;
-  __device__ FactorShared(unsigned char *smem, int ns)
+  int *piv, *pinv;
+  int ld;
+  __device__ FactorShared(unsigned char *smem, int ns) : ld(ns | 1)
   {
     buf0 = reinterpret_cast<double *>(smem);
-    buf1 = buf0 + (size_t)ns * ns;
-    ws = buf1 + (size_t)ns * ns;
-    piv = reinterpret_cast<int *>(ws + 2 * ns + 2);
+    buf1 = buf0 + (size_t)ns * ld;
+    ws = buf1 + (size_t)ns * ld;
+    piv = reinterpret_cast<int *>(ws + 2 * ns);
     pinv = piv + ns;
-    used = pinv + ns;
+  }
+  __device__ __forceinline__ double *invert(double *S, double *D, int ns)
+  {
+    return gj_inverse<true>(S, D, ns, ld, piv, pinv, ws, threadIdx.x, kFactorThreads, [] { __syncthreads(); });
   }
 };
+
+constexpr int kAhead = 8;  // elements of the next block each thread holds: all of a block of up to 55 x 55
 
 // One CTA per (flamelet, half): even CTAs eliminate blocks 0..m-1 downward, odd CTAs blocks nzi-1..m+1 upward.
 // Each half ends with the multiplier block that feeds block m (L_m, or U_{m+1}); btddod_middle_kernel then forms
@@ -466,13 +346,22 @@ __global__ void __launch_bounds__(kFactorThreads) btddod_factor_kernel(int nf, i
     const double *D0 = vals + (size_t)(down ? 0 : nb - 1) * bs2;
     for (int e = tid; e < bs2; e += nt) {
       const int c = e / ns, r = e - c * ns;
-      cur[r * ns + c] = D0[e];
+      cur[r * sh.ld + c] = D0[e];
     }
   }
   __syncthreads();
   for (int t = 0; t < len; ++t) {
     const int i = down ? t : nb - 1 - t;
-    double *Z = cta_gj_inverse(cur, other, ns, sh.piv, sh.pinv, sh.ws, sh.used);
+    // the next block of the chain is loaded while this one is eliminated
+    const bool more = t + 1 < len;
+    const double *Dn = vals + (size_t)(down ? i + 1 : i - 1) * bs2;
+    double dn[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int e = tid + u * kFactorThreads;
+      dn[u] = more && e < bs2 ? Dn[e] : 0.;
+    }
+    double *Z = sh.invert(cur, other, ns);
     double *nxt = Z == cur ? other : cur;  // the buffer the elimination no longer needs
     // multiplier: downward L_{i+1} = diag(sub_i) D_i^-1 at block i+1; upward U_i = diag(sup_{i-1}) T_i^-1 at block
     // i. Then the next block of the chain: D_{i+1} - L_{i+1} diag(sup_i), or D_{i-1} - U_i diag(sub_{i-1}).
@@ -480,16 +369,18 @@ __global__ void __launch_bounds__(kFactorThreads) btddod_factor_kernel(int nf, i
     const double *cs = down ? sup + (size_t)i * ns : sub + (size_t)(i - 1) * ns;
     double *Di = vals + (size_t)i * bs2;
     double *Lm = lv + (size_t)(down ? i + 1 : i) * bs2;
-    const double *Dn = vals + (size_t)(down ? i + 1 : i - 1) * bs2;
-    const bool more = t + 1 < len;
-    for (int e = tid; e < bs2; e += nt) {  // e: column-major index of the global arrays
+    auto element = [&](int e, double next) {  // e: column-major index of the global arrays
       const int c = e / ns, r = e - c * ns;
-      const double inv = Z[sh.piv[r] * ns + sh.pinv[c]];
+      const double inv = Z[sh.piv[r] * sh.ld + sh.pinv[c]];
       Di[e] = inv;
       const double l = inv * rs[r];
       Lm[e] = l;
-      if (more) nxt[r * ns + c] = Dn[e] + (-cs[c]) * l;
-    }
+      if (more) nxt[r * sh.ld + c] = next + (-cs[c]) * l;
+    };
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (tid + u * kFactorThreads < bs2) element(tid + u * kFactorThreads, dn[u]);
+    for (int e = tid + kAhead * kFactorThreads; e < bs2; e += nt) element(e, more ? Dn[e] : 0.);
     for (int k = tid; k < ns; k += nt) pv[(size_t)i * ns + k] = sh.piv[k];
     __syncthreads();
     cur = nxt;
@@ -523,112 +414,64 @@ __global__ void __launch_bounds__(kFactorThreads) btddod_middle_kernel(int nf, i
     double v = Dm[e];
     if (La) v = v + (-sup[(size_t)(m - 1) * ns + c]) * La[e];
     if (Ub) v = v + (-sub[(size_t)m * ns + c]) * Ub[e];
-    sh.buf0[r * ns + c] = v;
+    sh.buf0[r * sh.ld + c] = v;
   }
   __syncthreads();
-  const double *Z = cta_gj_inverse(sh.buf0, sh.buf1, ns, sh.piv, sh.pinv, sh.ws, sh.used);
+  const double *Z = sh.invert(sh.buf0, sh.buf1, ns);
   for (int e = tid; e < bs2; e += nt) {
     const int c = e / ns, r = e - c * ns;
-    Dm[e] = Z[sh.piv[r] * ns + sh.pinv[c]];
+    Dm[e] = Z[sh.piv[r] * sh.ld + sh.pinv[c]];
   }
   int *pv = perms + (size_t)(z0 + m) * ns;
   for (int k = tid; k < ns; k += nt) pv[k] = sh.piv[k];
 }
 
-// Per-lane asynchronous 8-byte copies global -> shared (cp.async, completion tracked by commit groups; no
-// mbarrier wait is involved).
+// Asynchronous 8-byte copies global -> shared by all threads of the block (cp.async, completion tracked by commit
+// groups; no mbarrier wait is involved).
 __device__ __forceinline__ void async_copy_doubles(double *dst, const double *src, int n)
 {
-  const int lane = threadIdx.x & 31;
-  for (int e = lane; e < n; e += 32)
+  for (int e = threadIdx.x; e < n; e += blockDim.x)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst + e)), "l"(src + e) : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 __device__ __forceinline__ void async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// Register-distributed vector of a warp: element k lives in lane k % 32, register k / 32 (R registers).
-template <int R>
-__device__ __forceinline__ double vec_get(const double (&v)[R], int k)
-{
-  double out = 0.;
-#pragma unroll
-  for (int s = 0; s < R; ++s) {
-    const double t = __shfl_sync(0xffffffffu, v[s], k & 31);
-    if ((k >> 5) == s) out = t;
-  }
-  return out;
-}
+// One CTA walks a chain of dependent block steps, each a matrix-vector product with a column-major ns x ns block staged
+// in shared memory (the next one is copied while the current one is used, where two fit). A product's rows are dealt
+// to the threads of whole warps and its columns cut into parts over the other warps: one warp alone takes two FP64
+// instructions per column at 64 cycles each, 6.8 us a step for ns = 53; twelve take 9 per step.
+constexpr int kSweepThreads = 384;
 
-template <int R>
-__device__ __forceinline__ void vec_load(double (&v)[R], const double *src, int ns)
-{
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int s = 0; s < R; ++s) {
-    const int k = lane + 32 * s;
-    v[s] = k < ns ? src[k] : 0.;
-  }
-}
-
-template <int R>
-__device__ __forceinline__ void vec_store(double *dst, const double (&v)[R], int ns)
-{
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int s = 0; s < R; ++s) {
-    const int k = lane + 32 * s;
-    if (k < ns) dst[k] = v[s];
-  }
-}
-
-// acc -= B y for the column-major ns x ns block B (shared memory) and register-distributed y.
-template <int R>
-__device__ __forceinline__ void vec_sub_matvec(const double *B, const double (&y)[R], int ns, double (&acc)[R])
-{
-  const int lane = threadIdx.x & 31;
-  for (int c = 0; c < ns; ++c) {
-    const double yc = vec_get<R>(y, c);
-#pragma unroll
-    for (int s = 0; s < R; ++s) {
-      const int k = lane + 32 * s;
-      if (k < ns) acc[s] += (-B[k + c * ns]) * yc;
-    }
-  }
-}
-
-// v <- B v for the column-major ns x ns block B (shared memory) and register-distributed v.
-template <int R>
-__device__ __forceinline__ void vec_apply(const double *B, int ns, double (&v)[R])
-{
-  const int lane = threadIdx.x & 31;
-  double acc[R];
-#pragma unroll
-  for (int s = 0; s < R; ++s) acc[s] = 0.;
-  for (int c = 0; c < ns; ++c) {
-    const double vc = vec_get<R>(v, c);
-#pragma unroll
-    for (int s = 0; s < R; ++s) {
-      const int k = lane + 32 * s;
-      if (k < ns) acc[s] += B[k + c * ns] * vc;
-    }
-  }
-#pragma unroll
-  for (int s = 0; s < R; ++s) v[s] = acc[s];
-}
-
-// Matrices of one warp's sweep, staged into shared memory: with two buffers the next block is copied while the
-// current one is used; with one (large blocks) each is copied when needed.
-struct SweepBuffers {
-  double *b0, *b1;
+struct Sweep {
+  double *b0, *b1, *part, *vec;
+  int ns, bs2, rows, parts, p, r, c0, c1;
   bool dbl;
-  int bs2;
-  __device__ __forceinline__ double *slot(int k) const { return (k & 1) ? b1 : b0; }  // parity, also for k < 0
-  template <class Src>
-  __device__ __forceinline__ const double *get(int t, int last, int step, Src src)
+  __device__ Sweep(unsigned char *smem, int ns_, bool dbl_) : ns(ns_), bs2(ns_ * ns_), dbl(dbl_)
   {
-    // blocks t, t + step, ... up to `last` inclusive are fetched in this order
-    __syncwarp();
+    b0 = reinterpret_cast<double *>(smem);
+    b1 = dbl ? b0 + bs2 : b0;
+    part = b1 + bs2;
+    vec = part + kSweepThreads;
+    rows = (ns + 31) & ~31;
+    parts = kSweepThreads / rows;
+    p = threadIdx.x / rows;
+    r = threadIdx.x - p * rows;
+    c0 = ns * p / parts;
+    c1 = ns * (p + 1) / parts;
+  }
+  static size_t bytes(int ns, bool dbl) { return ((size_t)(dbl ? 2 : 1) * ns * ns + kSweepThreads + ns) * 8; }
+  __device__ __forceinline__ double *slot(int t) const { return (t & 1) ? b1 : b0; }
+  template <class Src>
+  __device__ __forceinline__ void prime(int t, Src src) const
+  {
+    if (dbl) async_copy_doubles(slot(t), src(t), bs2);
+  }
+  // The block of step t (steps t, t + step, ..., last are fetched in this order); ends with the barrier that also makes
+  // the writes to vec visible.
+  template <class Src>
+  __device__ __forceinline__ const double *fetch(int t, int last, int step, Src src) const
+  {
     if (dbl) {
       if (t != last) {
         async_copy_doubles(slot(t + step), src(t + step), bs2);
@@ -640,165 +483,150 @@ struct SweepBuffers {
       async_copy_doubles(b0, src(t), bs2);
       async_wait_all();
     }
-    __syncwarp();
+    __syncthreads();
     return dbl ? slot(t) : b0;
   }
-  template <class Src>
-  __device__ __forceinline__ void prime(int t, Src src)
+  // Row r of B vec, complete in the threads below ns.
+  __device__ __forceinline__ double product(const double *B) const
   {
-    if (dbl) async_copy_doubles(slot(t), src(t), bs2);
+    double s = 0.;
+    if (p < parts && r < ns)
+      for (int c = c0; c < c1; ++c) s = fma(B[r + c * ns], vec[c], s);
+    if (p > 0 && p < parts) part[threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.x < ns)
+      for (int q = 1; q < parts; ++q) s += part[q * rows + threadIdx.x];
+    return s;
   }
 };
 
-// Solve with the twisted factors (the reference's btddod_matrix_kernels.cpp:82-119 sweeps, run from both ends):
-// one CTA of two warps per flamelet, warp 0 over blocks 0..m-1, warp 1 over blocks nzi-1..m+1, m = nzi/2.
-//   downward  y_0 = b_0, y_i = b_i - L_i y_{i-1};       upward  z_{nzi-1} = b_{nzi-1}, z_i = b_i - U_{i+1} z_{i+1}
-//   middle    x_m = M^-1 (b_m - L_m y_{m-1} - U_{m+1} z_{m+1})
-//   back      x_i = D_i^-1 (y_i - sup_i o x_{i+1}) for i < m;   x_i = T_i^-1 (z_i - sub_{i-1} o x_{i-1}) for i > m.
-// Every block step is a matrix-vector product (the factors hold the inverses). Vectors stay in registers; y and z are
-// parked in out_x until the back substitution overwrites them.
-template <int R>
-__global__ void __launch_bounds__(64) btddod_solve_kernel(int nf, int ns, const int *offz, const long long *offv,
-                                                          const double *values, const double *lvals,
-                                                          const int *perms, const double *rhs, double *x,
-                                                          const int *active, int double_buffer)
+// Solve with the twisted factors (the reference's btddod_matrix_kernels.cpp:82-119 sweeps, run from both ends), two
+// CTAs per flamelet, even ones over blocks 0..m-1, odd ones over blocks nzi-1..m+1, m = nzi/2, in three launches:
+//   1. sweeps toward block m: y_0 = b_0, y_i = b_i - L_i y_{i-1};   z_{nzi-1} = b_{nzi-1}, z_i = b_i - U_{i+1} z_{i+1}
+//   2. one CTA per flamelet:  x_m = M^-1 (b_m - L_m y_{m-1} - U_{m+1} z_{m+1})
+//   3. back substitution:     x_i = D_i^-1 (y_i - sup_i o x_{i+1}) for i < m;  x_i = T_i^-1 (z_i - sub_{i-1} o x_{i-1})
+// y and z are parked in x until the back substitution overwrites them.
+__global__ void __launch_bounds__(kSweepThreads) btddod_forward_kernel(int nf, int ns, const int *offz,
+                                                                       const double *lvals, const double *rhs,
+                                                                       double *x, const int *active, int double_buffer)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int f = blockIdx.x >> 1;
+  const bool down = (blockIdx.x & 1) == 0;
+  if (f >= nf || (active && !active[f])) return;
+  const int z0 = offz[f], nb = offz[f + 1] - z0, m = nb / 2;
+  const int len = down ? m : nb - 1 - m;
+  if (len == 0) return;
+  const Sweep sw(smem, ns, double_buffer != 0);
+  const double *lv = lvals + (size_t)z0 * sw.bs2;
+  const double *b = rhs + (size_t)z0 * ns;
+  double *xs = x + (size_t)z0 * ns;
+  const int tid = threadIdx.x;
+  auto at = [&](int t) { return (size_t)(down ? t : nb - 1 - t) * ns; };
+  auto src = [&](int t) { return lv + (size_t)(down ? t : nb - t) * sw.bs2; };
+  if (len > 1) sw.prime(1, src);
+  if (tid < ns) xs[at(0) + tid] = sw.vec[tid] = b[at(0) + tid];
+  for (int t = 1; t < len; ++t) {
+    const double *B = sw.fetch(t, len - 1, 1, src);
+    const double s = sw.product(B);
+    if (tid < ns) xs[at(t) + tid] = sw.vec[tid] = b[at(t) + tid] - s;
+  }
+}
+
+__global__ void __launch_bounds__(kSweepThreads) btddod_meet_kernel(int nf, int ns, const int *offz,
+                                                                    const long long *offv, const double *values,
+                                                                    const double *lvals, const double *rhs, double *x,
+                                                                    const int *active)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const int f = blockIdx.x;
   if (f >= nf || (active && !active[f])) return;
-  const int warp = threadIdx.x >> 5;
-  const bool down = warp == 0;
+  const int z0 = offz[f], nb = offz[f + 1] - z0, m = nb / 2;
+  const Sweep sw(smem, ns, false);
+  const double *lv = lvals + (size_t)z0 * sw.bs2;
+  double *xs = x + (size_t)z0 * ns;
+  const int tid = threadIdx.x;
+  double v = tid < ns ? rhs[(size_t)(z0 + m) * ns + tid] : 0.;
+  for (int side = 0; side < 2; ++side) {  // L_m y_{m-1}, then U_{m+1} z_{m+1}
+    const int i = side == 0 ? m - 1 : m + 1;
+    if (i < 0 || i >= nb) continue;
+    if (tid < ns) sw.vec[tid] = xs[(size_t)i * ns + tid];
+    const double *B = sw.fetch(0, 0, 1, [&](int) { return lv + (size_t)(m + side) * sw.bs2; });
+    v -= sw.product(B);
+    __syncthreads();
+  }
+  if (tid < ns) sw.vec[tid] = v;
+  const double *B = sw.fetch(0, 0, 1, [&](int) { return values + offv[f] + (size_t)m * sw.bs2; });
+  const double s = sw.product(B);
+  if (tid < ns) xs[(size_t)m * ns + tid] = s;
+}
+
+__global__ void __launch_bounds__(kSweepThreads) btddod_back_kernel(int nf, int ns, const int *offz,
+                                                                    const long long *offv, const double *values,
+                                                                    double *x, const int *active, int double_buffer)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int f = blockIdx.x >> 1;
+  const bool down = (blockIdx.x & 1) == 0;
+  if (f >= nf || (active && !active[f])) return;
   const int z0 = offz[f], nb = offz[f + 1] - z0, m = nb / 2;
   const int len = down ? m : nb - 1 - m;
-  const int bs2 = ns * ns;
-  double *sm = reinterpret_cast<double *>(smem);
-  const int nbuf = double_buffer ? 2 : 1;
-  SweepBuffers sb{sm + (size_t)(warp * nbuf) * bs2, sm + (size_t)(warp * nbuf + nbuf - 1) * bs2, double_buffer != 0,
-                  bs2};
-  double *feed = sm + (size_t)(2 * nbuf) * bs2;  // 2 ns doubles: -L_m y_{m-1} and -U_{m+1} z_{m+1}
-  double *xmid = feed + 2 * ns;                  // ns doubles
-  const double *vals = values + offv[f];
-  const double *lv = lvals + (size_t)z0 * bs2;
-  (void)perms;  // the pivot order of each block's elimination; the stored inverses need none
-  const double *sub = vals + (size_t)nb * bs2;
-  const double *sup = sub + (size_t)(nb - 1) * ns;
-  const double *b = rhs + (size_t)z0 * ns;
-  double *xs = x + (size_t)z0 * ns;
-  auto blk = [&](int t) { return down ? t : nb - 1 - t; };
-  // ---- sweeps toward block m: step t (1 <= t <= len) applies multiplier block blk(t) (+1 upward); step len feeds m
-  auto lsrc = [&](int t) { return lv + (size_t)(down ? t : nb - t) * bs2; };
-  double y[R];
-#pragma unroll
-  for (int s = 0; s < R; ++s) y[s] = 0.;
-  if (len > 0) {
-    sb.prime(1, lsrc);
-    vec_load<R>(y, b + (size_t)blk(0) * ns, ns);
-    vec_store<R>(xs + (size_t)blk(0) * ns, y, ns);
-    for (int t = 1; t <= len; ++t) {
-      const double *B = sb.get(t, len, 1, lsrc);
-      double acc[R];
-      if (t < len) {
-        vec_load<R>(acc, b + (size_t)blk(t) * ns, ns);
-      } else {
-#pragma unroll
-        for (int s = 0; s < R; ++s) acc[s] = 0.;
-      }
-      vec_sub_matvec<R>(B, y, ns, acc);
-#pragma unroll
-      for (int s = 0; s < R; ++s) y[s] = acc[s];
-      if (t < len) vec_store<R>(xs + (size_t)blk(t) * ns, y, ns);
-    }
-  }
-  vec_store<R>(feed + (size_t)warp * ns, y, ns);  // zero when this half is empty
-  __syncthreads();
-  // ---- block m
-  auto fsrc = [&](int i) { return vals + (size_t)i * bs2; };
-  if (down) {
-    sb.prime(m, fsrc);
-    const double *F = sb.get(m, m, 1, fsrc);  // single fetch (t == last)
-    double v[R], f0[R], f1[R];
-    vec_load<R>(v, b + (size_t)m * ns, ns);
-    vec_load<R>(f0, feed, ns);
-    vec_load<R>(f1, feed + ns, ns);
-#pragma unroll
-    for (int s = 0; s < R; ++s) v[s] = (v[s] + f0[s]) + f1[s];
-    vec_apply<R>(F, ns, v);
-    vec_store<R>(xs + (size_t)m * ns, v, ns);
-    vec_store<R>(xmid, v, ns);
-  }
-  __syncthreads();
   if (len == 0) return;
-  // ---- back substitution away from block m: blocks blk(len-1), ..., blk(0)
-  double xn[R];
-  vec_load<R>(xn, xmid, ns);
-  auto bsrc = [&](int t) { return vals + (size_t)blk(t) * bs2; };
-  sb.prime(len - 1, bsrc);
+  const Sweep sw(smem, ns, double_buffer != 0);
+  const double *vals = values + offv[f];
+  const double *sub = vals + (size_t)nb * sw.bs2;
+  const double *sup = sub + (size_t)(nb - 1) * ns;
+  double *xs = x + (size_t)z0 * ns;
+  const int tid = threadIdx.x;
+  auto blk = [&](int t) { return down ? t : nb - 1 - t; };
+  auto src = [&](int t) { return vals + (size_t)blk(t) * sw.bs2; };
+  sw.prime(len - 1, src);
+  double xn = tid < ns ? xs[(size_t)m * ns + tid] : 0.;
   for (int t = len - 1; t >= 0; --t) {
-    const double *F = sb.get(t, 0, -1, bsrc);
     const int i = blk(t);
     const double *cpl = down ? sup + (size_t)i * ns : sub + (size_t)(i - 1) * ns;
-    double v[R];
-    vec_load<R>(v, xs + (size_t)i * ns, ns);
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int s = 0; s < R; ++s) {
-      const int k = lane + 32 * s;
-      if (k < ns) v[s] = v[s] - cpl[k] * xn[s];
-    }
-    vec_apply<R>(F, ns, v);
-    vec_store<R>(xs + (size_t)i * ns, v, ns);
-#pragma unroll
-    for (int s = 0; s < R; ++s) xn[s] = v[s];
+    if (tid < ns) sw.vec[tid] = xs[(size_t)i * ns + tid] - cpl[tid] * xn;
+    const double *B = sw.fetch(t, 0, -1, src);
+    xn = sw.product(B);
+    if (tid < ns) xs[(size_t)i * ns + tid] = xn;
   }
 }
 
 // Block-triangular solves with the inverses of a block-diagonal factorization (btddod_matrix_kernels.cpp:386-428):
 //   lower  x_0 = F_0 b_0,               x_i = F_i (b_i - sub_{i-1} o x_{i-1})
 //   upper  x_{nb-1} = F_{nb-1} b_{nb-1}, x_i = F_i (b_i - sup_i o x_{i+1})
-// One warp per flamelet; F_i (column-major inverses, [points][ns*ns]) are streamed into shared memory one block
-// ahead, the vector stays in registers.
-template <int R>
-__global__ void __launch_bounds__(32) btddod_triangle_solve_kernel(int nf, int ns, const int *offz,
-                                                                   const long long *offv, const double *inverses,
-                                                                   const double *values, const double *rhs, double *x,
-                                                                   int upper, const int *active, int double_buffer)
+// One CTA per flamelet; F_i are column-major inverses, [points][ns*ns].
+__global__ void __launch_bounds__(kSweepThreads) btddod_triangle_solve_kernel(int nf, int ns, const int *offz,
+                                                                              const long long *offv,
+                                                                              const double *inverses,
+                                                                              const double *values, const double *rhs,
+                                                                              double *x, int upper, const int *active,
+                                                                              int double_buffer)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const int f = blockIdx.x;
   if (f >= nf || (active && !active[f])) return;
   const int z0 = offz[f], nb = offz[f + 1] - z0;
-  const int bs2 = ns * ns;
-  double *sm = reinterpret_cast<double *>(smem);
-  SweepBuffers sb{sm, sm + (double_buffer ? bs2 : 0), double_buffer != 0, bs2};
-  const double *vals = values + offv[f];
-  const double *sub = vals + (size_t)nb * bs2;
+  const Sweep sw(smem, ns, double_buffer != 0);
+  const double *sub = values + offv[f] + (size_t)nb * sw.bs2;
   const double *sup = sub + (size_t)(nb - 1) * ns;
   const double *b = rhs + (size_t)z0 * ns;
   double *xs = x + (size_t)z0 * ns;
+  const int tid = threadIdx.x;
   auto blk = [&](int t) { return upper ? nb - 1 - t : t; };
-  auto fsrc = [&](int t) { return inverses + (size_t)(z0 + blk(t)) * bs2; };
-  const int lane = threadIdx.x & 31;
-  double xp[R];
-#pragma unroll
-  for (int s = 0; s < R; ++s) xp[s] = 0.;
-  sb.prime(0, fsrc);
+  auto src = [&](int t) { return inverses + (size_t)(z0 + blk(t)) * sw.bs2; };
+  sw.prime(0, src);
+  double xp = 0.;
   for (int t = 0; t < nb; ++t) {
-    const double *F = sb.get(t, nb - 1, 1, fsrc);
     const int i = blk(t);
-    double v[R];
-    vec_load<R>(v, b + (size_t)i * ns, ns);
-    if (t > 0) {
-      const double *cpl = upper ? sup + (size_t)i * ns : sub + (size_t)(i - 1) * ns;
-#pragma unroll
-      for (int s = 0; s < R; ++s) {
-        const int k = lane + 32 * s;
-        if (k < ns) v[s] = v[s] - cpl[k] * xp[s];
-      }
+    if (tid < ns) {
+      double v = b[(size_t)i * ns + tid];
+      if (t > 0) v -= (upper ? sup[(size_t)i * ns + tid] : sub[(size_t)(i - 1) * ns + tid]) * xp;
+      sw.vec[tid] = v;
     }
-    vec_apply<R>(F, ns, v);
-    vec_store<R>(xs + (size_t)i * ns, v, ns);
-#pragma unroll
-    for (int s = 0; s < R; ++s) xp[s] = v[s];
+    const double *F = sw.fetch(t, nb - 1, 1, src);
+    xp = sw.product(F);
+    if (tid < ns) xs[(size_t)i * ns + tid] = xp;
   }
 }
 
@@ -817,14 +645,14 @@ __global__ void __launch_bounds__(kFactorThreads) blockdiag_inverse_kernel(int n
   const int tid = threadIdx.x, nt = blockDim.x;
   for (int e = tid; e < bs2; e += nt) {
     const int c = e / ns, r = e - c * ns;
-    sh.buf0[r * ns + c] = A[e];
+    sh.buf0[r * sh.ld + c] = A[e];
   }
   __syncthreads();
-  const double *Z = cta_gj_inverse(sh.buf0, sh.buf1, ns, sh.piv, sh.pinv, sh.ws, sh.used);
+  const double *Z = sh.invert(sh.buf0, sh.buf1, ns);
   double *O = out_inv + (size_t)blkid * bs2;
   for (int e = tid; e < bs2; e += nt) {
     const int c = e / ns, r = e - c * ns;
-    O[e] = Z[sh.piv[r] * ns + sh.pinv[c]];
+    O[e] = Z[sh.piv[r] * sh.ld + sh.pinv[c]];
   }
   for (int k = tid; k < ns; k += nt) pivots[(size_t)blkid * ns + k] = sh.piv[k];
 }
@@ -1007,27 +835,33 @@ int check_launch()
   return SF_OK;
 }
 
-template <int R>
+// Two staged blocks where they fit, else one
+bool sweep_double_buffer(int ns, int smem_max)
+{
+  if (Sweep::bytes(ns, false) > (size_t)smem_max)
+    throw sf_error(SF_ERR_UNSUPPORTED, "block size too large for the shared-memory block-Thomas solve");
+  return Sweep::bytes(ns, true) <= (size_t)smem_max;
+}
+
 int launch_solve(int nf, int ns, const int *offz, const long long *offv, const double *values,
-                 const double *l_values, const int *pivots, const double *rhs, double *out_x, const int *active,
-                 cudaStream_t st)
+                 const double *l_values, const double *rhs, double *out_x, const int *active, cudaStream_t st)
 {
   int dev, smem_max;
   CUDA_THROW(cudaGetDevice(&dev));
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  // two warps, each with two staged blocks (one when four do not fit), plus the middle block's feed vectors
-  const size_t extra = (size_t)3 * ns * 8;
-  const int dbl = (size_t)4 * ns * ns * 8 + extra <= (size_t)smem_max ? 1 : 0;
-  const size_t smem = (size_t)(dbl ? 4 : 2) * ns * ns * 8 + extra;
-  if (smem > (size_t)smem_max)
-    throw sf_error(SF_ERR_UNSUPPORTED, "block size too large for the shared-memory block-Thomas solve");
-  ensure_dynamic_smem((const void *)btddod_solve_kernel<R>, smem);
-  btddod_solve_kernel<R><<<nf, 64, smem, st>>>(nf, ns, offz, offv, values, l_values, pivots, rhs, out_x, active,
-                                               dbl);
+  const bool dbl = sweep_double_buffer(ns, smem_max);
+  const size_t smem = Sweep::bytes(ns, dbl), smem1 = Sweep::bytes(ns, false);
+  ensure_dynamic_smem((const void *)btddod_forward_kernel, smem);
+  ensure_dynamic_smem((const void *)btddod_meet_kernel, smem1);
+  ensure_dynamic_smem((const void *)btddod_back_kernel, smem);
+  btddod_forward_kernel<<<2 * nf, kSweepThreads, smem, st>>>(nf, ns, offz, l_values, rhs, out_x, active, dbl);
+  CUDA_THROW(cudaGetLastError());
+  btddod_meet_kernel<<<nf, kSweepThreads, smem1, st>>>(nf, ns, offz, offv, values, l_values, rhs, out_x, active);
+  CUDA_THROW(cudaGetLastError());
+  btddod_back_kernel<<<2 * nf, kSweepThreads, smem, st>>>(nf, ns, offz, offv, values, out_x, active, dbl);
   return check_launch();
 }
 
-template <int R>
 int launch_triangle(int nf, int ns, const int *offz, const long long *offv, const double *inverses,
                     const double *values, const double *rhs, double *out_x, int upper, const int *active,
                     cudaStream_t st)
@@ -1035,13 +869,11 @@ int launch_triangle(int nf, int ns, const int *offz, const long long *offv, cons
   int dev, smem_max;
   CUDA_THROW(cudaGetDevice(&dev));
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const int dbl = (size_t)2 * ns * ns * 8 <= (size_t)smem_max ? 1 : 0;
-  const size_t smem = (size_t)(dbl ? 2 : 1) * ns * ns * 8;
-  if (smem > (size_t)smem_max)
-    throw sf_error(SF_ERR_UNSUPPORTED, "block size too large for the shared-memory triangular solve");
-  ensure_dynamic_smem((const void *)btddod_triangle_solve_kernel<R>, smem);
-  btddod_triangle_solve_kernel<R><<<nf, 32, smem, st>>>(nf, ns, offz, offv, inverses, values, rhs, out_x, upper,
-                                                         active, dbl);
+  const bool dbl = sweep_double_buffer(ns, smem_max);
+  const size_t smem = Sweep::bytes(ns, dbl);
+  ensure_dynamic_smem((const void *)btddod_triangle_solve_kernel, smem);
+  btddod_triangle_solve_kernel<<<nf, kSweepThreads, smem, st>>>(nf, ns, offz, offv, inverses, values, rhs, out_x,
+                                                                upper, active, dbl);
   return check_launch();
 }
 
@@ -1100,10 +932,7 @@ int sf_btddod_triangle_solve_batch(int nf, int ns, const int *offz, const long l
   cudaStream_t st = (cudaStream_t)stream;
   const int up = upper ? 1 : 0;
   return guarded([&] {
-    if (ns <= 32) return launch_triangle<1>(nf, ns, offz, offv, inverses, values, rhs, out_x, up, active, st);
-    if (ns <= 64) return launch_triangle<2>(nf, ns, offz, offv, inverses, values, rhs, out_x, up, active, st);
-    if (ns <= 96) return launch_triangle<3>(nf, ns, offz, offv, inverses, values, rhs, out_x, up, active, st);
-    return launch_triangle<4>(nf, ns, offz, offv, inverses, values, rhs, out_x, up, active, st);
+    return launch_triangle(nf, ns, offz, offv, inverses, values, rhs, out_x, up, active, st);
   });
 }
 
@@ -1290,10 +1119,8 @@ int sf_btddod_solve_batch(int nf, int ns, const int *offz, const long long *offv
   (void)offz_host;
   cudaStream_t st = (cudaStream_t)stream;
   return guarded([&] {
-    if (ns <= 32) return launch_solve<1>(nf, ns, offz, offv, values, l_values, pivots, rhs, out_x, active, st);
-    if (ns <= 64) return launch_solve<2>(nf, ns, offz, offv, values, l_values, pivots, rhs, out_x, active, st);
-    if (ns <= 96) return launch_solve<3>(nf, ns, offz, offv, values, l_values, pivots, rhs, out_x, active, st);
-    return launch_solve<4>(nf, ns, offz, offv, values, l_values, pivots, rhs, out_x, active, st);
+    if ((long long)nf * 2 > 0x7fffffffLL) throw sf_error(SF_ERR_INVALID_ARGUMENT, "too many flamelets");
+    return launch_solve(nf, ns, offz, offv, values, l_values, rhs, out_x, active, st);
   });
 }
 

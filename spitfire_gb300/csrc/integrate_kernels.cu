@@ -19,6 +19,7 @@
 #include "sf_internal.h"
 #include "warp_lu.cuh"
 #include "esdirk64.cuh"
+#include "gj_device.cuh"
 
 namespace sfgb {
 namespace {
@@ -102,121 +103,7 @@ struct IterMatrixRows {
   }
 };
 
-// Inverse of the n x n row-major matrix in S (leading dimension ld) by Gauss-Jordan elimination with partial pivoting
-// by one wide group; the scheme of the block-Thomas factorization's elimination (flamelet_kernels.cu), one group
-// barrier per column: warp 0 forms the next column, chooses the next pivot (largest magnitude, lowest row on ties) and
-// its multipliers while the other warps update the block from S to D. Returns the buffer Z with inverse(r, c) =
-// Z[piv[r]][pinv[c]]. ws: 2n + 2 doubles; used: n ints; n <= 128. A zero pivot column gives no inverse (the step then
-// ends in values that are not finite and is rejected).
-template <int G>
-__device__ __forceinline__ double *group_gj_inverse(const Group<G> &grp, double *S, double *D, int n, int ld, int *piv,
-                                                    int *pinv, double *ws, int *used)
-{
-  const int lane = grp.lane & 31, warp = grp.warp;
-  double *ipb = ws + 2 * n;
-  auto choose = [&](int j, const double (&v)[4]) {
-    unsigned long long best = 0ull;
-    int bp = n;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = lane + 32 * s;
-      if (i < n && !used[i]) {
-        const unsigned long long key = abs_key(v[s]);
-        if (bp == n || key > best) { best = key; bp = i; }
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bp, o);
-      if (oi < n && (bp >= n || ob > best || (ob == best && oi < bp))) { best = ob; bp = oi; }
-    }
-    double pv = 0.;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const double t = __shfl_sync(0xffffffffu, v[s], bp & 31);
-      if ((bp >> 5) == s) pv = t;
-    }
-    const double ip = 1. / pv;
-    double *f = ws + (j & 1) * n;  // the negated multipliers
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = lane + 32 * s;
-      if (i < n) f[i] = -(v[s] * ip);
-    }
-    if (lane == 0) {
-      ipb[j & 1] = ip;
-      piv[j] = bp;
-      pinv[bp] = j;
-      used[bp] = 1;
-    }
-    __syncwarp();
-  };
-  if (warp == 0) {
-    for (int i = lane; i < n; i += 32) used[i] = 0;
-    __syncwarp();
-    double v[4];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int i = lane + 32 * s;
-      v[s] = i < n ? S[i * ld] : 0.;
-    }
-    choose(0, v);
-  }
-  grp.sync();
-  constexpr int stride = G - 32;
-  const int ut = grp.lane - 32;
-  const int i0 = ut / n, j0 = ut - i0 * n, di = stride / n, dj = stride - di * n;
-  for (int k = 0; k < n; ++k) {
-    const int p = piv[k];
-    const double ip = ipb[k & 1];
-    const double *nf = ws + (k & 1) * n;  // -f_i
-    const double *Sp = S + (size_t)p * ld;
-    if (warp == 0) {
-      if (k + 1 < n) {
-        const int j = k + 1;
-        const double spj = Sp[j];
-        double v[4];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          const int i = lane + 32 * s;
-          double val = 0.;
-          if (i < n) {
-            val = S[i * ld + j] + nf[i] * spj;
-            if (i == p) val = spj * ip;
-            D[i * ld + j] = val;
-          }
-          v[s] = val;
-        }
-        choose(j, v);
-      }
-    } else {
-      const int kn = k + 1;
-      int i = i0, j = j0;
-      while (i < n) {
-        if (j != kn) {  // column k+1 is warp 0's
-          const double nfi = nf[i];
-          double val = S[i * ld + j] + nfi * Sp[j];
-          if (j == k) val = nfi;
-          if (i == p) val = j == k ? ip : Sp[j] * ip;
-          D[i * ld + j] = val;
-        }
-        i += di;
-        j += dj;
-        if (j >= n) {
-          j -= n;
-          ++i;
-        }
-      }
-    }
-    grp.sync();
-    double *t = S;
-    S = D;
-    D = t;
-  }
-  return S;
-}
-
-// x[pinv[i]] = sum_k Z[i][k] b[piv[k]] for the permuted inverse of group_gj_inverse: the row sums are cut into parts
+// x[pinv[i]] = sum_k Z[i][k] b[piv[k]] for the permuted inverse of gj_inverse: the row sums are cut into parts
 // over the group's warps (part: G doubles), b permuted into xb first. Ends with a barrier; x is then complete.
 template <int G>
 __device__ __forceinline__ void group_apply_inverse(const Group<G> &grp, const double *Z, int n, int ld, const int *piv,
@@ -361,10 +248,10 @@ __global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) integrate_
   int *piv = reinterpret_cast<int *>(after + (p.prec == 1 ? lu32_doubles + neq : 0));
   double *dinv = after + (p.prec == 1 ? lu32_doubles + neq : 0) + (neq + 1) / 2 + 1;
   float *rf = xf + neq;
-  // WIDE: pivot order and its inverse, rows used, multipliers (3 neq ints, 2 neq + 2 doubles), parts (G doubles)
-  int *pinv = piv + neq, *used = pinv + neq;
-  double *ws = after + (3 * neq + 1) / 2 + 1;
-  double *part = ws + 2 * neq + 2;
+  // WIDE: pivot order and its inverse, multipliers (2 neq ints, 2 neq doubles), parts (G doubles)
+  int *pinv = piv + neq;
+  double *ws = after + neq;
+  double *part = ws + 2 * neq;
   const int Tidx = p.cfg.configuration == 1 ? 1 : 0;
   // feed mass fractions of a time table: the last ns doubles of the group's shared region
   double *ybuf = (p.ip.time_table && (p.ip.time_columns & SF_TIME_FEED_Y)) ? group_shared + p.per_warp - m.ns : nullptr;
@@ -405,7 +292,7 @@ __global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) integrate_
         if constexpr (WIDE) {
           IterMatrixRows im{A, ld, dt * kGamma};
           reactor_eval<G, true, int_unroll(G), OPEN>(m, b, L, scr, grp, y, pres, cf, p.pg, f, im);
-          const double *Z = group_gj_inverse<G>(grp, A, scr, neq, ld, piv, pinv, ws, used);
+          const double *Z = gj_inverse<false>(A, scr, neq, ld, piv, pinv, ws, lane, G, [&] { grp.sync(); });
           if (Z != A)  // an odd number of columns ends in the scratch, which the next right-hand side overwrites
             for (int e = lane; e < neq * ld; e += G) A[e] = Z[e];
         } else {
@@ -643,7 +530,7 @@ size_t wide_doubles(const HostMech &hm, int G, int neq, bool feed_y_table)
 {
   const size_t ld = neq | 1;
   return wide_group_doubles(G) + neq * ld + 12 * (size_t)neq + std::max<size_t>(hm.sl.total, neq * ld) +
-         (3 * (size_t)neq + 1) / 2 + 1 + 2 * (size_t)neq + 2 + G + (feed_y_table ? (size_t)hm.dm.ns : 0);
+         3 * (size_t)neq + G + (feed_y_table ? (size_t)hm.dm.ns : 0);
 }
 
 struct IntShape {
