@@ -1,9 +1,11 @@
 // Batched dense Newton algebra: LU factorization of A = gamma_h * J - I with partial pivoting and the matching
-// triangular solves, one warp per matrix, the matrix held in shared memory.
+// triangular solves, one warp per matrix.
 //
 // Replaces the scipy LAPACK calls of HomogeneousReactor (reactors.py:340-356): dgetrf on (prefactor*J - I) and
 // dgetrs per Newton iteration. The FP32 variant factorizes the same matrix in single precision (FP32 pipe) and
 // recovers FP64 accuracy in the solve by residual refinement r = b - A x with A in FP64.
+#include <algorithm>
+
 #include "sf_internal.h"
 #include "warp_lu.cuh"
 
@@ -11,129 +13,305 @@ namespace sfgb {
 
 namespace {
 
-constexpr int kWarpsPerCta = 4;
+// Matrices per CTA: three warps, so that three CTAs with a 55 x 55 FP64 matrix (odd leading dimension: the row swaps and
+// row reads then touch different banks) per warp fill an SM's shared memory.
+constexpr int kWarpsPerCta = 3;
 
-__global__ void lu64_kernel(int n, int m, const double *J, const double *gh, double *outA, double *outLU, int *piv,
-                            int *info)
+__host__ __device__ constexpr int lu_ld(int m) { return m | 1; }
+
+// Shared memory of a factorization CTA
+template <typename F>
+size_t lu_smem(int m)
+{
+  return (size_t)kWarpsPerCta * ((size_t)m * lu_ld(m) * sizeof(F) + (size_t)m * 4);
+}
+
+// A = gamma h J - I (also to outA if given) and its LU factors, one warp per matrix, F = double or float. Bound for FP64:
+// m^3 / 3 FMAs and a reciprocal per column, 1.05 ms for 8192 matrices of 54 x 54 at the FP64 issue rate.
+template <typename F>
+__global__ void __launch_bounds__(32 * kWarpsPerCta) lu_kernel(int n, int m, const double *J, const double *gh,
+                                                               double *outA, F *outLU, int *piv, int *info)
 {
   extern __shared__ __align__(16) unsigned char sm[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t mm = (size_t)m * m;
-  double *A = reinterpret_cast<double *>(sm) + (size_t)w * mm;
-  int *pv = reinterpret_cast<int *>(reinterpret_cast<double *>(sm) + (size_t)kWarpsPerCta * mm) + w * m;
+  const int mm = m * m, ld = lu_ld(m);
+  F *A = reinterpret_cast<F *>(sm) + (size_t)w * m * ld;
+  int *pv = reinterpret_cast<int *>(reinterpret_cast<F *>(sm) + (size_t)kWarpsPerCta * m * ld) + w * m;
+  const int dc = 32 / m, dr = 32 - dc * m, col0 = lane / m, row0 = lane - col0 * m;
   for (int s = blockIdx.x * kWarpsPerCta + w; s < n; s += gridDim.x * kWarpsPerCta) {
     const double g = gh[s];
-    const double *Js = J + s * mm;
-    for (size_t e = lane; e < mm; e += 32) {
-      const int col = (int)(e / m), row = (int)(e - (size_t)col * m);
-      const double v = g * Js[e] - (row == col ? 1. : 0.);
-      A[e] = v;
-      if (outA) outA[s * mm + e] = v;
+    const double *Js = J + (size_t)s * mm;
+    int row = row0, col = col0;
+#pragma unroll 4
+    for (int e = lane; e < mm; e += 32) {
+      const double v = fma(g, Js[e], row == col ? -1. : 0.);
+      A[row + col * ld] = (F)v;
+      if (outA) outA[(size_t)s * mm + e] = v;
+      row += dr;
+      col += dc;
+      if (row >= m) {
+        row -= m;
+        ++col;
+      }
     }
     __syncwarp();
-    const int inf = warp_lu(A, m, pv);
-    for (size_t e = lane; e < mm; e += 32) outLU[s * mm + e] = A[e];
+    const int inf = warp_lu_factor<false>(A, m, ld, pv, (F *)nullptr);
+    row = row0;
+    col = col0;
+#pragma unroll 4
+    for (int e = lane; e < mm; e += 32) {
+      outLU[(size_t)s * mm + e] = A[row + col * ld];
+      row += dr;
+      col += dc;
+      if (row >= m) {
+        row -= m;
+        ++col;
+      }
+    }
     for (int k = lane; k < m; k += 32) piv[(size_t)s * m + k] = pv[k];
     if (info && lane == 0) info[s] = inf;
     __syncwarp();
   }
 }
 
-__global__ void lu32_kernel(int n, int m, const double *J, const double *gh, double *outA, float *outLU, int *piv,
-                            int *info)
+// ------------------------------------------------------------------------------------------------------ solves
+// One warp per system, its vectors in registers (element i in lane i % 32, register i / 32; R registers), the factors
+// streamed from global memory a few columns ahead: every factor is used once per sweep, so staging it in shared memory
+// only limited the warps per SM.
+constexpr int kSolveWarps = 4;
+constexpr int kAheadCols = 4;
+
+template <int R, typename F>
+__device__ __forceinline__ F reg_get(const F (&v)[R], int k)
 {
-  extern __shared__ __align__(16) unsigned char sm[];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t mm = (size_t)m * m;
-  float *A = reinterpret_cast<float *>(sm) + (size_t)w * mm;
-  int *pv = reinterpret_cast<int *>(reinterpret_cast<float *>(sm) + (size_t)kWarpsPerCta * mm) + w * m;
-  for (int s = blockIdx.x * kWarpsPerCta + w; s < n; s += gridDim.x * kWarpsPerCta) {
-    const double g = gh[s];
-    const double *Js = J + s * mm;
-    for (size_t e = lane; e < mm; e += 32) {
-      const int col = (int)(e / m), row = (int)(e - (size_t)col * m);
-      const double v = g * Js[e] - (row == col ? 1. : 0.);
-      A[e] = (float)v;
-      outA[s * mm + e] = v;
+  F out = __shfl_sync(0xffffffffu, v[0], k & 31);
+#pragma unroll
+  for (int s = 1; s < R; ++s) {
+    const F t = __shfl_sync(0xffffffffu, v[s], k & 31);
+    if ((k >> 5) == s) out = t;
+  }
+  return out;
+}
+
+// The row order that the interchanges of the factorization give: perm element i is the original row that ends in row i.
+template <int R>
+__device__ __forceinline__ void reg_permutation(const int *piv, int m, int lane, int (&perm)[R])
+{
+  int pv[R];
+#pragma unroll
+  for (int s = 0; s < R; ++s) {
+    perm[s] = lane + 32 * s;
+    pv[s] = perm[s] < m ? piv[perm[s]] : 0;
+  }
+  for (int k = 0; k < m; ++k) {
+    const int p = reg_get<R>(pv, k);
+    const int a = reg_get<R>(perm, k), b = reg_get<R>(perm, p);
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+      if (lane + 32 * s == k) perm[s] = b;
+      if (lane + 32 * s == p) perm[s] = a;
     }
-    __syncwarp();
-    const int inf = warp_lu(A, m, pv);
-    for (size_t e = lane; e < mm; e += 32) outLU[s * mm + e] = A[e];
-    for (int k = lane; k < m; k += 32) piv[(size_t)s * m + k] = pv[k];
-    if (info && lane == 0) info[s] = inf;
-    __syncwarp();
   }
 }
 
-__global__ void solve64_kernel(int n, int m, const double *LU, const int *piv, const double *b, double *x)
+template <int R, typename F>
+__device__ __forceinline__ void reg_reciprocals(const F *LU, int m, int lane, F (&rd)[R])
 {
-  extern __shared__ __align__(16) unsigned char sm[];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t mm = (size_t)m * m;
-  double *L = reinterpret_cast<double *>(sm) + (size_t)w * (mm + m);
-  double *xs = L + mm;
-  int *pv = reinterpret_cast<int *>(reinterpret_cast<double *>(sm) + (size_t)kWarpsPerCta * (mm + m)) + w * m;
-  for (int s = blockIdx.x * kWarpsPerCta + w; s < n; s += gridDim.x * kWarpsPerCta) {
-    for (size_t e = lane; e < mm; e += 32) L[e] = LU[s * mm + e];
-    for (int k = lane; k < m; k += 32) {
-      xs[k] = b[(size_t)s * m + k];
-      pv[k] = piv[(size_t)s * m + k];
+#pragma unroll
+  for (int s = 0; s < R; ++s) {
+    const int i = lane + 32 * s;
+    rd[s] = lu_reciprocal(i < m ? LU[(size_t)i * (m + 1)] : (F)1);
+  }
+}
+
+template <int R, typename F>
+__device__ __forceinline__ void load_columns(F (&c)[kAheadCols][R], const F *M, int m, int lane, int j, int step)
+{
+#pragma unroll
+  for (int u = 0; u < kAheadCols; ++u) {
+    const int jj = j + u * step;
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+      const int i = lane + 32 * s;
+      c[u][s] = jj >= 0 && jj < m && i < m ? M[i + (size_t)jj * m] : (F)0;
     }
-    __syncwarp();
-    warp_lu_solve(L, m, pv, xs);
-    for (int k = lane; k < m; k += 32) x[(size_t)s * m + k] = xs[k];
-    __syncwarp();
+  }
+}
+
+// x <- (LU)^-1 x with x in the factors' row order and rd the reciprocals of U's diagonal.
+template <int R, typename F>
+__device__ __forceinline__ void reg_lu_solve(const F *LU, int m, int lane, const F (&rd)[R], F (&x)[R])
+{
+  F c[kAheadCols][R], nx[kAheadCols][R];
+  load_columns<R>(c, LU, m, lane, 0, 1);
+  for (int j0 = 0; j0 < m; j0 += kAheadCols) {
+    load_columns<R>(nx, LU, m, lane, j0 + kAheadCols, 1);
+#pragma unroll
+    for (int u = 0; u < kAheadCols; ++u) {
+      const int j = j0 + u;
+      if (j < m) {
+        const F xj = reg_get<R>(x, j);
+#pragma unroll
+        for (int s = 0; s < R; ++s)
+          if (32 * s + 31 > j && lane + 32 * s > j) x[s] = fma(-c[u][s], xj, x[s]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kAheadCols; ++u)
+#pragma unroll
+      for (int s = 0; s < R; ++s) c[u][s] = nx[u][s];
+  }
+  load_columns<R>(c, LU, m, lane, m - 1, -1);
+  for (int j0 = m - 1; j0 >= 0; j0 -= kAheadCols) {
+    load_columns<R>(nx, LU, m, lane, j0 - kAheadCols, -1);
+#pragma unroll
+    for (int u = 0; u < kAheadCols; ++u) {
+      const int j = j0 - u;
+      if (j >= 0) {
+        F xs = x[0], rs = rd[0];
+#pragma unroll
+        for (int s = 1; s < R; ++s)
+          if ((j >> 5) == s) {
+            xs = x[s];
+            rs = rd[s];
+          }
+        const F xj = __shfl_sync(0xffffffffu, xs * rs, j & 31);
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+          if (32 * s < j && lane + 32 * s < j) x[s] = fma(-c[u][s], xj, x[s]);
+          if (lane + 32 * s == j) x[s] = xj;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kAheadCols; ++u)
+#pragma unroll
+      for (int s = 0; s < R; ++s) c[u][s] = nx[u][s];
+  }
+}
+
+template <int R>
+__global__ void __launch_bounds__(32 * kSolveWarps) solve64_kernel(int n, int m, const double *LU, const int *piv,
+                                                                   const double *b, double *x)
+{
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int sys = blockIdx.x * kSolveWarps + w; sys < n; sys += gridDim.x * kSolveWarps) {
+    const double *L = LU + (size_t)sys * m * m;
+    int perm[R];
+    reg_permutation<R>(piv + (size_t)sys * m, m, lane, perm);
+    double rd[R], xr[R];
+    reg_reciprocals<R>(L, m, lane, rd);
+#pragma unroll
+    for (int s = 0; s < R; ++s) xr[s] = lane + 32 * s < m ? b[(size_t)sys * m + perm[s]] : 0.;
+    reg_lu_solve<R>(L, m, lane, rd, xr);
+#pragma unroll
+    for (int s = 0; s < R; ++s)
+      if (lane + 32 * s < m) x[(size_t)sys * m + lane + 32 * s] = xr[s];
   }
 }
 
 // FP32 triangular solves + FP64 residual refinement (r = b - A x, x += LU32^-1 r).
-__global__ void solve32_kernel(int n, int m, const double *A, const float *LU, const int *piv, int refine,
-                               const double *b, double *x)
+template <int R>
+__global__ void __launch_bounds__(32 * kSolveWarps) solve32_kernel(int n, int m, const double *A, const float *LU,
+                                                                   const int *piv, int refine, const double *b,
+                                                                   double *x)
 {
-  extern __shared__ __align__(16) unsigned char sm[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t mm = (size_t)m * m;
-  const size_t per = mm / 2 + 2 * (size_t)m + 2;  // doubles per warp: fp32 LU, x (fp64), r (fp32 in fp64 slots)
-  double *base = reinterpret_cast<double *>(sm) + (size_t)w * per;
-  float *L = reinterpret_cast<float *>(base);
-  double *xs = base + (mm + 1) / 2;
-  float *rs = reinterpret_cast<float *>(xs + m);
-  int *pv = reinterpret_cast<int *>(reinterpret_cast<double *>(sm) + (size_t)kWarpsPerCta * per) + w * m;
-  for (int s = blockIdx.x * kWarpsPerCta + w; s < n; s += gridDim.x * kWarpsPerCta) {
-    for (size_t e = lane; e < mm; e += 32) L[e] = LU[s * mm + e];
-    for (int k = lane; k < m; k += 32) {
-      rs[k] = (float)b[(size_t)s * m + k];
-      pv[k] = piv[(size_t)s * m + k];
+  for (int sys = blockIdx.x * kSolveWarps + w; sys < n; sys += gridDim.x * kSolveWarps) {
+    const float *L = LU + (size_t)sys * m * m;
+    const double *As = A + (size_t)sys * m * m;
+    int perm[R];
+    reg_permutation<R>(piv + (size_t)sys * m, m, lane, perm);
+    float rd[R], r[R];
+    reg_reciprocals<R>(L, m, lane, rd);
+    double bs[R], xs[R];
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+      bs[s] = lane + 32 * s < m ? b[(size_t)sys * m + lane + 32 * s] : 0.;
+      r[s] = lane + 32 * s < m ? (float)b[(size_t)sys * m + perm[s]] : 0.f;
     }
-    __syncwarp();
-    warp_lu_solve(L, m, pv, rs);
-    for (int k = lane; k < m; k += 32) xs[k] = (double)rs[k];
-    __syncwarp();
-    const double *As = A + s * mm;
+    reg_lu_solve<R>(L, m, lane, rd, r);
+#pragma unroll
+    for (int s = 0; s < R; ++s) xs[s] = (double)r[s];
     for (int it = 0; it < refine; ++it) {
       // residual in FP64, rows over lanes
-      for (int i = lane; i < m; i += 32) {
-        double r = b[(size_t)s * m + i];
-        for (int j = 0; j < m; ++j) r = fma(-As[i + (size_t)j * m], xs[j], r);
-        rs[i] = (float)r;
+      double res[R], c[kAheadCols][R], nx[kAheadCols][R];
+#pragma unroll
+      for (int s = 0; s < R; ++s) res[s] = bs[s];
+      load_columns<R>(c, As, m, lane, 0, 1);
+      for (int j0 = 0; j0 < m; j0 += kAheadCols) {
+        load_columns<R>(nx, As, m, lane, j0 + kAheadCols, 1);
+#pragma unroll
+        for (int u = 0; u < kAheadCols; ++u)
+          if (j0 + u < m) {
+            const double xj = reg_get<R>(xs, j0 + u);
+#pragma unroll
+            for (int s = 0; s < R; ++s) res[s] = fma(-c[u][s], xj, res[s]);
+          }
+#pragma unroll
+        for (int u = 0; u < kAheadCols; ++u)
+#pragma unroll
+          for (int s = 0; s < R; ++s) c[u][s] = nx[u][s];
       }
-      __syncwarp();
-      warp_lu_solve(L, m, pv, rs);
-      for (int k = lane; k < m; k += 32) xs[k] += (double)rs[k];
-      __syncwarp();
+      // into the factors' row order: element perm[s] of the residual
+      float rf[R];
+#pragma unroll
+      for (int s = 0; s < R; ++s) rf[s] = (float)res[s];
+#pragma unroll
+      for (int s = 0; s < R; ++s) {
+        r[s] = __shfl_sync(0xffffffffu, rf[0], perm[s] & 31);
+#pragma unroll
+        for (int q = 1; q < R; ++q) {
+          const float t = __shfl_sync(0xffffffffu, rf[q], perm[s] & 31);
+          if ((perm[s] >> 5) == q) r[s] = t;
+        }
+      }
+      reg_lu_solve<R>(L, m, lane, rd, r);
+#pragma unroll
+      for (int s = 0; s < R; ++s) xs[s] += (double)r[s];
     }
-    for (int k = lane; k < m; k += 32) x[(size_t)s * m + k] = xs[k];
-    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < R; ++s)
+      if (lane + 32 * s < m) x[(size_t)sys * m + lane + 32 * s] = xs[s];
   }
 }
 
-int grid_for(int n)
+int grid_for(int n, int per_cta, int ctas_per_sm)
 {
   int dev, nsm;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long need = ((long long)n + kWarpsPerCta - 1) / kWarpsPerCta;
-  return (int)std::max<long long>(1, std::min<long long>(need, (long long)nsm * 8));
+  const long long need = ((long long)n + per_cta - 1) / per_cta;
+  return (int)std::max<long long>(1, std::min<long long>(need, (long long)nsm * ctas_per_sm));
+}
+
+template <typename F>
+int launch_lu(int n, int m, const double *J, const double *gamma_h, double *out_A, F *out_lu, int *out_piv,
+              int *out_info, cudaStream_t st)
+{
+  const size_t smem = lu_smem<F>(m);
+  try {
+    ensure_dynamic_smem((const void *)lu_kernel<F>, smem);
+  } catch (sf_error &e) {
+    set_error(e.what());
+    return e.code;
+  }
+  // as many CTAs as the shared memory holds (233,472 bytes per SM, 1 KB of it per CTA), at most 10
+  const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(10, 233472 / (smem + 1024)));
+  lu_kernel<F><<<grid_for(n, kWarpsPerCta, per_sm), 32 * kWarpsPerCta, smem, st>>>(n, m, J, gamma_h, out_A, out_lu,
+                                                                                   out_piv, out_info);
+  return SF_OK;
+}
+
+template <int R>
+void launch_solve(int n, int m, const double *A, const void *lu, const int *piv, int precision, int refine,
+                  const double *b, double *out_x, cudaStream_t st)
+{
+  const int grid = grid_for(n, kSolveWarps, 8);
+  if (precision == 0)
+    solve64_kernel<R><<<grid, 32 * kSolveWarps, 0, st>>>(n, m, (const double *)lu, piv, b, out_x);
+  else
+    solve32_kernel<R><<<grid, 32 * kSolveWarps, 0, st>>>(n, m, A, (const float *)lu, piv, refine, b, out_x);
 }
 
 }  // namespace
@@ -156,27 +334,10 @@ int sf_newton_lu_batch(int n, int m, const double *J, const double *gamma_h, int
   }
   if (n == 0) return SF_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t mm = (size_t)m * m;
-  if (precision == 0) {
-    const size_t smem = kWarpsPerCta * (mm * 8 + m * 4);
-    try {
-      ensure_dynamic_smem((const void *)lu64_kernel, smem);
-    } catch (sf_error &e) {
-      set_error(e.what());
-      return e.code;
-    }
-    lu64_kernel<<<grid_for(n), 32 * kWarpsPerCta, smem, st>>>(n, m, J, gamma_h, out_A, (double *)out_lu, out_piv,
-                                                              out_info);
-  } else if (precision == 1) {
-    const size_t smem = kWarpsPerCta * (mm * 4 + m * 4);
-    try {
-      ensure_dynamic_smem((const void *)lu32_kernel, smem);
-    } catch (sf_error &e) {
-      set_error(e.what());
-      return e.code;
-    }
-    lu32_kernel<<<grid_for(n), 32 * kWarpsPerCta, smem, st>>>(n, m, J, gamma_h, out_A, (float *)out_lu, out_piv,
-                                                              out_info);
+  if (precision == 0 || precision == 1) {
+    const int rc = precision == 0 ? launch_lu<double>(n, m, J, gamma_h, out_A, (double *)out_lu, out_piv, out_info, st)
+                                  : launch_lu<float>(n, m, J, gamma_h, out_A, (float *)out_lu, out_piv, out_info, st);
+    if (rc != SF_OK) return rc;
   } else {
     set_error("sf_newton_lu_batch: precision must be 0 or 1");
     return SF_ERR_INVALID_ARGUMENT;
@@ -198,30 +359,17 @@ int sf_newton_solve_batch(int n, int m, const double *A, const void *lu, const i
   }
   if (n == 0) return SF_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t mm = (size_t)m * m;
-  if (precision == 0) {
-    const size_t smem = kWarpsPerCta * ((mm + m) * 8 + m * 4);
-    try {
-      ensure_dynamic_smem((const void *)solve64_kernel, smem);
-    } catch (sf_error &e) {
-      set_error(e.what());
-      return e.code;
-    }
-    solve64_kernel<<<grid_for(n), 32 * kWarpsPerCta, smem, st>>>(n, m, (const double *)lu, piv, b, out_x);
-  } else if (precision == 1) {
-    if (!A) {
+  if (precision == 0 || precision == 1) {
+    if (precision == 1 && !A) {
       set_error("sf_newton_solve_batch: precision 1 needs A");
       return SF_ERR_INVALID_ARGUMENT;
     }
-    const size_t per = mm / 2 + 2 * (size_t)m + 2;
-    const size_t smem = kWarpsPerCta * (per * 8 + m * 4);
-    try {
-      ensure_dynamic_smem((const void *)solve32_kernel, smem);
-    } catch (sf_error &e) {
-      set_error(e.what());
-      return e.code;
-    }
-    solve32_kernel<<<grid_for(n), 32 * kWarpsPerCta, smem, st>>>(n, m, A, (const float *)lu, piv, refine, b, out_x);
+    if (m <= 32)
+      launch_solve<1>(n, m, A, lu, piv, precision, refine, b, out_x, st);
+    else if (m <= 64)
+      launch_solve<2>(n, m, A, lu, piv, precision, refine, b, out_x, st);
+    else
+      launch_solve<3>(n, m, A, lu, piv, precision, refine, b, out_x, st);
   } else {
     set_error("sf_newton_solve_batch: precision must be 0 or 1");
     return SF_ERR_INVALID_ARGUMENT;
