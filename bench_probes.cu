@@ -13,8 +13,8 @@
 //                     the DFMA rate if the two share one FP64 unit, about twice it if they issue side by side
 //
 //   bench_exp         e^x throughput in register loops (8 blocks of 256 threads per SM, four independent sums per
-//                     thread): 0 the loop alone, 1 CUDA's exp, 2 the library's table-driven tab_exp
-//                     (spitfire_gb300/csrc/chem_device.cuh); the caller turns the times into FP64 instructions per call
+//                     thread): 0 the loop alone, 1 CUDA's exp, 2 the library's fixed-point fix_exp
+//                     (spitfire_gb300/csrc/chem_device.cuh), 3 its FP64 table-driven tab_exp; the caller turns the times into FP64 instructions per call
 //                     with the issue rate of bench_fp64_fma
 //   bench_exp_values  both exponentials of n device values, for their accuracy against a wider reference
 //
@@ -35,20 +35,22 @@
 
 namespace {
 
-__constant__ double cExpTab[128];  // sfgb::kExpTable, copied by exp_table_ready()
+__constant__ double cExpTab[384];  // sfgb::kExpTable, then kFixExpTable, copied by exp_table_ready()
 
 int exp_table_ready()
 {
   static bool done = false;
-  if (!done && cudaMemcpyToSymbol(cExpTab, sfgb::kExpTable, sizeof(sfgb::kExpTable)) == cudaSuccess) done = true;
+  if (!done && cudaMemcpyToSymbol(cExpTab, sfgb::kExpTable, sizeof(sfgb::kExpTable)) == cudaSuccess &&
+      cudaMemcpyToSymbol(cExpTab, sfgb::kFixExpTable, sizeof(sfgb::kFixExpTable), sizeof(sfgb::kExpTable)) == cudaSuccess)
+    done = true;
   return done ? 0 : 1;
 }
 
 template <int WHICH>
 __global__ void __launch_bounds__(256) exp_probe_kernel(int iters, double x0, double dx, double *sink)
 {
-  __shared__ __align__(16) double tab[128];
-  if (threadIdx.x < 128) tab[threadIdx.x] = cExpTab[threadIdx.x];
+  __shared__ __align__(16) double tab[384];
+  for (int k = threadIdx.x; k < 384; k += blockDim.x) tab[k] = cExpTab[k];
   __syncthreads();
   double x = x0 - 40. * (double)((blockIdx.x * blockDim.x + threadIdx.x) & 1023) / 1024.;
   double a0 = 0., a1 = 0., a2 = 0., a3 = 0.;
@@ -57,6 +59,9 @@ __global__ void __launch_bounds__(256) exp_probe_kernel(int iters, double x0, do
       a0 += x; a1 += x + dx; a2 += x + 2. * dx; a3 += x + 3. * dx;
     } else if (WHICH == 1) {
       a0 += exp(x); a1 += exp(x + dx); a2 += exp(x + 2. * dx); a3 += exp(x + 3. * dx);
+    } else if (WHICH == 2) {
+      a0 += sfgb::fix_exp(x, tab); a1 += sfgb::fix_exp(x + dx, tab);
+      a2 += sfgb::fix_exp(x + 2. * dx, tab); a3 += sfgb::fix_exp(x + 3. * dx, tab);
     } else {
       a0 += sfgb::tab_exp(x, tab); a1 += sfgb::tab_exp(x + dx, tab);
       a2 += sfgb::tab_exp(x + 2. * dx, tab); a3 += sfgb::tab_exp(x + 3. * dx, tab);
@@ -69,12 +74,12 @@ __global__ void __launch_bounds__(256) exp_probe_kernel(int iters, double x0, do
 
 __global__ void exp_values_kernel(const double *x, double *oc, double *ot, long long n)
 {
-  __shared__ __align__(16) double tab[128];
-  if (threadIdx.x < 128) tab[threadIdx.x] = cExpTab[threadIdx.x];
+  __shared__ __align__(16) double tab[384];
+  for (int k = threadIdx.x; k < 384; k += blockDim.x) tab[k] = cExpTab[k];
   __syncthreads();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     oc[i] = exp(x[i]);
-    ot[i] = sfgb::tab_exp(x[i], tab);
+    ot[i] = sfgb::fix_exp(x[i], tab);
   }
 }
 
@@ -280,10 +285,10 @@ int bench_fp64_mixed(int iters, double *out_tflops, double *sink, void *stream)
   return 0;
 }
 
-// Milliseconds of one exp_probe_kernel launch (4 iters exponentials per thread), which = 0, 1, 2 as above.
+// Milliseconds of one exp_probe_kernel launch (4 iters exponentials per thread), which = 0 to 3 as above.
 int bench_exp(int which, int iters, double *out_ms, double *sink, void *stream)
 {
-  if (which < 0 || which > 2 || iters < 1 || !out_ms || !sink) return 2;
+  if (which < 0 || which > 3 || iters < 1 || !out_ms || !sink) return 2;
   if (exp_table_ready()) return 1;
   int blocks, threads;
   shape(&blocks, &threads);
@@ -294,6 +299,7 @@ int bench_exp(int which, int iters, double *out_ms, double *sink, void *stream)
     if (which == 0) exp_probe_kernel<0><<<blocks, threads, 0, st>>>(n, -1., 1.e-6, sink);
     if (which == 1) exp_probe_kernel<1><<<blocks, threads, 0, st>>>(n, -1., 1.e-6, sink);
     if (which == 2) exp_probe_kernel<2><<<blocks, threads, 0, st>>>(n, -1., 1.e-6, sink);
+    if (which == 3) exp_probe_kernel<3><<<blocks, threads, 0, st>>>(n, -1., 1.e-6, sink);
   }, &ms);
   *out_ms = ms;
   return rc;

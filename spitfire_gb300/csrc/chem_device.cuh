@@ -382,18 +382,102 @@ __device__ __forceinline__ double tab_exp(double x, const double *tab)
   return exp_finish(x, t.x + fma(t.x, p, t.y), N);
 }
 
+// ----------------------------------------------------------------------------- fixed-point exponential
+// e^x on the integer pipes. A warp FP64 instruction takes its scheduler's FP64 unit 76 cycles, an integer multiply-add
+// 2 to 5, so that tab_exp above (11.7 FP64 instructions) costs about 890 cycles of the unit that bounds these kernels
+// and the form below about 200 issue slots that the scheduler otherwise leaves empty. The method is the same
+// (Tang's table plus polynomial), in fixed point:
+//   y = x log2(e) = N + f with f in [0, 1) as a 64-bit fraction, from the 53-bit mantissa of x times log2(e) to 96 bits;
+//   2^f = T_j (1 + p): T_j = 2^(j/256) to 64 bits, j the leading 8 bits of f, and 256 p = W(v) = v (c1 + v (c2 + ...)),
+//   v the other 56 bits as a fraction. The terms shrink by 2^-8 each, so c3 .. c5 need only 32-bit products.
+// The 64-bit result is within 20 units of 2^-63 before it is rounded: at most 0.51 ulp like tab_exp, NaN and |x| >= 708
+// go to tab_exp. tab: the 128 doubles of tab_exp's table, then the 256 words of 2^(j/256).
+
+// High 64 bits of a b without the product of the low words (within 3 units).
+__device__ __forceinline__ unsigned long long fix_mulhi(unsigned long long a, unsigned long long b)
+{
+  const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a, bh = (unsigned)(b >> 32), bl = (unsigned)b;
+  return (unsigned long long)ah * bh + ((unsigned long long)__umulhi(ah, bl) + __umulhi(al, bh));
+}
+
+// x log2(e) = N + f 2^-64 for |x| < 1024
+__device__ __forceinline__ void fix_reduce(double x, int &N, unsigned long long &f)
+{
+  typedef unsigned long long u64;
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const unsigned m1 = ((((unsigned)hi & 0xfffffu) | 0x100000u) << 11) | (lo >> 21), m0 = lo << 11;
+  // the leading 96 bits of the 64 x 96 bit product
+  const u64 t1 = (u64)m0 * kFixLog2e1;
+  const u64 t2 = (u64)m1 * kFixLog2e0 + (unsigned)t1;
+  const u64 t3 = (u64)m1 * kFixLog2e1 + (unsigned)(t1 >> 32);
+  const u64 t4 = (u64)m0 * kFixLog2e2 + (unsigned)t3;
+  const u64 s2 = (u64)(unsigned)t4 + (unsigned)(t2 >> 32);
+  const u64 t5 = (u64)m1 * kFixLog2e2 + ((u64)(unsigned)(t3 >> 32) + (unsigned)(t4 >> 32) + (unsigned)(s2 >> 32));
+  const unsigned p2 = (unsigned)(t5 >> 32), p1 = (unsigned)t5, p0 = (unsigned)s2;
+  // shifted right by 30 - exponent (21 to 95) bits: 32 integer bits above 64 fraction bits
+  int sh = 30 + 1023 - ((hi >> 20) & 0x7ff);
+  sh = sh > 95 ? 95 : sh;
+  const bool q1 = sh >= 32, q2 = sh >= 64;
+  const unsigned w2 = q1 ? 0u : p2, w1 = q2 ? 0u : (q1 ? p2 : p1), w0 = q2 ? p2 : (q1 ? p1 : p0);
+  const unsigned f0 = __funnelshift_r(w0, w1, sh), f1 = __funnelshift_r(w1, w2, sh), n = w2 >> (sh & 31);
+  f = ((u64)f1 << 32) | f0;
+  N = (int)n;
+  if (hi < 0) {  // -(N + f) = (-N - 1) + (1 - f), or -N when f = 0
+    N = f ? ~N : -N;
+    f = 0ull - f;
+  }
+}
+
+// 2^(f 2^-64) 2^63
+__device__ __forceinline__ unsigned long long fix_exp2(unsigned long long f, const unsigned long long *tab)
+{
+  typedef unsigned long long u64;
+  const u64 T = tab[(unsigned)(f >> 56)];
+  const u64 v = f << 8;
+  const unsigned vh = (unsigned)(v >> 32);
+  const unsigned a4 = (unsigned)kFixC4 + __umulhi(vh, (unsigned)kFixC5);
+  const unsigned a3 = (unsigned)kFixC3 + __umulhi(vh, a4);
+  const u64 a2 = kFixC2 + (((u64)vh * a3) >> 20);
+  const u64 W = fix_mulhi(v, kFixC1 + fix_mulhi(v, a2));
+  return T + (fix_mulhi(T, W) >> 8);
+}
+
+// R 2^-63 2^N, R in [2^63, 2^64), rounded to nearest, as a normal double
+__device__ __forceinline__ double fix_to_double(unsigned long long R, int N)
+{
+  const unsigned long long m = (R >> 11) + ((unsigned)(R >> 10) & 1u);  // 53 bits; the leading one adds to the exponent
+  return __longlong_as_double((long long)(m + ((unsigned long long)(unsigned)(N + 1022) << 52)));
+}
+
+__device__ __forceinline__ double fix_exp(double x, const double *tab)
+{
+  if ((((unsigned)__double2hiint(x)) & 0x7fffffffu) >= 0x40862000u) return tab_exp(x, tab);  // |x| >= 708 or NaN
+  int N;
+  unsigned long long f;
+  fix_reduce(x, N, f);
+  return fix_to_double(fix_exp2(f, reinterpret_cast<const unsigned long long *>(tab + 128)), N);
+}
+
 // exp(-g/RT) of one species as m 2^k, formed once per state so that the equilibrium factor of every reversible
 // reaction, exp(-sum_i nu_i g_i/RT), becomes a product of mantissas and an exact power-of-two scaling instead of one
-// exponential per reaction. With x = -g/RT = (64 k + j) ln2/64 + r (the reduction of tab_exp):
-//   m = 2^(j/64) e^r in [1, 2) (to rounding), and the reciprocal mantissa 2^(-j/64) e^-r = m^-1 (the factor of a
-//   product: every m^-1 2^-k is e^-x), from the same reduction: 2^(-j/64) = T_(64-j) / 2 for j > 0, and e^r, e^-r
-//   from the even and odd parts of the polynomial, without a division.
-// The power of two stays an integer (k = N >> 6), so any |x| below 2^31 ln2/64 = 2.3e7, where N fits an int, is
-// represented exactly; g/RT of a species is at most a few thousand even at 10 K.
+// exponential per reaction: m = 2^f in [1, 2) with x = -g/RT = (k + f) ln2, and the reciprocal mantissa 2^-f in
+// (0.5, 1] (the factor of a product: every m^-1 2^-k is e^-x) from the same reduction. For |x| >= 1024, which a species
+// reaches only far below 100 K, both come from the FP64 reduction of tab_exp, whose integer N fits |x| up to 2.3e7.
 template <class S>
 __device__ __forceinline__ void store_gibbs_factor(S scr, const ScratchLayout &L, int i, double gRT, const double *tab)
 {
   const double x = -gRT;
+  if ((((unsigned)__double2hiint(x)) & 0x7fffffffu) < 0x40900000u) {
+    const unsigned long long *t2 = reinterpret_cast<const unsigned long long *>(tab + 128);
+    int N;
+    unsigned long long f;
+    fix_reduce(x, N, f);
+    scr[L.gm + i] = fix_to_double(fix_exp2(f, t2), 0);
+    scr[L.gmi + i] = fix_to_double(fix_exp2(0ull - f, t2), f ? -1 : 0);
+    scr[L.gk + i] = __hiloint2double(0, N);
+    return;
+  }
   double r;
   int N;
   exp_parts(x, r, N);
@@ -553,7 +637,7 @@ __device__ __forceinline__ double forward_constant(const DevMech &m, const Blob 
   case 1: return kc[0] * s.T;
   case 2: return kc[0] * (s.T * s.T);
   case 3: return kc[0] * s.invT;
-  default: return kc[0] * tab_exp(fma(kc[1], s.logT, -(kc[2] * s.invT)), b.d + m.d_exptab);
+  default: return kc[0] * fix_exp(fma(kc[1], s.logT, -(kc[2] * s.invT)), b.d + m.d_exptab);
   }
 }
 
@@ -567,19 +651,19 @@ __device__ __forceinline__ double troe_center(const DevMech &m, const Blob &b, c
   Tdfc = 0.;
   if (terms & 1) {
     const double x = s.T * tr[1];
-    const double e = (1. - tr[0]) * tab_exp(x, b.d + m.d_exptab);
+    const double e = (1. - tr[0]) * fix_exp(x, b.d + m.d_exptab);
     fc += e;
     if (JAC) Tdfc = x * e;
   }
   if (terms & 2) {
     const double x = s.T * tr[2];
-    const double e = tr[0] * tab_exp(x, b.d + m.d_exptab);
+    const double e = tr[0] * fix_exp(x, b.d + m.d_exptab);
     fc += e;
     if (JAC) Tdfc = fma(x, e, Tdfc);
   }
   if (terms & 4) {
     const double x = -(s.invT * tr[3]);
-    const double e = tab_exp(x, b.d + m.d_exptab);
+    const double e = fix_exp(x, b.d + m.d_exptab);
     fc += e;
     if (JAC) Tdfc = fma(-x, e, Tdfc);
   }
@@ -628,7 +712,7 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
     } else {
       const int f = b.i[m.i_fall + r];
       const double *kp = b.d + m.d_kp + 3 * f;  // the ratio k0 / kinf as A, b, E/R
-      const double kpf = kp[0] * tab_exp(fma(kp[1], s.logT, -(kp[2] * s.invT)), b.d + m.d_exptab);
+      const double kpf = kp[0] * fix_exp(fma(kp[1], s.logT, -(kp[2] * s.invT)), b.d + m.d_exptab);
       const double pr = kpf * M;
       const double i1 = 1. / (1. + pr), hf = pr * i1;
       const double Tdlogk = fma(kp[2], s.invT, kp[1]);
@@ -652,7 +736,7 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
         const double b2 = bb * bb;
         const double iq = 1. / fma(a, a, b2);
         const double gt = b2 * iq;
-        const double F = tab_exp(gt * lnfc, b.d + m.d_exptab);
+        const double F = fix_exp(gt * lnfc, b.d + m.d_exptab);
         Ctbaf = F * hf;
         if (JAC) {
           const double dlfc = Tdfc / fc;

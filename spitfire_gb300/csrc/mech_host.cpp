@@ -248,8 +248,9 @@ void HostMech::build(const sf_mech_desc *d)
   m.d_smallint = dsec(64);
   for (int k = 0; k < 64; ++k) D[m.d_smallint + k] = k - 32;
   while (D.size() % 2) D.push_back(0.);  // 16-byte boundary: the table is read as (head, tail) pairs
-  m.d_exptab = dsec(128);
+  m.d_exptab = dsec(128 + 256);
   std::copy(kExpTable, kExpTable + 128, D.begin() + m.d_exptab);
+  std::memcpy(&D[m.d_exptab + 128], kFixExpTable, sizeof kFixExpTable);
   m.i_info = isec(nr);
   m.i_orig = isec(nr);
   for (int r = 0; r < nr; ++r) I[m.i_orig + r] = orig_index[r];
