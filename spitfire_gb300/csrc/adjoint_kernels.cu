@@ -42,8 +42,7 @@ __device__ double falloff_factor(const DevMech &m, const Blob &b, const ScratchL
 {
   const double M = third_body(m, b, s, r, scr + L.C);
   const int f = b.i[m.i_fall + r];
-  const double *kp = b.d + m.d_kp + 3 * f;
-  const double pr = kp[0] * fix_exp(fma(kp[1], s.logT, -(kp[2] * s.invT)), b.d + m.d_exptab) * M;
+  const double pr = falloff_ratio(m, b, s, f) * M;
   double fac = pr / (1. + pr);
   if (kind == 4 && pr > 1.e-300) {
     double Tdfc;

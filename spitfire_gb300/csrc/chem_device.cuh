@@ -382,6 +382,21 @@ __device__ __forceinline__ double tab_exp(double x, const double *tab)
   return exp_finish(x, t.x + fma(t.x, p, t.y), N);
 }
 
+// x 2^K, exact unless the result leaves the normal range; |K| beyond 2044 already takes any factor of a rate
+// expression to 0 or infinity. A normal x whose result is normal has K added to its exponent field.
+__device__ __forceinline__ double scale_pow2(double x, long long K)
+{
+  const int e = (__double2hiint(x) >> 20) & 0x7ff;
+  const int k = (int)(K < -4096 ? -4096 : (K > 4096 ? 4096 : K));
+  if ((unsigned)(e - 1) < 2046u && (unsigned)(e + k - 1) < 2046u)
+    return __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
+  const int kc = k < -2044 ? -2044 : (k > 2046 ? 2046 : k);
+  const int k1 = kc / 2, k2 = kc - k1;  // both within [-1022, 1023]
+  const double f1 = __longlong_as_double((long long)(k1 + 1023) << 52);
+  const double f2 = __longlong_as_double((long long)(k2 + 1023) << 52);
+  return x * f1 * f2;
+}
+
 // ----------------------------------------------------------------------------- fixed-point exponential
 // e^x on the integer pipes. A warp FP64 instruction takes its scheduler's FP64 unit 76 cycles, an integer multiply-add
 // 2 to 5, so that tab_exp above (11.7 FP64 instructions) costs about 890 cycles of the unit that bounds these kernels
@@ -400,7 +415,7 @@ __device__ __forceinline__ unsigned long long fix_mulhi(unsigned long long a, un
   return (unsigned long long)ah * bh + ((unsigned long long)__umulhi(ah, bl) + __umulhi(al, bh));
 }
 
-// x log2(e) = N + f 2^-64 for |x| < 1024
+// x log2(e) = N + f 2^-64 for |x| < 2^20
 __device__ __forceinline__ void fix_reduce(double x, int &N, unsigned long long &f)
 {
   typedef unsigned long long u64;
@@ -415,7 +430,7 @@ __device__ __forceinline__ void fix_reduce(double x, int &N, unsigned long long 
   const u64 s2 = (u64)(unsigned)t4 + (unsigned)(t2 >> 32);
   const u64 t5 = (u64)m1 * kFixLog2e2 + ((u64)(unsigned)(t3 >> 32) + (unsigned)(t4 >> 32) + (unsigned)(s2 >> 32));
   const unsigned p2 = (unsigned)(t5 >> 32), p1 = (unsigned)t5, p0 = (unsigned)s2;
-  // shifted right by 30 - exponent (21 to 95) bits: 32 integer bits above 64 fraction bits
+  // shifted right by 30 - exponent (at most 95) bits: 32 integer bits above 64 fraction bits
   int sh = 30 + 1023 - ((hi >> 20) & 0x7ff);
   sh = sh > 95 ? 95 : sh;
   const bool q1 = sh >= 32, q2 = sh >= 64;
@@ -459,54 +474,69 @@ __device__ __forceinline__ double fix_exp(double x, const double *tab)
   return fix_to_double(fix_exp2(f, reinterpret_cast<const unsigned long long *>(tab + 128)), N);
 }
 
-// exp(-g/RT) of one species as m 2^k, formed once per state so that the equilibrium factor of every reversible
-// reaction, exp(-sum_i nu_i g_i/RT), becomes a product of mantissas and an exact power-of-two scaling instead of one
-// exponential per reaction: m = 2^f in [1, 2) with x = -g/RT = (k + f) ln2, and the reciprocal mantissa 2^-f in
-// (0.5, 1] (the factor of a product: every m^-1 2^-k is e^-x) from the same reduction. For |x| >= 1024, which a species
-// reaches only far below 100 K, both come from the FP64 reduction of tab_exp, whose integer N fits |x| up to 2.3e7.
-template <class S>
-__device__ __forceinline__ void store_gibbs_factor(S scr, const ScratchLayout &L, int i, double gRT, const double *tab)
+// Logarithms to base 2 in fixed point: 32 integer bits (signed) over 64 fraction bits. A rate constant is kept as its
+// logarithm until the one fix_exp2 that forms it: log2 k = log2 A + b log2 T - (E/R) log2(e) / T, and the reverse
+// constant's logarithm adds the species' -g/RT log2(e), so that the two constants of a reaction take no FP64 instruction
+// (8 before, with the exponential already in fixed point). Sums wrap only beyond 2^31, far outside the range of doubles.
+struct Fix96 {
+  unsigned f0, f1;
+  int n;
+};
+__device__ __forceinline__ Fix96 fix96(int n, unsigned long long f) { return Fix96{(unsigned)f, (unsigned)(f >> 32), n}; }
+__device__ __forceinline__ Fix96 operator+(Fix96 a, Fix96 b)
 {
-  const double x = -gRT;
-  if ((((unsigned)__double2hiint(x)) & 0x7fffffffu) < 0x40900000u) {
-    const unsigned long long *t2 = reinterpret_cast<const unsigned long long *>(tab + 128);
+  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+      : "+r"(a.f0), "+r"(a.f1), "+r"(a.n)
+      : "r"(b.f0), "r"(b.f1), "r"(b.n));
+  return a;
+}
+__device__ __forceinline__ Fix96 operator-(Fix96 a, Fix96 b)
+{
+  asm("sub.cc.u32 %0, %0, %3;\n\tsubc.cc.u32 %1, %1, %4;\n\tsubc.u32 %2, %2, %5;"
+      : "+r"(a.f0), "+r"(a.f1), "+r"(a.n)
+      : "r"(b.f0), "r"(b.f1), "r"(b.n));
+  return a;
+}
+
+// a b 2^-32 2^-SHIFT as a Fix96 (SHIFT 1 to 31) for 64-bit a, b; the dropped bits are below the result's last one.
+template <int SHIFT>
+__device__ __forceinline__ Fix96 fix_product(unsigned long long a, unsigned long long b)
+{
+  typedef unsigned long long u64;
+  const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a, bh = (unsigned)(b >> 32), bl = (unsigned)b;
+  const u64 t2 = (u64)ah * bl + __umulhi(al, bl);
+  const u64 t3 = (u64)al * bh + (unsigned)t2;
+  const u64 t4 = (u64)ah * bh + ((u64)(unsigned)(t2 >> 32) + (unsigned)(t3 >> 32));
+  const unsigned p1 = (unsigned)t3, p2 = (unsigned)t4, p3 = (unsigned)(t4 >> 32);
+  return Fix96{__funnelshift_r(p1, p2, SHIFT), __funnelshift_r(p2, p3, SHIFT), (int)(p3 >> SHIFT)};
+}
+
+// 2^y as a double, 0 or infinity beyond its range
+__device__ __forceinline__ double fix96_exp2(Fix96 y, const unsigned long long *tab)
+{
+  const unsigned long long R = fix_exp2(((unsigned long long)y.f1 << 32) | y.f0, tab);
+  if ((unsigned)(y.n + 1022) < 2045u) return fix_to_double(R, y.n);
+  return scale_pow2(fix_to_double(R, 0), y.n);
+}
+
+// The species' contribution to the reverse constants, formed once per state: x = -g/RT as x log2(e) in fixed point
+// (fraction in gm, integer part in gk). A state whose temperature is outside the fixed-point range keeps x itself.
+template <class S>
+__device__ __forceinline__ void store_gibbs_factor(S scr, const ScratchLayout &L, int i, double gRT, bool fixed)
+{
+  double x = -gRT;
+  if (fixed) {
     int N;
     unsigned long long f;
     fix_reduce(x, N, f);
-    scr[L.gm + i] = fix_to_double(fix_exp2(f, t2), 0);
-    scr[L.gmi + i] = fix_to_double(fix_exp2(0ull - f, t2), f ? -1 : 0);
+    if ((((unsigned)__double2hiint(x)) & 0x7fffffffu) >= 0x41300000u) {  // |x| >= 2^20: 0 or infinity in any product
+      N = __double2hiint(x) < 0 ? -(1 << 20) : 1 << 20;
+      f = 0;
+    }
+    x = __longlong_as_double((long long)f);
     scr[L.gk + i] = __hiloint2double(0, N);
-    return;
   }
-  double r;
-  int N;
-  exp_parts(x, r, N);
-  const double r2 = r * r;
-  const double E = r2 * fma(r2, fma(r2, 1. / 720., 1. / 24.), 0.5);          // r^2/2 + r^4/24 + r^6/720
-  const double O = fma(r * r2, fma(r2, 1. / 120., 1. / 6.), r);              // r + r^3/6 + r^5/120
-  const int j = N & 63;
-  const double2 t = reinterpret_cast<const double2 *>(tab)[j];
-  const double2 u = reinterpret_cast<const double2 *>(tab)[(64 - j) & 63];
-  const double ui = j ? 0.5 : 1.;                                             // exact
-  const double ep = O + E, em = E - O;                                        // e^r - 1, e^-r - 1
-  scr[L.gm + i] = t.x + fma(t.x, ep, t.y);
-  scr[L.gmi + i] = ui * (u.x + fma(u.x, em, u.y));
-  scr[L.gk + i] = __hiloint2double(0, N >> 6);
-}
-
-// x 2^K, exact unless the result leaves the normal range; |K| beyond 2044 already takes any factor of a rate
-// expression to 0 or infinity. A normal x whose result is normal has K added to its exponent field.
-__device__ __forceinline__ double scale_pow2(double x, long long K)
-{
-  const int e = (__double2hiint(x) >> 20) & 0x7ff;
-  const int k = (int)(K < -4096 ? -4096 : (K > 4096 ? 4096 : K));
-  if ((unsigned)(e - 1) < 2046u && (unsigned)(e + k - 1) < 2046u)
-    return __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
-  const int kc = k < -2044 ? -2044 : (k > 2046 ? 2046 : k);
-  const int k1 = kc / 2, k2 = kc - k1;  // both within [-1022, 1023]
-  const double f1 = __longlong_as_double((long long)(k1 + 1023) << 52);
-  const double f2 = __longlong_as_double((long long)(k2 + 1023) << 52);
-  return x * f1 * f2;
+  scr[L.gm + i] = x;
 }
 
 // A small integer (a stoichiometric coefficient or a sum of them) as a double: from the blob's table when within
@@ -520,7 +550,9 @@ __device__ __forceinline__ double small_int(const double *table, int k)
 // Per-state quantities every reaction needs.
 struct StateCtx {
   double T, logT, invT, rho, invRho, mmw, invM, ct;
-  double port, invport;  // p_ref / (R T) and its reciprocal
+  double port;  // p_ref / (R T)
+  bool fixed;   // 16 < T < 65536: rate constants in fixed point
+  unsigned long long l60, u68;  // log2 T 2^60, 2^68 / T
   int option;  // rates-sensitivity option: 0 / 2 exact, 1 without third-body/falloff derivatives
 };
 
@@ -628,17 +660,63 @@ __device__ __forceinline__ double special_orders(const DevMech &m, Blob b, int r
   return v;
 }
 
-// Forward rate constant of reaction r (chemistry_kernels.cpp:140-157).
-__device__ __forceinline__ double forward_constant(const DevMech &m, const Blob &b, const StateCtx &s, int r, int kform)
+// The fixed-point terms of a state: log2 T from its logarithm, 1/T.
+__device__ __forceinline__ bool fixed_temperature(double T)
 {
-  const double *kc = b.d + m.d_kf + 3 * r;
+  return __double_as_longlong(T) > 0x4030000000000000ll && __double_as_longlong(T) < 0x40f0000000000000ll;
+}
+__device__ __forceinline__ unsigned long long fixed_log2(double logT)
+{
+  int N;
+  unsigned long long f;
+  fix_reduce(logT, N, f);
+  return ((unsigned long long)(unsigned)N << 60) | (f >> 4);
+}
+__device__ __forceinline__ unsigned long long fixed_reciprocal(double invT)
+{
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(invT);
+  const int e = (int)(bits >> 52);  // 1007 to 1018 for T in range
+  return ((bits & 0xfffffffffffffull) | 0x10000000000000ull) << ((e - 1007) & 15);
+}
+
+// log2 of an Arrhenius expression: w = (fraction of log2 A, b 2^58, (E/R) log2(e) 2^44) and the integer part of log2 A.
+__device__ __forceinline__ Fix96 fixed_arrhenius(const double *w, int n, const StateCtx &s)
+{
+  Fix96 y = fix96(n, (unsigned long long)__double_as_longlong(w[0]));
+  const long long bb = __double_as_longlong(w[1]), ee = __double_as_longlong(w[2]);
+  if (bb) {
+    const Fix96 p = fix_product<22>((unsigned long long)(bb < 0 ? -bb : bb), s.l60);  // 118 - 32 - 22 = 64
+    y = bb < 0 ? y - p : y + p;
+  }
+  if (ee) {
+    const Fix96 p = fix_product<16>((unsigned long long)(ee < 0 ? -ee : ee), s.u68);  // 112 - 32 - 16 = 64
+    y = ee < 0 ? y + p : y - p;
+  }
+  return y;
+}
+
+// Forward rate constant of reaction r (chemistry_kernels.cpp:140-157) in FP64: states and reactions outside the
+// fixed-point ranges.
+static __device__ __noinline__ double forward_constant(const double *kc, const double *tab, double T, double logT, double invT,
+                                                int kform)
+{
   switch (kform) {
   case 0: return kc[0];
-  case 1: return kc[0] * s.T;
-  case 2: return kc[0] * (s.T * s.T);
-  case 3: return kc[0] * s.invT;
-  default: return kc[0] * fix_exp(fma(kc[1], s.logT, -(kc[2] * s.invT)), b.d + m.d_exptab);
+  case 1: return kc[0] * T;
+  case 2: return kc[0] * (T * T);
+  case 3: return kc[0] * invT;
+  default: return kc[0] * fix_exp(fma(kc[1], logT, -(kc[2] * invT)), tab);
   }
+}
+
+// k0 / kinf of falloff reaction f
+__device__ __forceinline__ double falloff_ratio(const DevMech &m, const Blob &b, const StateCtx &s, int f)
+{
+  const int n = b.i[m.i_fixp + f];
+  if (s.fixed && n != kFixNone)
+    return fix96_exp2(fixed_arrhenius(b.d + m.d_fixp + 3 * f, n, s),
+                      reinterpret_cast<const unsigned long long *>(b.d + m.d_exptab + 128));
+  return forward_constant(b.d + m.d_kp + 3 * f, b.d + m.d_exptab, s.T, s.logT, s.invT, 4);
 }
 
 // F_cent of a Troe reaction and, with JAC, T dF_cent/dT. d_troe holds (a, -1/T3, -1/T1, T2).
@@ -699,8 +777,20 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
   const bool has_ord = (info >> RI_ORD_BIT) & 1;
   const auto C = scr + L.C;
   const double *smallint = b.d + m.d_smallint;
-  const double kf = forward_constant(m, b, s, r, (info >> RI_KFORM_SHIFT) & 7);
   const double *kc = b.d + m.d_kf + 3 * r;
+  const unsigned long long *exp2tab = reinterpret_cast<const unsigned long long *>(b.d + m.d_exptab + 128);
+  const int kform = (info >> RI_KFORM_SHIFT) & 7;
+  const int fixn = b.i[m.i_fixn + r];
+  const bool fixed = s.fixed && fixn != kFixNone;
+  Fix96 y;
+  double kf;
+  if (fixed) {
+    y = fixed_arrhenius(b.d + m.d_fix + 3 * r, fixn, s);
+    kf = kform == 0 ? kc[0] : fix96_exp2(y, exp2tab);
+  } else {
+    kf = forward_constant(kc, b.d + m.d_exptab, s.T, s.logT, s.invT, kform);
+    y = fix96(0, 0);
+  }
   const double Tdlogkf = fma(kc[2], s.invT, kc[1]);  // T d ln kf / dT
   // third-body / falloff factor (chemistry_kernels.cpp:158-314; rates_sensitivities_exact.cpp:826-1000); K = dCtbaf/dM
   double Ctbaf = 1., TdCdT = 0., K = 0., M = 0.;
@@ -712,7 +802,7 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
     } else {
       const int f = b.i[m.i_fall + r];
       const double *kp = b.d + m.d_kp + 3 * f;  // the ratio k0 / kinf as A, b, E/R
-      const double kpf = kp[0] * fix_exp(fma(kp[1], s.logT, -(kp[2] * s.invT)), b.d + m.d_exptab);
+      const double kpf = falloff_ratio(m, b, s, f);
       const double pr = kpf * M;
       const double i1 = 1. / (1. + pr), hf = pr * i1;
       const double Tdlogk = fma(kp[2], s.invT, kp[1]);
@@ -773,20 +863,28 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
     }
     // rates of a special-order reaction have no reverse part (chemistry_kernels.cpp:316-326)
     if (rev && !has_ord) {
-      // kr = kf exp(sum_nu ln(p_ref/RT) - sum_i nu_i g_i/RT) (chemistry_kernels.cpp:327-341), with
-      // exp(-g_i/RT) = gm_i 2^gk_i
-      nkr = -kf;
-      if (sum_nu) nkr *= sum_nu > 0 ? ipow(s.port, sum_nu) : ipow(s.invport, -sum_nu);
-      long long Kp = 0;
-      for (int j = n0; j < n1; ++j) {
-        const int e = b.i[m.i_net + j];
-        const int sp = e & 0xFFFF, nu = (e >> 16) - 128;
-        const double mi = scr[(nu > 0 ? L.gm : L.gmi) + sp];
-        const int a = nu > 0 ? nu : -nu;
-        nkr *= a == 1 ? mi : ipow(mi, a);
-        Kp += (long long)nu * __double2loint(scr[L.gk + sp]);
+      // kr = kf exp(sum_nu ln(p_ref/RT) - sum_i nu_i g_i/RT) (chemistry_kernels.cpp:327-341), as logarithms
+      if (s.fixed) {
+        if (sum_nu) {
+          const Fix96 lp = fix96(m.log2_port_n, m.log2_port_f) - fix96((int)(s.l60 >> 60), s.l60 << 4);  // log2(p_ref/RT)
+          for (int j = sum_nu < 0 ? -sum_nu : sum_nu; j > 0; --j) y = sum_nu > 0 ? y + lp : y - lp;
+        }
+        for (int j = n0; j < n1; ++j) {
+          const int e = b.i[m.i_net + j];
+          const int sp = e & 0xFFFF, nu = (e >> 16) - 128;
+          const Fix96 g = fix96(__double2loint(scr[L.gk + sp]), (unsigned long long)__double_as_longlong(scr[L.gm + sp]));
+          for (int q = nu < 0 ? -nu : nu; q > 0; --q) y = nu > 0 ? y + g : y - g;
+        }
+        nkr = -fix96_exp2(y, exp2tab);
+        if (!fixed) nkr *= kf;
+      } else {
+        double x = sum_nu ? (double)sum_nu * log(s.port) : 0.;
+        for (int j = n0; j < n1; ++j) {
+          const int e = b.i[m.i_net + j];
+          x += (double)((e >> 16) - 128) * scr[L.gm + (e & 0xFFFF)];
+        }
+        nkr = -kf * fix_exp(x, b.d + m.d_exptab);
       }
-      nkr = scale_pow2(nkr, Kp);
       if (short_lists) {
         fp = side3<JAC>(pl, npr, C, nkr, smallint);
         nRr = fp.R;

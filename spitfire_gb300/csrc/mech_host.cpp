@@ -21,6 +21,61 @@ namespace sfgb {
 
 static int pack_sp(int s, int hi) { return (s & 0xFFFF) | (hi << 16); }
 
+namespace {
+typedef unsigned long long u64;
+typedef unsigned __int128 u128;
+
+// log2(x) = n + f 2^-64 of a positive normal x, in integers (the same on every host) within 2^-59: x = 2^e m with m in
+// [2^-1/2, 2^1/2), ln m = 2 atanh(z), z = (m - 1) / (m + 1), |z| < 0.172.
+void fixed_log2_of(double x, int *n, u64 *f)
+{
+  int e;
+  double m = std::frexp(x, &e);  // [0.5, 1)
+  if (m < 0.70710678118654752) { m *= 2.; --e; }
+  const bool below = m < 1.;
+  const u64 one = 1ull << 53, mi = (u64)std::ldexp(m, 53);
+  const u64 num = below ? one - mi : mi - one, den = one + mi;
+  const u64 z = (u64)(((u128)num << 64) / den);
+  const u64 z2 = (u64)(((u128)z * z) >> 64);
+  u128 sum = z;
+  u64 term = z;
+  for (int k = 3; term; k += 2) {
+    term = (u64)(((u128)term * z2) >> 64);
+    sum += term / k;
+  }
+  // log2 m = 2 sum log2(e): log2(e) 2^63 rounded
+  const u64 l2e63 = ((u64)kFixLog2e2 << 32) | kFixLog2e1;
+  const u64 l = (u64)((sum * l2e63) >> 62);  // |log2 m| < 1/2 in units of 2^-64
+  *n = e;
+  *f = l;
+  if (below && l) {
+    *f = 0ull - l;
+    --*n;
+  }
+}
+
+// Fixed-point form of A T^b exp(-c/T): false where it has none (A not positive, b or c too large)
+bool fixed_arrhenius_of(const double *k, double *w, int *n)
+{
+  if (!(k[0] > 1e-300 && k[0] < 1e300) || !(std::abs(k[1]) < 31.) || !(std::abs(k[2]) < 7.0e5)) return false;
+  u64 f;
+  fixed_log2_of(k[0], n, &f);
+  const long long b = (long long)std::ldexp(k[1], 58);
+  // |c| log2(e) 2^44 from the 53-bit mantissa of c and log2(e) 2^63
+  int e;
+  const u64 mi = (u64)std::ldexp(std::frexp(std::abs(k[2]), &e), 53);  // |c| = mi 2^(e - 53)
+  const u64 l2e63 = ((u64)kFixLog2e2 << 32) | kFixLog2e1;
+  const int sh = 53 - e + 63 - 44;  // mi l2e63 2^-sh
+  const u128 prod = (u128)mi * l2e63;
+  long long c = sh < 128 ? (long long)((prod + (((u128)1 << sh) >> 1)) >> sh) : 0;
+  if (k[2] < 0.) c = -c;
+  std::memcpy(&w[0], &f, 8);
+  std::memcpy(&w[1], &b, 8);
+  std::memcpy(&w[2], &c, 8);
+  return true;
+}
+}  // namespace
+
 HostMech::~HostMech()
 {
   for (auto &kv : programs) {
@@ -44,7 +99,6 @@ void HostMech::build(const sf_mech_desc *d)
   m.Ru = d->gas_constant;
   m.invRu = 1. / d->gas_constant;
   m.pref = d->ref_pressure;
-  m.ipref = 1. / m.pref;
 
   // ---------------- species
   invmw.resize(ns);
@@ -220,6 +274,11 @@ void HostMech::build(const sf_mech_desc *d)
   }
   m.d_kf = dsec(3 * nr);
   m.d_kp = dsec(3 * n_fall);
+  m.d_fix = dsec(3 * nr);
+  m.d_fixp = dsec(3 * n_fall);
+  m.i_fixn = isec(nr);
+  m.i_fixp = isec(n_fall);
+  fixed_log2_of(m.pref / m.Ru, &m.log2_port_n, &m.log2_port_f);
   m.d_troe = dsec(4 * n_fall);
   m.d_beff = dsec(nr);
   for (int r = 0; r < nr; ++r) {
@@ -228,9 +287,12 @@ void HostMech::build(const sf_mech_desc *d)
     if (x.fall >= 0) {
       D[m.d_kp + 3 * x.fall] = x.kp[0] / x.kf[0];
       for (int j = 1; j < 3; ++j) D[m.d_kp + 3 * x.fall + j] = x.kp[j] - x.kf[j];
+      if (!fixed_arrhenius_of(&D[m.d_kp + 3 * x.fall], &D[m.d_fixp + 3 * x.fall], &I[m.i_fixp + x.fall]))
+        I[m.i_fixp + x.fall] = kFixNone;
       const double tr[4] = {x.troe[0], -1. / x.troe[1], -1. / x.troe[2], x.troe[3]};
       for (int j = 0; j < 4; ++j) D[m.d_troe + 4 * x.fall + j] = tr[j];
     }
+    if (!fixed_arrhenius_of(x.kf, &D[m.d_fix + 3 * r], &I[m.i_fixn + r])) I[m.i_fixn + r] = kFixNone;
     D[m.d_beff + r] = x.beff;
   }
   int ntb = 0, nnet = 0, nord = 0, nslot = 0, nreac = 0, nprod = 0;
@@ -322,7 +384,7 @@ void HostMech::build(const sf_mech_desc *d)
   auto take = [&](int n) { const int r = o; o += (n + 1) & ~1; return r; };
   L.misc = take(16);
   L.y = take(ns); L.C = take(ns); L.eh = take(ns); L.cpv = take(ns); L.w = take(ns);
-  L.gm = take(ns); L.gmi = take(ns); L.gk = take(ns);
+  L.gm = take(ns); L.gk = take(ns);
   L.q = take(nr);
   L.total_rhs = o;
   L.dB = take(ns); L.dcp = take(ns); L.Srho = take(ns); L.ST = take(ns); L.P = take(ns); L.Q = take(ns);

@@ -51,7 +51,7 @@ __device__ __forceinline__ SpeciesSums prep_species(const DevMech &m, const Blob
     const SpeciesThermo th = species_thermo(m, b, i, s.T, s.logT, s.invT, JAC);
     if (gibbs) {
       scr[L.C + i] = yi * s.rho * invmw;
-      store_gibbs_factor(scr, L, i, th.g * (s.invT * m.invRu), b.d + m.d_exptab);
+      store_gibbs_factor(scr, L, i, th.g * (s.invT * m.invRu), s.fixed);
       // gather destinations start at zero: an entry with no contributions (an inert species) is never written
       scr[L.w + i] = 0.;
       if (JAC) {
@@ -109,10 +109,12 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &
     }
     s.ct = s.rho * sim;
     s.port = m.pref * s.invT * m.invRu;
-    s.invport = T * (m.Ru * m.ipref);
+    s.u68 = fixed_reciprocal(s.invT);
   };
+  s.fixed = fixed_temperature(T);
   if constexpr (G <= 32) {
     s.logT = log(T);
+    s.l60 = fixed_log2(s.logT);
     scalars(grp);
   } else {
     double *sh = grp.scalars;
@@ -125,11 +127,15 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &
         sh[3] = s.invRho;
         sh[4] = s.ct;
         sh[5] = s.port;
-        sh[6] = s.invport;
+        sh[6] = __longlong_as_double((long long)s.u68);
       }
     } else if (grp.warp == 1) {
       s.logT = log(T);
-      if (grp.lane == 32) sh[7] = s.logT;
+      s.l60 = fixed_log2(s.logT);
+      if (grp.lane == 32) {
+        sh[7] = s.logT;
+        sh[11] = __longlong_as_double((long long)s.l60);
+      }
     }
     grp.sync();
     s.invT = sh[0];
@@ -138,8 +144,9 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &
     s.invRho = sh[3];
     s.ct = sh[4];
     s.port = sh[5];
-    s.invport = sh[6];
+    s.u68 = (unsigned long long)__double_as_longlong(sh[6]);
     s.logT = sh[7];
+    s.l60 = (unsigned long long)__double_as_longlong(sh[11]);
   }
   return s;
 }

@@ -9,6 +9,7 @@
 namespace sfgb {
 
 constexpr int kMaxSpecies = 1024;   // species indices are stored in 16 bits in the gather programs
+constexpr int kFixNone = 0x7fffffff;  // no fixed-point form of a rate constant
 constexpr int kMaxNet = 8;          // Griffon's NSR (combustion_kernels.h:518)
 
 // per-reaction packed info word (int section, o_info)
@@ -31,13 +32,17 @@ struct DevMech {
   int blob_doubles; // size of the double section
   int blob_ints;    // size of the int section
   int blob_bytes;   // total, multiple of 16
-  double Ru, invRu, pref, ipref;
+  double Ru, invRu, pref;
+  int log2_port_n;                  // log2(pref / Ru) in fixed point: integer part and 64-bit fraction
+  unsigned long long log2_port_f;
 
   // ---- double section offsets ----
   int d_nasa;    // [ns][15] Griffon NASA7 storage (chemistry_setup.cpp:102-130); const-cp: [T0, h0, s0, cp, ...]
   int d_tmin, d_tmax, d_invmw, d_mw, d_u;  // [ns]; u_s = 1/M_s - 1/M_{ns-1}
   int d_kf;      // [nr][3] A, b, Ea/R
   int d_kp;      // [n_fall][3] the ratio k0 / kinf: A0/A, b0 - b, (E0 - E)/R
+  int d_fix;     // [nr][3] fixed-point forward constant: fraction of log2 A, b 2^58, (E/R) log2(e) 2^44 (64-bit words)
+  int d_fixp;    // [n_fall][3] the same of k0 / kinf
   int d_troe;    // [n_fall][4] a, -1/T3, -1/T1, T2
   int d_beff;    // [nr] default third-body efficiency
   int d_tbeff;   // [tb entries] eff - default
@@ -51,6 +56,8 @@ struct DevMech {
 
   // ---- int section offsets ----
   int i_info;    // [nr]
+  int i_fixn;    // [nr] integer part of log2 A, or kFixNone where the constant is outside the fixed-point range
+  int i_fixp;    // [n_fall] the same of k0 / kinf
   int i_orig;    // [nr] index of each device-order reaction in the order the mechanism was described
   int i_sums;    // [nr] sum_nu (low 16 bits, signed) | sum_reac_nu << 16 (8 bits) | sum_prod_nu << 24
   int i_fall;    // [nr] falloff index or -1
@@ -85,8 +92,9 @@ constexpr int GATHER_UNROLL = 8;  // items per batch of the device runner; each 
 // Per-state scratch layout (doubles), shared by every kernel of one mechanism.
 struct ScratchLayout {
   int y, C, dB, eh, cpv, dcp;          // species arrays [ns]
-  int gm, gmi, gk;                     // [ns] exp(-g/RT) = gm * 2^gk (gk an int in the low word), gmi = 1 / gm; dead
-                                       // after the reactions: partial sums of the species gathers
+  int gm, gk;                          // [ns] -g/RT log2(e): 64-bit fraction, and its integer part in the low word (or
+                                       // -g/RT itself in gm); dead after the reactions: partial sums of the species
+                                       // gathers
   int w, Srho, ST, P, Q, trow;         // gather destinations [ns]
   int q, dqdrho, dqdT, E;              // reaction arrays [nr]; dqdrho, dqdT: dead after the species gathers, then
                                        // partial sums of the Jacobian gathers
