@@ -159,7 +159,7 @@ void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pre
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
   int groups = (int)std::min<size_t>(avail / per, (G > 32 ? 512 : 256) / G);
   if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the parameter-adjoint kernel");
-  groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)n_items + nsm - 1) / nsm));
+  groups = balanced_groups(groups, n_items, nsm);
   p.groups_per_cta = groups;
   const size_t smem = hm.dm.blob_bytes + per * groups;
   auto kern = G == 256 ? rate_param_adjoint_kernel<256>

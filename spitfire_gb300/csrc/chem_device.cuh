@@ -760,7 +760,7 @@ __device__ __forceinline__ double third_body(const DevMech &m, const Blob &b, co
 
 // Evaluate reaction r. Always writes its net rate q[r]; with JAC also
 //   dqdrho = rho dq/drho, dqdT = T dq/dT, the sparse slots D_j = dq/dC_j (concentration C = rho Y / M), the dense
-//   coefficients alpha, beta of dq/dY_k / rho = D_k / M_k + alpha u_k + beta, and E = sum_i c_ir e_i.
+//   coefficients alpha, beta of dq/dY_k / rho = D_k / M_k + alpha u_k + beta.
 // The kernels are bound by FP64 instructions, so the scaled forms were chosen for what they leave out: the factors 1/M,
 // 1/rho and 1/T belong to a species or a state and are applied once there (1/M in the gather programs' coefficients),
 // a reaction without a third body multiplies by no such factor, the products of a side are shared by its rate and
@@ -769,7 +769,7 @@ __device__ __forceinline__ double third_body(const DevMech &m, const Blob &b, co
 // factor in place took 110.
 template <bool JAC, class S>
 __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const ScratchLayout &L, S scr,
-                                              const StateCtx &s, int r, double *Eacc_a, double *Eacc_b)
+                                              const StateCtx &s, int r)
 {
   const int info = b.i[m.i_info + r];
   const int kind = (info >> RI_KIND_SHIFT) & 7;
@@ -960,9 +960,6 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
     scr[L.D + j] = v;
   }
   const int di = b.i[m.i_dense + r];
-  double Er = 0.;
-  for (int j = n0; j < n1; ++j) Er = fma(b.d[m.d_netc + j], scr[L.eh + (b.i[m.i_net + j] & 0xFFFF)], Er);
-  scr[L.E + r] = Er;
   if (di >= 0) {
     // closure species ns-1 and third-body terms common to every Y column (all divided by rho)
     double closure = 0.;  // -d (Rf - Rr) / d C_{ns-1}
@@ -994,8 +991,23 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
     beta *= b.d[m.d_invmw + ns - 1];
     scr[L.alpha + di] = alpha;
     scr[L.beta + di] = beta;
-    *Eacc_a = fma(Er, alpha, *Eacc_a);
-    *Eacc_b = fma(Er, beta, *Eacc_b);
+  }
+}
+
+// E_r = sum_i c_ir e_i of reaction r, for the temperature row: after the species gathers, in the place of q. The dense
+// terms' share of the row's sums goes to Ea and Eb.
+template <class S>
+__device__ __forceinline__ void reaction_energy(const DevMech &m, const Blob &b, const ScratchLayout &L, S scr, int r,
+                                                double &Ea, double &Eb)
+{
+  const int n0 = b.i[m.i_net_off + r], n1 = b.i[m.i_net_off + r + 1];
+  double Er = 0.;
+  for (int j = n0; j < n1; ++j) Er = fma(b.d[m.d_netc + j], scr[L.eh + (b.i[m.i_net + j] & 0xFFFF)], Er);
+  scr[L.E + r] = Er;
+  const int di = b.i[m.i_dense + r];
+  if (di >= 0) {
+    Ea = fma(Er, scr[L.alpha + di], Ea);
+    Eb = fma(Er, scr[L.beta + di], Eb);
   }
 }
 

@@ -95,7 +95,7 @@ __device__ __forceinline__ void eval_state(const KParams &p, const DevMech &m, c
   sim = grp.sum(sim);
   const StateCtx s = state_ctx<G>(m, grp, T, rho, sim, 0., true, p.option);
   prep_species<G, JAC>(m, b, L, scr, grp, s, false, MODE == MODE_SENS);
-  reactions_and_gathers<G, JAC>(m, b, L, scr, grp, s, pg);
+  reactions_and_gathers<G, JAC>(m, b, L, scr, grp, s, pg, false);
   if (MODE == MODE_RATES) {
     for (int i = lane; i < ns; i += G) p.out_w[(size_t)st * ns + i] = scr[L.w + i];
     grp.sync();
@@ -136,7 +136,7 @@ __device__ __forceinline__ ReactorCfg cfg_of(const KParams &p)
 }
 
 template <int G, int MODE>
-__global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) chem_kernel(const KParams p)
+__global__ void __launch_bounds__(512, 1) chem_kernel(const KParams p)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t bar;
@@ -215,8 +215,9 @@ size_t tps_scratch_bytes(const HostMech &hm, int mode, long long n)
 // SM holds at once. Measured on 152 SMs (microseconds, GRI-3.0, 53 species / 325 reactions; h2-burke, 11 / 27):
 //   GRI Jacobians   n = 1: 41 with 256 threads, 135 with 32; 608: 90 (128), 88 (64), 139 (32); 2432: 337 (128), 380
 //                   (64), 569 (32); 4864: 652 (64), 668 (128); 65,536: 8,108 (64), 12,266 (32), 9,129 (thread per state)
-//   GRI rates       n = 152: 28 (128), 55 (32); 608: 44 (64), 58 (32); 1216: 75 (64), 83 (32), 90 (16); 4864: 248 (16),
-//                   278 (64), 297 (32); 20,011: 1,049 (8), 1,094 (16); 65,536: 2,961 (8), 3,262 (16)
+//   GRI rates       n = 304: 25 (256), 27 (128), 30 (64); 608: 36 (64), 46 (256), 50 (32); 1216: 53 (64), 63 (32), 75
+//                   (16); 1824: 79 (32), 83 (64), 85 (16); 3040: 109 (16), 134 (32); 20,011: 652 (16), 786 (8), 792
+//                   (32); 65,536: 2,155 (16), 2,291 (8)
 //   h2 Jacobians    n = 1: 33 (64), 40 (16); 1216: 42 (16), 53 (64); 4096: 74 (8), 96 (16); 65,536: 677 (1), 1,063 (8)
 //   h2 rates        n = 1216: 25 (16), 30 (8); 4096: 41 (8), 63 (16); 20,000: 155 (1), 204 (8)
 // The lines lie at the SM count times the states of one SM; thread per state only where the caller's workspace has its
@@ -226,11 +227,19 @@ int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_all
   const long long per_sm = (n + nsm - 1) / nsm;
   if (m.nr >= 96 || m.ns >= 24) {
     if (jac) return per_sm <= 2 ? 256 : (per_sm <= 24 ? 128 : 64);
-    return per_sm <= 1 ? 128 : (per_sm <= 10 ? 64 : (per_sm <= 80 ? 16 : 8));
+    return per_sm <= 2 ? 256 : (per_sm <= 8 ? 64 : (per_sm <= 14 ? 32 : 16));
   }
   if (per_sm <= 2 && jac) return 64;
   if (per_sm <= 16) return 16;
   return per_sm > 100 && tps_allowed ? 1 : 8;
+}
+
+// Groups per block for n items on nsm blocks when `fit` groups fit: the passes that `fit` needs, taken evenly (a last
+// pass with few items would otherwise cost as much as a full one).
+int balanced_groups(int fit, long long n, int nsm)
+{
+  const long long f = std::max(fit, 1), per_sm = std::max<long long>(1, (n + nsm - 1) / nsm), passes = (per_sm + f - 1) / f;
+  return (int)((per_sm + passes - 1) / passes);
 }
 
 // ------------------------------------------------------------------------------------------------ launchers
@@ -291,9 +300,8 @@ int launch_mode(const HostMech &hm, KParams &p, cudaStream_t st, int G_req, void
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
   if ((size_t)smem_max <= (size_t)hm.dm.blob_bytes + per_group)
     throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the shared-memory kernels");
-  int groups = (int)std::min<size_t>(avail / per_group, (G > 32 ? 512 : 256) / G);
-  // no more groups per block than spread the states over all SMs
-  groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)p.n + nsm - 1) / nsm));
+  int groups = (int)std::min<size_t>(avail / per_group, 512 / G);
+  groups = balanced_groups(groups, p.n, nsm);
   p.groups_per_cta = groups;
   const size_t smem = hm.dm.blob_bytes + per_group * groups;
   const int threads = groups * G;

@@ -120,7 +120,7 @@ __device__ __forceinline__ void heat_loss_cfg(const FlmParams &p, const Group<G>
 }
 
 template <int G, bool JAC>
-__global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) flamelet_point_kernel(const FlmParams p)
+__global__ void __launch_bounds__(512, 1) flamelet_point_kernel(const FlmParams p)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint64_t bar;
@@ -756,15 +756,16 @@ int launch_points(HostMech &hm, FlmParams &p, bool jac, cudaStream_t st)
   const int shared = wide_group_doubles(G);
   const size_t per = (size_t)((jac ? hm.sl.total : hm.sl.total_rhs) + hm.dm.ns + 2 + shared) * 8;
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
-  int groups = (int)std::min<size_t>(avail / per, (G > 32 ? 512 : 256) / G);
+  int groups = (int)std::min<size_t>(avail / per, 512 / G);
   if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the flamelet kernels");
-  groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)p.n_points + nsm - 1) / nsm));
+  groups = balanced_groups(groups, p.n_points, nsm);
   p.groups_per_cta = groups;
   const size_t smem = hm.dm.blob_bytes + per * groups;
   void (*k)(const FlmParams);
   switch (G) {
   case 8: k = jac ? flamelet_point_kernel<8, true> : flamelet_point_kernel<8, false>; break;
   case 16: k = jac ? flamelet_point_kernel<16, true> : flamelet_point_kernel<16, false>; break;
+  case 32: k = jac ? flamelet_point_kernel<32, true> : flamelet_point_kernel<32, false>; break;
   case 64: k = jac ? flamelet_point_kernel<64, true> : flamelet_point_kernel<64, false>; break;
   case 128: k = jac ? flamelet_point_kernel<128, true> : flamelet_point_kernel<128, false>; break;
   default: k = jac ? flamelet_point_kernel<256, true> : flamelet_point_kernel<256, false>; break;

@@ -387,9 +387,11 @@ void HostMech::build(const sf_mech_desc *d)
   L.gm = take(ns); L.gk = take(ns);
   L.q = take(nr);
   L.total_rhs = o;
-  L.dB = take(ns); L.dcp = take(ns); L.Srho = take(ns); L.ST = take(ns); L.P = take(ns); L.Q = take(ns);
-  L.trow = take(ns);
-  L.dqdrho = take(nr); L.dqdT = take(nr); L.E = take(nr);
+  L.dB = take(ns); L.dcp = take(ns); L.P = take(ns); L.Q = take(ns);
+  L.dqdrho = take(nr); L.dqdT = take(nr);
+  // arrays that take the place of dead ones: C and dB after the reactions, S_rho after the rho column, q after the
+  // species gathers
+  L.Srho = L.C; L.ST = L.dB; L.trow = L.Srho; L.E = L.q;
   L.alpha = take(n_dense); L.beta = take(n_dense);
   L.D = take(nslot);
   L.total = o;
@@ -583,6 +585,10 @@ void HostMech::build_programs(int G)
     }
     for (Entry *e : {&ew, &er, &et, &ep, &eq}) E[1].push_back(*e);
   }
+  // an entry with no contributions (an inert species) is written as zero
+  for (int k = 0; k < 2; ++k)
+    for (Entry &e : E[k])
+      if (e.items.empty()) e.items.push_back(item(0., L.y));
   // program 2: the Y block (rows/cols 0..ns-2) and the T-row sums; program 3: every species row (the (ns+1)^2
   // sensitivity block of prod_rates_primitive_sensitivities)
   {
@@ -618,7 +624,7 @@ void HostMech::build_programs(int G)
   Programs P;
   for (int k = 0; k < 4; ++k) {
     // partial sums: the Gibbs factors are dead after the reactions, dqdrho and dqdT after the species gathers
-    const int part = k < 2 ? L.gm : L.dqdrho, cap = k < 2 ? L.q - L.gm : L.E - L.dqdrho;
+    const int part = k < 2 ? L.gm : L.dqdrho, cap = k < 2 ? L.q - L.gm : L.alpha - L.dqdrho;
     std::vector<Entry> fix;
     const std::vector<Entry> main = split_entries(E[k], G, part, cap, &fix);
     auto upload = [&](const std::vector<Entry> &entries, int *len) -> const GatherItem * {

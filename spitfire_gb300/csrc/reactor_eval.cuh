@@ -52,14 +52,6 @@ __device__ __forceinline__ SpeciesSums prep_species(const DevMech &m, const Blob
     if (gibbs) {
       scr[L.C + i] = yi * s.rho * invmw;
       store_gibbs_factor(scr, L, i, th.g * (s.invT * m.invRu), s.fixed);
-      // gather destinations start at zero: an entry with no contributions (an inert species) is never written
-      scr[L.w + i] = 0.;
-      if (JAC) {
-        scr[L.Srho + i] = 0.;
-        scr[L.ST + i] = 0.;
-        scr[L.P + i] = 0.;
-        scr[L.Q + i] = 0.;
-      }
     }
     if (caloric) {
       if (want_eh) {
@@ -151,28 +143,38 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &
   return s;
 }
 
-// P2 + P3: reaction rates (and derivatives) and the species gathers. Returns (EA, EB) of the T-row dense terms.
+// The reactions of a group's lanes. In a wide group the last reactions in device order, the falloff ones, cost several
+// times the others: the first warps take those in the first pass, and the last warps start the second.
+template <int G, class F>
+__device__ __forceinline__ void for_reactions(const Group<G> &grp, int nr, F f)
+{
+  if constexpr (G <= 32) {
+    for (int r = grp.lane; r < nr; r += G) f(r);
+  } else {
+    for (int p = 0; p * G < nr; ++p) {
+      const int r = nr - 1 - p * G - ((p & 1) ? G - 1 - grp.lane : grp.lane);
+      if (r >= 0) f(r);
+    }
+  }
+}
+
+// P2 + P3: reaction rates (and derivatives) and the species gathers. energy: also the reactions' E (after the gathers,
+// in the place of their rates) and (EA, EB), the T-row sums of the dense terms.
 template <int G, bool JAC, int U = default_unroll(G), class S>
 __device__ __forceinline__ double2 reactions_and_gathers(const DevMech &m, const Blob &b, const ScratchLayout &L,
                                                          S scr, const Group<G> &grp, const StateCtx &s,
-                                                         const Progs &pg)
+                                                         const Progs &pg, bool energy)
 {
-  double EA = 0., EB = 0.;
-  if constexpr (G <= 32) {
-    for (int r = grp.lane; r < m.nr; r += G) eval_reaction<JAC>(m, b, L, scr, s, r, &EA, &EB);
-  } else {
-    // the last reactions in device order, the falloff ones, cost several times the others: the first warps take
-    // those in the first pass, and the last warps start the second
-    for (int p = 0; p * G < m.nr; ++p) {
-      const int r = m.nr - 1 - p * G - ((p & 1) ? G - 1 - grp.lane : grp.lane);
-      if (r >= 0) eval_reaction<JAC>(m, b, L, scr, s, r, &EA, &EB);
-    }
-  }
-  if (JAC) grp.sum2(EA, EB);
-  if (G <= 32 || !JAC) grp.sync();  // a wide group's reduction has a barrier of its own
+  for_reactions<G>(grp, m.nr, [&](int r) { eval_reaction<JAC>(m, b, L, scr, s, r); });
+  grp.sync();
   NoJ noj;
   run_program<G, U>(JAC ? pg.full : pg.w, grp, scr, L.Q, noj);
   grp.sync();
+  double EA = 0., EB = 0.;
+  if (JAC && energy) {
+    for_reactions<G>(grp, m.nr, [&](int r) { reaction_energy(m, b, L, scr, r, EA, EB); });
+    grp.sum2(EA, EB);
+  }
   return make_double2(EA, EB);
 }
 
@@ -224,7 +226,7 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
     iC = 1. / cmix;
     if ((lane & 31) == 0) grp.scalars[8] = iC;
   }
-  const double2 E = reactions_and_gathers<G, JAC, U>(m, b, L, scr, grp, s, pg);
+  const double2 E = reactions_and_gathers<G, JAC, U>(m, b, L, scr, grp, s, pg, true);
   const double EA = E.x, EB = E.y;
   if constexpr (G > 32) iC = grp.scalars[8];
   const double iRC = iC * invRho;

@@ -78,6 +78,8 @@ void ensure_dynamic_smem(const void *kernel, size_t bytes);
 size_t tps_resident_warps(const HostMech &hm);
 // Threads per state (8 to 256, or 1) of the chemistry kernels for n states when none was set.
 int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_allowed);
+// Groups per block that take n items on nsm blocks in even passes when `fit` groups fit one block.
+int balanced_groups(int fit, long long n, int nsm);
 // sf_reactor_jac_batch with an explicit lane width G (8, 16 or 32; no workspace). Throws sf_error.
 void reactor_jac_lanes(const sf_mech *mech, const sf_reactor_params *rp, int rates_option, int n, const double *q,
                        const double *pressures, double *out_rhs, double *out_jac, int G, cudaStream_t st);

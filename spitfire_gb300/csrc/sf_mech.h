@@ -95,8 +95,8 @@ struct ScratchLayout {
   int gm, gk;                          // [ns] -g/RT log2(e): 64-bit fraction, and its integer part in the low word (or
                                        // -g/RT itself in gm); dead after the reactions: partial sums of the species
                                        // gathers
-  int w, Srho, ST, P, Q, trow;         // gather destinations [ns]
-  int q, dqdrho, dqdT, E;              // reaction arrays [nr]; dqdrho, dqdT: dead after the species gathers, then
+  int w, Srho, ST, P, Q, trow;         // gather destinations [ns]; Srho in the place of C, ST of dB, trow of Srho
+  int q, dqdrho, dqdT, E;              // reaction arrays [nr]; E in the place of q; dqdrho, dqdT: dead after the species gathers, then
                                        // partial sums of the Jacobian gathers
   int alpha, beta;                     // [n_dense]
   int D;                               // [n_slots]
