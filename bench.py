@@ -729,7 +729,8 @@ def build_probes():
     out_dir = os.path.join(ROOT, '_build')
     lib = os.path.join(out_dir, 'libbench_probes.so')
     stamp = lib + '.stamp'
-    deps = [src] + [os.path.join(B.CSRC, f) for f in ('chem_device.cuh', 'exp_table.h', 'sf_mech.h')]
+    deps = [src] + [os.path.join(B.CSRC, f) for f in ('chem_device.cuh', 'fixed_point.cuh', 'exp_table.h',
+                                                  'sf_mech.h')]
     h = hashlib.sha256(b''.join(open(f, 'rb').read() for f in deps) + ' '.join(B.ARCH).encode() +
                        os.uname().machine.encode()).hexdigest()
     if os.path.exists(lib) and os.path.exists(stamp) and open(stamp).read() == h:

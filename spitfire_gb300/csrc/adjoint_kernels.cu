@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) rate_param
         cmix += scr[L.y + i] * scr[L.cpv + i];
       }
       grp.sum2(sim, cmix, ns);
-      const StateCtx s = state_ctx<G>(m, grp, T, isochoric ? qs[0] : 0., sim, pres, isochoric, 0);
-      const double icmix = 1. / cmix;
+      const StateCtx s = state_ctx<G>(m, b, grp, T, isochoric ? qs[0] : 0., sim, pres, isochoric, 0);
+      const double icmix = fix_reciprocal(cmix);
       for (int r = lane; r < nr; r += G) {
         const int info = b.i[m.i_info + r];
         const int kind = (info >> RI_KIND_SHIFT) & 7;

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "exp_table.h"
+#include "fixed_point.cuh"
 #include "sf_mech.h"
 
 namespace sfgb {
@@ -141,17 +142,17 @@ struct Group {
     c = __shfl_sync(mask, r, Q, G);
     d = __shfl_sync(mask, r, H + Q, G);
   }
-  // reciprocals of three values that all lanes hold: one division instruction sequence for all three where the
-  // group has lanes to share it (an FP64 division is about eight FP64 instructions)
+  // reciprocals of three values that all lanes hold: one instruction sequence for all three where the group has lanes
+  // to share it
   __device__ __forceinline__ void recip3(double a, double b, double c, double &ia, double &ib, double &ic) const
   {
     if (G < 4) {
-      ia = 1. / a;
-      ib = 1. / b;
-      ic = 1. / c;
+      ia = fix_reciprocal(a);
+      ib = fix_reciprocal(b);
+      ic = fix_reciprocal(c);
       return;
     }
-    const double r = 1. / (lane == 1 ? b : (lane == 2 ? c : a));
+    const double r = fix_reciprocal(lane == 1 ? b : (lane == 2 ? c : a));
     ia = __shfl_sync(mask, r, 0, G);
     ib = __shfl_sync(mask, r, 1, G);
     ic = __shfl_sync(mask, r, G < 4 ? 0 : 2, G);
@@ -382,89 +383,6 @@ __device__ __forceinline__ double tab_exp(double x, const double *tab)
   return exp_finish(x, t.x + fma(t.x, p, t.y), N);
 }
 
-// x 2^K, exact unless the result leaves the normal range; |K| beyond 2044 already takes any factor of a rate
-// expression to 0 or infinity. A normal x whose result is normal has K added to its exponent field.
-__device__ __forceinline__ double scale_pow2(double x, long long K)
-{
-  const int e = (__double2hiint(x) >> 20) & 0x7ff;
-  const int k = (int)(K < -4096 ? -4096 : (K > 4096 ? 4096 : K));
-  if ((unsigned)(e - 1) < 2046u && (unsigned)(e + k - 1) < 2046u)
-    return __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
-  const int kc = k < -2044 ? -2044 : (k > 2046 ? 2046 : k);
-  const int k1 = kc / 2, k2 = kc - k1;  // both within [-1022, 1023]
-  const double f1 = __longlong_as_double((long long)(k1 + 1023) << 52);
-  const double f2 = __longlong_as_double((long long)(k2 + 1023) << 52);
-  return x * f1 * f2;
-}
-
-// ----------------------------------------------------------------------------- fixed-point exponential
-// e^x on the integer pipes. A warp FP64 instruction takes its scheduler's FP64 unit 76 cycles, an integer multiply-add
-// 2 to 5, so that tab_exp above (11.7 FP64 instructions) costs about 890 cycles of the unit that bounds these kernels
-// and the form below about 200 issue slots that the scheduler otherwise leaves empty. The method is the same
-// (Tang's table plus polynomial), in fixed point:
-//   y = x log2(e) = N + f with f in [0, 1) as a 64-bit fraction, from the 53-bit mantissa of x times log2(e) to 96 bits;
-//   2^f = T_j (1 + p): T_j = 2^(j/256) to 64 bits, j the leading 8 bits of f, and 256 p = W(v) = v (c1 + v (c2 + ...)),
-//   v the other 56 bits as a fraction. The terms shrink by 2^-8 each, so c3 .. c5 need only 32-bit products.
-// The 64-bit result is within 20 units of 2^-63 before it is rounded: at most 0.51 ulp like tab_exp, NaN and |x| >= 708
-// go to tab_exp. tab: the 128 doubles of tab_exp's table, then the 256 words of 2^(j/256).
-
-// High 64 bits of a b without the product of the low words (within 3 units).
-__device__ __forceinline__ unsigned long long fix_mulhi(unsigned long long a, unsigned long long b)
-{
-  const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a, bh = (unsigned)(b >> 32), bl = (unsigned)b;
-  return (unsigned long long)ah * bh + ((unsigned long long)__umulhi(ah, bl) + __umulhi(al, bh));
-}
-
-// x log2(e) = N + f 2^-64 for |x| < 2^20
-__device__ __forceinline__ void fix_reduce(double x, int &N, unsigned long long &f)
-{
-  typedef unsigned long long u64;
-  const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
-  const unsigned m1 = ((((unsigned)hi & 0xfffffu) | 0x100000u) << 11) | (lo >> 21), m0 = lo << 11;
-  // the leading 96 bits of the 64 x 96 bit product
-  const u64 t1 = (u64)m0 * kFixLog2e1;
-  const u64 t2 = (u64)m1 * kFixLog2e0 + (unsigned)t1;
-  const u64 t3 = (u64)m1 * kFixLog2e1 + (unsigned)(t1 >> 32);
-  const u64 t4 = (u64)m0 * kFixLog2e2 + (unsigned)t3;
-  const u64 s2 = (u64)(unsigned)t4 + (unsigned)(t2 >> 32);
-  const u64 t5 = (u64)m1 * kFixLog2e2 + ((u64)(unsigned)(t3 >> 32) + (unsigned)(t4 >> 32) + (unsigned)(s2 >> 32));
-  const unsigned p2 = (unsigned)(t5 >> 32), p1 = (unsigned)t5, p0 = (unsigned)s2;
-  // shifted right by 30 - exponent (at most 95) bits: 32 integer bits above 64 fraction bits
-  int sh = 30 + 1023 - ((hi >> 20) & 0x7ff);
-  sh = sh > 95 ? 95 : sh;
-  const bool q1 = sh >= 32, q2 = sh >= 64;
-  const unsigned w2 = q1 ? 0u : p2, w1 = q2 ? 0u : (q1 ? p2 : p1), w0 = q2 ? p2 : (q1 ? p1 : p0);
-  const unsigned f0 = __funnelshift_r(w0, w1, sh), f1 = __funnelshift_r(w1, w2, sh), n = w2 >> (sh & 31);
-  f = ((u64)f1 << 32) | f0;
-  N = (int)n;
-  if (hi < 0) {  // -(N + f) = (-N - 1) + (1 - f), or -N when f = 0
-    N = f ? ~N : -N;
-    f = 0ull - f;
-  }
-}
-
-// 2^(f 2^-64) 2^63
-__device__ __forceinline__ unsigned long long fix_exp2(unsigned long long f, const unsigned long long *tab)
-{
-  typedef unsigned long long u64;
-  const u64 T = tab[(unsigned)(f >> 56)];
-  const u64 v = f << 8;
-  const unsigned vh = (unsigned)(v >> 32);
-  const unsigned a4 = (unsigned)kFixC4 + __umulhi(vh, (unsigned)kFixC5);
-  const unsigned a3 = (unsigned)kFixC3 + __umulhi(vh, a4);
-  const u64 a2 = kFixC2 + (((u64)vh * a3) >> 20);
-  const u64 W = fix_mulhi(v, kFixC1 + fix_mulhi(v, a2));
-  return T + (fix_mulhi(T, W) >> 8);
-}
-
-// R 2^-63 2^N, R in [2^63, 2^64), rounded to nearest, as a normal double
-__device__ __forceinline__ double fix_to_double(unsigned long long R, int N)
-{
-  const unsigned long long m = (R >> 11) + ((unsigned)(R >> 10) & 1u);  // 53 bits; the leading one adds to the exponent
-  return __longlong_as_double((long long)(m + ((unsigned long long)(unsigned)(N + 1022) << 52)));
-}
-
 __device__ __forceinline__ double fix_exp(double x, const double *tab)
 {
   if ((((unsigned)__double2hiint(x)) & 0x7fffffffu) >= 0x40862000u) return tab_exp(x, tab);  // |x| >= 708 or NaN
@@ -472,51 +390,6 @@ __device__ __forceinline__ double fix_exp(double x, const double *tab)
   unsigned long long f;
   fix_reduce(x, N, f);
   return fix_to_double(fix_exp2(f, reinterpret_cast<const unsigned long long *>(tab + 128)), N);
-}
-
-// Logarithms to base 2 in fixed point: 32 integer bits (signed) over 64 fraction bits. A rate constant is kept as its
-// logarithm until the one fix_exp2 that forms it: log2 k = log2 A + b log2 T - (E/R) log2(e) / T, and the reverse
-// constant's logarithm adds the species' -g/RT log2(e), so that the two constants of a reaction take no FP64 instruction
-// (8 before, with the exponential already in fixed point). Sums wrap only beyond 2^31, far outside the range of doubles.
-struct Fix96 {
-  unsigned f0, f1;
-  int n;
-};
-__device__ __forceinline__ Fix96 fix96(int n, unsigned long long f) { return Fix96{(unsigned)f, (unsigned)(f >> 32), n}; }
-__device__ __forceinline__ Fix96 operator+(Fix96 a, Fix96 b)
-{
-  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
-      : "+r"(a.f0), "+r"(a.f1), "+r"(a.n)
-      : "r"(b.f0), "r"(b.f1), "r"(b.n));
-  return a;
-}
-__device__ __forceinline__ Fix96 operator-(Fix96 a, Fix96 b)
-{
-  asm("sub.cc.u32 %0, %0, %3;\n\tsubc.cc.u32 %1, %1, %4;\n\tsubc.u32 %2, %2, %5;"
-      : "+r"(a.f0), "+r"(a.f1), "+r"(a.n)
-      : "r"(b.f0), "r"(b.f1), "r"(b.n));
-  return a;
-}
-
-// a b 2^-32 2^-SHIFT as a Fix96 (SHIFT 1 to 31) for 64-bit a, b; the dropped bits are below the result's last one.
-template <int SHIFT>
-__device__ __forceinline__ Fix96 fix_product(unsigned long long a, unsigned long long b)
-{
-  typedef unsigned long long u64;
-  const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a, bh = (unsigned)(b >> 32), bl = (unsigned)b;
-  const u64 t2 = (u64)ah * bl + __umulhi(al, bl);
-  const u64 t3 = (u64)al * bh + (unsigned)t2;
-  const u64 t4 = (u64)ah * bh + ((u64)(unsigned)(t2 >> 32) + (unsigned)(t3 >> 32));
-  const unsigned p1 = (unsigned)t3, p2 = (unsigned)t4, p3 = (unsigned)(t4 >> 32);
-  return Fix96{__funnelshift_r(p1, p2, SHIFT), __funnelshift_r(p2, p3, SHIFT), (int)(p3 >> SHIFT)};
-}
-
-// 2^y as a double, 0 or infinity beyond its range
-__device__ __forceinline__ double fix96_exp2(Fix96 y, const unsigned long long *tab)
-{
-  const unsigned long long R = fix_exp2(((unsigned long long)y.f1 << 32) | y.f0, tab);
-  if ((unsigned)(y.n + 1022) < 2045u) return fix_to_double(R, y.n);
-  return scale_pow2(fix_to_double(R, 0), y.n);
 }
 
 // The species' contribution to the reverse constants, formed once per state: x = -g/RT as x log2(e) in fixed point
@@ -660,17 +533,18 @@ __device__ __forceinline__ double special_orders(const DevMech &m, Blob b, int r
   return v;
 }
 
-// The fixed-point terms of a state: log2 T from its logarithm, 1/T.
+// The fixed-point terms of a state: the logarithm of T (natural, and to base 2 in fixed point), 1/T.
 __device__ __forceinline__ bool fixed_temperature(double T)
 {
   return __double_as_longlong(T) > 0x4030000000000000ll && __double_as_longlong(T) < 0x40f0000000000000ll;
 }
-__device__ __forceinline__ unsigned long long fixed_log2(double logT)
+__device__ __forceinline__ double state_log(double T, const unsigned long long *tab, unsigned long long &l60)
 {
-  int N;
-  unsigned long long f;
-  fix_reduce(logT, N, f);
-  return ((unsigned long long)(unsigned)N << 60) | (f >> 4);
+  l60 = 0;
+  if (!fixed_temperature(T)) return log(T);
+  const Fix96 y = fix_log2(T, tab);
+  l60 = ((unsigned long long)(unsigned)y.n << 60) | ((unsigned long long)y.f1 << 28) | (y.f0 >> 4);
+  return fix96_ln(y);
 }
 __device__ __forceinline__ unsigned long long fixed_reciprocal(double invT)
 {
@@ -748,6 +622,12 @@ __device__ __forceinline__ double troe_center(const DevMech &m, const Blob &b, c
   return fc;
 }
 
+// max(x, 1e-300), on the integer pipe
+__device__ __forceinline__ double at_least_tiny(double x)
+{
+  return __double_as_longlong(x) < 0x01a56e1fc2f8f359ll ? 1.e-300 : x;
+}
+
 // Third-body concentration of reaction r: the default efficiency times the total plus the listed excesses.
 template <class SC>
 __device__ __forceinline__ double third_body(const DevMech &m, const Blob &b, const StateCtx &s, int r, const SC &C)
@@ -804,7 +684,7 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
       const double *kp = b.d + m.d_kp + 3 * f;  // the ratio k0 / kinf as A, b, E/R
       const double kpf = falloff_ratio(m, b, s, f);
       const double pr = kpf * M;
-      const double i1 = 1. / (1. + pr), hf = pr * i1;
+      const double i1 = fix_reciprocal(1. + pr), hf = pr * i1;
       const double Tdlogk = fma(kp[2], s.invT, kp[1]);
       if (kind == 3) {
         Ctbaf = hf;
@@ -816,20 +696,20 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
         double Tdfc;
         const double fc = troe_center<JAC>(m, b, s, f, (info >> RI_TROE_SHIFT) & 7, Tdfc);
         constexpr double kLog10e = 0.43429448190325176;
-        const double l10pr = log(fmax(pr, 1.e-300)) * kLog10e;
+        const double l10pr = fix_log(at_least_tiny(pr), exp2tab) * kLog10e;
         // Fc clamped at 1e-300 in the sensitivities (rates_sensitivities_exact.cpp:949-985), not in the rates
         // (chemistry_kernels.cpp:280-312): log10 F = log10 Fc / (1 + (a / bb)^2)
-        const double lnfc = log(JAC ? fmax(fc, 1.e-300) : fc);
+        const double lnfc = fix_log(JAC ? at_least_tiny(fc) : fc, exp2tab);
         const double l10fc = lnfc * kLog10e;
         const double a = l10pr - 0.67 * l10fc - 0.4;
         const double bb = 0.806 - 0.14 * l10pr - 1.1762 * l10fc;
         const double b2 = bb * bb;
-        const double iq = 1. / fma(a, a, b2);
+        const double iq = fix_reciprocal(fma(a, a, b2));
         const double gt = b2 * iq;
         const double F = fix_exp(gt * lnfc, b.d + m.d_exptab);
         Ctbaf = F * hf;
         if (JAC) {
-          const double dlfc = Tdfc / fc;
+          const double dlfc = Tdfc * fix_reciprocal(fc);
           const double c1 = (-2. * kLog10e) * lnfc * (a * bb) * (iq * iq);
           const double p1 = fma(0.14, a, bb) * c1;
           const double TdlnF = fma(gt, dlfc, fma(p1, Tdlogk, -(c1 * (0.67 * bb - 1.1762 * a) * dlfc)));

@@ -93,7 +93,7 @@ __device__ __forceinline__ void eval_state(const KParams &p, const DevMech &m, c
   double sim = 0.;
   for (int i = lane; i < ns; i += G) sim += scr[L.y + i] * b.d[m.d_invmw + i];
   sim = grp.sum(sim);
-  const StateCtx s = state_ctx<G>(m, grp, T, rho, sim, 0., true, p.option);
+  const StateCtx s = state_ctx<G>(m, b, grp, T, rho, sim, 0., true, p.option);
   prep_species<G, JAC>(m, b, L, scr, grp, s, false, MODE == MODE_SENS);
   reactions_and_gathers<G, JAC>(m, b, L, scr, grp, s, pg, false);
   if (MODE == MODE_RATES) {

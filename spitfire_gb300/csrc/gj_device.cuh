@@ -3,24 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
-namespace sfgb {
+#include "fixed_point.cuh"
 
-// 1 / p: two Newton steps from the FP32 reciprocal of the leading 23 mantissa bits, four FP64 instructions (a division
-// takes about nine, and this one stands on the elimination's serial chain); within an ulp. The mantissa goes to FP32 and
-// back and the exponent to the result as integers. Zeros, subnormals and values that are not finite divide.
-__device__ __forceinline__ double rcp_newton(double p)
-{
-  const int hi = __double2hiint(p), lo = __double2loint(p);
-  const int e = (hi >> 20) & 0x7ff;
-  if ((unsigned)(e - 1) >= 2044u) return 1. / p;
-  const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, lo);  // [1, 2)
-  const float f = __frcp_rn(__int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29)));
-  const int fb = __float_as_int(f);
-  double x = __hiloint2double((fb >> 3) + ((1023 - 127) << 20), fb << 29);
-  x = fma(x, fma(-m, x, 1.), x);
-  x = fma(x, fma(-m, x, 1.), x);
-  return __hiloint2double((__double2hiint(x) - ((e - 1023) << 20)) | (hi & 0x80000000), __double2loint(x));
-}
+namespace sfgb {
 
 // Inverse of the n x n row-major matrix in S (leading dimension ld, odd: rows then start in different banks) by
 // Gauss-Jordan elimination with partial pivoting (G. H. Golub and C. F. Van Loan, "Matrix Computations", section 3.2;
@@ -76,7 +61,7 @@ __device__ __forceinline__ double *gj_inverse(double *S, double *D, int n, int l
       }
     }
     const bool zero = ZERO_PIVOT && (__double_as_longlong(pv) << 1) == 0;
-    const double ip = zero ? 0. : rcp_newton(pv);
+    const double ip = zero ? 0. : fix_reciprocal(pv);
     double *f = ws + (j & 1) * n;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {

@@ -55,7 +55,7 @@ __device__ void plain_state(const DevMech &m, const Blob &b, const ScratchLayout
     T = qs[0];
   }
   const Group<1> one;
-  const StateCtx s = state_ctx<1>(m, one, T, rho, sim, pressure, iso, 0);
+  const StateCtx s = state_ctx<1>(m, b, one, T, rho, sim, pressure, iso, 0);
   rho = s.rho;
   const double mmw = s.mmw;
   double cpmix = 0., cpsens = 0.;

@@ -82,9 +82,10 @@ __device__ __forceinline__ SpeciesSums prep_species(const DevMech &m, const Blob
 // Scalars of a state: three reciprocals in one division sequence, everything else products. In a wide group the first
 // warp forms them and the second one the logarithm, for all.
 template <int G>
-__device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &grp, double T, double rho, double sim,
-                                              double pres, bool isochoric, int option)
+__device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Blob &b, const Group<G> &grp, double T,
+                                              double rho, double sim, double pres, bool isochoric, int option)
 {
+  const unsigned long long *exp2tab = reinterpret_cast<const unsigned long long *>(b.d + m.d_exptab + 128);
   StateCtx s;
   s.T = T;
   s.invM = sim;
@@ -105,8 +106,7 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &
   };
   s.fixed = fixed_temperature(T);
   if constexpr (G <= 32) {
-    s.logT = log(T);
-    s.l60 = fixed_log2(s.logT);
+    s.logT = state_log(T, exp2tab, s.l60);
     scalars(grp);
   } else {
     double *sh = grp.scalars;
@@ -122,8 +122,7 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Group<G> &
         sh[6] = __longlong_as_double((long long)s.u68);
       }
     } else if (grp.warp == 1) {
-      s.logT = log(T);
-      s.l60 = fixed_log2(s.logT);
+      s.logT = state_log(T, exp2tab, s.l60);
       if (grp.lane == 32) {
         sh[7] = s.logT;
         sh[11] = __longlong_as_double((long long)s.l60);
@@ -212,7 +211,7 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
   if (lane == 0) scr[L.y + ns - 1] = 1. - sy;
   if (G <= 32) grp.sync();  // else the barrier in state_ctx
   sim += b.d[m.d_invmw + ns - 1];
-  const StateCtx s = state_ctx<G>(m, grp, T, rho, sim, pres, isochoric, c.option);
+  const StateCtx s = state_ctx<G>(m, b, grp, T, rho, sim, pres, isochoric, c.option);
   rho = s.rho;
   const double mmw = s.mmw;
   // ---------------- P1-P3
@@ -221,9 +220,9 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
   const double invRho = s.invRho;
   double iC;
   if constexpr (G <= 32) {
-    iC = 1. / cmix;
+    iC = fix_reciprocal(cmix);
   } else if (grp.warp == Group<G>::W / 2) {  // read after the reactions' barrier
-    iC = 1. / cmix;
+    iC = fix_reciprocal(cmix);
     if ((lane & 31) == 0) grp.scalars[8] = iC;
   }
   const double2 E = reactions_and_gathers<G, JAC, U>(m, b, L, scr, grp, s, pg, true);

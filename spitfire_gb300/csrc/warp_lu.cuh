@@ -32,7 +32,7 @@ __device__ __forceinline__ bool larger_abs(float a, float b)
 {
   return ((unsigned)__float_as_int(a) << 1) > ((unsigned)__float_as_int(b) << 1);
 }
-__device__ __forceinline__ double lu_reciprocal(double p) { return rcp_newton(p); }
+__device__ __forceinline__ double lu_reciprocal(double p) { return fix_reciprocal(p); }
 __device__ __forceinline__ float lu_reciprocal(float p) { return 1.f / p; }
 
 // A[i, j] -= A[i, k] A[k, j] for i, j > k. FP64: the elements are dealt to the lanes in column-major order, so that no
