@@ -17,7 +17,8 @@
 //                     (spitfire_gb300/csrc/chem_device.cuh), 3 its FP64 table-driven tab_exp; the caller turns the times into FP64 instructions per call
 //                     with the issue rate of bench_fp64_fma
 //   bench_exp_values  both exponentials of n device values, for their accuracy against a wider reference
-//   bench_fixed_values  the library's fixed-point exponential, logarithm and reciprocal of n device values
+//   bench_fixed_values  the library's fixed-point exponential, logarithm, reciprocal and reciprocal square root of n
+//                     device values
 //
 //   bench_store       stores from the SMs into a buffer, device memory or pinned host memory reached over the host
 //                     link (the device address of a pinned allocation comes from cudaHostGetDevicePointer, and the
@@ -84,7 +85,7 @@ __global__ void exp_values_kernel(const double *x, double *oc, double *ot, long 
   }
 }
 
-__global__ void fixed_values_kernel(const double *x, double *oe, double *ol, double *orc, long long n)
+__global__ void fixed_values_kernel(const double *x, double *oe, double *ol, double *orc, double *os, long long n)
 {
   __shared__ __align__(16) double tab[384];
   for (int k = threadIdx.x; k < 384; k += blockDim.x) tab[k] = cExpTab[k];
@@ -93,6 +94,7 @@ __global__ void fixed_values_kernel(const double *x, double *oe, double *ol, dou
     oe[i] = sfgb::fix_exp(x[i], tab);
     ol[i] = sfgb::fix_log(x[i], reinterpret_cast<const unsigned long long *>(tab + 128));
     orc[i] = sfgb::fix_reciprocal(x[i]);
+    os[i] = sfgb::fix_rsqrt(x[i]);
   }
 }
 
@@ -298,13 +300,14 @@ int bench_fp64_mixed(int iters, double *out_tflops, double *sink, void *stream)
   return 0;
 }
 
-int bench_fixed_values(const double *x, double *out_exp, double *out_log, double *out_rcp, long long n, void *stream)
+int bench_fixed_values(const double *x, double *out_exp, double *out_log, double *out_rcp, double *out_rsqrt, long long n,
+                       void *stream)
 {
-  if (!x || !out_exp || !out_log || !out_rcp || n < 0) return 2;
+  if (!x || !out_exp || !out_log || !out_rcp || !out_rsqrt || n < 0) return 2;
   if (exp_table_ready()) return 1;
   int blocks, threads;
   shape(&blocks, &threads);
-  fixed_values_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>(x, out_exp, out_log, out_rcp, n);
+  fixed_values_kernel<<<blocks, threads, 0, (cudaStream_t)stream>>>(x, out_exp, out_log, out_rcp, out_rsqrt, n);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

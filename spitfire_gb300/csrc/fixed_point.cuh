@@ -1,4 +1,4 @@
-// Fixed-point arithmetic on the integer pipes: exponential, logarithm and reciprocal of doubles.
+// Fixed-point arithmetic on the integer pipes: exponential, logarithm, reciprocal and reciprocal square root of doubles.
 //
 // A warp FP64 instruction takes its scheduler's FP64 unit 64 to 76 cycles on GB300, an integer multiply-add 2 to 5, and
 // the two pipes run side by side, so that the functions below cost no time in a kernel that the FP64 unit bounds.
@@ -169,6 +169,29 @@ __device__ __forceinline__ double fix_reciprocal(double x)
   const unsigned long long M = ((unsigned long long)__double_as_longlong(x) << 11) | 0x8000000000000000ull;
   const double y = fix_to_double(fix_rcp(M), 1022 - e);
   return __hiloint2double(__double2hiint(y) | (hi & 0x80000000), __double2loint(y));
+}
+
+// 1 / sqrt(x) to within 0.51 ulp, the same way: a 2^(2q) = x with a in [1/4, 1), the FP32 reciprocal square root and two
+// Newton steps y + y (1 - a y^2) / 2. Arguments that are not normal and positive go to rsqrt.
+__device__ __forceinline__ double fix_rsqrt(double x)
+{
+  typedef unsigned long long u64;
+  const int hi = __double2hiint(x);
+  if ((unsigned)(hi - 0x00100000) >= 0x7fe00000u) return rsqrt(x);
+  const u64 M = ((u64)__double_as_longlong(x) << 11) | 0x8000000000000000ull;
+  const int e1 = (hi >> 20) - 1022;  // x = M 2^-64 2^e1
+  const int odd = e1 & 1, q = (e1 + odd) >> 1;
+  const u64 a = M >> odd;
+  const float f = rsqrtf(__int_as_float(((126 - odd) << 23) | (int)((unsigned)(M >> 40) & 0x7fffffu)));
+  const unsigned y0 = __float2uint_rz(f * 2147483648.f);  // saturates at 2^32 - 1
+  const long long d0 = (long long)(0x4000000000000000ull - fix_mulhi(a, (u64)y0 * y0));
+  const long long c0 = (long long)(int)(d0 >> 11) * (int)(y0 >> 1);
+  const u64 s1 = ((u64)y0 << 32) + (u64)(c0 >> 19);
+  const u64 y1 = y0 > 0xff000000u && (s1 >> 63) == 0 ? ~0ull : s1;  // past 2
+  const long long d1 = (long long)(0x4000000000000000ull - fix_mulhi(a, fix_mulhi(y1, y1)));
+  const long long c1 = (long long)(int)d1 * (int)(unsigned)(y1 >> 33);
+  const u64 s2 = y1 + (u64)(c1 >> 30);
+  return fix_to_double(y1 > 0xff00000000000000ull && (s2 >> 63) == 0 ? ~0ull : s2, -q);
 }
 
 // log2 of a normal positive x as a Fix96, within 2^-58.9: from the FP32 logarithm k 2^-24 of the mantissa m by one Newton

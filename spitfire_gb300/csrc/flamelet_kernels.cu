@@ -233,20 +233,31 @@ __global__ void __launch_bounds__(512, 1) flamelet_point_kernel(const FlmParams 
 // enthalpy-flux correction is applied to the block. One warp per point, the block in shared memory. The result is
 // exactly 0 whenever every eigenvalue lies left of d; the scaled-Gershgorin (M-matrix) test proves that for a large
 // share of the points at a small fraction of the QR iteration's cost, which then runs only for the rest.
-__global__ void flamelet_expeig_kernel(int n_points, int nf, int ns, const int *offz, const long long *offv,
+template <int G>
+__global__ void __launch_bounds__(256) flamelet_expeig_kernel(int n_points, int nf, int ns, const int *offz, const long long *offv,
                                        double *values, const double *cmajor, double diffterm,
                                        const double *diffterm_f, const int *active, double *expeig, int *status,
-                                       int warps, int *next_point)
+                                       int *next_point)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double *A = reinterpret_cast<double *>(smem) + (size_t)w * (ns * ns + 2 * ns);
+  const int w = threadIdx.x / G;
+  double *shared = reinterpret_cast<double *>(smem) + (size_t)w * (ns * ns + 2 * ns + Group<G>::kShared);
+  double *A = shared + Group<G>::kShared;
+  const Group<G> g(shared, w);
+  const int lane = g.lane;
   double *work = A + ns * ns;
   // points are taken dynamically (whether a point needs the QR iteration is known only once it is examined)
   for (;;) {
     int pt = 0;
     if (lane == 0) pt = atomicAdd(next_point, 1);
-    pt = __shfl_sync(0xffffffffu, pt, 0);
+    if constexpr (G > 32) {
+      if (lane == 0) g.scalars[0] = (double)pt;
+      g.sync();
+      pt = (int)g.scalars[0];
+      g.sync();
+    } else {
+      pt = __shfl_sync(0xffffffffu, pt, 0);
+    }
     if (pt >= n_points) break;
     const int f = find_flamelet(offz, nf, pt);
     if (active && !active[f]) continue;
@@ -254,27 +265,27 @@ __global__ void flamelet_expeig_kernel(int n_points, int nf, int ns, const int *
     const double d = diffterm_f ? diffterm_f[f] : diffterm;
     double *blk = values + offv[f] + (size_t)iz * ns * ns;
     auto load = [&]() {
-      for (int e = lane; e < ns * ns; e += 32) {
+      for (int e = lane; e < ns * ns; e += G) {
         const int col = e / ns, row = e - col * ns;
         A[e] = blk[e] - (row == col ? cmajor[(size_t)pt * ns + row] : 0.);
       }
-      __syncwarp();
+      g.sync();
     };
     load();
     double mx = d;
     bool ok = true;
-    if (!warp_hmatrix_below(A, ns, d, work)) {
-      __syncwarp();
+    if (!group_hmatrix_below<G>(g, A, ns, d, work)) {
+      g.sync();
       load();
-      ok = warp_max_real_eig(A, ns, work, &mx, d);
+      ok = group_max_real_eig<G>(g, A, ns, work, &mx, d);
     }
     if (!ok && lane == 0) report_error(status, DEVERR_WAIT_TIMEOUT);
     const double corr = expeig[(size_t)pt * ns];
-    __syncwarp();
+    g.sync();
     const double e = fmax(mx - d, 0.);
-    for (int q = lane; q < ns; q += 32) expeig[(size_t)pt * ns + q] = e;
+    for (int q = lane; q < ns; q += G) expeig[(size_t)pt * ns + q] = e;
     if (lane == 0) blk[0] -= corr;
-    __syncwarp();
+    g.sync();
   }
 }
 
@@ -1055,22 +1066,26 @@ int sf_flamelet_jac_batch(const sf_mech *mech, const sf_flamelet_batch *fb, cons
       CUDA_THROW(cudaGetDevice(&dev));
       CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
       CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-      const size_t per = (size_t)(ns * ns + 2 * ns) * 8;
-      const int warps = (int)std::min<size_t>(8, (size_t)smem_max / per);
-      if (warps < 1) throw sf_error(SF_ERR_UNSUPPORTED, "block too large for the eigenvalue kernel");
-      ensure_dynamic_smem((const void *)flamelet_expeig_kernel, per * warps);
+      // Up to two points per SM two warps work on one point (a row or column of a 53 x 53 block is then one pass) and every
+      // point has the FP64 unit of an SM, or half of it, to itself: with eight points per block, 120 points had filled 15
+      // SMs and taken 2.7 ms.
+      const bool two = p.n_points <= 2 * nsm;
+      const size_t per = (size_t)(ns * ns + 2 * ns + (two ? Group<64>::kShared : 0)) * 8;
+      int groups = (int)std::min<size_t>(two ? 2 : 8, (size_t)smem_max / per);
+      if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "block too large for the eigenvalue kernel");
+      groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)p.n_points + nsm - 1) / nsm));
+      const int threads = groups * (two ? 64 : 32);
+      auto kern = two ? flamelet_expeig_kernel<64> : flamelet_expeig_kernel<32>;
+      ensure_dynamic_smem((const void *)kern, per * groups);
       int per_sm = 0;
-      CUDA_THROW(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flamelet_expeig_kernel, 32 * warps,
-                                                               per * warps));
+      CUDA_THROW(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, per * groups));
       const int grid = (int)std::max<long long>(1, std::min<long long>((long long)nsm * std::max(1, per_sm),
-                                                                       ((long long)p.n_points + warps - 1) / warps));
+                                                                       ((long long)p.n_points + groups - 1) / groups));
       // the points are handed out by an atomic counter in the caller's workspace, zeroed on the stream first
       int *counter = static_cast<int *>(workspace);
       CUDA_THROW(cudaMemsetAsync(counter, 0, sizeof(int), st));
-      flamelet_expeig_kernel<<<grid, 32 * warps, per * warps, st>>>(p.n_points, p.n_flamelets, ns, p.offz, p.offv,
-                                                                    out_values, p.cmajor, diffterm, fb->diffterm,
-                                                                    fb->active, out_expeig, hm.d_status, warps,
-                                                                    counter);
+      kern<<<grid, threads, per * groups, st>>>(p.n_points, p.n_flamelets, ns, p.offz, p.offv, out_values, p.cmajor,
+                                                diffterm, fb->diffterm, fb->active, out_expeig, hm.d_status, counter);
       CUDA_THROW(cudaGetLastError());
     }
     return SF_OK;
