@@ -40,13 +40,13 @@ struct AdjParams {
 __device__ double falloff_factor(const DevMech &m, const Blob &b, const ScratchLayout &L, const double *scr,
                                  const StateCtx &s, int r, int kind, int info)
 {
-  const double M = third_body(m, b, s, r, scr + L.C);
+  const double M = third_body<false>(m, b, s, r, scr + L.C);
   const int f = b.i[m.i_fall + r];
   const double pr = falloff_ratio(m, b, s, f) * M;
   double fac = pr / (1. + pr);
   if (kind == 4 && pr > 1.e-300) {
     double Tdfc;
-    const double fc = troe_center<false>(m, b, s, f, (info >> RI_TROE_SHIFT) & 7, Tdfc);
+    const double fc = troe_center<false, false>(m, b, s, f, (info >> RI_TROE_SHIFT) & 7, Tdfc);
     const double lfc = log10(fc);
     const double nn = 0.75 - 1.27 * lfc;
     const double lpc = log10(pr) + (-0.4 - 0.67 * lfc);

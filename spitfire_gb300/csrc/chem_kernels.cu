@@ -110,7 +110,6 @@ __device__ __forceinline__ void eval_state(const KParams &p, const DevMech &m, c
     Sb[n1 + i] = scr[L.ST + i] * s.invT;
   }
   for (int k = lane; k < n1; k += G) Sb[k * n1 + ns] = 0.;
-  grp.sync();
   JWriter<G> jw{Sb, n1, 0, 2, rho};
   run_program<G>(p.prog_j, grp, scr, L.Q, jw);
   grp.sync();
@@ -229,7 +228,7 @@ int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_all
     if (jac) return per_sm <= 2 ? 256 : (per_sm <= 24 ? 128 : 64);
     return per_sm <= 2 ? 256 : (per_sm <= 8 ? 64 : (per_sm <= 14 ? 32 : 16));
   }
-  if (per_sm <= 2 && jac) return 64;
+  if (per_sm <= (jac ? 2 : 4)) return 64;
   if (per_sm <= 16) return 16;
   return per_sm > 100 && tps_allowed ? 1 : 8;
 }

@@ -220,32 +220,34 @@ __device__ __forceinline__ double fix96_ln(Fix96 y)
   typedef unsigned long long u64;
   const bool neg = y.n < 0;
   if (neg) y = Fix96{0u, 0u, 0} - y;
-  // the leading 64 bits of |y|
-  u64 top = ((u64)y.f1 << 32) | y.f0;
-  int e = -1;
-  if (y.n) {
-    const int c = __clz(y.n);
-    top = ((u64)__funnelshift_l(y.f1, (unsigned)y.n, c) << 32) | __funnelshift_l(y.f0, y.f1, c);
-    e = 31 - c;
-  } else {
-    if (!top) return 0.;
-    const int c = __clzll((long long)top);
-    top <<= c;
-    e -= c;
+  // the leading 64 bits of |y|, past up to two zero words (selects, so that two logarithms can run interleaved)
+  unsigned w2 = (unsigned)y.n, w1 = y.f1, w0 = y.f0;
+  int e = 31;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const bool z = w2 == 0;
+    w2 = z ? w1 : w2;
+    w1 = z ? w0 : w1;
+    w0 = z ? 0u : w0;
+    e = z ? e - 32 : e;
   }
+  const int c = __clz((int)w2);
+  const u64 top = ((u64)__funnelshift_l(w1, w2, c) << 32) | __funnelshift_l(w0, w1, c);
+  e -= c;
   u64 R = fix_mulhi(top, 0xb17217f7d1cf79acull);  // ln 2 2^64
   if (!(R >> 63)) {
     R <<= 1;
     --e;
   }
-  const double v = fix_to_double(R, e);
+  const double v = w2 ? fix_to_double(R, e) : 0.;
   return neg ? -v : v;
 }
+__device__ __forceinline__ bool fix_normal(double x) { return (unsigned)(__double2hiint(x) - 0x00100000) < 0x7fe00000u; }
 
 // ln x, absolute error below 2^-58 (and half an ulp); arguments that are not normal and positive go to log.
 __device__ __forceinline__ double fix_log(double x, const unsigned long long *tab)
 {
-  if ((unsigned)(__double2hiint(x) - 0x00100000) >= 0x7fe00000u) return log(x);
+  if (!fix_normal(x)) return log(x);
   return fix96_ln(fix_log2(x, tab));
 }
 

@@ -78,7 +78,7 @@ __device__ void plain_state(const DevMech &m, const Blob &b, const ScratchLayout
     for (int i = 0; i < n1 * n1; ++i) S[i] = 0.;
   for (int i = 0; i < ns; ++i) scr[L.w + i] = 0.;
   for (int r = 0; r < nr; ++r) {
-    eval_reaction<JAC>(m, b, L, scr, s, r);
+    eval_reaction<JAC, false>(m, b, L, scr, s, r);
     if (JAC) {
       // dense dq/dY over all columns
       const int di = b.i[m.i_dense + r];

@@ -164,8 +164,7 @@ __device__ __forceinline__ double2 reactions_and_gathers(const DevMech &m, const
                                                          S scr, const Group<G> &grp, const StateCtx &s,
                                                          const Progs &pg, bool energy)
 {
-  for_reactions<G>(grp, m.nr, [&](int r) { eval_reaction<JAC>(m, b, L, scr, s, r); });
-  grp.sync();
+  for_reactions<G>(grp, m.nr, [&](int r) { eval_reaction<JAC, (G > 32 && !JAC)>(m, b, L, scr, s, r); });
   NoJ noj;
   run_program<G, U>(JAC ? pg.full : pg.w, grp, scr, L.Q, noj);
   grp.sync();
@@ -305,7 +304,6 @@ __device__ void reactor_eval(const DevMech &m, const Blob &b, const ScratchLayou
     }
   }
   for (int k = lane; k < ns; k += G) scr[L.trow + k] = 0.;
-  grp.sync();
 
   // ---------------- P5: Y block (species rows/columns) and T-row sums; an open reactor's feed adds -mfac on the
   // diagonal (rho_in / (tau rho) isochoric, 1 / tau isobaric)
