@@ -600,42 +600,51 @@ __device__ __forceinline__ double troe_center(const DevMech &m, const Blob &b, c
 {
   const double *tr = b.d + m.d_troe + 4 * f;
   const double *tab = b.d + m.d_exptab;
-  const double x[3] = {s.T * tr[1], s.T * tr[2], -(s.invT * tr[3])};
-  double e[3];
-  // PAIR: the three exponentials interleave where all arguments are in the fixed-point range
-  bool in = PAIR;
-  if (PAIR) {
+  double fc = 0.;
+  Tdfc = 0.;
+  if constexpr (PAIR) {  // the three exponentials interleave where all arguments are in the fixed-point range
+    const double x[3] = {s.T * tr[1], s.T * tr[2], -(s.invT * tr[3])};
+    bool in = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k)
       in = in && (!(terms >> k & 1) || (((unsigned)__double2hiint(x[k])) & 0x7fffffffu) < 0x40862000u);
-  }
-  if (in) {
+    if (in) {
+      double e[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      int N;
-      unsigned long long f64;
-      fix_reduce((terms >> k & 1) ? x[k] : 0., N, f64);
-      e[k] = fix_to_double(fix_exp2(f64, reinterpret_cast<const unsigned long long *>(tab + 128)), N);
+      for (int k = 0; k < 3; ++k) {
+        int N;
+        unsigned long long f64;
+        fix_reduce((terms >> k & 1) ? x[k] : 0., N, f64);
+        e[k] = fix_to_double(fix_exp2(f64, reinterpret_cast<const unsigned long long *>(tab + 128)), N);
+      }
+      const double w[3] = {1. - tr[0], tr[0], 1.};
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (terms >> k & 1) {
+          const double t = k == 2 ? e[k] : w[k] * e[k];
+          fc += t;
+          if (JAC) Tdfc = fma(k == 2 ? -x[k] : x[k], t, Tdfc);
+        }
+      return fc;
     }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      if (terms >> k & 1) e[k] = fix_exp(x[k], tab);
   }
-  double fc = 0.;
-  Tdfc = 0.;
   if (terms & 1) {
-    fc = (1. - tr[0]) * e[0];
-    if (JAC) Tdfc = x[0] * fc;
+    const double x = s.T * tr[1];
+    const double e = (1. - tr[0]) * fix_exp(x, tab);
+    fc += e;
+    if (JAC) Tdfc = x * e;
   }
   if (terms & 2) {
-    const double t = tr[0] * e[1];
-    fc += t;
-    if (JAC) Tdfc = fma(x[1], t, Tdfc);
+    const double x = s.T * tr[2];
+    const double e = tr[0] * fix_exp(x, tab);
+    fc += e;
+    if (JAC) Tdfc = fma(x, e, Tdfc);
   }
   if (terms & 4) {
-    fc += e[2];
-    if (JAC) Tdfc = fma(-x[2], e[2], Tdfc);
+    const double x = -(s.invT * tr[3]);
+    const double e = fix_exp(x, tab);
+    fc += e;
+    if (JAC) Tdfc = fma(-x, e, Tdfc);
   }
   return fc;
 }
@@ -652,18 +661,21 @@ __device__ __forceinline__ double third_body(const DevMech &m, const Blob &b, co
 {
   const int t0 = b.i[m.i_tb_off + r], t1 = b.i[m.i_tb_off + r + 1];
   double M = b.d[m.d_beff + r] * s.ct;
-  constexpr int U = PAIR ? 4 : 1;
-  for (int j = t0; j < t1; j += U) {
-    double e[U], c[U];
+  if constexpr (PAIR) {
+    for (int j = t0; j < t1; j += 4) {
+      double e[4], c[4];
 #pragma unroll
-    for (int k = 0; k < U; ++k) {
-      const bool in = j + k < t1;
-      e[k] = in ? b.d[m.d_tbeff + j + k] : 0.;
-      c[k] = in ? C[b.i[m.i_tb + j + k]] : 0.;
+      for (int k = 0; k < 4; ++k) {
+        const bool in = j + k < t1;
+        e[k] = in ? b.d[m.d_tbeff + j + k] : 0.;
+        c[k] = in ? C[b.i[m.i_tb + j + k]] : 0.;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (j + k < t1) M = fma(e[k], c[k], M);
     }
-#pragma unroll
-    for (int k = 0; k < U; ++k)
-      if (j + k < t1) M = fma(e[k], c[k], M);
+  } else {
+    for (int j = t0; j < t1; ++j) M = fma(b.d[m.d_tbeff + j], C[b.i[m.i_tb + j]], M);
   }
   return M;
 }
@@ -733,15 +745,16 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
         // Fc clamped at 1e-300 in the sensitivities (rates_sensitivities_exact.cpp:949-985), not in the rates
         // (chemistry_kernels.cpp:280-312): log10 F = log10 Fc / (1 + (a / bb)^2)
         const double prc = at_least_tiny(pr), fcc = JAC ? at_least_tiny(fc) : fc;
-        double lnpr, lnfc;
+        double l10pr, lnfc;
         if (PAIR && fix_normal(prc) && fix_normal(fcc)) {  // the two logarithms interleave
-          lnpr = fix96_ln(fix_log2(prc, exp2tab));
+          const double lnpr = fix96_ln(fix_log2(prc, exp2tab));
           lnfc = fix96_ln(fix_log2(fcc, exp2tab));
+          l10pr = lnpr * kLog10e;
         } else {
-          lnpr = fix_log(prc, exp2tab);
+          l10pr = fix_log(prc, exp2tab) * kLog10e;
           lnfc = fix_log(fcc, exp2tab);
         }
-        const double l10pr = lnpr * kLog10e, l10fc = lnfc * kLog10e;
+        const double l10fc = lnfc * kLog10e;
         const double a = l10pr - 0.67 * l10fc - 0.4;
         const double bb = 0.806 - 0.14 * l10pr - 1.1762 * l10fc;
         const double b2 = bb * bb;
