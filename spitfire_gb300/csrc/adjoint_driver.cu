@@ -7,10 +7,10 @@
 // reactor across the sweep, no compaction or scatter between steps. Per step m, over the na(m) reactors with more
 // than m steps:
 //   1. gather the recorded step (h, six stage states) of each reactor;
-//   2. right-hand sides and Jacobians at the 6 na stage states (the 32-lane batched chemistry kernel);
+//   2. right-hand sides and Jacobians at the 6 na stage states (the batched chemistry kernel at its own group width);
 //   3. the factors of the transposed implicit stage systems h gamma J_s^T - I, s = 1..5 (one warp per system);
 //   4. the clamp mask of the step update (entries the forward step clamped at 0 carry no derivative);
-//   5. the stage recursion, backwards over the stages, one warp per reactor for all outputs:
+//   5. the stage recursion, backwards over the stages, one CTA per reactor for all outputs:
 //        c_s = h b_s lam' + sum_{l>s} h a_ls Ybar_l (+ h gamma qd_s),   w_s = solve(h gamma J_s^T - I, -c_s)
 //        (w_0 = c_0),   Ybar_s = J_s^T w_s + qd_s,   lam = lam' + sum_s Ybar_s,
 //      qd_s the smoothed-delay quadrature term h b_s g'(T_s) e_T;
@@ -131,23 +131,31 @@ __global__ void k_adj_lamp(AdjBufs B, int na)
   }
 }
 
-// the stage recursion of one reactor for all outputs, one warp
-__global__ void k_adj_stages(AdjBufs B, int na)
+// The stage recursion of one reactor for all outputs, one CTA of kWarps warps per reactor: a warp solves for the outputs
+// w, w + kWarps, ..., and the products with J_s^T are spread over all threads. The factors and J_s are staged in shared
+// memory together, once per stage for all outputs. Bound: the serial sweeps of the solves. With one warp per reactor, the
+// outputs one after another and the columns of J_s read from global memory by single lanes, a step of 64 GRI reactors
+// (two outputs) took 320 us; 116 us now.
+__global__ void __launch_bounds__(32 * kWarps) k_adj_stages(AdjBufs B, int na)
 {
   extern __shared__ __align__(16) unsigned char sm[];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x, nt = 32 * kWarps;
   const int m = B.neq, O = B.O, tix = B.tix;
   const size_t mm = (size_t)m * m;
-  double *LU = reinterpret_cast<double *>(sm) + (size_t)w * (mm + 3 * m);
-  double *x = LU + mm, *cv = x + m, *di = cv + m;
-  int *pv = reinterpret_cast<int *>(reinterpret_cast<double *>(sm) + (size_t)kWarps * (mm + 3 * m)) + w * m;
-  for (int a = blockIdx.x * kWarps + w; a < na; a += gridDim.x * kWarps) {
+  double *LU = reinterpret_cast<double *>(sm);
+  double *J = LU + mm, *di = J + mm, *X = di + m, *cw = X + (size_t)O * m + (size_t)w * m;  // X: [O][m]
+  int *pv = reinterpret_cast<int *>(X + (size_t)(O + kWarps) * m);
+  for (int a = blockIdx.x; a < na; a += gridDim.x) {
     const double h = B.h[a];
     for (int s = 5; s >= 0; --s) {
+      const double *Js = B.J6 + ((size_t)a * 6 + s) * mm;
+      const size_t sys = (size_t)a * 5 + s - 1;
+      for (size_t e = tid; e < mm; e += nt) {
+        J[e] = Js[e];
+        if (s >= 1) LU[e] = B.LU[sys * mm + e];
+      }
       if (s >= 1) {
-        const size_t sys = (size_t)a * 5 + s - 1;
-        for (size_t e = lane; e < mm; e += 32) LU[e] = B.LU[sys * mm + e];
-        for (int k = lane; k < m; k += 32) {
+        for (int k = tid; k < m; k += nt) {
           pv[k] = B.perm[sys * m + k];
           di[k] = B.dinv[sys * m + k];
         }
@@ -155,46 +163,49 @@ __global__ void k_adj_stages(AdjBufs B, int na)
       const double Ts = B.Y6[((size_t)a * 6 + s) * m + tix];
       const double sg = 1. / (1. + exp(-((Ts - B.T0s[a] - kDtIgn) / kWidth)));
       const double dg = -sg * (1. - sg) / kWidth;
-      const double *J = B.J6 + ((size_t)a * 6 + s) * mm;
-      for (int o = 0; o < O; ++o) {
-        const size_t base = ((size_t)a * O + o);
+      __syncthreads();
+      for (int o = w; o < O; o += kWarps) {
+        const size_t base = (size_t)a * O + o;
         const double qdT = ((h * c_b[s]) * dg) * B.quad[o];
-        __syncwarp();
+        double *x = X + (size_t)o * m;
         for (int j = lane; j < m; j += 32) {
           double c = (h * c_b[s]) * B.lamp[base * m + j];
           for (int l = s + 1; l < 6; ++l)
             if (c_a[l][s] != 0.) c = c + (h * c_a[l][s]) * B.Ybar[(base * 6 + l) * m + j];
           if (s >= 1) c = c + (h * kGamma) * (j == tix ? qdT : 0.);
-          cv[j] = s >= 1 ? -c : c;
+          (s >= 1 ? cw : x)[j] = s >= 1 ? -c : c;
         }
         __syncwarp();
         if (s >= 1) {  // (h gamma J_s^T - I) w = -c, the right-hand side loaded in pivot order
-          for (int i = lane; i < m; i += 32) x[i] = cv[pv[i]];
-          warp_lu_solve_pd(LU, m, di, x);
-        } else {
-          for (int i = lane; i < m; i += 32) x[i] = cv[i];
+          for (int i = lane; i < m; i += 32) x[i] = cw[pv[i]];
+          __syncwarp();
+          if (m <= 32) warp_lu_solve_regs<1>(LU, m, di, x);
+          else if (m <= 64) warp_lu_solve_regs<2>(LU, m, di, x);
+          else warp_lu_solve_pd(LU, m, di, x);
         }
-        __syncwarp();
         for (int j = lane; j < m; j += 32) B.W[(base * 6 + s) * m + j] = x[j];
-        // Ybar_s = J_s^T w + qd_s: lane i walks column i of J (contiguous)
-        for (int i = lane; i < m; i += 32) {
-          const double *col = J + (size_t)i * m;
-          double acc = 0.;
-          for (int j = 0; j < m; ++j) acc = fma(col[j], x[j], acc);
-          B.Ybar[(base * 6 + s) * m + i] = acc + (i == tix ? qdT : 0.);
-        }
         __syncwarp();
       }
-    }
-    for (int o = 0; o < O; ++o) {
-      const size_t base = (size_t)a * O + o;
-      for (int j = lane; j < m; j += 32) {
-        double sum = 0.;
-        for (int s = 0; s < 6; ++s) sum += B.Ybar[(base * 6 + s) * m + j];
-        B.lam[base * m + j] = B.lamp[base * m + j] + sum;
+      __syncthreads();
+      // Ybar_s = J_s^T w + qd_s, a thread per output and column of J_s
+      for (int e = tid; e < O * m; e += nt) {
+        const int o = e / m, i = e - o * m;
+        const double *col = J + (size_t)i * m, *x = X + (size_t)o * m;
+        const double qdT = ((h * c_b[s]) * dg) * B.quad[o];
+        double acc = 0.;
+        for (int j = 0; j < m; ++j) acc = fma(col[j], x[j], acc);
+        B.Ybar[(((size_t)a * O + o) * 6 + s) * m + i] = acc + (i == tix ? qdT : 0.);
       }
+      __syncthreads();
     }
-    __syncwarp();
+    for (int e = tid; e < O * m; e += nt) {
+      const int o = e / m, j = e - o * m;
+      const size_t base = (size_t)a * O + o;
+      double sum = 0.;
+      for (int s = 0; s < 6; ++s) sum += B.Ybar[(base * 6 + s) * m + j];
+      B.lam[base * m + j] = B.lamp[base * m + j] + sum;
+    }
+    __syncthreads();
   }
 }
 
@@ -337,7 +348,7 @@ int sf_adjoint_batch(const sf_mech *mech, const sf_reactor_params *params, int n
     CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const size_t mm = (size_t)B.neq * B.neq;
     const size_t smem_lu = kWarps * ((mm + B.neq) * 8 + B.neq * 4);
-    const size_t smem_st = kWarps * ((mm + 3 * B.neq) * 8 + B.neq * 4);
+    const size_t smem_st = (2 * mm + (size_t)(1 + n_outputs + kWarps) * B.neq) * 8 + (size_t)B.neq * 4;
     ensure_dynamic_smem((const void *)k_adj_lu, smem_lu);
     ensure_dynamic_smem((const void *)k_adj_stages, smem_st);
     const int nmax = sorted_steps[0];
@@ -346,17 +357,14 @@ int sf_adjoint_batch(const sf_mech *mech, const sf_reactor_params *params, int n
       while (na > 0 && sorted_steps[na - 1] <= m) --na;
       k_adj_gather<<<na, 128, 0, st>>>(B, m, na);
       CUDA_THROW(cudaGetLastError());
-      // 32 lanes per state: a few thousand stage states are too few for the thread-per-state kernels
-      reactor_jac_lanes(mech, params, 0, 6 * na, B.Y6, params->configuration == 0 ? B.pres6 : nullptr, B.K6, B.J6,
-                        32, st);
+      reactor_jac_groups(mech, params, 0, 6 * na, B.Y6, params->configuration == 0 ? B.pres6 : nullptr, B.K6, B.J6, st);
       const long long lu_need = ((long long)na * 5 + kWarps - 1) / kWarps;
       k_adj_lu<<<(int)std::min<long long>(lu_need, (long long)nsm * 8), 32 * kWarps, smem_lu, st>>>(B, na);
       CUDA_THROW(cudaGetLastError());
       const long long lp = ((long long)na * B.neq + 255) / 256;
       k_adj_lamp<<<(int)std::min<long long>(lp, 4096), 256, 0, st>>>(B, na);
       CUDA_THROW(cudaGetLastError());
-      const long long st_need = ((long long)na + kWarps - 1) / kWarps;
-      k_adj_stages<<<(int)std::min<long long>(st_need, (long long)nsm * 8), 32 * kWarps, smem_st, st>>>(B, na);
+      k_adj_stages<<<std::min(na, nsm * 8), 32 * kWarps, smem_st, st>>>(B, na);
       CUDA_THROW(cudaGetLastError());
       launch_rate_param_adjoint(hm, params->configuration, params->pressure, na, n_outputs, 6, B.Y6,
                                 params->configuration == 0 ? B.ps : nullptr, B.W, B.grad, st);

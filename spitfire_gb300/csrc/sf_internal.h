@@ -80,9 +80,9 @@ size_t tps_resident_warps(const HostMech &hm);
 int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_allowed);
 // Groups per block that take n items on nsm blocks in even passes when `fit` groups fit one block.
 int balanced_groups(int fit, long long n, int nsm);
-// sf_reactor_jac_batch with an explicit lane width G (8, 16 or 32; no workspace). Throws sf_error.
-void reactor_jac_lanes(const sf_mech *mech, const sf_reactor_params *rp, int rates_option, int n, const double *q,
-                       const double *pressures, double *out_rhs, double *out_jac, int G, cudaStream_t st);
+// sf_reactor_jac_batch at the library's own group width (default_group; no workspace). Throws sf_error.
+void reactor_jac_groups(const sf_mech *mech, const sf_reactor_params *rp, int rates_option, int n, const double *q,
+                        const double *pressures, double *out_rhs, double *out_jac, cudaStream_t st);
 // Parameter adjoint of closed adiabatic reactors (sf_rate_param_adjoint_batch) with `wsets` adjoint vector sets per
 // state: w [n_items][wsets][stages][neq], out [n_items][wsets][2 nr] (accumulated). Throws sf_error.
 void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pressure, int n_items, int wsets,

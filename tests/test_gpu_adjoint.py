@@ -242,3 +242,22 @@ def test_native_backward_matches_host_loop(cuda, name, configuration, outputs):
             err = np.max(np.abs(x[:, o] - y[:, o])) / scale
             assert err < 1e-9, (key, o, err)
     assert spec.griffon.device_status() == 0
+
+
+@pytest.mark.parametrize('copies', [1, 4, 5, 8])
+def test_outputs_beyond_one_per_warp(cuda, copies):
+    """The stage recursion gives each output to a warp: a gradient does not depend on how many outputs are taken with it
+    (initial-state gradients bit for bit, the parameter sums to rounding), up to the largest number of outputs."""
+    import torch
+    from spitfire_gb300.adjoint import ReactorAdjoint
+    spec, _ = pair('h2-burke')
+    adj = ReactorAdjoint(spec, 'isobaric')
+    tr = adj.forward(_h2_reactors(spec, 3), pressures=np.full(3, 101325.), t_end=3.e-4)
+    one = {o: adj.backward(tr, outputs=(o,)) for o in ('T_end', 'tau_s')}
+    outputs = tuple(('T_end', 'tau_s')[k % 2] for k in range(copies))
+    many = adj.backward(tr, outputs=outputs)
+    for k, o in enumerate(outputs):
+        assert torch.equal(many['q0'][:, k], one[o]['q0'][:, 0])
+        x, y = many['theta'][:, k], one[o]['theta'][:, 0]
+        assert torch.all((x - y).abs().amax((1, 2)) <= 1e-13 * y.abs().amax((1, 2)))
+    assert spec.griffon.device_status() == 0
