@@ -300,7 +300,7 @@ def bench_newton(q, rhs, J, gamma_h, stream):
 
 
 # integrator memory placement knob: Griffon scratch and iteration matrix in shared memory or L2-resident global slots
-PLACEMENT = {3: 'shared', 1: 'global scratch', 2: 'global scratch + matrix'}
+PLACEMENT = {0: 'library rule', 3: 'shared', 1: 'global scratch', 2: 'global scratch + matrix'}
 
 
 def bench_ignition(spec, rank, stream, cpu):
@@ -619,7 +619,7 @@ def bench_flamelet(spec, rank, stream, cpu):
                       'achieved_gbs': rhs_bytes / (k['rhs_ms'] * 1e-3) / 1e9,
                       'points_per_s': pts / (k['rhs_ms'] * 1e-3)},
         'jacobian': {'points_per_s': pts / (k['jacobian_ms'] * 1e-3),
-                     'fp64_tflops_executed_est': FP64_PER_STATE[32]['flops'] * pts / (k['jacobian_ms'] * 1e-3)
+                     'fp64_tflops_executed_est': FP64_PER_STATE[0]['flops'] * pts / (k['jacobian_ms'] * 1e-3)
                      / 1e12},
         'factor': {'bound': 'fp64 (critical path: the longest flamelet)', 'flops_per_point': 2. * ns ** 3,
                    'achieved_tflops': fac_flops / (k['factor_ms'] * 1e-3) / 1e12}}

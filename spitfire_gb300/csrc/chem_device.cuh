@@ -240,7 +240,7 @@ struct Group<G, true> {
   }
 };
 
-inline int wide_group_doubles(int G)
+inline __host__ __device__ int wide_group_doubles(int G)
 {
   return G == 256 ? Group<256>::kShared : (G == 128 ? Group<128>::kShared : (G == 64 ? Group<64>::kShared : 0));
 }

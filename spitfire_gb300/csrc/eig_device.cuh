@@ -1,5 +1,5 @@
-// Largest real part of the eigenvalues of a small real nonsymmetric matrix, by one state group (a warp, or two where
-// there are fewer matrices than SMs: a row or column of up to 64 entries is then one pass), in shared memory:
+// Largest real part of the eigenvalues of a small real nonsymmetric matrix, by one state group (a warp where there
+// are many matrices, two or eight where there are about as many as SMs), in shared memory:
 // Parlett-Reinsch balancing (diagonal similarity by powers of two, exact in floating point), Householder reduction
 // to upper Hessenberg form, then the implicit double-shift (Francis) QR iteration with deflation on the active
 // window only (eigenvalues, no Schur vectors). Published algorithms: B. N. Parlett and C. Reinsch, "Balancing a
@@ -33,34 +33,78 @@ __device__ __forceinline__ double scale_pow2(double x, int k, double fac)
   return __longlong_as_double(b + ((long long)k << 52));
 }
 
+// Sums of the magnitudes of column i and row i of A without the diagonal, n <= 64, one warp: the terms as integers on the
+// scale of the largest (53 bits, the rest cut off), added by integer warp reductions in two halves. False where an exponent
+// is near the ends of the range (or a sum is zero); c and r are then untouched.
+__device__ __forceinline__ bool abs_sums(const double *A, int n, int i, int lane, double &c, double &r)
+{
+  unsigned long long b[2][2];
+  unsigned hi[2] = {0u, 0u};
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const int j = lane + 32 * s;
+    const bool in = j < n && j != i;
+    b[0][s] = in ? (unsigned long long)__double_as_longlong(A[j + i * n]) & 0x7fffffffffffffffull : 0ull;
+    b[1][s] = in ? (unsigned long long)__double_as_longlong(A[i + j * n]) & 0x7fffffffffffffffull : 0ull;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) hi[q] = max(hi[q], (unsigned)(b[q][s] >> 32));
+  }
+  int e[2];
+  unsigned long long x[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) e[q] = (int)(__reduce_max_sync(0xffffffffu, hi[q]) >> 20);
+  if (e[0] < 64 || e[1] < 64 || e[0] > 0x7b0 || e[1] > 0x7b0) return false;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    x[q] = 0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int ex = (int)(b[q][s] >> 52), sh = e[q] - ex;
+      const unsigned long long m = (b[q][s] & 0xfffffffffffffull) | 0x10000000000000ull;
+      x[q] += ex && sh < 64 ? m >> sh : 0ull;  // subnormals are below the last bit
+    }
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)x[q] & 0x7ffffffu);
+    const unsigned up = __reduce_add_sync(0xffffffffu, (unsigned)(x[q] >> 27));
+    x[q] = lo + ((unsigned long long)up << 27);
+    const int z = __clzll((long long)x[q]);
+    (q ? r : c) = fix_to_double(x[q] << z, 63 - z + e[q] - 1075);
+  }
+  return true;
+}
+
 // Parlett-Reinsch balancing with radix 2 (scaling only): repeat until no row/column pair changes by more than
 // 5%, at most `max_sweeps` sweeps. Column-major A, leading dimension n.
 // GB300 issues FP64 at one warp instruction per 76 cycles per scheduler, so the scalings by powers of two (exact)
 // run on the integer pipe: non-negative finite doubles order like their bit patterns, and a factor 4 or 1/4 on a
 // normal value is a change of 2 in its exponent field. The results are those of the plain FP64 form bit for bit;
 // values near the ends of the exponent range take the FP64 form.
-template <int G>
-__device__ void group_balance(const Group<G> &g, double *A, int n, int max_sweeps = 32)
+// One warp, also where the matrix has several: a row/column pair is a serial step, and the exchange between warps cost more
+// than it gained. The sums are integer sums (abs_sums) and a pair that needs no scaling (m = 0) is left at once: a 53 x 53
+// block takes nine sweeps of 53 pairs, about 1700 cycles a pair in FP64 with two warps.
+__device__ void warp_balance(double *A, int n, int max_sweeps = 32)
 {
+  const Group<32> g;
   const int lane = g.lane;
   constexpr long long kExp1 = 1LL << 52;
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     bool changed = false;
     for (int i = 0; i < n; ++i) {
       double c = 0., r = 0.;
-      for (int j = lane; j < n; j += G)
-        if (j != i) {
-          c += fabs(A[j + i * n]);
-          r += fabs(A[i + j * n]);
-        }
-      g.sum2(c, r, n);
+      if (n > 64 || !abs_sums(A, n, i, lane, c, r)) {
+        for (int j = lane; j < n; j += 32)
+          if (j != i) {
+            c += fabs(A[j + i * n]);
+            r += fabs(A[i + j * n]);
+          }
+        g.sum2(c, r, n);
+      }
       // c, r >= 0: zero when the bit pattern is zero, not finite when the exponent field is all ones
       const long long cb = __double_as_longlong(c), rb = __double_as_longlong(r);
       const int ce = (int)(cb >> 52), re = (int)(rb >> 52);
       if (cb == 0 || rb == 0 || ce == 0x7ff || re == 0x7ff) continue;
       // the scaling f = 2^m: the smallest m >= 0 with c 4^m >= r / 2, else the m < 0 that brings c below 2 r
       int m = 0;
-      const double s = c + r;
+      const double c0 = c;
       if (ce > 4 && ce < 0x7f0 && re > 4 && re < 0x7f0) {
         long long cc = cb;
         const long long g1 = rb - kExp1, g2 = rb + kExp1;  // r / 2, 2 r
@@ -85,6 +129,8 @@ __device__ void group_balance(const Group<G> &g, double *A, int n, int max_sweep
           --m;
         }
       }
+      if (m == 0) continue;  // nothing to scale
+      const double s = c0 + r;
       const bool normal = m >= -1000 && m <= 1000;
       const double f = normal ? __longlong_as_double((long long)(1023 + m) << 52) : ldexp(1., m);
       const double fi = normal ? __longlong_as_double((long long)(1023 - m) << 52) : 1. / f;
@@ -96,7 +142,7 @@ __device__ void group_balance(const Group<G> &g, double *A, int n, int max_sweep
                                : (normal ? t * fi : t / f) < lim;
       if (shrink) {
         changed = true;
-        for (int j = lane; j < n; j += G) {
+        for (int j = lane; j < n; j += 32) {
           if (normal) {
             A[i + j * n] = scale_pow2(A[i + j * n], -m, fi);
             A[j + i * n] = scale_pow2(A[j + i * n], m, f);
@@ -125,6 +171,8 @@ template <int G>
 __device__ bool group_hmatrix_below(const Group<G> &g, double *A, int n, double cutoff, double *dg)
 {
   const int lane = g.lane;
+  constexpr int W = G > 64 ? 64 : G;  // lanes over rows; the columns are dealt to the parts of a larger group
+  const int slot = lane % W, part = lane / W;
   bool ok = true;
   for (int e = lane; e < n * n; e += G) {
     const int c = e / n, r = e - c * n;
@@ -144,9 +192,9 @@ __device__ bool group_hmatrix_below(const Group<G> &g, double *A, int n, double 
     const double p = A[k + k * n];
     if (!(p > 1e-10 * dg[k])) return false;  // the same value in every lane: a warp-uniform exit
     const double ip = fix_reciprocal(p);
-    for (int i = k + 1 + lane; i < n; i += G) {
+    for (int i = k + 1 + slot; i < n; i += W) {
       const double l = A[i + k * n] * ip;
-      for (int j = k + 1; j < n; ++j) {
+      for (int j = k + 1 + part; j < n; j += G / W) {
         const double mkj = A[k + j * n];
         if ((__double_as_longlong(mkj) << 1) != 0) A[i + j * n] -= l * mkj;
       }
@@ -203,42 +251,70 @@ __device__ double group_gershgorin_bound(const Group<G> &g, const double *A, int
   return fmin(r, c);
 }
 
-// Reduce the n x n column-major A to upper Hessenberg form in place. v: n doubles, s: n doubles of shared work.
+// Reduce the n x n column-major A to upper Hessenberg form in place. v: n doubles; s: G doubles, sc: 8 doubles of shared
+// work for a group of more than 64 threads. Such a group has 64 lanes over columns (rows), and the inner products and
+// updates of a column are cut into G / 64 parts: FP64 instructions cost the same on each of an SM's four schedulers, and
+// two warps use two of them. 144 points of
+// 53 x 53, hardest point: 1.77 ms with two warps per point, 1.32 ms with eight and the balancing above.
 template <int G>
-__device__ void group_hessenberg(const Group<G> &g, double *A, int n, double *v, double *s)
+__device__ void group_hessenberg(const Group<G> &g, double *A, int n, double *v, double *s, double *sc)
 {
-  const int lane = g.lane;
-  for (int k = 0; k + 2 < n; ++k) {
-    double ss = 0.;
-    for (int i = k + 2 + lane; i < n; i += G) ss += A[i + k * n] * A[i + k * n];
-    ss = g.sum(ss, n);
-    if (ss == 0.) continue;  // already zero below the subdiagonal
-    const double x0 = A[(k + 1) + k * n];
-    const double s2 = x0 * x0 + ss, nrm = s2 * fix_rsqrt(s2);
-    const double alpha = -copysign(nrm, x0);
-    const double tau = fix_reciprocal(nrm * (nrm + fabs(x0)));  // 2 / (u^T u) for u = x - alpha e1
-    for (int i = k + 1 + lane; i < n; i += G) v[i] = (i == k + 1) ? x0 - alpha : A[i + k * n];
-    g.sync();
-    // left: A[k+1:, j] -= tau u (u^T A[k+1:, j]), lanes over columns j > k; column k becomes alpha e1
-    for (int j = k + 1 + lane; j < n; j += G) {
+  constexpr int W = G > 64 ? 64 : G, P = G / W;
+  const int lane = g.lane, slot = lane % W, part = lane / W;
+  // x[base + i stride] -= tau (x . v) v over i = k+1 .. n-1 for the lines base = 0 .. lines-1 of this group
+  auto reflect = [&](int k, int first, int base, int stride, double tau) {
+    const int m = n - k - 1, a = k + 1 + m * part / P, e = k + 1 + m * (part + 1) / P;
+    for (int j0 = first; j0 < n; j0 += W) {
+      const int j = j0 + slot;
+      double *x = A + (size_t)j * base;
       double d = 0.;
-      for (int i = k + 1; i < n; ++i) d += v[i] * A[i + j * n];
+      if (j < n)
+        for (int i = a; i < e; ++i) d += v[i] * x[i * stride];
+      if (P > 1) {
+        s[lane] = d;
+        g.sync();
+        d = s[slot];
+#pragma unroll
+        for (int q = 1; q < P; ++q) d += s[q * W + slot];
+      }
       d *= tau;
-      for (int i = k + 1; i < n; ++i) A[i + j * n] -= d * v[i];
+      if (j < n)
+        for (int i = a; i < e; ++i) x[i * stride] -= d * v[i];
+      if (P > 1 && j0 + W < n) g.sync();
     }
+  };
+  for (int k = 0; k + 2 < n; ++k) {
+    double tau = 0., alpha = 0.;
+    if (P == 1 || lane < 32) {
+      double ss = 0.;
+      for (int i = k + 2 + (P > 1 ? lane & 31 : lane); i < n; i += P > 1 ? 32 : G) ss += A[i + k * n] * A[i + k * n];
+      ss = P > 1 ? Group<32>().sum(ss) : g.sum(ss, n);
+      if (ss != 0.) {  // else already zero below the subdiagonal
+        const double x0 = A[(k + 1) + k * n];
+        const double s2 = x0 * x0 + ss, nrm = s2 * fix_rsqrt(s2);
+        alpha = -copysign(nrm, x0);
+        tau = fix_reciprocal(nrm * (nrm + fabs(x0)));  // 2 / (u^T u) for u = x - alpha e1
+        for (int i = k + 1 + lane; i < n; i += P > 1 ? 32 : G) v[i] = (i == k + 1) ? x0 - alpha : A[i + k * n];
+      }
+      if (P > 1 && lane == 0) {
+        sc[4 * (k & 1)] = tau;
+        sc[4 * (k & 1) + 1] = alpha;
+      }
+    }
+    if (P > 1) {
+      g.sync();
+      tau = sc[4 * (k & 1)];
+      alpha = sc[4 * (k & 1) + 1];
+    }
+    if (tau == 0. && alpha == 0.) continue;
+    if (P == 1) g.sync();
+    reflect(k, k + 1, n, 1, tau);  // left: A[k+1:, j] for the columns j > k; column k becomes alpha e1
     if (lane == 0) A[(k + 1) + k * n] = alpha;
     for (int i = k + 2 + lane; i < n; i += G) A[i + k * n] = 0.;
     g.sync();
-    // right: A[i, k+1:] -= tau (A[i, k+1:] u) u^T, lanes over rows
-    for (int i = lane; i < n; i += G) {
-      double d = 0.;
-      for (int l = k + 1; l < n; ++l) d += A[i + l * n] * v[l];
-      d *= tau;
-      for (int l = k + 1; l < n; ++l) A[i + l * n] -= d * v[l];
-    }
+    reflect(k, 0, 1, n, tau);      // right: A[i, k+1:] for all rows i
     g.sync();
   }
-  (void)s;
 }
 
 // Householder reflector P = I - v v^T mapping (x, y[, z]) to a multiple of e1: v = u / sqrt(beta) with
@@ -311,26 +387,13 @@ __device__ __forceinline__ int group_find_lo(const Group<G> &g, double *H, int n
   return 0;
 }
 
-// Largest real part of the eigenvalues of the n x n matrix A (destroyed; A is balanced first). work: 2n doubles
-// of shared memory. If cutoff is given and the balanced matrix's Gershgorin bound is <= cutoff, the function
-// returns that bound instead of running QR (every eigenvalue is then known to have real part <= cutoff).
-// With a cutoff the QR iteration also stops early: after every second sweep on an unreduced block, the block is
-// tested with group_hess_hmatrix_below, and a block whose eigenvalues are all proven left of the cutoff is set aside
-// without computing them. The returned maximum then covers only the eigenvalues computed, so it is exact whenever
-// it exceeds the cutoff, and at most the cutoff otherwise, which is all max(lambda_max - cutoff, 0) needs.
-// Returns false if the QR iteration did not converge within its budget (the largest real part of the diagonal
-// found so far is returned then).
+// Shared doubles beside the n of `work`: partial sums, two scalars per parity, the result.
+__host__ __device__ constexpr int eig_work_doubles(int G) { return G > 64 ? G + 8 + 2 : 0; }
+
+// QR iteration of group_max_real_eig on the Hessenberg matrix A; work: n doubles.
 template <int G>
-__device__ bool group_max_real_eig(const Group<G> &g, double *A, int n, double *work, double *out_max, double cutoff = -INFINITY)
+__device__ bool group_qr_max_real(const Group<G> &g, double *A, int n, double *work, double *out_max, double cutoff)
 {
-  group_balance<G>(g, A, n);
-  g.sync();
-  const double gb = group_gershgorin_bound<G>(g, A, n);
-  if (gb <= cutoff) {
-    *out_max = gb;
-    return true;
-  }
-  group_hessenberg<G>(g, A, n, work, work + n);
   double *H = A;
   double vmax = -INFINITY;
   int hi = n - 1, iter = 0, total = 0;
@@ -398,6 +461,48 @@ __device__ bool group_max_real_eig(const Group<G> &g, double *A, int n, double *
   }
   *out_max = vmax;
   return ok;
+}
+
+// Largest real part of the eigenvalues of the n x n matrix A (destroyed; A is balanced first). work: n +
+// eig_work_doubles(G) doubles of shared memory. If cutoff is given and the balanced matrix's Gershgorin bound is <= cutoff, the function
+// returns that bound instead of running QR (every eigenvalue is then known to have real part <= cutoff).
+// With a cutoff the QR iteration also stops early: after every second sweep on an unreduced block, the block is
+// tested with group_hess_hmatrix_below, and a block whose eigenvalues are all proven left of the cutoff is set aside
+// without computing them. The returned maximum then covers only the eigenvalues computed, so it is exact whenever
+// it exceeds the cutoff, and at most the cutoff otherwise, which is all max(lambda_max - cutoff, 0) needs.
+// Returns false if the QR iteration did not converge within its budget (the largest real part of the diagonal
+// found so far is returned then).
+template <int G>
+__device__ bool group_max_real_eig(const Group<G> &g, double *A, int n, double *work, double *out_max, double cutoff = -INFINITY)
+{
+  if (g.lane < 32) warp_balance(A, n);
+  g.sync();
+  const double gb = group_gershgorin_bound<G>(g, A, n);
+  if (gb <= cutoff) {
+    *out_max = gb;
+    return true;
+  }
+  double *wide = work + n;
+  group_hessenberg<G>(g, A, n, work, wide, wide + G);
+  if constexpr (G <= 64) {
+    return group_qr_max_real<G>(g, A, n, work, out_max, cutoff);
+  } else {
+    // the sweeps are a serial chain with a row and a column of work per step: the first two warps
+    double *res = wide + G + 8;
+    if (g.lane < 64) {
+      Group<64> two(wide, 0);
+      two.id = g.id + 8;  // a barrier of its own
+      double m;
+      const bool ok = group_qr_max_real<64>(two, A, n, work, &m, cutoff);
+      if (g.lane == 0) {
+        res[0] = m;
+        res[1] = ok ? 1. : 0.;
+      }
+    }
+    g.sync();
+    *out_max = res[0];
+    return res[1] != 0.;
+  }
 }
 
 }  // namespace sfgb

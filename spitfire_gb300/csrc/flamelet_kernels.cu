@@ -230,9 +230,14 @@ __global__ void __launch_bounds__(512, 1) flamelet_point_kernel(const FlmParams 
 // Pseudo-time-step eigenvalue bound (flamelet_kernels.cpp:1329-1341): for each point, max(max Re(lambda) - d, 0)
 // of the transformed isobaric chemistry block (the block before the diffusion diagonal and the enthalpy-flux
 // correction are added), d the flamelet's diffusion term, written to all ns entries of the point; then the held-back
-// enthalpy-flux correction is applied to the block. One warp per point, the block in shared memory. The result is
+// enthalpy-flux correction is applied to the block. A warp, two or eight per point, the block in shared memory. The result is
 // exactly 0 whenever every eigenvalue lies left of d; the scaled-Gershgorin (M-matrix) test proves that for a large
 // share of the points at a small fraction of the QR iteration's cost, which then runs only for the rest.
+inline __host__ __device__ size_t expeig_doubles(int G, int ns)
+{
+  return (size_t)ns * ns + 2 * ns + wide_group_doubles(G) + eig_work_doubles(G);
+}
+
 template <int G>
 __global__ void __launch_bounds__(256) flamelet_expeig_kernel(int n_points, int nf, int ns, const int *offz, const long long *offv,
                                        double *values, const double *cmajor, double diffterm,
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(256) flamelet_expeig_kernel(int n_points, int 
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const int w = threadIdx.x / G;
-  double *shared = reinterpret_cast<double *>(smem) + (size_t)w * (ns * ns + 2 * ns + Group<G>::kShared);
+  double *shared = reinterpret_cast<double *>(smem) + (size_t)w * expeig_doubles(G, ns);
   double *A = shared + Group<G>::kShared;
   const Group<G> g(shared, w);
   const int lane = g.lane;
@@ -1066,16 +1071,16 @@ int sf_flamelet_jac_batch(const sf_mech *mech, const sf_flamelet_batch *fb, cons
       CUDA_THROW(cudaGetDevice(&dev));
       CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
       CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-      // Up to two points per SM two warps work on one point (a row or column of a 53 x 53 block is then one pass) and every
-      // point has the FP64 unit of an SM, or half of it, to itself: with eight points per block, 120 points had filled 15
-      // SMs and taken 2.7 ms.
-      const bool two = p.n_points <= 2 * nsm;
-      const size_t per = (size_t)(ns * ns + 2 * ns + (two ? Group<64>::kShared : 0)) * 8;
-      int groups = (int)std::min<size_t>(two ? 2 : 8, (size_t)smem_max / per);
+      // One point per SM: eight warps work on it (all four schedulers for the reduction to Hessenberg form); up to two
+      // points per SM two warps each: every point has the FP64 unit of an SM, or half of it, to itself. With eight points
+      // per block, 120 points had filled 15 SMs and taken 2.7 ms.
+      const int G = p.n_points <= nsm ? 256 : (p.n_points <= 2 * nsm ? 64 : 32);
+      const size_t per = expeig_doubles(G, ns) * 8;
+      int groups = (int)std::min<size_t>(G == 256 ? 1 : (G == 64 ? 2 : 8), (size_t)smem_max / per);
       if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "block too large for the eigenvalue kernel");
       groups = (int)std::max<long long>(1, std::min<long long>(groups, ((long long)p.n_points + nsm - 1) / nsm));
-      const int threads = groups * (two ? 64 : 32);
-      auto kern = two ? flamelet_expeig_kernel<64> : flamelet_expeig_kernel<32>;
+      const int threads = groups * G;
+      auto kern = G == 256 ? flamelet_expeig_kernel<256> : (G == 64 ? flamelet_expeig_kernel<64> : flamelet_expeig_kernel<32>);
       ensure_dynamic_smem((const void *)kern, per * groups);
       int per_sm = 0;
       CUDA_THROW(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, per * groups));
