@@ -52,15 +52,14 @@ N_REACTORS = 8192
 N_FLAMELETS = 64
 N_ADJOINT = 2048
 TUNE_REACTORS = 4096
-# Per GRI state of each Jacobian kernel the autotuner can choose, from ncu on the profiling cases
-# (python bench.py --profile-case jac | jac_tps): executed FP64 flops (thread-level DADD + DMUL + 2*DFMA),
-# warp-level FP64 instructions (smsp__inst_executed_pipe_fp64.sum / states) and DRAM bytes
-# (dram__bytes_read.sum + dram__bytes_write.sum / states; the 8192-state case of the lane-group kernel keeps part of
-# its Jacobians in L2 at the end, so its figure is a lower bound; it was captured before the table-driven exponential,
-# which took the thread-per-state kernel from 79,842 to 76,159 flops and from 1,733 to 1,727 instructions).
+# Per GRI state of the Jacobian kernels, from ncu on the profiling cases (python bench.py --profile-case jac | jac_tps):
+# executed FP64 flops (thread-level DADD + DMUL + 2*DFMA), warp-level FP64 instructions
+# (smsp__inst_executed_pipe_fp64.sum / states) and DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum / states; the
+# 8192-state case keeps part of its Jacobians in L2 at the end, so its figure is a lower bound). Key: the group_jac knob;
+# 0 is the library's rule, 64 threads per state at the headline's batch.
 FP64_PER_STATE = {
-    32: {'kernel': 'chem_kernel<32, MODE_JAC>', 'flops': 86953., 'warp_instr': 2816., 'dram_bytes': 18725.},
-    1: {'kernel': 'chem_kernel_tps<MODE_JAC>', 'flops': 76159., 'warp_instr': 1727., 'dram_bytes': 124181.},
+    0: {'kernel': 'chem_kernel<64, MODE_JAC>', 'flops': 51814., 'warp_instr': 1403., 'dram_bytes': 24344.},
+    1: {'kernel': 'chem_kernel_tps<MODE_JAC>', 'flops': 46143., 'warp_instr': 933., 'dram_bytes': 118607.},
 }
 
 

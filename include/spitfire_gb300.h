@@ -122,15 +122,17 @@ int sf_mech_info(const sf_mech *mech, int *n_species, int *n_reactions, int *cou
  * the candidates on the device). 0 restores the built-in choice. Knobs and values:
  *   SF_TUNE_GROUP_{RATES,SENS,RHS,JAC}: lanes per state of the batched kernels, 8, 16 or 32, or 1 for the
  *     thread-per-state kernels (each lane one state, scratch interleaved across the warp in the caller's
- *     workspace, whose size sf_chem_workspace_size reports; no knob allocates anything);
- *   SF_TUNE_INTEGRATE_WARPS: warps (reactors) per block of sf_integrate_batch, 1..8 (0: as many as fit);
+ *     workspace, whose size sf_chem_workspace_size reports; no knob allocates anything); 0 lets the library choose by
+ *     the batch size, from 256 threads per state to one (the last only with a workspace);
+ *   SF_TUNE_INTEGRATE_WARPS: warps (reactors) per block of sf_integrate_batch, 1..8 (0: as many as fit; with both
+ *     integrator knobs 0, small FP64 batches of mechanisms with more than 64 reactions run eight warps per reactor);
  *   SF_TUNE_INTEGRATE_SCRATCH: where each integrating warp keeps its data: 3 all in shared memory; 1 its Griffon
  *     scratch in global memory (L2-resident), so that more warps fit per SM; 2 also its iteration matrix and FP32
  *     factors (0: the built-in choice, 2);
  *   SF_TUNE_TPS_CTAS: resident 4-warp blocks per SM of the thread-per-state kernels, 1..16 (0: as many as fit);
  *     fewer keep more of their interleaved scratch in L2.
- * The integrator knobs do not change results; the lane-group width changes the order of per-species sums, so those
- * results agree to rounding. No reference counterpart.
+ * The integrator knobs of one-warp shapes do not change results; the width of a group (and eight warps per reactor)
+ * changes the order of per-species sums, so those results agree to rounding. No reference counterpart.
  * Concurrency: a mechanism holds no scratch, so calls on one sf_mech may run on several streams at once, each with
  * its own workspace. Set knobs while no call that uses the mechanism is being issued. */
 enum sf_tune_knob {
@@ -153,10 +155,10 @@ int sf_thermo_batch(const sf_mech *mech, int what, int n, const double *T, const
 
 /* --------------------------------------------------------------------------------------------------- kinetics */
 /* Device workspace of the batched chemistry calls below, in bytes, for n states: the thread-per-state kernels
- * (lanes-per-state knob 1) interleave each warp's per-state scratch in it, at most one slot per warp that can be
- * resident (GRI-3.0 Jacobians: about 1.2 GB for a full device); the lane-group kernels keep their scratch in shared
- * memory and need none (0; the workspace pointer may then be NULL). The size depends on the mechanism's current
- * knobs: query it after tuning. One workspace must not be used by two calls that run at the same time. */
+ * (lanes-per-state knob 1, or the library's choice for large batches of small mechanisms) interleave each warp's
+ * per-state scratch in it, at most one slot per warp that can be resident; the state-group kernels keep their scratch
+ * in shared memory and need none (0). The workspace pointer may be NULL unless the knob is 1: the library then chooses
+ * a group. The size depends on the mechanism's current knobs: query it after tuning. One workspace must not be used by two calls that run at the same time. */
 enum sf_chem_kind { SF_CHEM_RATES = 0, SF_CHEM_SENS = 1, SF_CHEM_RHS = 2, SF_CHEM_JAC = 3 };
 size_t sf_chem_workspace_size(const sf_mech *mech, int kind, int n);
 

@@ -1,6 +1,7 @@
 // Device building blocks of the Griffon hot path on sm_103a.
 //
-// Execution model: one *state group* of G lanes (G = 8, 16 or 32) evaluates one thermochemical state at a time.
+// Execution model: one *state group* of G lanes evaluates one thermochemical state at a time: 8, 16 or 32 lanes of a warp, or
+// 64, 128 or 256 threads of a block (and one lane, in the thread-per-state kernels).
 // Lanes split species (thermodynamics, gathers by species) and reactions (rate evaluation), and a static gather
 // program assembles Jacobian entries with one FP64 FMA per item. The packed mechanism is copied into shared
 // memory once per CTA with a bulk-async (TMA) copy; every state group keeps its own scratch area in shared memory.
@@ -85,7 +86,7 @@ __device__ inline bool stage_to_smem(void *dst, const void *src, uint32_t bytes,
 // transposed reduction below adds four 32-lane sums in 6 instructions instead of 20 (the first two exchanges leave
 // each quarter of the lanes with one of the four sums).
 //
-// Group<G>, G <= 32: part of a warp. Group<G>, G = 128 or 256: several warps of a block, for launches with too few
+// Group<G>, G <= 32: part of a warp. Group<G>, G = 64, 128 or 256: several warps of a block, for launches with too few
 // states to give every scheduler of the GPU a warp of its own (below).
 template <int G, bool WIDE = (G > 32)>
 struct Group {
@@ -159,7 +160,7 @@ struct Group {
   }
 };
 
-// A state group of several whole warps of one block (G = 128 or 256 threads). An SM's FP64 rate is shared by four
+// A state group of several whole warps of one block (G = 64, 128 or 256 threads). An SM's FP64 rate is shared by four
 // schedulers and one warp can use only its own scheduler's quarter, so a launch whose states are fewer than about
 // four per SM runs each of them on all four. Warps meet at the group's own named barrier; a reduction goes through
 // shared memory, with two alternating buffers so that one barrier per reduction is enough (a thread reuses a buffer only

@@ -7,7 +7,7 @@
 // Points of all flamelets are flattened: flamelet f owns interior points offsets_z[f] .. offsets_z[f+1]-1. One state
 // group evaluates one point (isobaric chemistry via reactor_eval, then the mixture-fraction stencils). The
 // block-Thomas factorization and solve are sequential in mixture fraction; they run from both ends of a flamelet
-// toward its middle block, two CTAs (factorization) or two warps (solve) per flamelet, parallel within each block.
+// toward its middle block, two CTAs per flamelet, parallel within each block.
 #include "reactor_eval.cuh"
 #include "sf_internal.h"
 #include "eig_device.cuh"
@@ -1074,7 +1074,8 @@ int sf_flamelet_jac_batch(const sf_mech *mech, const sf_flamelet_batch *fb, cons
       // One point per SM: eight warps work on it (all four schedulers for the reduction to Hessenberg form); up to two
       // points per SM two warps each: every point has the FP64 unit of an SM, or half of it, to itself. With eight points
       // per block, 120 points had filled 15 SMs and taken 2.7 ms.
-      const int G = p.n_points <= nsm ? 256 : (p.n_points <= 2 * nsm ? 64 : 32);
+      int G = p.n_points <= nsm ? 256 : (p.n_points <= 2 * nsm ? 64 : 32);
+      while (G > 32 && expeig_doubles(G, ns) * 8 > (size_t)smem_max) G = G == 256 ? 64 : 32;  // the largest blocks
       const size_t per = expeig_doubles(G, ns) * 8;
       int groups = (int)std::min<size_t>(G == 256 ? 1 : (G == 64 ? 2 : 8), (size_t)smem_max / per);
       if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "block too large for the eigenvalue kernel");

@@ -1,8 +1,8 @@
 // Batched adaptive ESDIRK64 integration of closed homogeneous reactors in one persistent launch.
 //
-// One warp integrates one reactor at a time and takes the next unfinished reactor from an atomic work queue when
-// it is done, so reactors with ten times more steps than others do not hold the rest back. Everything a reactor
-// needs between steps lives in the warp's shared memory: the state, the six stage derivatives, the Newton
+// A group of threads, one warp or eight, integrates one reactor at a time and takes the next unfinished reactor from an
+// atomic work queue when it is done, so reactors with ten times more steps than others do not hold the rest back.
+// Everything a reactor needs between steps lives in the group's shared memory: the state, the six stage derivatives, the Newton
 // iteration matrix A = dt*gamma*J - I and its LU factors, and the Griffon scratch of the right-hand side and
 // Jacobian evaluations.
 //
