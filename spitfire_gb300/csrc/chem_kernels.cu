@@ -613,7 +613,14 @@ int sf_reactor_jac_host_batch(const sf_mech *mech, const sf_reactor_params *rp, 
     void *kws = w + io_bytes;  // the kernel's scratch: every chunk runs on `stream`, one after another
     const size_t kws_bytes = workspace_bytes - io_bytes;
     cudaStream_t st = (cudaStream_t)stream;
-    const int G = group_of(hm, SF_TUNE_GROUP_JAC);
+    // the group width of the whole batch for every chunk: the results are those of one device call, bit for bit
+    int G = group_of(hm, SF_TUNE_GROUP_JAC);
+    if (G == 0) {
+      int dev, nsm;
+      CUDA_THROW(cudaGetDevice(&dev));
+      CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+      G = default_group(hm.dm, true, n, nsm, kws_bytes >= tps_scratch_bytes(hm, MODE_JAC, n));
+    }
     // chunk: by default the states one wave of the thread-per-state kernel covers (its resident warps), else half
     int chunk = chunk_states;
     if (chunk <= 0) chunk = G == 1 ? (int)std::min<size_t>((size_t)n, tps_resident_warps(hm) * 32) : (n + 1) / 2;
