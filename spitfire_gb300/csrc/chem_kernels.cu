@@ -212,24 +212,25 @@ size_t tps_scratch_bytes(const HostMech &hm, int mode, long long n)
 // Threads per state for n states when no lane width was set: narrow groups waste the fewest FP64 instructions on empty
 // lanes, wide ones put few states on all four schedulers of every SM, and the shared memory decides how many states an
 // SM holds at once. Measured on 152 SMs (microseconds, GRI-3.0, 53 species / 325 reactions; h2-burke, 11 / 27):
-//   GRI Jacobians   n = 1: 41 with 256 threads, 135 with 32; 608: 90 (128), 88 (64), 139 (32); 2432: 337 (128), 380
-//                   (64), 569 (32); 4864: 652 (64), 668 (128); 65,536: 8,108 (64), 12,266 (32), 9,129 (thread per state)
-//   GRI rates       n = 304: 25 (256), 27 (128), 30 (64); 608: 36 (64), 46 (256), 50 (32); 1216: 53 (64), 63 (32), 75
-//                   (16); 1824: 79 (32), 83 (64), 85 (16); 3040: 109 (16), 134 (32); 20,011: 652 (16), 786 (8), 792
-//                   (32); 65,536: 2,155 (16), 2,291 (8)
-//   h2 Jacobians    n = 1: 33 (64), 40 (16); 1216: 42 (16), 53 (64); 4096: 74 (8), 96 (16); 65,536: 677 (1), 1,063 (8)
-//   h2 rates        n = 1216: 25 (16), 30 (8); 4096: 41 (8), 63 (16); 20,000: 155 (1), 204 (8)
+//   GRI Jacobians   n = 304: 62 (256), 456: 63 (128), 74 (64), 92 (256); 608: 73 (128), 82 (64); 2432: 274 (128), 279
+//                   (64); 3648: 368 (64), 408 (128); 65,536: 6,590 (64), 8,140 (thread per state), 9,540 (32)
+//   GRI rates       n = 304: 24 (256, 128), 27 (64), 44 (32); 456: 28 (128, 64); 912: 39 (64), 49 (32); 1216: 44 (64), 52
+//                   (32); 1824: 62 (32), 73 (64), 76 (16); 3040: 92 (16), 112 (32, 64); 20,011: 589 (16)
+//   h2 Jacobians    n = 304: 31 (64), 37 (16); 608: 34 (64), 37 (16); 1216: 38 (16), 42 (64); 3000: 47 (16), 54 (8); 4096:
+//                   59 (16), 60 (8); 9728: 102 (8), 133 (16); 65,536: 677 (1), 1,063 (8), before fixed-point rate constants
+//   h2 rates        n = 912: 22 (64), 23 (16); 1216: 22 (16), 24 (64); 3000: 24.6 (16), 25.3 (8); 4096: 28 (8), 30 (16);
+//                   20,000: 155 (1), 204 (8), before fixed-point rate constants
 // The lines lie at the SM count times the states of one SM; thread per state only where the caller's workspace has its
 // scratch (allowed), and for small mechanisms: GRI's 29 KB of scratch per state do not stay in L2.
 int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_allowed)
 {
   const long long per_sm = (n + nsm - 1) / nsm;
   if (m.nr >= 96 || m.ns >= 24) {
-    if (jac) return per_sm <= 2 ? 256 : (per_sm <= 24 ? 128 : 64);
+    if (jac) return per_sm <= 2 ? 256 : (per_sm <= 16 ? 128 : 64);
     return per_sm <= 2 ? 256 : (per_sm <= 8 ? 64 : (per_sm <= 14 ? 32 : 16));
   }
-  if (per_sm <= (jac ? 2 : 4)) return 64;
-  if (per_sm <= 16) return 16;
+  if (per_sm <= (jac ? 4 : 6)) return 64;
+  if (per_sm <= (jac ? 27 : 20)) return 16;
   return per_sm > 100 && tps_allowed ? 1 : 8;
 }
 

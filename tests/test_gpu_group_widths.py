@@ -16,7 +16,7 @@ def _sm_count():
 
 @pytest.mark.parametrize('mech', ['h2-burke', 'methane-gri30'])
 @pytest.mark.parametrize('conf', ['isobaric', 'isochoric'])
-@pytest.mark.parametrize('states', [(0, 1), (1, 1), (2, 1), (10, 1), (16, 1), (24, 1), (80, 1), (101, 3)])
+@pytest.mark.parametrize('states', [(0, 1), (1, 1), (2, 1), (4, 1), (6, 1), (10, 1), (16, 1), (20, 1), (24, 1), (27, 1), (80, 1), (101, 3)])
 def test_group_widths_agree(cuda, mech, conf, states):
     """States per SM up to and one past a line of the rule (the second number: states above that multiple of the SM
     count). Every width sums the same terms in another order: 1e-13 row-normwise, as between any two widths."""
