@@ -54,10 +54,11 @@ void fixed_log2_of(double x, int *n, u64 *f)
   }
 }
 
-// Fixed-point form of A T^b exp(-c/T): false where it has none (A not positive, b or c too large)
+// Fixed-point form of A T^b exp(-c/T): false where it has none (A not positive, b or c too large). The signed words hold
+// |b| 2^58 up to 32 and |c| log2(e) 2^44 up to 2^19 / log2(e) = 363,408 K.
 bool fixed_arrhenius_of(const double *k, double *w, int *n)
 {
-  if (!(k[0] > 1e-300 && k[0] < 1e300) || !(std::abs(k[1]) < 31.) || !(std::abs(k[2]) < 7.0e5)) return false;
+  if (!(k[0] > 1e-300 && k[0] < 1e300) || !(std::abs(k[1]) < 31.) || !(std::abs(k[2]) < 3.6e5)) return false;
   u64 f;
   fixed_log2_of(k[0], n, &f);
   const long long b = (long long)std::ldexp(k[1], 58);
@@ -67,7 +68,9 @@ bool fixed_arrhenius_of(const double *k, double *w, int *n)
   const u64 l2e63 = ((u64)kFixLog2e2 << 32) | kFixLog2e1;
   const int sh = 53 - e + 63 - 44;  // mi l2e63 2^-sh
   const u128 prod = (u128)mi * l2e63;
-  long long c = sh < 128 ? (long long)((prod + (((u128)1 << sh) >> 1)) >> sh) : 0;
+  const u128 rounded = sh < 128 ? (prod + (((u128)1 << sh) >> 1)) >> sh : 0;
+  if (rounded >> 63) return false;
+  long long c = (long long)rounded;
   if (k[2] < 0.) c = -c;
   std::memcpy(&w[0], &f, 8);
   std::memcpy(&w[1], &b, 8);
