@@ -584,6 +584,16 @@ static __device__ __noinline__ double forward_constant(const double *kc, const d
   }
 }
 
+// k e^x, with the power of two apart from the rest: e^x may lie outside the range of doubles where the product does not
+static __device__ __noinline__ double times_exp(double k, double x, const unsigned long long *exp2tab)
+{
+  int N = x < 0. ? -(1 << 20) : 1 << 20;  // beyond 2^20: 0 or infinity times k
+  unsigned long long f = 0;
+  if (isnan(x)) return x;
+  if (fabs(x) < 1048576.) fix_reduce(x, N, f);
+  return scale_pow2(k * fix_to_double(fix_exp2(f, exp2tab), 0), N);
+}
+
 // k0 / kinf of falloff reaction f
 __device__ __forceinline__ double falloff_ratio(const DevMech &m, const Blob &b, const StateCtx &s, int f)
 {
@@ -810,15 +820,17 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
           const Fix96 g = fix96(__double2loint(scr[L.gk + sp]), (unsigned long long)__double_as_longlong(scr[L.gm + sp]));
           for (int q = nu < 0 ? -nu : nu; q > 0; --q) y = nu > 0 ? y + g : y - g;
         }
-        nkr = -fix96_exp2(y, exp2tab);
-        if (!fixed) nkr *= kf;
+        if (fixed)
+          nkr = -fix96_exp2(y, exp2tab);
+        else  // 2^y may lie outside the range of doubles where its product with kf does not
+          nkr = -scale_pow2(kf * fix_to_double(fix_exp2(((unsigned long long)y.f1 << 32) | y.f0, exp2tab), 0), y.n);
       } else {
         double x = sum_nu ? (double)sum_nu * log(s.port) : 0.;
         for (int j = n0; j < n1; ++j) {
           const int e = b.i[m.i_net + j];
           x += (double)((e >> 16) - 128) * scr[L.gm + (e & 0xFFFF)];
         }
-        nkr = -kf * fix_exp(x, b.d + m.d_exptab);
+        nkr = -times_exp(kf, x, exp2tab);
       }
       if (short_lists) {
         fp = side3<JAC>(pl, npr, C, nkr, smallint);

@@ -33,6 +33,21 @@ def _log_k(A, b, theta, T):
         return np.sign(A), np.log(np.abs(LD(A))) + LD(b) * np.log(LD(T)) - LD(theta) / LD(T)
 
 
+def _g_over_RT(md, s, T):
+    _, _, tmid, _, lo, hi = md['species'][s]['cp']
+    a = [LD(v) for v in (lo if T <= tmid else hi)]
+    T = LD(T)
+    h = a[0] + T * (a[1] / 2 + T * (a[2] / 3 + T * (a[3] / 4 + T * a[4] / 5))) + a[5] / T
+    return h - (a[0] * np.log(T) + T * (a[1] + T * (a[2] / 2 + T * (a[3] / 3 + T * a[4] / 4))) + a[6])
+
+
+def _log_Kc(md, reac, prod, T):
+    """ln of kr / kf"""
+    nu = {s: reac.get(s, 0) - prod.get(s, 0) for s in SPECIES}
+    port = LD(md['ref_pressure']) / (LD(md['gas_constant']) * LD(T))
+    return sum(nu.values()) * np.log(port) - sum(v * _g_over_RT(md, s, T) for s, v in nu.items() if v)
+
+
 def _state(present):
     Y = np.array([1. if s in present else 0. for s in SPECIES])
     return Y / Y.sum()
@@ -126,3 +141,61 @@ def test_falloff_ratio(cuda, A0, b0, theta):
     for w in _evaluate(spec, np.array(T), np.ones(len(T)), np.tile(Y, (len(T), 1))):
         err = np.abs(w[:, 0] / (-q * LD(mw)) - 1.).astype(float)
         assert (err <= np.array(tol)).all(), (err, T)
+
+
+def _g_terms(md, s, T):
+    """Sum of the magnitudes of the terms of g/RT."""
+    _, _, tmid, _, lo, hi = md['species'][s]['cp']
+    a = np.abs(lo if T <= tmid else hi)
+    return sum(a[k] * T ** k for k in range(5)) * 2. + a[0] * np.log(T) + a[5] / T + a[6]
+
+
+def _reaction(sides, A, T):
+    """reactants -> products at temperature T with kr / kf far out of range where the sides' energies differ enough: E/R halves
+    what ln(kr) would be with none."""
+    reac, prod = ({s: side.count(s) for s in side} for side in sides)
+    from spitfire_gb300.mechanism import ChemicalMechanismSpec
+    md = ChemicalMechanismSpec.bundled(BASE).mech_data
+    mid = float(_log_Kc(md, reac, prod, T)) / 2. + np.log(abs(A) if A else 1.)
+    return reac, prod, True, A, 0., max(0., mid * T)
+
+
+REVERSIBLE = [(sides, T, A) for A in (1e10, -1e10) for sides, temps in
+              ((('ABDD', 'NNNC'), (15.9, 17., 300., 1500.)), (('BD', 'NC'), (15.9, 17., 300., 1500.)),
+               (('CC', 'D'), (300., 1500.))) for T in temps] + \
+    [(('ABDD', 'NNNC'), T, 1e-302) for T in (15.9, 17., 300., 1500.)] + \
+    [(sides, T, 0.) for sides in (('ABDD', 'NNNC'), ('NNNC', 'ABDD'), ('BD', 'NC'), ('CC', 'D'))
+     for T in (15.9, 17., 300., 1500., 66000.)]
+
+
+@pytest.mark.parametrize('sides,T,A', REVERSIBLE)
+def test_reverse_constant(cuda, sides, T, A):
+    """A state of products alone, so that the rate is the reverse one. E/R is chosen so that kf and kr are normal numbers
+    although kr / kf may lie far above the range; A = 0 gives no rate whatever kr / kf is. Below 16 K and above 65,536 K both
+    constants are formed in FP64, between them kf alone where A is not positive or out of range. The Gibbs energies'
+    terms are rounded to 53 bits at most six times each."""
+    spec = _mechanism([_reaction(sides, A, T)])
+    md = spec.mech_data
+    reac, prod = md['reactions'][0][1], md['reactions'][0][2]
+    theta = md['reactions'][0][6] / md['gas_constant']
+    Y = _state(''.join(prod))
+    c = _conc(spec, 1., Y)
+    product = np.prod([c[s] ** v for s, v in prod.items()])
+    net = {s: reac.get(s, 0) - prod.get(s, 0) for s in SPECIES}
+    i = SPECIES.index(next(iter(prod)))
+    mw = LD(spec.griffon._rec.species_mw[i])
+    runs = _evaluate(spec, np.array([T]), np.ones(1), Y[None])
+    w, S = spec.griffon.rates_sens_batch(np.ones(1), np.array([T]), Y[None])
+    assert bool(S.isfinite().all())
+    if A == 0.:
+        for w in runs:
+            assert (w == 0.).all()
+        return
+    sign, lk = _log_k(A, 0., theta, T)
+    lkr = lk + _log_Kc(md, reac, prod, T)
+    assert abs(lk) < 700. and abs(lkr) < 700.
+    expect = -net[SPECIES[i]] * mw * -sign * np.exp(lkr) * product
+    size = abs(np.log(abs(A))) + abs(theta) / T + abs(sum(net.values())) * 10. + \
+        sum(abs(v) * _g_terms(md, s, T) for s, v in net.items())
+    for w in runs:
+        assert abs(float(w[0, i] / expect - 1.)) <= 6. * 2.3e-16 * float(size) + 1e-14, (w[0, i], expect)
