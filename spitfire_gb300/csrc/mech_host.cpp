@@ -287,15 +287,19 @@ void HostMech::build(const sf_mech_desc *d)
   for (int r = 0; r < nr; ++r) {
     const HRxn &x = rx[r];
     for (int j = 0; j < 3; ++j) D[m.d_kf + 3 * r + j] = x.kf[j];
+    // the constant that the temperature forms 0 to 3 mean: b = 0, 1, 2, -1 and no E, whatever the last digits of b and E
+    static const double form_b[4] = {0., 1., 2., -1.};
+    const bool arrhenius = x.kform == 4;
+    const double kf[3] = {x.kf[0], arrhenius ? x.kf[1] : form_b[x.kform], arrhenius ? x.kf[2] : 0.};
     if (x.fall >= 0) {
-      D[m.d_kp + 3 * x.fall] = x.kp[0] / x.kf[0];
-      for (int j = 1; j < 3; ++j) D[m.d_kp + 3 * x.fall + j] = x.kp[j] - x.kf[j];
+      D[m.d_kp + 3 * x.fall] = x.kp[0] / kf[0];
+      for (int j = 1; j < 3; ++j) D[m.d_kp + 3 * x.fall + j] = x.kp[j] - kf[j];
       if (!fixed_arrhenius_of(&D[m.d_kp + 3 * x.fall], &D[m.d_fixp + 3 * x.fall], &I[m.i_fixp + x.fall]))
         I[m.i_fixp + x.fall] = kFixNone;
       const double tr[4] = {x.troe[0], -1. / x.troe[1], -1. / x.troe[2], x.troe[3]};
       for (int j = 0; j < 4; ++j) D[m.d_troe + 4 * x.fall + j] = tr[j];
     }
-    if (!fixed_arrhenius_of(x.kf, &D[m.d_fix + 3 * r], &I[m.i_fixn + r])) I[m.i_fixn + r] = kFixNone;
+    if (!fixed_arrhenius_of(kf, &D[m.d_fix + 3 * r], &I[m.i_fixn + r])) I[m.i_fixn + r] = kFixNone;
     D[m.d_beff + r] = x.beff;
   }
   int ntb = 0, nnet = 0, nord = 0, nslot = 0, nreac = 0, nprod = 0;

@@ -199,3 +199,27 @@ def test_reverse_constant(cuda, sides, T, A):
         sum(abs(v) * _g_terms(md, s, T) for s, v in net.items())
     for w in runs:
         assert abs(float(w[0, i] / expect - 1.)) <= 6. * 2.3e-16 * float(size) + 1e-14, (w[0, i], expect)
+
+
+@pytest.mark.parametrize('b,theta', [(5e-7, 0.), (1. + 5e-7, 0.), (2. - 5e-7, 5e-7), (-1. + 9e-7, -9e-7), (0., 9e-7)])
+def test_temperature_forms(cuda, b, theta):
+    """b within 1e-6 of 0, 1, 2 or -1 and E/R below 1e-6 mean exactly A, A T, A T^2 or A / T, in the forward constant, in
+    the reverse one and under a falloff ratio."""
+    form = round(b)
+    T = np.array([300., 1500., 3000.])
+    for falloff in (False, True):
+        reac, prod = {'B': 1, 'D': 1}, {'N': 1, 'C': 1}
+        spec = _mechanism([(reac, prod, True, 1e8, b, theta) + ((1e12, -0.3, 100.) if falloff else ())])
+        md = spec.mech_data
+        for present in ('BD', 'CN'):
+            Y = _state(present)
+            c = _conc(spec, 1., Y)
+            k = LD(1e8) * LD(1.) * np.array([LD(t) for t in T]) ** form
+            if falloff:
+                pr = np.array([np.exp(_log_k(1e12, -0.3, 100., t)[1]) for t in T]) / k * sum(c.values())
+                k = k * pr / (1. + pr)
+            if present == 'CN':
+                k = -k * np.array([np.exp(_log_Kc(md, reac, prod, t)) for t in T])
+            expect = -k * c[present[0]] * c[present[1]] * LD(spec.griffon._rec.species_mw[1])
+            for w in _evaluate(spec, T, np.ones(3), np.tile(Y, (3, 1))):
+                assert np.abs((w[:, 1] / expect - 1.).astype(float)).max() <= 6. * 2.3e-16 * 200. + 1e-14
