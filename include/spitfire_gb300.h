@@ -349,7 +349,9 @@ int sf_integrate_plain_batch(const sf_mech *mech, const sf_reactor_params *param
 /* sf_integrate_batch that also records every accepted step for adjoint sensitivities: trajectory is DEVICE
  * [n][capacity_steps][2 + 6*neq] doubles, per step (t_n, dt_n, Y_1..Y_6) with Y_1 = y_n and Y_2..Y_6 the converged
  * ESDIRK64 stage values (in the integrator's order). A reactor that needs more steps than the capacity stops with
- * SF_INT_RECORD_FULL. No reference counterpart (the reference computes no parameter sensitivities). */
+ * SF_INT_RECORD_FULL. With the same knobs a reactor's recorded integration does not depend on the rest of its batch, bit for
+ * bit, so that those reactors can be integrated again by themselves. No reference counterpart (the reference computes no
+ * parameter sensitivities). */
 int sf_integrate_record_batch(const sf_mech *mech, const sf_reactor_params *params, const sf_integrate_params *iparams,
                               int n, const double *q0, const double *pressures, double *out_q, double *out_t,
                               int *out_counts, int *out_status, void *workspace, size_t workspace_bytes,

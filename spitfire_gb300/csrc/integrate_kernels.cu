@@ -539,8 +539,10 @@ struct IntShape {
   size_t per_warp, smem, scratch_bytes, mat_bytes;
 };
 
-// Warps per block and grid of the persistent launch (autotuned knobs, else as many warps as fit)
-IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed_y_table = false)
+// Warps per block and grid of the persistent launch (autotuned knobs, else as many warps as fit). record: the steps are
+// recorded, and a caller integrates the reactors whose record was too short again, by themselves: the two launches belong
+// together only if the algorithm does not depend on the number of reactors.
+IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed_y_table, bool record)
 {
   int dev, smem_max, nsm;
   CUDA_THROW(cudaGetDevice(&dev));
@@ -551,8 +553,8 @@ IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed
   // was set (the autotuner's) or the factors are FP32. (GRI-3.0 to 20 us: one reactor 4.0 ms against 13.0 with one
   // warp, 300 16.7 against 66.1, 1000 38.1 against 66.9, 2000 64.0 against 89.0; ignitions to 0.1 s: 2048 reactors
   // 0.88 s against 0.90, 8192 3.29 against 2.73. h2-burke's 27 reactions fit one warp: 1000 reactors 171 ms with one,
-  // 243 with eight.)
-  if (prec == 0 && hm.dm.nr > 64 && n <= 12 * nsm && hm.tune[SF_TUNE_INTEGRATE_SCRATCH] == 0 && hm.tune[SF_TUNE_INTEGRATE_WARPS] == 0) {
+  // 243 with eight.) Recordings take them at every size.
+  if (prec == 0 && hm.dm.nr > 64 && (record || n <= 12 * nsm) && hm.tune[SF_TUNE_INTEGRATE_SCRATCH] == 0 && hm.tune[SF_TUNE_INTEGRATE_WARPS] == 0) {
     constexpr int wg = kWideG;
     s.per_warp = wide_doubles(hm, wg, neq, feed_y_table);
     const int fit = (int)std::min<size_t>(512 / wg, ((size_t)smem_max - hm.dm.blob_bytes - 64) / (s.per_warp * 8));
@@ -598,7 +600,7 @@ size_t sf_integrate_workspace_size(const sf_mech *mech, const sf_reactor_params 
     size_t most = 0;
     for (int prec = 0; prec <= 1; ++prec)
       for (int fy = 0; fy <= 1; ++fy) {
-        const IntShape a = integrate_shape(hm, neq, prec, n < 1 ? 1 : n, fy != 0);
+        const IntShape a = integrate_shape(hm, neq, prec, n < 1 ? 1 : n, fy != 0, false);
         most = std::max(most, a.scratch_bytes + a.mat_bytes);
       }
     return 256 + most;
@@ -677,8 +679,8 @@ static int integrate_impl(const sf_mech *mech, const sf_reactor_params *rp, cons
     p.queue = static_cast<unsigned int *>(workspace);
     p.rec = record;
     p.rec_cap = record_cap;
-    const IntShape sh = integrate_shape(hm, p.neq, p.prec, n,
-                                        ip->time_table && (ip->time_columns & SF_TIME_FEED_Y));
+    const IntShape sh = integrate_shape(hm, p.neq, p.prec, n, ip->time_table && (ip->time_columns & SF_TIME_FEED_Y),
+                                        record != nullptr);
     if (workspace_bytes < 256 + sh.scratch_bytes + sh.mat_bytes)
       throw sf_error(SF_ERR_WORKSPACE, "workspace smaller than sf_integrate_workspace_size reports");
     const auto &progs = hm.programs_for(sh.group);

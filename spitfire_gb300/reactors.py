@@ -211,7 +211,7 @@ class BatchIntegrator:
         """Recording integration (sf_integrate_record_batch) of every row of q0, into a record of `capacity` steps per
         reactor to start with. Reactors that fill their record (status 7) are integrated again, by themselves, into a
         record of twice the capacity, until every reactor fits; the others keep the results of the first launch. A
-        reactor's integration does not depend on the rest of its batch, so the results are those of a single run
+        recorded integration does not depend on the rest of its batch, so the results are those of a single run
         with the final capacity, without integrating the whole batch again. Returns (out, record)."""
         torch = _torch()
         n, neq = q0.shape
