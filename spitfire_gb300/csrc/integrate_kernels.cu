@@ -541,8 +541,9 @@ struct IntShape {
 
 // Warps per block and grid of the persistent launch (autotuned knobs, else as many warps as fit). record: the steps are
 // recorded, and a caller integrates the reactors whose record was too short again, by themselves: the two launches belong
-// together only if the algorithm does not depend on the number of reactors.
-IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed_y_table, bool record)
+// together only if the algorithm does not depend on the number of reactors. one_warp: the shape without wide groups, whose
+// scratch a workspace holds whatever n it is asked for.
+IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed_y_table, bool record, bool one_warp = false)
 {
   int dev, smem_max, nsm;
   CUDA_THROW(cudaGetDevice(&dev));
@@ -554,7 +555,7 @@ IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed
   // warp, 300 16.7 against 66.1, 1000 38.1 against 66.9, 2000 64.0 against 89.0; ignitions to 0.1 s: 2048 reactors
   // 0.88 s against 0.90, 8192 3.29 against 2.73. h2-burke's 27 reactions fit one warp: 1000 reactors 171 ms with one,
   // 243 with eight.) Recordings take them at every size.
-  if (prec == 0 && hm.dm.nr > 64 && (record || n <= 12 * nsm) && hm.tune[SF_TUNE_INTEGRATE_SCRATCH] == 0 && hm.tune[SF_TUNE_INTEGRATE_WARPS] == 0) {
+  if (!one_warp && prec == 0 && hm.dm.nr > 64 && (record || n <= 12 * nsm) && hm.tune[SF_TUNE_INTEGRATE_SCRATCH] == 0 && hm.tune[SF_TUNE_INTEGRATE_WARPS] == 0) {
     constexpr int wg = kWideG;
     s.per_warp = wide_doubles(hm, wg, neq, feed_y_table);
     const int fit = (int)std::min<size_t>(512 / wg, ((size_t)smem_max - hm.dm.blob_bytes - 64) / (s.per_warp * 8));
@@ -596,11 +597,11 @@ size_t sf_integrate_workspace_size(const sf_mech *mech, const sf_reactor_params 
   try {
     const HostMech &hm = mech->m;
     const int neq = params->configuration == 1 ? hm.dm.ns + 1 : hm.dm.ns;
-    // both linear precisions, with or without a feed mass-fraction table: the largest scratch need
+    // both linear precisions, with or without a feed mass-fraction table: the largest scratch need, for every n
     size_t most = 0;
     for (int prec = 0; prec <= 1; ++prec)
       for (int fy = 0; fy <= 1; ++fy) {
-        const IntShape a = integrate_shape(hm, neq, prec, n < 1 ? 1 : n, fy != 0, false);
+        const IntShape a = integrate_shape(hm, neq, prec, n < 1 ? 1 : n, fy != 0, false, true);
         most = std::max(most, a.scratch_bytes + a.mat_bytes);
       }
     return 256 + most;
