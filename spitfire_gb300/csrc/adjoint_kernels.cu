@@ -132,7 +132,9 @@ void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pre
   CUDA_THROW(cudaGetDevice(&dev));
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const int G = n_items <= 2 * nsm ? 256 : (n_items <= 8 * nsm ? 64 : 32);
+  const size_t scr_doubles = (size_t)hm.sl.total_rhs + hm.dm.ns + (configuration == 1 ? 1 : 0) + 2;
+  int G = fitting_group(hm.dm, n_items <= 2 * nsm ? 256 : (n_items <= 8 * nsm ? 64 : 32), scr_doubles, smem_max);
+  if (G == 128) G = 64;  // no kernel of that width
   const auto &progs = hm.programs_for(G);
   AdjParams p{};
   p.m = hm.dm;
@@ -155,7 +157,7 @@ void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pre
   p.w = w;
   p.out = out;
   const int shared = wide_group_doubles(G);
-  const size_t per = (size_t)(hm.sl.total_rhs + p.neq + 2 + shared) * 8;
+  const size_t per = (scr_doubles + shared) * 8;
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
   int groups = (int)std::min<size_t>(avail / per, (G > 32 ? 512 : 256) / G);
   if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the parameter-adjoint kernel");

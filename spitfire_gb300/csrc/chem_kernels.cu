@@ -234,6 +234,12 @@ int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_all
   return per_sm > 100 && tps_allowed ? 1 : 8;
 }
 
+int fitting_group(const DevMech &m, int G, size_t doubles, int smem_max)
+{
+  while (G > 32 && (size_t)m.blob_bytes + (doubles + wide_group_doubles(G)) * 8 + 64 > (size_t)smem_max) G /= 2;
+  return G;
+}
+
 // Groups per block for n items on nsm blocks when `fit` groups fit: the passes that `fit` needs, taken evenly (a last
 // pass with few items would otherwise cost as much as a full one).
 int balanced_groups(int fit, long long n, int nsm)
@@ -275,6 +281,18 @@ int launch_tps(const HostMech &hm, KParams &p, cudaStream_t st, void *ws, size_t
   return SF_OK;
 }
 
+// Width of the groups (or 1) that a call with no lane width set takes for n states. room: the caller's workspace has the
+// scratch of the thread-per-state kernels.
+int chosen_group(const HostMech &hm, int mode, long long n, bool room)
+{
+  int dev, nsm, smem_max;
+  CUDA_THROW(cudaGetDevice(&dev));
+  CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  return fitting_group(hm.dm, default_group(hm.dm, jac_mode(mode), n, nsm, room),
+                       jac_mode(mode) ? hm.sl.total : hm.sl.total_rhs, smem_max);
+}
+
 template <int MODE>
 int launch_mode(const HostMech &hm, KParams &p, cudaStream_t st, int G_req, void *ws, size_t ws_bytes)
 {
@@ -283,8 +301,7 @@ int launch_mode(const HostMech &hm, KParams &p, cudaStream_t st, int G_req, void
   int smem_max, nsm;
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const bool room = ws && ws_bytes >= tps_scratch_bytes(hm, MODE, p.n);
-  const int G = G_req > 0 ? G_req : default_group(hm.dm, jac_mode(MODE), p.n, nsm, room);
+  const int G = G_req > 0 ? G_req : chosen_group(hm, MODE, p.n, ws && ws_bytes >= tps_scratch_bytes(hm, MODE, p.n));
   if (G == 1) return launch_tps<MODE>(hm, p, st, ws, ws_bytes);
   const auto &progs = hm.programs_for(G);
   p.m = hm.dm;
@@ -566,11 +583,8 @@ size_t sf_chem_workspace_size(const sf_mech *mech, int kind, int n)
   static const int knob[4] = {SF_TUNE_GROUP_RATES, SF_TUNE_GROUP_SENS, SF_TUNE_GROUP_RHS, SF_TUNE_GROUP_JAC};
   static const int mode[4] = {MODE_RATES, MODE_SENS, MODE_RHS, MODE_JAC};
   try {
-    int dev, nsm;
-    CUDA_THROW(cudaGetDevice(&dev));
-    CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int g = group_of(mech->m, knob[kind]);
-    if ((g ? g : default_group(mech->m.dm, jac_mode(mode[kind]), n, nsm, true)) != 1) return 0;
+    if ((g ? g : chosen_group(mech->m, mode[kind], n, true)) != 1) return 0;
     return tps_scratch_bytes(mech->m, mode[kind], n);
   } catch (sf_error &e) {
     t_err = e.what();
@@ -616,12 +630,7 @@ int sf_reactor_jac_host_batch(const sf_mech *mech, const sf_reactor_params *rp, 
     cudaStream_t st = (cudaStream_t)stream;
     // the group width of the whole batch for every chunk: the results are those of one device call, bit for bit
     int G = group_of(hm, SF_TUNE_GROUP_JAC);
-    if (G == 0) {
-      int dev, nsm;
-      CUDA_THROW(cudaGetDevice(&dev));
-      CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-      G = default_group(hm.dm, true, n, nsm, kws_bytes >= tps_scratch_bytes(hm, MODE_JAC, n));
-    }
+    if (G == 0) G = chosen_group(hm, MODE_JAC, n, kws_bytes >= tps_scratch_bytes(hm, MODE_JAC, n));
     // chunk: by default the states one wave of the thread-per-state kernel covers (its resident warps), else half
     int chunk = chunk_states;
     if (chunk <= 0) chunk = G == 1 ? (int)std::min<size_t>((size_t)n, tps_resident_warps(hm) * 32) : (n + 1) / 2;

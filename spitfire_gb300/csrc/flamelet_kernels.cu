@@ -760,7 +760,8 @@ int launch_points(HostMech &hm, FlmParams &p, bool jac, cudaStream_t st)
   CUDA_THROW(cudaGetDevice(&dev));
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const int G = default_group(hm.dm, jac, p.n_points, nsm, false);
+  const size_t scr_doubles = (size_t)(jac ? hm.sl.total : hm.sl.total_rhs) + hm.dm.ns + 2;
+  const int G = fitting_group(hm.dm, default_group(hm.dm, jac, p.n_points, nsm, false), scr_doubles, smem_max);
   const auto &progs = hm.programs_for(G);
   p.m = hm.dm;
   p.blob = hm.d_blob;
@@ -770,7 +771,7 @@ int launch_points(HostMech &hm, FlmParams &p, bool jac, cudaStream_t st)
   p.pg.full = progs.progs[1];
   p.pg.j = progs.progs[2];
   const int shared = wide_group_doubles(G);
-  const size_t per = (size_t)((jac ? hm.sl.total : hm.sl.total_rhs) + hm.dm.ns + 2 + shared) * 8;
+  const size_t per = (scr_doubles + shared) * 8;
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
   int groups = (int)std::min<size_t>(avail / per, 512 / G);
   if (groups < 1) throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the flamelet kernels");

@@ -78,6 +78,9 @@ void ensure_dynamic_smem(const void *kernel, size_t bytes);
 size_t tps_resident_warps(const HostMech &hm);
 // Threads per state (8 to 256, or 1) of the chemistry kernels for n states when none was set.
 int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_allowed);
+// The widest group, G or narrower (halved down to one warp), of which one fits a block's shared memory beside the blob: `doubles`
+// of scratch per group, and what a wide group's reductions take. Below 64 threads G is returned as it is.
+int fitting_group(const DevMech &m, int G, size_t doubles, int smem_max);
 // Groups per block that take n items on nsm blocks in even passes when `fit` groups fit one block.
 int balanced_groups(int fit, long long n, int nsm);
 // sf_reactor_jac_batch at the library's own group width (default_group; no workspace). Throws sf_error.
