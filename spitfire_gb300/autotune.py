@@ -190,7 +190,7 @@ def _fitting_warps(integrator):
     props = torch.cuda.get_device_properties(torch.cuda.current_device())
     smem = getattr(props, 'shared_memory_per_block_optin', 232448)
     h = integrator.mech.griffon
-    # per-warp doubles as the integrator lays them out (integrate_kernels.cu per_warp_doubles)
+    # per-warp doubles as the integrator lays them out (integrate_kernels.cu integrate_warp_doubles)
     lay = h.scratch_layout()
     neq = integrator.mech.n_species + (1 if integrator.configuration == 'isochoric' else 0)
     v = get_tuning(integrator.mech, 'integrate_scratch')

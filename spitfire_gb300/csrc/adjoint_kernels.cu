@@ -41,7 +41,7 @@ __device__ double falloff_factor(const DevMech &m, const Blob &b, const ScratchL
                                  const StateCtx &s, int r, int kind, int info)
 {
   const double M = third_body<false>(m, b, s, r, scr + L.C);
-  const int f = b.i[m.i_fall + r];
+  const int f = r - (m.nr - m.n_fall);
   const double pr = falloff_ratio(m, b, s, f) * M;
   double fac = pr / (1. + pr);
   if (kind == 4 && pr > 1.e-300) {

@@ -425,7 +425,7 @@ __device__ __forceinline__ double small_int(const double *table, int k)
 struct StateCtx {
   double T, logT, invT, rho, invRho, mmw, invM, ct;
   double port;  // p_ref / (R T)
-  bool fixed;   // 16 < T < 65536: rate constants in fixed point
+  bool fixed;   // rate constants in fixed point: 16 < T < 65536 and the blob holds them
   unsigned long long l60, u68;  // log2 T 2^60, 2^68 / T
   int option;  // rates-sensitivity option: 0 / 2 exact, 1 without third-body/falloff derivatives
 };
@@ -737,7 +737,7 @@ __device__ __forceinline__ void eval_reaction(const DevMech &m, Blob b, const Sc
       Ctbaf = M;
       K = 1.;
     } else {
-      const int f = b.i[m.i_fall + r];
+      const int f = r - (m.nr - m.n_fall);
       const double *kp = b.d + m.d_kp + 3 * f;  // the ratio k0 / kinf as A, b, E/R
       const double kpf = falloff_ratio(m, b, s, f);
       const double pr = kpf * M;

@@ -496,6 +496,20 @@ __global__ void __launch_bounds__(G > 32 ? 512 : 256, G > 32 ? 1 : 2) integrate_
   }
 }
 
+}  // namespace
+
+size_t integrate_warp_doubles(const HostMech &hm, int neq, int prec, bool global_scratch, bool global_matrix,
+                              bool feed_y_table)
+{
+  const size_t n2 = (size_t)neq * neq;
+  return (global_matrix ? 0 : n2) + 12 * (size_t)neq + (global_scratch ? 0 : hm.sl.total) +
+         (prec == 1 ? (global_matrix ? 0 : (n2 + 1) / 2) + (size_t)neq : 0) + ((size_t)neq + 1) / 2 + 2 +
+         (size_t)neq +                           // reciprocals of U's diagonal
+         (feed_y_table ? (size_t)hm.dm.ns : 0);  // interpolated feed mass fractions
+}
+
+namespace {
+
 // Memory placement of an integrating warp's data: 0 all in shared memory, 1 the Griffon scratch in a global
 // (L2-resident) slot, 2 the iteration matrix and FP32 factors there too. The built-in choice (knob value 0) is 2:
 // with 8 warps per block it ran the 8192-reactor GRI ignition batch at 2,292 ignitions/s, against 1,771 for
@@ -504,18 +518,6 @@ int integrate_placement(const HostMech &hm)
 {
   const int v = hm.tune[SF_TUNE_INTEGRATE_SCRATCH];
   return v == 0 ? 2 : (v == 3 ? 0 : v);
-}
-
-// Shared memory per warp. global_scratch: the Griffon scratch lives in a global slot; global_matrix: the iteration
-// matrix and the FP32 factors too, leaving the vectors and pivots in shared memory.
-size_t per_warp_doubles(const HostMech &hm, int neq, int prec, bool global_scratch, bool global_matrix,
-                        bool feed_y_table = false)
-{
-  const size_t n2 = (size_t)neq * neq;
-  return (global_matrix ? 0 : n2) + 12 * (size_t)neq + (global_scratch ? 0 : hm.sl.total) +
-         (prec == 1 ? (global_matrix ? 0 : (n2 + 1) / 2) + (size_t)neq : 0) + ((size_t)neq + 1) / 2 + 2 +
-         (size_t)neq +                           // reciprocals of U's diagonal
-         (feed_y_table ? (size_t)hm.dm.ns : 0);  // interpolated feed mass fractions
 }
 
 size_t matrix_doubles(int neq, int prec)
@@ -570,7 +572,7 @@ IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed
   s.group = 32;
   const int place = integrate_placement(hm);
   const bool gs = place >= 1, gm = place == 2;
-  s.per_warp = per_warp_doubles(hm, neq, prec, gs, gm, feed_y_table);
+  s.per_warp = integrate_warp_doubles(hm, neq, prec, gs, gm, feed_y_table);
   const size_t avail = (size_t)smem_max - hm.dm.blob_bytes - 64;
   int fit = (int)std::min<size_t>(8, avail / (s.per_warp * 8));
   if (fit < 1) throw sf_error(SF_ERR_UNSUPPORTED, "mechanism too large for the shared-memory integrator");

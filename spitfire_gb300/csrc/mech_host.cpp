@@ -77,6 +77,15 @@ bool fixed_arrhenius_of(const double *k, double *w, int *n)
   std::memcpy(&w[2], &c, 8);
   return true;
 }
+
+// The forward constant that a reaction's temperature form means: forms 0 to 3 have b = 0, 1, 2, -1 and no E, whatever the
+// last digits of the b and E that selected them.
+std::array<double, 3> form_constant(const HRxn &x)
+{
+  static const double form_b[4] = {0., 1., 2., -1.};
+  if (x.kform == 4) return {x.kf[0], x.kf[1], x.kf[2]};
+  return {x.kf[0], form_b[x.kform], 0.};
+}
 }  // namespace
 
 HostMech::~HostMech()
@@ -277,29 +286,19 @@ void HostMech::build(const sf_mech_desc *d)
   }
   m.d_kf = dsec(3 * nr);
   m.d_kp = dsec(3 * n_fall);
-  m.d_fix = dsec(3 * nr);
-  m.d_fixp = dsec(3 * n_fall);
-  m.i_fixn = isec(nr);
-  m.i_fixp = isec(n_fall);
   fixed_log2_of(m.pref / m.Ru, &m.log2_port_n, &m.log2_port_f);
   m.d_troe = dsec(4 * n_fall);
   m.d_beff = dsec(nr);
   for (int r = 0; r < nr; ++r) {
     const HRxn &x = rx[r];
     for (int j = 0; j < 3; ++j) D[m.d_kf + 3 * r + j] = x.kf[j];
-    // the constant that the temperature forms 0 to 3 mean: b = 0, 1, 2, -1 and no E, whatever the last digits of b and E
-    static const double form_b[4] = {0., 1., 2., -1.};
-    const bool arrhenius = x.kform == 4;
-    const double kf[3] = {x.kf[0], arrhenius ? x.kf[1] : form_b[x.kform], arrhenius ? x.kf[2] : 0.};
     if (x.fall >= 0) {
+      const std::array<double, 3> kf = form_constant(x);
       D[m.d_kp + 3 * x.fall] = x.kp[0] / kf[0];
       for (int j = 1; j < 3; ++j) D[m.d_kp + 3 * x.fall + j] = x.kp[j] - kf[j];
-      if (!fixed_arrhenius_of(&D[m.d_kp + 3 * x.fall], &D[m.d_fixp + 3 * x.fall], &I[m.i_fixp + x.fall]))
-        I[m.i_fixp + x.fall] = kFixNone;
       const double tr[4] = {x.troe[0], -1. / x.troe[1], -1. / x.troe[2], x.troe[3]};
       for (int j = 0; j < 4; ++j) D[m.d_troe + 4 * x.fall + j] = tr[j];
     }
-    if (!fixed_arrhenius_of(kf, &D[m.d_fix + 3 * r], &I[m.i_fixn + r])) I[m.i_fixn + r] = kFixNone;
     D[m.d_beff + r] = x.beff;
   }
   int ntb = 0, nnet = 0, nord = 0, nslot = 0, nreac = 0, nprod = 0;
@@ -312,8 +311,6 @@ void HostMech::build(const sf_mech_desc *d)
   m.d_tbeff = dsec(ntb);
   m.d_netc = dsec(nnet);
   m.d_ord = dsec(nord);
-  m.d_one = dsec(1);
-  D[m.d_one] = 1.;
   m.d_smallint = dsec(64);
   for (int k = 0; k < 64; ++k) D[m.d_smallint + k] = k - 32;
   while (D.size() % 2) D.push_back(0.);  // 16-byte boundary: the table is read as (head, tail) pairs
@@ -324,7 +321,6 @@ void HostMech::build(const sf_mech_desc *d)
   m.i_orig = isec(nr);
   for (int r = 0; r < nr; ++r) I[m.i_orig + r] = orig_index[r];
   m.i_sums = isec(nr);
-  m.i_fall = isec(nr);
   m.i_dense = isec(nr);
   m.i_reac_off = isec(nr + 1); m.i_reac = isec(nreac);
   m.i_prod_off = isec(nr + 1); m.i_prod = isec(nprod);
@@ -343,7 +339,6 @@ void HostMech::build(const sf_mech_desc *d)
                       (x.reversible ? 1 << RI_REV_BIT : 0) | (x.has_orders ? 1 << RI_ORD_BIT : 0) |
                       (x.dense ? 1 << RI_DENSE_BIT : 0);
     I[m.i_sums + r] = (x.sum_nu & 0xFFFF) | ((x.sum_reac_nu & 0xFF) << 16) | ((x.sum_prod_nu & 0xFF) << 24);
-    I[m.i_fall + r] = x.fall;
     I[m.i_dense + r] = x.dense_idx;
     I[m.i_reac_off + r] = cr;
     for (size_t i = 0; i < x.reac.size(); ++i) I[m.i_reac + cr++] = pack_sp(x.reac[i], x.reac_nu[i]);
@@ -377,19 +372,10 @@ void HostMech::build(const sf_mech_desc *d)
   }
   I[m.i_reac_off + nr] = cr; I[m.i_prod_off + nr] = cp; I[m.i_net_off + nr] = cn;
   I[m.i_tb_off + nr] = ct; I[m.i_ord_off + nr] = co; I[m.i_slot_off + nr] = cs;
-  while (D.size() % 2) D.push_back(0.);  // 16-byte boundary for the int section
-  while (I.size() % 4) I.push_back(0);   // 16-byte total
-  m.blob_doubles = (int)D.size();
-  m.blob_ints = (int)I.size();
-  m.blob_bytes = m.blob_doubles * 8 + m.blob_ints * 4;
-  host_dbl = D;
-  host_int = I;
-
   // ---------------- scratch layout (RHS-only path uses the prefix up to total_rhs)
   ScratchLayout &L = sl;
   int o = 0;
   auto take = [&](int n) { const int r = o; o += (n + 1) & ~1; return r; };
-  L.misc = take(16);
   L.y = take(ns); L.C = take(ns); L.eh = take(ns); L.cpv = take(ns); L.w = take(ns);
   L.gm = take(ns); L.gk = take(ns);
   L.q = take(nr);
@@ -403,6 +389,41 @@ void HostMech::build(const sf_mech_desc *d)
   L.D = take(nslot);
   L.total = o;
 
+  // ---------------- fixed-point rate constants, 28 bytes per reaction and falloff ratio: left out (the rates are then formed
+  // in FP64) where some kernel's narrowest group fits a block's shared memory only without them
+  CUDA_THROW(cudaGetDevice(&device));
+  {
+    int smem_max;
+    CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    std::vector<size_t> need = {0, (size_t)L.total_rhs, (size_t)L.total, (size_t)L.total_rhs + ns + 3, (size_t)L.total + ns + 2};
+    for (int neq : {ns, ns + 1})
+      for (int place = 0; place <= 2; ++place)
+        for (int prec = 0; prec <= 1; ++prec)
+          need.push_back(integrate_warp_doubles(*this, neq, prec, place >= 1, place == 2, true));
+    const size_t base = D.size() * 8 + I.size() * 4 + 32, fix = (size_t)28 * (nr + n_fall);
+    m.fixed_rates = 1;
+    for (size_t n : need)
+      if (base + 8 * n + 64 <= (size_t)smem_max && base + fix + 8 * n + 64 > (size_t)smem_max) m.fixed_rates = 0;
+  }
+  if (m.fixed_rates) {
+    m.d_fix = dsec(3 * nr);
+    m.d_fixp = dsec(3 * n_fall);
+    m.i_fixn = isec(nr);
+    m.i_fixp = isec(n_fall);
+    for (int r = 0; r < nr; ++r) {
+      const int f = rx[r].fall;
+      if (!fixed_arrhenius_of(form_constant(rx[r]).data(), &D[m.d_fix + 3 * r], &I[m.i_fixn + r])) I[m.i_fixn + r] = kFixNone;
+      if (f >= 0 && !fixed_arrhenius_of(&D[m.d_kp + 3 * f], &D[m.d_fixp + 3 * f], &I[m.i_fixp + f])) I[m.i_fixp + f] = kFixNone;
+    }
+  }
+  while (D.size() % 2) D.push_back(0.);  // 16-byte boundary for the int section
+  while (I.size() % 4) I.push_back(0);   // 16-byte total
+  m.blob_doubles = (int)D.size();
+  m.blob_ints = (int)I.size();
+  m.blob_bytes = m.blob_doubles * 8 + m.blob_ints * 4;
+  host_dbl = D;
+  host_int = I;
+
   // ---------------- upload
   CUDA_THROW(cudaMalloc(&d_blob, m.blob_bytes));
   std::vector<unsigned char> bytes(m.blob_bytes);
@@ -411,7 +432,6 @@ void HostMech::build(const sf_mech_desc *d)
   CUDA_THROW(cudaMemcpy(d_blob, bytes.data(), m.blob_bytes, cudaMemcpyHostToDevice));
   CUDA_THROW(cudaMalloc(&d_status, 16));
   CUDA_THROW(cudaMemset(d_status, 0, 16));
-  CUDA_THROW(cudaGetDevice(&device));
   // every gather program the kernels use, built here so that no evaluation call builds or allocates one
   for (int G : {1, 8, 16, 32, 64, 128, 256}) build_programs(G);
 }

@@ -104,7 +104,7 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Blob &b, c
     s.port = m.pref * s.invT * m.invRu;
     s.u68 = fixed_reciprocal(s.invT);
   };
-  s.fixed = fixed_temperature(T);
+  s.fixed = m.fixed_rates && fixed_temperature(T);
   if constexpr (G <= 32) {
     s.logT = state_log(T, exp2tab, s.l60);
     scalars(grp);

@@ -92,6 +92,10 @@ void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pre
                                int stages, const double *q, const double *pressures, const double *w, double *out,
                                cudaStream_t st);
 size_t tps_scratch_bytes(const HostMech &hm, int mode, long long n);
+// Shared memory (doubles) of one integrating warp. global_scratch: the Griffon scratch lives in a global slot;
+// global_matrix: the iteration matrix and the FP32 factors too, leaving the vectors and pivots in shared memory.
+size_t integrate_warp_doubles(const HostMech &hm, int neq, int prec, bool global_scratch, bool global_matrix,
+                              bool feed_y_table);
 
 }  // namespace sfgb
 

@@ -25,7 +25,8 @@ enum : int {
 struct DevMech {
   int ns, nr;
   int n_dense;      // reactions with a dense Jacobian part
-  int n_fall;       // Lindemann + Troe
+  int n_fall;       // Lindemann + Troe: the last reactions in device order, so that falloff index f is reaction nr - n_fall + f
+  int fixed_rates;  // 1 if the blob holds the fixed-point rate constants (d_fix, d_fixp, i_fixn, i_fixp)
   int n_slots;      // total sparse Jacobian slots over all reactions
   int n_net_total;
   int all_nasa7;    // 1 if every species is NASA7 (else some are constant-cp)
@@ -48,7 +49,6 @@ struct DevMech {
   int d_tbeff;   // [tb entries] eff - default
   int d_netc;    // [net entries] -nu*M (coefficient of q_r in w_i)
   int d_ord;     // [order entries] special orders
-  int d_one;     // 1.0
   int d_smallint;  // [64] the integer k - 32 at index k (stoichiometric coefficients without conversions); kept
                    // small because every kernel stages the blob into shared memory
   int d_exptab;    // [128] 2^(j/64) as (head, tail) pairs, j = 0..63, for the table-driven exponential
@@ -60,7 +60,6 @@ struct DevMech {
   int i_fixp;    // [n_fall] the same of k0 / kinf
   int i_orig;    // [nr] index of each device-order reaction in the order the mechanism was described
   int i_sums;    // [nr] sum_nu (low 16 bits, signed) | sum_reac_nu << 16 (8 bits) | sum_prod_nu << 24
-  int i_fall;    // [nr] falloff index or -1
   int i_dense;   // [nr] dense index or -1
   int i_reac_off, i_reac;   // [nr+1], entries: species | nu << 16
   int i_prod_off, i_prod;   // [nr+1], entries: species | nu << 16
@@ -100,7 +99,6 @@ struct ScratchLayout {
                                        // partial sums of the Jacobian gathers
   int alpha, beta;                     // [n_dense]
   int D;                               // [n_slots]
-  int misc;                            // 16 scalars
   int total;                           // doubles per state
   int total_rhs;                       // doubles per state needed by the RHS-only path (prefix of the layout)
 };

@@ -102,3 +102,38 @@ def test_flamelet_points(cuda, kind):
     assert bool(torch.isfinite(out[0]).all())
     assert float((out[0] - out[1]).abs().max()) <= 1e-12 * float(out[1].abs().max())
     assert spec.griffon.device_status() == 0
+
+
+@pytest.mark.parametrize('which', [0, 1])
+def test_tables_up_to_the_plain_layout(cuda, which):
+    """The largest mechanism whose FP64 tables and plain scratch fit a block (0: right-hand sides, 1: Jacobians) runs, the
+    fixed-point constants' tables or not, in every kernel shape, and an integration of it. 1e-10 row-normwise against the
+    CPU oracle: rates near equilibrium cancel to about 1e-4 of their terms."""
+    import oracle as orc
+    import torch
+    from helpers import colmajor, rownorm_err
+    from spitfire_gb300 import autotune as AT
+    from spitfire_gb300 import workloads as W
+    from spitfire_gb300._desc import reactor_params
+    from spitfire_gb300.reactors import BatchIntegrator
+    k = LM.search(lambda k: LM.plain_need(LM.mechanism(k))[which], LM.SMEM - 64, 400, 1600)
+    spec = LM.mechanism(k)
+    og = orc.OracleGriffon()
+    spec._populate_griffon(og)
+    g = spec.griffon
+    d = W.gri_states(spec, 3, seed=9)
+    q = W.isobaric_state(d)
+    P = reactor_params('isobaric')
+    ref, refJ = og.reactor_jac_batch(P, q, pressures=d['p'])
+    for knob in (0, 8, 16, 32):
+        AT.set_tuning(spec, 'group_rhs', knob)
+        AT.set_tuning(spec, 'group_jac', knob)
+        for n in (1, 3):
+            r = g.reactor_rhs_batch(P, q[:n], pressures=d['p'][:n]).cpu().numpy()
+            assert rownorm_err(r[:, None, :], ref[:n, None, :]) < 1e-10
+            if which == 1:
+                J = g.reactor_jac_batch(P, q[:n], pressures=d['p'][:n])[1].cpu().numpy()
+                assert rownorm_err(colmajor(J, NS), colmajor(refJ[:n], NS)) < 1e-10
+    out = BatchIntegrator(spec, 'isobaric').run(q, pressures=d['p'], stop_at_time=1.e-9, first_time_step=1.e-9)
+    assert bool(torch.isfinite(out['q']).all())
+    assert g.device_status() == 0
