@@ -168,14 +168,16 @@ __device__ __forceinline__ void reg_lu_solve(const F *LU, int m, int lane, const
     for (int u = 0; u < kAheadCols; ++u) {
       const int j = j0 - u;
       if (j >= 0) {
-        F xs = x[0], rs = rd[0];
+        F xs = x[0], rs = rd[0], d = c[u][0];
 #pragma unroll
         for (int s = 1; s < R; ++s)
           if ((j >> 5) == s) {
             xs = x[s];
             rs = rd[s];
+            d = c[u][s];
           }
-        const F xj = __shfl_sync(0xffffffffu, xs * rs, j & 31);
+        // a pivot whose reciprocal leaves the normal numbers divides (lane j holds it)
+        const F xj = __shfl_sync(0xffffffffu, lu_normal(rs) ? xs * rs : xs / d, j & 31);
 #pragma unroll
         for (int s = 0; s < R; ++s) {
           if (32 * s < j && lane + 32 * s < j) x[s] = fma(-c[u][s], xj, x[s]);

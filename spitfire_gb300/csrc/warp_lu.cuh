@@ -34,6 +34,9 @@ __device__ __forceinline__ bool larger_abs(float a, float b)
 }
 __device__ __forceinline__ double lu_reciprocal(double p) { return fix_reciprocal(p); }
 __device__ __forceinline__ float lu_reciprocal(float p) { return 1.f / p; }
+// A reciprocal of full precision: neither infinite (of a subnormal pivot) nor itself subnormal.
+__device__ __forceinline__ bool lu_normal(double r) { return (unsigned)(((__double2hiint(r) >> 20) & 0x7ff) - 1) < 2046u; }
+__device__ __forceinline__ bool lu_normal(float r) { return (unsigned)(((__float_as_int(r) >> 23) & 0xff) - 1) < 254u; }
 
 // A[i, j] -= A[i, k] A[k, j] for i, j > k. FP64: the elements are dealt to the lanes in column-major order, so that no
 // FP64 instruction leaves lanes empty (an instruction costs the same with one lane as with 32); the position advances
