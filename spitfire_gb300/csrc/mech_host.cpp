@@ -12,8 +12,11 @@
 
 #include <algorithm>
 #include <cmath>
+#include <deque>
+#include <functional>
 #include <map>
 #include <numeric>
+#include <queue>
 #include <stdexcept>
 #include <string>
 
@@ -90,9 +93,7 @@ std::array<double, 3> form_constant(const HRxn &x)
 
 HostMech::~HostMech()
 {
-  for (auto &kv : programs) {
-    for (GatherItem *p : kv.second.owned) cudaFree(p);
-  }
+  if (d_items) cudaFree(d_items);
   if (d_blob) cudaFree(d_blob);
   if (d_status) cudaFree(d_status);
   for (cudaEvent_t e : events) cudaEventDestroy(e);
@@ -433,7 +434,7 @@ void HostMech::build(const sf_mech_desc *d)
   CUDA_THROW(cudaMalloc(&d_status, 16));
   CUDA_THROW(cudaMemset(d_status, 0, 16));
   // every gather program the kernels use, built here so that no evaluation call builds or allocates one
-  for (int G : {1, 8, 16, 32, 64, 128, 256}) build_programs(G);
+  build_programs();
 }
 
 const HostMech::Programs &HostMech::programs_for(int G) const
@@ -468,55 +469,55 @@ struct Entry {
   uint32_t dst;  // IT_JAC | row | col << IT_COL_SHIFT, or a scratch index
 };
 
+typedef std::vector<const Entry *> EntryList;
+
 // The device runner loads operands ahead of the stores of earlier items, so a program must never read a scratch
 // location that it writes (as a destination or through an entry's initial value).
-void check_no_read_after_write(const std::vector<Entry> &entries, int qoff)
+void check_no_read_after_write(const EntryList &entries, int qoff, int scratch)
 {
-  std::vector<uint32_t> written;
-  for (const Entry &e : entries)
-    if (!(e.dst & IT_JAC)) written.push_back(e.dst);
-  std::sort(written.begin(), written.end());
-  auto check = [&](uint32_t idx) {
-    if (std::binary_search(written.begin(), written.end(), idx))
-      throw sf_error(SF_ERR_MECHANISM, "internal: gather program reads what it writes");
-  };
-  for (const Entry &e : entries) {
-    if (e.dst & IT_JAC) check(qoff + (e.dst & IT_ROW_MASK));
-    for (const Item &it : e.items) {
-      check(it.ref);
-      if (it.pair >= 0) check(it.pair);
-    }
+  std::vector<char> written(scratch, 0);
+  for (const Entry *e : entries)
+    if (!(e->dst & IT_JAC)) written[e->dst] = 1;
+  bool bad = false;
+  for (const Entry *e : entries) {
+    if (e->dst & IT_JAC) bad |= written[qoff + (e->dst & IT_ROW_MASK)] != 0;
+    for (const Item &it : e->items) bad |= written[it.ref] || (it.pair >= 0 && written[it.pair]);
   }
+  if (bad) throw sf_error(SF_ERR_MECHANISM, "internal: gather program reads what it writes");
 }
 
 // Assignment of entries to G lanes and the interleaved item array, each lane's items padded with no-ops to a
 // multiple of the device runner's batch. G > 1: longest-processing-time assignment (balanced lanes). G = 1 (one
 // lane per state): entries in destination order, Jacobian entries column-major, so that each thread writes its
 // Jacobian block sequentially through memory.
-std::vector<GatherItem> schedule(const std::vector<Entry> &entries, int G, int qoff, int *len_out)
+std::vector<GatherItem> schedule(const EntryList &entries, int G, int qoff, int scratch, int *len_out)
 {
-  check_no_read_after_write(entries, qoff);
+  check_no_read_after_write(entries, qoff, scratch);
   std::vector<int> order(entries.size());
   std::iota(order.begin(), order.end(), 0);
   if (G == 1) {
     auto key = [&](int e) {
-      const uint32_t d = entries[e].dst;
+      const uint32_t d = entries[e]->dst;
       const uint64_t jac = (d & IT_JAC) ? 0 : 1;  // the Jacobian first
       return jac << 32 | (d & IT_DST_MASK);       // col << 13 | row: column-major
     };
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key(a) < key(b); });
   } else {
     std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return entries[a].items.size() > entries[b].items.size(); });
+                     [&](int a, int b) { return entries[a]->items.size() > entries[b]->items.size(); });
   }
   std::vector<std::vector<int>> lane(G);
   std::vector<size_t> load(G, 0);
+  typedef std::pair<size_t, int> Load;  // (items, lane): the least loaded lane, the lowest on ties
+  std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+  for (int l = 0; l < G; ++l) least.push({0, l});
   for (int e : order) {
-    if (entries[e].items.empty()) continue;
-    int best = 0;
-    for (int l = 1; l < G; ++l) if (load[l] < load[best]) best = l;
+    if (entries[e]->items.empty()) continue;
+    const int best = least.top().second;
+    least.pop();
     lane[best].push_back(e);
-    load[best] += entries[e].items.size();
+    load[best] += entries[e]->items.size();
+    least.push({load[best], best});
   }
   size_t len = 0;
   for (int l = 0; l < G; ++l) len = std::max(len, load[l]);
@@ -525,7 +526,7 @@ std::vector<GatherItem> schedule(const std::vector<Entry> &entries, int G, int q
   for (int l = 0; l < G; ++l) {
     size_t j = 0;
     for (int e : lane[l]) {
-      const Entry &E = entries[e];
+      const Entry &E = *entries[e];
       for (size_t k = 0; k < E.items.size(); ++k, ++j) {
         const Item &x = E.items[k];
         GatherItem it{x.c, x.ref, E.dst};
@@ -547,39 +548,47 @@ std::vector<GatherItem> schedule(const std::vector<Entry> &entries, int G, int q
 // Entries longer than a lane's share are cut into parts of about that share, which sum into the scratch slots
 // part .. part + cap - 1 and are added up by the entries put into `fix`. (GRI-3.0's species rates on 32 lanes: 137
 // items for H against a share of 39.) A Jacobian entry's first item, u_k P_i on top of Q_i, stays in its fix entry.
-std::vector<Entry> split_entries(const std::vector<Entry> &entries, int G, int part, int cap, std::vector<Entry> *fix)
+// own holds the entries made here.
+EntryList split_entries(const std::vector<Entry> &entries, int G, int part, int cap, std::deque<Entry> *own, EntryList *fix)
 {
-  if (G == 1) return entries;
+  EntryList out;
+  out.reserve(entries.size());
+  if (G == 1) {
+    for (const Entry &e : entries) out.push_back(&e);
+    return out;
+  }
   size_t total = 0;
   for (const Entry &e : entries) total += e.items.size();
   for (size_t share = std::max<size_t>(4, (total + G - 1) / G);; share += (share + 3) / 4) {
-    std::vector<Entry> out;
+    out.clear();
     fix->clear();
+    own->clear();
     int used = 0;
     for (const Entry &e : entries) {
       const size_t keep = (e.dst & IT_JAC) ? 1 : 0, n = e.items.size() - std::min(keep, e.items.size());
       if (e.items.size() <= share + share / 8) {
-        out.push_back(e);
+        out.push_back(&e);
         continue;
       }
       const size_t parts = (n + share - 1) / share;
       Entry f{{e.items.begin(), e.items.begin() + keep}, e.dst};
       for (size_t p = 0; p < parts; ++p) {
         const size_t a = keep + n * p / parts, b = keep + n * (p + 1) / parts;
-        out.push_back(Entry{{e.items.begin() + a, e.items.begin() + b}, (uint32_t)(part + used)});
+        own->push_back(Entry{{e.items.begin() + a, e.items.begin() + b}, (uint32_t)(part + used)});
+        out.push_back(&own->back());
         f.items.push_back(Item{1., (uint32_t)(part + used), -1});
         ++used;
       }
-      fix->push_back(f);
+      own->push_back(std::move(f));
+      fix->push_back(&own->back());
     }
     if (used <= cap) return out;
   }
 }
 }  // namespace
 
-void HostMech::build_programs(int G)
+void HostMech::build_programs()
 {
-  if (programs.count(G)) return;
   const int ns = dm.ns, nr = dm.nr;
   const ScratchLayout &L = sl;
   // species -> list of (reaction, coefficient of its rate) in increasing reaction order
@@ -648,27 +657,32 @@ void HostMech::build_programs(int G)
         }
     }
   }
-  Programs P;
-  for (int k = 0; k < 4; ++k) {
-    // partial sums: the Gibbs factors are dead after the reactions, dqdrho and dqdT after the species gathers
-    const int part = k < 2 ? L.gm : L.dqdrho, cap = k < 2 ? L.q - L.gm : L.alpha - L.dqdrho;
-    std::vector<Entry> fix;
-    const std::vector<Entry> main = split_entries(E[k], G, part, cap, &fix);
-    auto upload = [&](const std::vector<Entry> &entries, int *len) -> const GatherItem * {
-      const std::vector<GatherItem> items = schedule(entries, G, L.Q, len);
-      GatherItem *dptr = nullptr;
-      CUDA_THROW(cudaMalloc(&dptr, std::max<size_t>(items.size(), 1) * sizeof(GatherItem)));
-      P.owned.push_back(dptr);
-      if (!items.empty())
-        CUDA_THROW(cudaMemcpy(dptr, items.data(), items.size() * sizeof(GatherItem), cudaMemcpyHostToDevice));
-      return dptr;
-    };
-    P.progs[k].items = upload(main, &P.progs[k].len);
-    P.progs[k].fix_items = nullptr;
-    P.progs[k].fix_len = 0;
-    if (!fix.empty()) P.progs[k].fix_items = upload(fix, &P.progs[k].fix_len);
+  // every program's items in one device array: offsets until it exists
+  std::vector<GatherItem> all;
+  auto add = [&](const EntryList &entries, int G, int *len) {
+    const std::vector<GatherItem> items = schedule(entries, G, L.Q, L.total, len);
+    const size_t at = all.size();
+    all.insert(all.end(), items.begin(), items.end());
+    return at;
+  };
+  std::vector<std::pair<const GatherItem **, size_t>> places;
+  for (int G : {1, 8, 16, 32, 64, 128, 256}) {
+    Programs &P = programs[G];
+    for (int k = 0; k < 4; ++k) {
+      // partial sums: the Gibbs factors are dead after the reactions, dqdrho and dqdT after the species gathers
+      const int part = k < 2 ? L.gm : L.dqdrho, cap = k < 2 ? L.q - L.gm : L.alpha - L.dqdrho;
+      std::deque<Entry> own;
+      EntryList fix;
+      const EntryList main = split_entries(E[k], G, part, cap, &own, &fix);
+      places.push_back({&P.progs[k].items, add(main, G, &P.progs[k].len)});
+      P.progs[k].fix_items = nullptr;
+      P.progs[k].fix_len = 0;
+      if (!fix.empty()) places.push_back({&P.progs[k].fix_items, add(fix, G, &P.progs[k].fix_len)});
+    }
   }
-  programs.emplace(G, std::move(P));
+  CUDA_THROW(cudaMalloc(&d_items, std::max<size_t>(all.size(), 1) * sizeof(GatherItem)));
+  if (!all.empty()) CUDA_THROW(cudaMemcpy(d_items, all.data(), all.size() * sizeof(GatherItem), cudaMemcpyHostToDevice));
+  for (auto &p : places) *p.first = d_items + p.second;
 }
 
 }  // namespace sfgb

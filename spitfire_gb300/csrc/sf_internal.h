@@ -54,16 +54,16 @@ struct HostMech {
 
   struct Programs {
     DevProgram progs[4]{};  // 0: w only, 1: w/S_rho/S_T/P/Q, 2: Y block + T row, 3: all species rows (sens)
-    std::vector<GatherItem *> owned;  // device allocations of the items
   };
   std::map<int, Programs> programs;
+  GatherItem *d_items = nullptr;  // the items of all programs, on the device
 
   void build(const sf_mech_desc *d);
-  const Programs &programs_for(int G) const;  // the gather programs of group width G (1, 8, 16, 32, 128 or 256), built by build()
+  const Programs &programs_for(int G) const;  // the gather programs of group width G (1, 8, 16, 32, 64, 128 or 256), built by build()
   ~HostMech();
 
  private:
-  void build_programs(int G);
+  void build_programs();
 };
 
 // Launch helpers implemented in the .cu files (return an sf_status code).
