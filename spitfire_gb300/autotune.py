@@ -9,10 +9,11 @@ CUDA events and applies the fastest through ``sf_mech_set_tuning``:
     share a block, against the library's own choice (0, 0), which for large mechanisms is eight warps per reactor.
 The knobs change launch shapes only. The integrator's one-warp candidates produce bit-identical results; the group
 width changes the order of the per-species sums, so other candidates agree to rounding (the tuner checks both).
-Choices are cached per (mechanism, device) in spitfire_gb300/_tuning (created on first use).
+Choices are cached per (mechanism, device, kernel sources) in spitfire_gb300/_tuning (created on first use).
 """
 
 import ctypes as C
+import glob
 import hashlib
 import json
 import os
@@ -20,6 +21,7 @@ import os
 import numpy as np
 
 from . import _native as N
+from . import build
 
 KNOBS = {'group_rates': 0, 'group_sens': 1, 'group_rhs': 2, 'group_jac': 3, 'integrate_warps': 4,
          'integrate_scratch': 5, 'tps_ctas': 6}
@@ -57,11 +59,22 @@ def _time(fn, reps=3):
     return best
 
 
+def _kernels():
+    """Digest of the kernels' sources: choices measured with other kernels are not applied."""
+    h = hashlib.sha1()
+    for p in sorted(glob.glob(os.path.join(build.CSRC, '*'))):
+        if p.endswith(('.cu', '.cuh', '.h', '.cpp')):
+            h.update(os.path.basename(p).encode())
+            with open(p, 'rb') as f:
+                h.update(f.read())
+    return h.hexdigest()[:16]
+
+
 def _key(mech):
     torch = _torch()
     h = hashlib.sha1(json.dumps(mech.mech_data_json(), sort_keys=True).encode()).hexdigest()[:16]
     dev = torch.cuda.get_device_name().replace(' ', '_')
-    return f'{h}_{dev}'
+    return f'{h}_{dev}_{_kernels()}'
 
 
 def tune_chemistry(mech, states, pressures=None, configuration='isochoric', kinds=('rates', 'rhs', 'jac'), reps=3,

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from spitfire_gb300 import autotune as AT
+from spitfire_gb300 import build
 
 
 class FakeIntegrator:
@@ -54,3 +55,27 @@ def test_knobs_restored_when_a_launch_fails(tuner, fail_at):
     with pytest.raises(ValueError):
         tuner(f, {})
     assert f.shape() == (2, 5)
+
+
+def test_saved_choices_belong_to_the_kernels_that_were_timed(monkeypatch, tmp_path):
+    """load() finds what save() wrote, and no longer once a kernel source has changed."""
+    src = tmp_path / 'csrc'
+    src.mkdir()
+    (src / 'a.cu').write_text('one')
+    (src / 'note.txt').write_text('no kernel')
+    monkeypatch.setattr(build, 'CSRC', str(src))
+    monkeypatch.setattr(AT, 'CACHE_DIR', str(tmp_path / 'tuning'))
+    monkeypatch.setattr(AT, '_torch', lambda: types.SimpleNamespace(
+        cuda=types.SimpleNamespace(get_device_name=lambda: 'a GPU')))
+    knobs = {name: 0 for name in AT.KNOBS}
+    knobs['group_jac'] = 16
+    monkeypatch.setattr(AT, 'get_tuning', lambda mech, k: knobs[k])
+    applied = {}
+    monkeypatch.setattr(AT, 'set_tuning', lambda mech, k, v: applied.__setitem__(k, v))
+    mech = types.SimpleNamespace(mech_data_json=lambda: {'species': 2})
+    AT.save(mech, {})
+    assert AT.load(mech) == knobs and applied == knobs
+    (src / 'note.txt').write_text('still none')
+    assert AT.load(mech) == knobs
+    (src / 'a.cu').write_text('two')
+    assert AT.load(mech) is None
