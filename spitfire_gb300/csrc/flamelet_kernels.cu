@@ -442,65 +442,72 @@ __global__ void __launch_bounds__(kFactorThreads) btddod_middle_kernel(int nf, i
   for (int k = tid; k < ns; k += nt) pv[k] = sh.piv[k];
 }
 
-// Asynchronous 8-byte copies global -> shared by all threads of the block (cp.async, completion tracked by commit
+// Asynchronous 8-byte copies global -> shared by `threads` threads, t among them (cp.async, completion tracked by commit
 // groups; no mbarrier wait is involved).
-__device__ __forceinline__ void async_copy_doubles(double *dst, const double *src, int n)
+__device__ __forceinline__ void async_copy_doubles(double *dst, const double *src, int n, int t, int threads)
 {
-  for (int e = threadIdx.x; e < n; e += blockDim.x)
+  for (int e = t; e < n; e += threads)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst + e)), "l"(src + e) : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 __device__ __forceinline__ void async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// One CTA walks a chain of dependent block steps, each a matrix-vector product with a column-major ns x ns block staged
-// in shared memory (the next one is copied while the current one is used, where two fit). A product's rows are dealt
-// to the threads of whole warps and its columns cut into parts over the other warps: one warp alone takes two FP64
+// A group of whole warps walks a chain of dependent block steps, each a matrix-vector product with a column-major ns x ns
+// block staged in shared memory (the next one is copied while the current one is used, where two fit). A product's rows are
+// dealt to the threads of whole warps and its columns cut into parts over the other warps: one warp alone takes two FP64
 // instructions per column at 64 cycles each, 6.8 us a step for ns = 53; twelve take 9 per step.
 constexpr int kSweepThreads = 384;
+constexpr int kSmallSolveBlock = 32;    // blocks up to this size: both halves of a flamelet in one CTA,
+constexpr int kSmallSolveThreads = 128; // on this many threads each
 
 struct Sweep {
   double *b0, *b1, *part, *vec;
-  int ns, bs2, rows, parts, p, r, c0, c1;
+  int ns, bs2, rows, parts, p, r, c0, c1, t, threads, id;
   bool dbl;
-  __device__ Sweep(unsigned char *smem, int ns_, bool dbl_) : ns(ns_), bs2(ns_ * ns_), dbl(dbl_)
+  __device__ Sweep(unsigned char *smem, int ns_, bool dbl_, int t_, int threads_, int barrier)
+      : ns(ns_), bs2(ns_ * ns_), t(t_), threads(threads_), id(barrier), dbl(dbl_)
   {
     b0 = reinterpret_cast<double *>(smem);
     b1 = dbl ? b0 + bs2 : b0;
     part = b1 + bs2;
-    vec = part + kSweepThreads;
+    vec = part + threads;
     rows = (ns + 31) & ~31;
-    parts = kSweepThreads / rows;
-    p = threadIdx.x / rows;
-    r = threadIdx.x - p * rows;
+    parts = threads / rows;
+    p = t / rows;
+    r = t - p * rows;
     c0 = ns * p / parts;
     c1 = ns * (p + 1) / parts;
   }
-  static size_t bytes(int ns, bool dbl) { return ((size_t)(dbl ? 2 : 1) * ns * ns + kSweepThreads + ns) * 8; }
-  __device__ __forceinline__ double *slot(int t) const { return (t & 1) ? b1 : b0; }
-  template <class Src>
-  __device__ __forceinline__ void prime(int t, Src src) const
+  __host__ __device__ static size_t bytes(int ns, bool dbl, int threads = kSweepThreads)
   {
-    if (dbl) async_copy_doubles(slot(t), src(t), bs2);
+    return ((size_t)(dbl ? 2 : 1) * ns * ns + threads + ns) * 8;
   }
-  // The block of step t (steps t, t + step, ..., last are fetched in this order); ends with the barrier that also makes
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+  __device__ __forceinline__ double *slot(int k) const { return (k & 1) ? b1 : b0; }
+  template <class Src>
+  __device__ __forceinline__ void prime(int k, Src src) const
+  {
+    if (dbl) async_copy_doubles(slot(k), src(k), bs2, t, threads);
+  }
+  // The block of step k (steps k, k + step, ..., last are fetched in this order); ends with the barrier that also makes
   // the writes to vec visible.
   template <class Src>
-  __device__ __forceinline__ const double *fetch(int t, int last, int step, Src src) const
+  __device__ __forceinline__ const double *fetch(int k, int last, int step, Src src) const
   {
     if (dbl) {
-      if (t != last) {
-        async_copy_doubles(slot(t + step), src(t + step), bs2);
+      if (k != last) {
+        async_copy_doubles(slot(k + step), src(k + step), bs2, t, threads);
         async_wait_all_but_one();
       } else {
         async_wait_all();
       }
     } else {
-      async_copy_doubles(b0, src(t), bs2);
+      async_copy_doubles(b0, src(k), bs2, t, threads);
       async_wait_all();
     }
-    __syncthreads();
-    return dbl ? slot(t) : b0;
+    sync();
+    return dbl ? slot(k) : b0;
   }
   // Row r of B vec, complete in the threads below ns.
   __device__ __forceinline__ double product(const double *B) const
@@ -508,45 +515,90 @@ struct Sweep {
     double s = 0.;
     if (p < parts && r < ns)
       for (int c = c0; c < c1; ++c) s = fma(B[r + c * ns], vec[c], s);
-    if (p > 0 && p < parts) part[threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.x < ns)
-      for (int q = 1; q < parts; ++q) s += part[q * rows + threadIdx.x];
+    if (p > 0 && p < parts) part[t] = s;
+    sync();
+    if (t < ns)
+      for (int q = 1; q < parts; ++q) s += part[q * rows + t];
     return s;
   }
 };
 
-// Solve with the twisted factors (the reference's btddod_matrix_kernels.cpp:82-119 sweeps, run from both ends), two
-// CTAs per flamelet, even ones over blocks 0..m-1, odd ones over blocks nzi-1..m+1, m = nzi/2, in three launches:
+// Solve with the twisted factors (the reference's btddod_matrix_kernels.cpp:82-119 sweeps, run from both ends), one half over
+// blocks 0..m-1, the other over blocks nzi-1..m+1, m = nzi/2, in three parts:
 //   1. sweeps toward block m: y_0 = b_0, y_i = b_i - L_i y_{i-1};   z_{nzi-1} = b_{nzi-1}, z_i = b_i - U_{i+1} z_{i+1}
-//   2. one CTA per flamelet:  x_m = M^-1 (b_m - L_m y_{m-1} - U_{m+1} z_{m+1})
+//   2. the middle:            x_m = M^-1 (b_m - L_m y_{m-1} - U_{m+1} z_{m+1})
 //   3. back substitution:     x_i = D_i^-1 (y_i - sup_i o x_{i+1}) for i < m;  x_i = T_i^-1 (z_i - sub_{i-1} o x_{i-1})
-// y and z are parked in x until the back substitution overwrites them.
+// y and z are parked in x until the back substitution overwrites them. The parts are launches of their own with a CTA per
+// half; blocks of up to kSmallSolveBlock have steps so short that the two further launches cost more than the wider halves
+// gain, so there one CTA takes the halves and all parts. 11 species: one flamelet of 30 blocks 50 us in three launches, 29 in
+// one (40 with the two warps per flamelet before), eight of up to 95 blocks 122 and 80 (114), 64 of up to 126 156 and 107
+// (155); 30 species, eight of up to 95 blocks: 118 in one (245).
+__device__ __forceinline__ void solve_forward(const Sweep &sw, bool down, int nb, int m, const double *lv, const double *b,
+                                              double *xs)
+{
+  const int len = down ? m : nb - 1 - m, ns = sw.ns, t = sw.t;
+  if (len == 0) return;
+  auto at = [&](int k) { return (size_t)(down ? k : nb - 1 - k) * ns; };
+  auto src = [&](int k) { return lv + (size_t)(down ? k : nb - k) * sw.bs2; };
+  if (len > 1) sw.prime(1, src);
+  if (t < ns) xs[at(0) + t] = sw.vec[t] = b[at(0) + t];
+  for (int k = 1; k < len; ++k) {
+    const double *B = sw.fetch(k, len - 1, 1, src);
+    const double s = sw.product(B);
+    if (t < ns) xs[at(k) + t] = sw.vec[t] = b[at(k) + t] - s;
+  }
+}
+
+__device__ __forceinline__ void solve_meet(const Sweep &sw, int nb, int m, const double *lv, const double *Dm, const double *b,
+                                           double *xs)
+{
+  const int ns = sw.ns, t = sw.t;
+  double v = t < ns ? b[(size_t)m * ns + t] : 0.;
+  for (int side = 0; side < 2; ++side) {  // L_m y_{m-1}, then U_{m+1} z_{m+1}
+    const int i = side == 0 ? m - 1 : m + 1;
+    if (i < 0 || i >= nb) continue;
+    if (t < ns) sw.vec[t] = xs[(size_t)i * ns + t];
+    const double *B = sw.fetch(0, 0, 1, [&](int) { return lv + (size_t)(m + side) * sw.bs2; });
+    v -= sw.product(B);
+    sw.sync();
+  }
+  if (t < ns) sw.vec[t] = v;
+  const double *B = sw.fetch(0, 0, 1, [&](int) { return Dm; });
+  const double s = sw.product(B);
+  if (t < ns) xs[(size_t)m * ns + t] = s;
+}
+
+__device__ __forceinline__ void solve_back(const Sweep &sw, bool down, int nb, int m, const double *vals, double *xs)
+{
+  const int len = down ? m : nb - 1 - m, ns = sw.ns, t = sw.t;
+  if (len == 0) return;
+  const double *sub = vals + (size_t)nb * sw.bs2;
+  const double *sup = sub + (size_t)(nb - 1) * ns;
+  auto blk = [&](int k) { return down ? k : nb - 1 - k; };
+  auto src = [&](int k) { return vals + (size_t)blk(k) * sw.bs2; };
+  sw.prime(len - 1, src);
+  double xn = t < ns ? xs[(size_t)m * ns + t] : 0.;
+  for (int k = len - 1; k >= 0; --k) {
+    const int i = blk(k);
+    const double *cpl = down ? sup + (size_t)i * ns : sub + (size_t)(i - 1) * ns;
+    if (t < ns) sw.vec[t] = xs[(size_t)i * ns + t] - cpl[t] * xn;
+    const double *B = sw.fetch(k, 0, -1, src);
+    xn = sw.product(B);
+    if (t < ns) xs[(size_t)i * ns + t] = xn;
+  }
+}
+
 __global__ void __launch_bounds__(kSweepThreads) btddod_forward_kernel(int nf, int ns, const int *offz,
                                                                        const double *lvals, const double *rhs,
                                                                        double *x, const int *active, int double_buffer)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const int f = blockIdx.x >> 1;
-  const bool down = (blockIdx.x & 1) == 0;
   if (f >= nf || (active && !active[f])) return;
-  const int z0 = offz[f], nb = offz[f + 1] - z0, m = nb / 2;
-  const int len = down ? m : nb - 1 - m;
-  if (len == 0) return;
-  const Sweep sw(smem, ns, double_buffer != 0);
-  const double *lv = lvals + (size_t)z0 * sw.bs2;
-  const double *b = rhs + (size_t)z0 * ns;
-  double *xs = x + (size_t)z0 * ns;
-  const int tid = threadIdx.x;
-  auto at = [&](int t) { return (size_t)(down ? t : nb - 1 - t) * ns; };
-  auto src = [&](int t) { return lv + (size_t)(down ? t : nb - t) * sw.bs2; };
-  if (len > 1) sw.prime(1, src);
-  if (tid < ns) xs[at(0) + tid] = sw.vec[tid] = b[at(0) + tid];
-  for (int t = 1; t < len; ++t) {
-    const double *B = sw.fetch(t, len - 1, 1, src);
-    const double s = sw.product(B);
-    if (tid < ns) xs[at(t) + tid] = sw.vec[tid] = b[at(t) + tid] - s;
-  }
+  const int z0 = offz[f], nb = offz[f + 1] - z0;
+  const Sweep sw(smem, ns, double_buffer != 0, threadIdx.x, kSweepThreads, 0);
+  solve_forward(sw, (blockIdx.x & 1) == 0, nb, nb / 2, lvals + (size_t)z0 * sw.bs2, rhs + (size_t)z0 * ns,
+                x + (size_t)z0 * ns);
 }
 
 __global__ void __launch_bounds__(kSweepThreads) btddod_meet_kernel(int nf, int ns, const int *offz,
@@ -558,23 +610,9 @@ __global__ void __launch_bounds__(kSweepThreads) btddod_meet_kernel(int nf, int 
   const int f = blockIdx.x;
   if (f >= nf || (active && !active[f])) return;
   const int z0 = offz[f], nb = offz[f + 1] - z0, m = nb / 2;
-  const Sweep sw(smem, ns, false);
-  const double *lv = lvals + (size_t)z0 * sw.bs2;
-  double *xs = x + (size_t)z0 * ns;
-  const int tid = threadIdx.x;
-  double v = tid < ns ? rhs[(size_t)(z0 + m) * ns + tid] : 0.;
-  for (int side = 0; side < 2; ++side) {  // L_m y_{m-1}, then U_{m+1} z_{m+1}
-    const int i = side == 0 ? m - 1 : m + 1;
-    if (i < 0 || i >= nb) continue;
-    if (tid < ns) sw.vec[tid] = xs[(size_t)i * ns + tid];
-    const double *B = sw.fetch(0, 0, 1, [&](int) { return lv + (size_t)(m + side) * sw.bs2; });
-    v -= sw.product(B);
-    __syncthreads();
-  }
-  if (tid < ns) sw.vec[tid] = v;
-  const double *B = sw.fetch(0, 0, 1, [&](int) { return values + offv[f] + (size_t)m * sw.bs2; });
-  const double s = sw.product(B);
-  if (tid < ns) xs[(size_t)m * ns + tid] = s;
+  const Sweep sw(smem, ns, false, threadIdx.x, kSweepThreads, 0);
+  solve_meet(sw, nb, m, lvals + (size_t)z0 * sw.bs2, values + offv[f] + (size_t)m * sw.bs2, rhs + (size_t)z0 * ns,
+             x + (size_t)z0 * ns);
 }
 
 __global__ void __launch_bounds__(kSweepThreads) btddod_back_kernel(int nf, int ns, const int *offz,
@@ -583,29 +621,34 @@ __global__ void __launch_bounds__(kSweepThreads) btddod_back_kernel(int nf, int 
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const int f = blockIdx.x >> 1;
-  const bool down = (blockIdx.x & 1) == 0;
   if (f >= nf || (active && !active[f])) return;
+  const int z0 = offz[f], nb = offz[f + 1] - z0;
+  const Sweep sw(smem, ns, double_buffer != 0, threadIdx.x, kSweepThreads, 0);
+  solve_back(sw, (blockIdx.x & 1) == 0, nb, nb / 2, values + offv[f], x + (size_t)z0 * ns);
+}
+
+__global__ void __launch_bounds__(2 * kSmallSolveThreads) btddod_small_solve_kernel(int nf, int ns, const int *offz,
+                                                                                    const long long *offv,
+                                                                                    const double *values,
+                                                                                    const double *lvals,
+                                                                                    const double *rhs, double *x,
+                                                                                    const int *active)
+{
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int f = blockIdx.x;
+  if (f >= nf || (active && !active[f])) return;
+  const int half = threadIdx.x / kSmallSolveThreads, t = threadIdx.x - half * kSmallSolveThreads;
   const int z0 = offz[f], nb = offz[f + 1] - z0, m = nb / 2;
-  const int len = down ? m : nb - 1 - m;
-  if (len == 0) return;
-  const Sweep sw(smem, ns, double_buffer != 0);
-  const double *vals = values + offv[f];
-  const double *sub = vals + (size_t)nb * sw.bs2;
-  const double *sup = sub + (size_t)(nb - 1) * ns;
+  unsigned char *own = smem + half * Sweep::bytes(ns, true, kSmallSolveThreads);
+  const Sweep sw(own, ns, true, t, kSmallSolveThreads, 1 + half);
+  const double *lv = lvals + (size_t)z0 * sw.bs2, *vals = values + offv[f], *b = rhs + (size_t)z0 * ns;
   double *xs = x + (size_t)z0 * ns;
-  const int tid = threadIdx.x;
-  auto blk = [&](int t) { return down ? t : nb - 1 - t; };
-  auto src = [&](int t) { return vals + (size_t)blk(t) * sw.bs2; };
-  sw.prime(len - 1, src);
-  double xn = tid < ns ? xs[(size_t)m * ns + tid] : 0.;
-  for (int t = len - 1; t >= 0; --t) {
-    const int i = blk(t);
-    const double *cpl = down ? sup + (size_t)i * ns : sub + (size_t)(i - 1) * ns;
-    if (tid < ns) sw.vec[tid] = xs[(size_t)i * ns + tid] - cpl[tid] * xn;
-    const double *B = sw.fetch(t, 0, -1, src);
-    xn = sw.product(B);
-    if (tid < ns) xs[(size_t)i * ns + tid] = xn;
-  }
+  solve_forward(sw, half == 0, nb, m, lv, b, xs);
+  __syncthreads();
+  if (half == 0)
+    solve_meet(Sweep(own, ns, false, t, kSmallSolveThreads, 1), nb, m, lv, vals + (size_t)m * sw.bs2, b, xs);
+  __syncthreads();
+  solve_back(sw, half == 0, nb, m, vals, xs);
 }
 
 // Block-triangular solves with the inverses of a block-diagonal factorization (btddod_matrix_kernels.cpp:386-428):
@@ -623,7 +666,7 @@ __global__ void __launch_bounds__(kSweepThreads) btddod_triangle_solve_kernel(in
   const int f = blockIdx.x;
   if (f >= nf || (active && !active[f])) return;
   const int z0 = offz[f], nb = offz[f + 1] - z0;
-  const Sweep sw(smem, ns, double_buffer != 0);
+  const Sweep sw(smem, ns, double_buffer != 0, threadIdx.x, kSweepThreads, 0);
   const double *sub = values + offv[f] + (size_t)nb * sw.bs2;
   const double *sup = sub + (size_t)(nb - 1) * ns;
   const double *b = rhs + (size_t)z0 * ns;
@@ -867,6 +910,13 @@ int launch_solve(int nf, int ns, const int *offz, const long long *offv, const d
   int dev, smem_max;
   CUDA_THROW(cudaGetDevice(&dev));
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  if (ns <= kSmallSolveBlock) {
+    const size_t smem = 2 * Sweep::bytes(ns, true, kSmallSolveThreads);
+    ensure_dynamic_smem((const void *)btddod_small_solve_kernel, smem);
+    btddod_small_solve_kernel<<<nf, 2 * kSmallSolveThreads, smem, st>>>(nf, ns, offz, offv, values, l_values, rhs, out_x,
+                                                                        active);
+    return check_launch();
+  }
   const bool dbl = sweep_double_buffer(ns, smem_max);
   const size_t smem = Sweep::bytes(ns, dbl), smem1 = Sweep::bytes(ns, false);
   ensure_dynamic_smem((const void *)btddod_forward_kernel, smem);
