@@ -23,10 +23,10 @@ def test_regrown_record_equals_one_fitting_run(cuda, per_sm):
     T = np.linspace(1100., 1900., n)
     q0 = torch.tensor(np.hstack([T[:, None], Y[:, :-1]]), device='cuda')
     bi = BatchIntegrator(spec, 'isobaric', pressure=10. * 101325.)
-    ip = bi.controls(stop_at_time=3.e-5)
-    one, rec = bi.record(q0, None, ip, 256)
+    ip = bi.controls(stop_at_time=3.e-5, max_attempts=1024)
+    one, rec = bi.record(q0, None, ip, 1024)
     steps = one['counts'][:, 0].cpu().numpy()
-    assert steps.max() <= 256 and (one['status'].cpu().numpy() != 7).all()
+    assert (one['status'].cpu().numpy() != 7).all()
     capacity = int(np.quantile(steps, 0.95))  # about one reactor in twenty is integrated again
     assert steps.max() > capacity
     out, grown = bi.record(q0, None, ip, capacity)
