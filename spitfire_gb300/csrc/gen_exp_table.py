@@ -8,13 +8,13 @@
 * kExpTable[2j], kExpTable[2j+1] = head and tail of 2^(j/64), j = 0..63 (head: 2^(j/64) rounded; tail: the
   rounded remainder), interleaved so that one 16-byte load fetches both.
 
-The fixed-point exponential's constants (chem_device.cuh: fix_exp2):
+The fixed-point exponential's constants (fixed_point.cuh: fix_exp2):
 * kFixLog2e2, 1, 0: the three 32-bit words of log2(e) 2^95, truncated;
 * kFixExpTable[j] = 2^(j/256) 2^63, rounded, j = 0..255;
 * kFixC1 .. kFixC5: the polynomial of W(v) = 256 (2^(v/256) - 1) = v (c1 + v (c2 + ...)) on [0, 1], the Chebyshev fit of
-  degree 4 of W(v)/v, as integers scaled by 2^64 (c1, c2) and 2^52 (c3, c4, c5). The device's shifts and high products
-  truncate; kFixC3 + 1 and kFixC2 + 1300 center the error that leaves (within 20 units of 2^-63 of the result's
-  mantissa, 0.0098 ulp, before the final rounding).
+  degree 4 of W(v)/v, as integers scaled by 2^64 (c1, c2), 2^52 (c3) and 2^60 (c4, c5). The device's shifts and high
+  products truncate; 2700 added to kFixC2 centers the error that leaves (within 16 units of 2^-63 of the result's mantissa,
+  0.0079 ulp, before the final rounding).
 """
 import os
 
@@ -50,7 +50,7 @@ def header_text():
     lines += [f'constexpr unsigned kFixLog2e{k} = {hex((l96 >> (32 * k)) & 0xffffffff)}u;' for k in (2, 1, 0)]
     w = lambda v: ln2 if v == 0 else 256 * (mp.power(2, v / 256) - 1) / v
     c = mp.chebyfit(w, [mp.mpf(10) ** -30, 1], 5)[::-1]
-    fix = [int(mp.nint(c[k] * mp.mpf(2) ** (64 if k < 2 else 52))) + (0, 1300, 1, 0, 0)[k] for k in range(5)]
+    fix = [int(mp.nint(c[k] * mp.mpf(2) ** (64, 64, 52, 60, 60)[k])) + (0, 2700, 0, 0, 0)[k] for k in range(5)]
     lines += [f'constexpr unsigned long long kFixC{k + 1} = {hex(fix[k])}ull;' for k in range(5)]
     lines += ['constexpr unsigned long long kFixExpTable[256] = {']
     for j in range(0, 256, 4):
