@@ -423,7 +423,7 @@ __device__ __forceinline__ double small_int(const double *table, int k)
 // ------------------------------------------------------------------------------------------ reaction phase
 // Per-state quantities every reaction needs.
 struct StateCtx {
-  double T, logT, invT, rho, invRho, mmw, invM, ct;
+  double T, logT, invT, rho, invRho, mmw, ct;
   double port;  // p_ref / (R T)
   bool fixed;   // rate constants in fixed point: 16 < T < 65536 and the blob holds them
   unsigned long long l60, u68;  // log2 T 2^60, 2^68 / T

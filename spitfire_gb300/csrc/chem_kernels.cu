@@ -683,9 +683,8 @@ int sf_device_status(const sf_mech *mech, int clear)
 
 }  // extern "C"
 
-// Reactor right-hand sides and Jacobians with an explicit lane width G (8, 16 or 32 lanes per state: shared-memory
-// scratch, no workspace), for callers whose batch is too small for the thread-per-state shape the autotuner may have
-// chosen for large batches.
+// Reactor right-hand sides and Jacobians at the library's own group width (no workspace), for callers whose batch is too
+// small for the shape the autotuner may have chosen for large batches.
 void sfgb::reactor_jac_groups(const sf_mech *mech, const sf_reactor_params *rp, int rates_option, int n,
                               const double *q, const double *pressures, double *out_rhs, double *out_jac,
                               cudaStream_t st)

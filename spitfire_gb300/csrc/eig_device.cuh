@@ -76,8 +76,9 @@ __device__ __forceinline__ bool abs_sums(const double *A, int n, int i, int lane
 // 5%, at most `max_sweeps` sweeps. Column-major A, leading dimension n.
 // GB300 issues FP64 at one warp instruction per 76 cycles per scheduler, so the scalings by powers of two (exact)
 // run on the integer pipe: non-negative finite doubles order like their bit patterns, and a factor 4 or 1/4 on a
-// normal value is a change of 2 in its exponent field. The results are those of the plain FP64 form bit for bit;
-// values near the ends of the exponent range take the FP64 form.
+// normal value is a change of 2 in its exponent field; values near the ends of the exponent range take the FP64 form. The
+// scalings themselves are exact. The sums of up to 64 rows are cut to 53 bits of their largest term (abs_sums), so that a
+// choice of scaling can differ from the FP64 form's where a comparison ties within that cut.
 // One warp, also where the matrix has several: a row/column pair is a serial step, and the exchange between warps cost more
 // than it gained. The sums are integer sums (abs_sums) and a pair that needs no scaling (m = 0) is left at once: a 53 x 53
 // block takes nine sweeps of 53 pairs, about 1700 cycles a pair in FP64 with two warps.

@@ -3,7 +3,7 @@
 //
 // Derivations restated from src/spitfire/griffon/src/chemistry_setup.cpp:
 //   NASA7 storage scaled by R and 1/2, 1/6, 1/12, 1/20          (:102-130)
-//   third-body efficiencies stored as invM*(eff - default)        (:406-419)
+//   third-body efficiencies stored as eff - default               (:406-419)
 //   net stoichiometry over species in ascending index order       (:459-541), 2 <= n_net <= 8 enforced
 //   dense/sparse sensitivity classification                       (:543-602)
 //   rate-constant temperature form and Troe term flags            (:670-730)

@@ -88,7 +88,6 @@ __device__ __forceinline__ StateCtx state_ctx(const DevMech &m, const Blob &b, c
   const unsigned long long *exp2tab = reinterpret_cast<const unsigned long long *>(b.d + m.d_exptab + 128);
   StateCtx s;
   s.T = T;
-  s.invM = sim;
   s.option = option;
   auto scalars = [&](const auto &g) {
     double ix;  // 1 / rho isochoric, 1 / p isobaric
