@@ -654,7 +654,9 @@ __global__ void __launch_bounds__(2 * kSmallSolveThreads) btddod_small_solve_ker
 // Block-triangular solves with the inverses of a block-diagonal factorization (btddod_matrix_kernels.cpp:386-428):
 //   lower  x_0 = F_0 b_0,               x_i = F_i (b_i - sub_{i-1} o x_{i-1})
 //   upper  x_{nb-1} = F_{nb-1} b_{nb-1}, x_i = F_i (b_i - sup_i o x_{i+1})
-// One CTA per flamelet; F_i are column-major inverses, [points][ns*ns].
+// One CTA per flamelet, of four warps for small blocks, whose few columns cost less than a barrier of twelve (one chain of 30
+// blocks of 11 rows 27 us against 37, of 30 rows 37 against 45; one warp had taken 36 and 68); F_i are column-major
+// inverses, [points][ns*ns].
 __global__ void __launch_bounds__(kSweepThreads) btddod_triangle_solve_kernel(int nf, int ns, const int *offz,
                                                                               const long long *offv,
                                                                               const double *inverses,
@@ -666,7 +668,7 @@ __global__ void __launch_bounds__(kSweepThreads) btddod_triangle_solve_kernel(in
   const int f = blockIdx.x;
   if (f >= nf || (active && !active[f])) return;
   const int z0 = offz[f], nb = offz[f + 1] - z0;
-  const Sweep sw(smem, ns, double_buffer != 0, threadIdx.x, kSweepThreads, 0);
+  const Sweep sw(smem, ns, double_buffer != 0, threadIdx.x, blockDim.x, 0);
   const double *sub = values + offv[f] + (size_t)nb * sw.bs2;
   const double *sup = sub + (size_t)(nb - 1) * ns;
   const double *b = rhs + (size_t)z0 * ns;
@@ -940,8 +942,9 @@ int launch_triangle(int nf, int ns, const int *offz, const long long *offv, cons
   const bool dbl = sweep_double_buffer(ns, smem_max);
   const size_t smem = Sweep::bytes(ns, dbl);
   ensure_dynamic_smem((const void *)btddod_triangle_solve_kernel, smem);
-  btddod_triangle_solve_kernel<<<nf, kSweepThreads, smem, st>>>(nf, ns, offz, offv, inverses, values, rhs, out_x,
-                                                                upper, active, dbl);
+  const int threads = ns <= kSmallSolveBlock ? kSmallSolveThreads : kSweepThreads;
+  btddod_triangle_solve_kernel<<<nf, threads, smem, st>>>(nf, ns, offz, offv, inverses, values, rhs, out_x, upper, active,
+                                                          dbl);
   return check_launch();
 }
 
