@@ -133,7 +133,13 @@ void launch_rate_param_adjoint(const HostMech &hm, int configuration, double pre
   CUDA_THROW(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CUDA_THROW(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const size_t scr_doubles = (size_t)hm.sl.total_rhs + hm.dm.ns + (configuration == 1 ? 1 : 0) + 2;
-  int G = fitting_group(hm.dm, n_items <= 2 * nsm ? 256 : (n_items <= 8 * nsm ? 64 : 32), scr_doubles, smem_max);
+  // Threads per item. Measured with one stage each, microseconds: GRI-3.0 (325 reactions) n = 304: 35 (256), 44 (64), 70
+  // (32); 456: 46 (64), 65 (256), 70 (32); 1216: 76 (64), 87 (32); 1824: 107 (32), 122 (64); 2432: 144 (64), 165 (32).
+  // methane-lu30 (184) n = 304: 30 (256), 34 (64), 46 (32); 1216: 50 (64), 56 (32); 1824: 68 (32), 83 (64). h2-burke (27), whose
+  // reactions one warp takes in a single pass, n = 1: 25 (32), 26 (64), 27 (256); 304: 26 (32), 28 (64), 29 (256); 1216: 34
+  // (32), 39 (64).
+  const int width = hm.dm.nr <= 32 || n_items > 8 * nsm ? 32 : (n_items <= 2 * nsm ? 256 : 64);
+  int G = fitting_group(hm.dm, width, scr_doubles, smem_max);
   if (G == 128) G = 64;  // no kernel of that width
   const auto &progs = hm.programs_for(G);
   AdjParams p{};

@@ -217,9 +217,12 @@ size_t tps_scratch_bytes(const HostMech &hm, int mode, long long n)
 //   GRI rates       n = 304: 24 (256, 128), 27 (64), 44 (32); 456: 28 (128, 64); 912: 39 (64), 49 (32); 1216: 44 (64), 52
 //                   (32); 1824: 62 (32), 73 (64), 76 (16); 3040: 92 (16), 112 (32, 64); 20,011: 589 (16)
 //   h2 Jacobians    n = 304: 31 (64), 37 (16); 608: 34 (64), 37 (16); 1216: 38 (16), 42 (64); 3000: 47 (16), 54 (8); 4096:
-//                   59 (16), 60 (8); 9728: 102 (8), 133 (16); 65,536: 677 (1), 1,063 (8), before fixed-point rate constants
+//                   59 (16), 60 (8); 9728: 102 (8), 133 (16); 20,011: 211 (8), 273 (1); 28,500: 275 (8), 278 (1); 30,400:
+//                   280 (1), 322 (8); 65,536: 623 (1), 638 (8); 200,000: 1,333 (1), 1,921 (8)
 //   h2 rates        n = 912: 22 (64), 23 (16); 1216: 22 (16), 24 (64); 3000: 24.6 (16), 25.3 (8); 4096: 28 (8), 30 (16);
-//                   20,000: 155 (1), 204 (8), before fixed-point rate constants
+//                   20,011: 95 (8), 102 (1); 22,800: 103 (1), 107 (8); 65,536: 209 (1), 275 (8)
+//   methane-lu30 (30 species / 184 reactions), right-hand sides n = 9728: 152 (16), 169 (8), 194 (32); Jacobians n = 65,536:
+//                   3,780 (32), 3,803 (64), 4,259 (1)
 // The lines lie at the SM count times the states of one SM; thread per state only where the caller's workspace has its
 // scratch (allowed), and for small mechanisms: GRI's 29 KB of scratch per state do not stay in L2.
 int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_allowed)
@@ -231,7 +234,7 @@ int default_group(const DevMech &m, bool jac, long long n, int nsm, bool tps_all
   }
   if (per_sm <= (jac ? 4 : 6)) return 64;
   if (per_sm <= (jac ? 27 : 20)) return 16;
-  return per_sm > 100 && tps_allowed ? 1 : 8;
+  return per_sm > (jac ? 190 : 140) && tps_allowed ? 1 : 8;
 }
 
 int fitting_group(const DevMech &m, int G, size_t doubles, int smem_max)

@@ -511,9 +511,9 @@ size_t integrate_warp_doubles(const HostMech &hm, int neq, int prec, bool global
 namespace {
 
 // Memory placement of an integrating warp's data: 0 all in shared memory, 1 the Griffon scratch in a global
-// (L2-resident) slot, 2 the iteration matrix and FP32 factors there too. The built-in choice (knob value 0) is 2:
-// with 8 warps per block it ran the 8192-reactor GRI ignition batch at 2,292 ignitions/s, against 1,771 for
-// placement 1 and 5 warps; placement 0 leaves room for two warps per block. Knob value 3 selects placement 0.
+// (L2-resident) slot, 2 the iteration matrix and FP32 factors there too. The built-in choice (knob value 0) is 2: 8192 GRI
+// reactors to 20 us take 240 ms with it at 8 warps per block (220 at 6, of which two blocks fit an SM), 268 with placement 1
+// and 5 warps, 408 with placement 0 and 2 warps. Knob value 3 selects placement 0.
 int integrate_placement(const HostMech &hm)
 {
   const int v = hm.tune[SF_TUNE_INTEGRATE_SCRATCH];
@@ -555,7 +555,8 @@ IntShape integrate_shape(const HostMech &hm, int neq, int prec, int n, bool feed
   // A mechanism of more than 64 reactions runs eight warps per reactor up to 12 reactors per SM, unless a launch shape
   // was set (the autotuner's) or the factors are FP32. (GRI-3.0 to 20 us: one reactor 4.0 ms against 13.0 with one
   // warp, 300 16.7 against 66.1, 1000 38.1 against 66.9, 2000 64.0 against 89.0; ignitions to 0.1 s: 2048 reactors
-  // 0.88 s against 0.90, 8192 3.29 against 2.73. h2-burke's 27 reactions fit one warp: 1000 reactors 171 ms with one,
+  // 0.88 s against 0.90, 8192 3.29 against 2.73. methane-lu30, 184 reactions, to 20 us: 300 reactors 10.3 ms against 22.4,
+  // 1400 27.2 against 31.1, 1824 36.1 against 34.5. h2-burke's 27 reactions fit one warp: 1000 reactors 171 ms with one,
   // 243 with eight.) Recordings take them at every size.
   if (!one_warp && prec == 0 && hm.dm.nr > 64 && (record || n <= 12 * nsm) && hm.tune[SF_TUNE_INTEGRATE_SCRATCH] == 0 && hm.tune[SF_TUNE_INTEGRATE_WARPS] == 0) {
     constexpr int wg = kWideG;
