@@ -114,14 +114,19 @@ __device__ __forceinline__ void reg_permutation(const int *piv, int m, int lane,
   }
 }
 
+// The reciprocals of U's diagonal; true where one is not a normal number (of a subnormal or zero pivot, or of one so large that
+// its reciprocal is subnormal): the system is then solved by reg_lu_solve_dividing.
 template <int R, typename F>
-__device__ __forceinline__ void reg_reciprocals(const F *LU, int m, int lane, F (&rd)[R])
+__device__ __forceinline__ bool reg_reciprocals(const F *LU, int m, int lane, F (&rd)[R])
 {
+  bool odd = false;
 #pragma unroll
   for (int s = 0; s < R; ++s) {
     const int i = lane + 32 * s;
     rd[s] = lu_reciprocal(i < m ? LU[(size_t)i * (m + 1)] : (F)1);
+    odd = odd || !lu_normal(rd[s]);
   }
+  return __any_sync(0xffffffffu, odd);
 }
 
 template <int R, typename F>
@@ -168,16 +173,14 @@ __device__ __forceinline__ void reg_lu_solve(const F *LU, int m, int lane, const
     for (int u = 0; u < kAheadCols; ++u) {
       const int j = j0 - u;
       if (j >= 0) {
-        F xs = x[0], rs = rd[0], d = c[u][0];
+        F xs = x[0], rs = rd[0];
 #pragma unroll
         for (int s = 1; s < R; ++s)
           if ((j >> 5) == s) {
             xs = x[s];
             rs = rd[s];
-            d = c[u][s];
           }
-        // a pivot whose reciprocal leaves the normal numbers divides (lane j holds it)
-        const F xj = __shfl_sync(0xffffffffu, lu_normal(rs) ? xs * rs : xs / d, j & 31);
+        const F xj = __shfl_sync(0xffffffffu, xs * rs, j & 31);
 #pragma unroll
         for (int s = 0; s < R; ++s) {
           if (32 * s < j && lane + 32 * s < j) x[s] = fma(-c[u][s], xj, x[s]);
@@ -192,6 +195,29 @@ __device__ __forceinline__ void reg_lu_solve(const F *LU, int m, int lane, const
   }
 }
 
+// The same with a division per pivot and without columns held ahead, so that beside the sweeps above it needs no registers of
+// its own (as a choice in every step of those, division cost them eight and a quarter of the FP32 solves' time).
+template <int R, typename F>
+__device__ __forceinline__ void reg_lu_solve_dividing(const F *LU, int m, int lane, F (&x)[R])
+{
+#pragma unroll 1
+  for (int j = 0; j < m; ++j) {
+    const F xj = reg_get<R>(x, j);
+#pragma unroll
+    for (int s = 0; s < R; ++s)
+      if (lane + 32 * s > j && lane + 32 * s < m) x[s] = fma(-LU[lane + 32 * s + (size_t)j * m], xj, x[s]);
+  }
+#pragma unroll 1
+  for (int j = m - 1; j >= 0; --j) {
+    const F xj = reg_get<R>(x, j) / LU[(size_t)j * (m + 1)];
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+      if (lane + 32 * s < j) x[s] = fma(-LU[lane + 32 * s + (size_t)j * m], xj, x[s]);
+      if (lane + 32 * s == j) x[s] = xj;
+    }
+  }
+}
+
 template <int R>
 __global__ void __launch_bounds__(32 * kSolveWarps) solve64_kernel(int n, int m, const double *LU, const int *piv,
                                                                    const double *b, double *x)
@@ -202,10 +228,13 @@ __global__ void __launch_bounds__(32 * kSolveWarps) solve64_kernel(int n, int m,
     int perm[R];
     reg_permutation<R>(piv + (size_t)sys * m, m, lane, perm);
     double rd[R], xr[R];
-    reg_reciprocals<R>(L, m, lane, rd);
+    const bool odd = reg_reciprocals<R>(L, m, lane, rd);
 #pragma unroll
     for (int s = 0; s < R; ++s) xr[s] = lane + 32 * s < m ? b[(size_t)sys * m + perm[s]] : 0.;
-    reg_lu_solve<R>(L, m, lane, rd, xr);
+    if (odd)
+      reg_lu_solve_dividing<R>(L, m, lane, xr);
+    else
+      reg_lu_solve<R>(L, m, lane, rd, xr);
 #pragma unroll
     for (int s = 0; s < R; ++s)
       if (lane + 32 * s < m) x[(size_t)sys * m + lane + 32 * s] = xr[s];
@@ -225,14 +254,17 @@ __global__ void __launch_bounds__(32 * kSolveWarps) solve32_kernel(int n, int m,
     int perm[R];
     reg_permutation<R>(piv + (size_t)sys * m, m, lane, perm);
     float rd[R], r[R];
-    reg_reciprocals<R>(L, m, lane, rd);
+    const bool odd = reg_reciprocals<R>(L, m, lane, rd);
     double bs[R], xs[R];
 #pragma unroll
     for (int s = 0; s < R; ++s) {
       bs[s] = lane + 32 * s < m ? b[(size_t)sys * m + lane + 32 * s] : 0.;
       r[s] = lane + 32 * s < m ? (float)b[(size_t)sys * m + perm[s]] : 0.f;
     }
-    reg_lu_solve<R>(L, m, lane, rd, r);
+    if (odd)
+      reg_lu_solve_dividing<R>(L, m, lane, r);
+    else
+      reg_lu_solve<R>(L, m, lane, rd, r);
 #pragma unroll
     for (int s = 0; s < R; ++s) xs[s] = (double)r[s];
     for (int it = 0; it < refine; ++it) {
@@ -268,7 +300,10 @@ __global__ void __launch_bounds__(32 * kSolveWarps) solve32_kernel(int n, int m,
           if ((perm[s] >> 5) == q) r[s] = t;
         }
       }
-      reg_lu_solve<R>(L, m, lane, rd, r);
+      if (odd)
+        reg_lu_solve_dividing<R>(L, m, lane, r);
+      else
+        reg_lu_solve<R>(L, m, lane, rd, r);
 #pragma unroll
       for (int s = 0; s < R; ++s) xs[s] += (double)r[s];
     }
