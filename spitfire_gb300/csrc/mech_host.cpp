@@ -287,7 +287,6 @@ void HostMech::build(const sf_mech_desc *d)
   }
   m.d_kf = dsec(3 * nr);
   m.d_kp = dsec(3 * n_fall);
-  fixed_log2_of(m.pref / m.Ru, &m.log2_port_n, &m.log2_port_f);
   m.d_troe = dsec(4 * n_fall);
   m.d_beff = dsec(nr);
   for (int r = 0; r < nr; ++r) {
@@ -391,7 +390,8 @@ void HostMech::build(const sf_mech_desc *d)
   L.total = o;
 
   // ---------------- fixed-point rate constants, 28 bytes per reaction and falloff ratio: left out (the rates are then formed
-  // in FP64) where some kernel's narrowest group fits a block's shared memory only without them
+  // in FP64) where some kernel's narrowest group fits a block's shared memory only without them, and where the Gibbs energies
+  // or the reference concentration are no finite numbers, which a fixed-point word cannot hold
   CUDA_THROW(cudaGetDevice(&device));
   {
     int smem_max;
@@ -405,8 +405,12 @@ void HostMech::build(const sf_mech_desc *d)
     m.fixed_rates = 1;
     for (size_t n : need)
       if (base + 8 * n + 64 <= (size_t)smem_max && base + fix + 8 * n + 64 > (size_t)smem_max) m.fixed_rates = 0;
+    for (double c : nasa)
+      if (!std::isfinite(c)) m.fixed_rates = 0;
+    if (!std::isnormal(m.pref / m.Ru) || !(m.pref / m.Ru > 0.)) m.fixed_rates = 0;
   }
   if (m.fixed_rates) {
+    fixed_log2_of(m.pref / m.Ru, &m.log2_port_n, &m.log2_port_f);
     m.d_fix = dsec(3 * nr);
     m.d_fixp = dsec(3 * n_fall);
     m.i_fixn = isec(nr);

@@ -223,3 +223,29 @@ def test_temperature_forms(cuda, b, theta):
             expect = -k * c[present[0]] * c[present[1]] * LD(spec.griffon._rec.species_mw[1])
             for w in _evaluate(spec, T, np.ones(3), np.tile(Y, (3, 1))):
                 assert np.abs((w[:, 1] / expect - 1.).astype(float)).max() <= 6. * 2.3e-16 * 200. + 1e-14
+
+
+def test_thermodynamics_without_numbers(cuda):
+    """A species whose polynomials hold no number makes the reverse rates of its reactions none, in every kernel shape, and leaves
+    the irreversible ones alone; a reference pressure of zero makes reverse constants zero where moles are lost."""
+    for case in ('nan', 'zero pressure'):
+        spec = _mechanism([({'A': 1, 'D': 1}, {'B': 1, 'E': 1}, True, 1e8, 0., 0.), ({'A': 1}, {'C': 1}, False, 1e3, 0., 0.),
+                           ({'A': 2}, {'D': 1}, True, 1e3, 0., 0.)])
+        md = copy.deepcopy(spec.mech_data)
+        if case == 'nan':
+            md['species']['E']['cp'] = tuple(md['species']['E']['cp'][:4]) + ([float('nan')] * 7, [float('nan')] * 7)
+        else:
+            md['ref_pressure'] = 0.
+        spec = type(spec)(mech_data=md)
+        Y = np.full(6, 1. / 6.)
+        for w in _evaluate(spec, np.array([300., 1500.]), np.ones(2), np.tile(Y, (2, 1))):
+            if case == 'nan':
+                assert np.isnan(w[:, SPECIES.index('B')]).all() and np.isnan(w[:, SPECIES.index('E')]).all()
+                assert np.isfinite(w[:, SPECIES.index('C')]).all()
+            else:  # 2 A <=> D: one mole lost, so kr has a factor p_ref; A + D <=> B + E has none
+                c = _conc(spec, 1., Y)
+                q = 1e3 * c['A'] ** 2
+                kr = np.array([np.exp(_log_Kc(md | {'ref_pressure': 1.}, {'A': 1, 'D': 1}, {'B': 1, 'E': 1}, T)) for T in (300., 1500.)])
+                r = 1e8 * (c['A'] * c['D'] - kr * c['B'] * c['E'])
+                mw = LD(spec.griffon._rec.species_mw[SPECIES.index('D')])
+                assert np.abs((w[:, SPECIES.index('D')] / (mw * (q - r)) - 1.).astype(float)).max() < 1e-11
