@@ -4,6 +4,11 @@ The hot path has no exchange step: every state, reactor and flamelet is independ
 contiguous slices, one per rank; each rank runs its slice on its own GPU and the only collective is a host-side
 concatenation of the per-rank results (and a max of per-rank times for measurement). The process group may be
 gloo (host tensors) or nccl (the caller passes device tensors).
+
+The concatenated results are those of the whole batch to rounding, not bit for bit: the kernels choose how many threads share
+a state, and the integrator whether one warp or eight share a reactor, by the number of units in a call, and that orders the
+sums. With the same launch shapes set on every rank (autotune.set_tuning: group_rates, group_sens, group_rhs, group_jac,
+integrate_scratch) states and reactors do not depend on the slice they are in.
 """
 
 import os
