@@ -1224,7 +1224,7 @@ def main():
            'ms_each_step': [round(x, 3) for x in e2e_steps],
            'h2d_bytes_per_step': qpin.numel() * 8, 'd2h_bytes_per_step': (rhs_h.numel() + J_h.numel()) * 8,
            'api': 'PyCombustionKernels.reactor_jac_host_batch -> sf_reactor_jac_host_batch (pinned host buffers; '
-                  'chunks of one resident wave, device-to-host copies overlapping the next chunk)'}
+                  'chunks whose device-to-host copies overlap the next chunk)'}
 
     # ---------------- comparison point: the plain single-state GPU form on the same states
     ws = torch.empty(N.load().sf_reactor_jac_plain_workspace_size(g.handle, N_STATES) // 8 + 1,

@@ -249,3 +249,54 @@ def test_thermodynamics_without_numbers(cuda):
                 r = 1e8 * (c['A'] * c['D'] - kr * c['B'] * c['E'])
                 mw = LD(spec.griffon._rec.species_mw[SPECIES.index('D')])
                 assert np.abs((w[:, SPECIES.index('D')] / (mw * (q - r)) - 1.).astype(float)).max() < 1e-11
+
+
+@pytest.mark.parametrize('knob', [0, 8, 16, 32, 1])
+def test_jacobians_with_constants_of_both_forms(cuda, knob):
+    """h2-burke with reversible duplicates whose A is negative, whose b or E/R is beyond the fixed-point range, and a falloff
+    reaction whose k0/kinf is: rates, right-hand sides and Jacobians against the CPU oracle, 1e-10 row-normwise as for the
+    mechanism itself, for one state (a wide group) and several."""
+    import oracle as orc
+    from helpers import colmajor, rownorm_err
+    from spitfire_gb300 import autotune as AT
+    from spitfire_gb300 import workloads as W
+    from spitfire_gb300._desc import reactor_params
+    from spitfire_gb300.mechanism import ChemicalMechanismSpec
+    md = copy.deepcopy(ChemicalMechanismSpec.bundled('h2-burke').mech_data)
+    Ru = md['gas_constant']
+    rx = [list(r) for r in md['reactions']]
+    simple = [r for r in rx if r[0] == 'simple' and r[3]]
+    troe = [list(r) for r in rx if r[0] == 'Troe']
+    for k, change in enumerate(('negative', 'b', 'E')):
+        r = list(simple[k])
+        if change == 'negative':
+            r[4] = -0.3 * r[4]
+        elif change == 'b':
+            r[4], r[5] = r[4] * 1e-99, r[5] + 32.
+        else:
+            r[6] = -3.7e5 * Ru
+            r[4] = r[4] * 1e-150
+        rx.insert(k, r)
+    troe[0][10] = troe[0][5] + 32.  # the ratio's exponent
+    troe[0][9] = troe[0][9] * 1e-99
+    rx = [r for r in rx if r[0] != 'Troe'] + troe
+    md['reactions'] = [tuple(r) for r in rx]
+    spec = ChemicalMechanismSpec(mech_data=md)
+    og = orc.OracleGriffon()
+    spec._populate_griffon(og)
+    g = spec.griffon
+    d = W.h2_states(spec, 40, seed=4)
+    q = W.isochoric_state(d)
+    P = reactor_params('isochoric')
+    neq = q.shape[1]
+    ref, refJ = og.reactor_jac_batch(P, q)
+    for name in ('group_rates', 'group_rhs', 'group_jac'):
+        AT.set_tuning(spec, name, knob)
+    w = g.production_rates_batch(d['T'], d['rho'], d['Y']).cpu().numpy()
+    assert rownorm_err(w, og.production_rates_batch(d['T'], d['rho'], d['Y'])) < 1e-10
+    for n in (1, 40):
+        rhs, J = g.reactor_jac_batch(P, q[:n])
+        assert rownorm_err(g.reactor_rhs_batch(P, q[:n]).cpu().numpy()[:, None, :], ref[:n, None, :]) < 1e-10
+        assert rownorm_err(rhs.cpu().numpy()[:, None, :], ref[:n, None, :]) < 1e-10
+        assert rownorm_err(colmajor(J.cpu().numpy(), neq), colmajor(refJ[:n], neq)) < 1e-10
+    assert g.device_status() == 0
