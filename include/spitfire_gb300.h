@@ -125,7 +125,8 @@ int sf_mech_info(const sf_mech *mech, int *n_species, int *n_reactions, int *cou
  *     workspace, whose size sf_chem_workspace_size reports; no knob allocates anything); 0 lets the library choose by
  *     the batch size, from 256 threads per state to one (the last only with a workspace);
  *   SF_TUNE_INTEGRATE_WARPS: warps (reactors) per block of sf_integrate_batch, 1..8 (0: as many as fit; with both
- *     integrator knobs 0, small FP64 batches of mechanisms with more than 64 reactions run eight warps per reactor);
+ *     integrator knobs 0, small FP64 batches of mechanisms with more than 64 reactions, and recordings of any size, run
+ *     eight warps per reactor);
  *   SF_TUNE_INTEGRATE_SCRATCH: where each integrating warp keeps its data: 3 all in shared memory; 1 its Griffon
  *     scratch in global memory (L2-resident), so that more warps fit per SM; 2 also its iteration matrix and FP32
  *     factors (0: the built-in choice, 2);
@@ -325,9 +326,10 @@ enum sf_integrate_status {
   SF_INT_NAN = 5, SF_INT_NO_IGNITION = 6, SF_INT_RECORD_FULL = 7
 };
 
+/* Device workspace of the two integration calls below, in bytes, the same for every n >= 1 with the same knobs. */
 size_t sf_integrate_workspace_size(const sf_mech *mech, const sf_reactor_params *params, int n);
 /* Integrate n independent reactors of the same configuration and feed from q0 (state-major; isobaric reactors
- * may each have their own pressure). One persistent launch works through the batch: each warp takes the next
+ * may each have their own pressure). One persistent launch works through the batch: each warp (or eight) takes the next
  * unfinished reactor from a queue, so reactors with 10x more steps do not stall the rest. Outputs: final states
  * out_q, final time out_t, per-reactor counters out_counts[n][4] = steps, Newton iterations, Jacobian setups,
  * failed steps, and status codes. out_t of an ignition run is the ignition delay (the end time of the first
